@@ -1,73 +1,163 @@
 // C[M,N] = A[M,K] * W[N,K]^T in true 32-bit: float inputs, float FMA accumulation on
 // CUDA cores, no tensor-core mode of reduced precision.  This is the matrix product
 // of the float32 path of the whole model (the reference has no such path: it lets
-// float matmuls run as TF32, mstar/engine/__init__.py:6).  Every output element is
-// one sequential sum over K, so a row's result does not depend on what else is in
-// the batch.
+// float matmuls run as TF32, mstar/engine/__init__.py:6).
+//
+// Every output element is two sequential sums over K, one of the even and one of the odd
+// positions, added at the end: the pair is one packed FMA (fma.rn.f32x2: two IEEE FMAs an
+// instruction, which is what the FMA pipe needs for its full rate), and both its factors lie
+// side by side in the row-major operands.  All tile shapes below sum in this order, so a row's
+// result does not depend on what else is in the batch.
+//
+// What bounds it: the shared loads that feed the FMA pipe where there are tiles for every SM (a
+// thread's 8 x 4 outputs take 12 loads of 16 bytes for 64 packed FMAs; 46 of the pipe's 74
+// TFLOP/s), the stream of W and the depth of the copies where there are few rows.  Both operands come by cp.async, STAGES k-blocks deep, in their own
+// row-major order; rows are BK + 4 floats apart in shared memory, so that eight threads reading
+// 16 bytes of eight neighbouring rows meet no bank twice, and nothing has to be transposed.
 #include "common.cuh"
+#include "mma_util.cuh"
 
-#define SG_BM 64
-#define SG_BN 64
-#define SG_BK 16
+__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+// 4 bytes global -> shared (rows that do not lie on 16 bytes); bytes 0: zeros
+__device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
+}
 
-__global__ void __launch_bounds__(256)
+// A block of (BM / TM) x (BN / TN) threads makes a BM x BN tile; thread (ty, tx) has rows
+// ty + i (BM / TM) and columns tx + j (BN / TN).  VEC: rows of both operands start on 16 bytes
+// and K is a multiple of 4.
+template <int BM, int BN, int TM, int TN, int BK, int STAGES, bool VEC>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
 sgemm_nt_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
                 int M, int N, int K, int lda, int ldw, int ldc) {
-    __shared__ __align__(16) float As[SG_BK][SG_BM + 4];
-    __shared__ __align__(16) float Ws[SG_BK][SG_BN + 4];
-    const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;
-    const int m0 = blockIdx.y * SG_BM, n0 = blockIdx.x * SG_BN;
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    constexpr int TY = BM / TM, TX = BN / TN, THREADS = TY * TX, LD = BK + 4;
+    constexpr int STAGE = (BM + BN) * LD;          // floats: the A rows, then the W rows
+    extern __shared__ __align__(16) float sg_smem[];
+    const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
 
-    for (int k0 = 0; k0 < K; k0 += SG_BK) {
+    auto load_stage = [&](int stage, int k0) {
+        float* dst = sg_smem + stage * STAGE;
+        if (VEC) {
+            constexpr int PER_ROW = BK / 4;
 #pragma unroll
-        for (int it = 0; it < 4; ++it) {
-            const int idx = tid + it * 256;      // 0..1023
-            const int r = idx >> 4, kk = idx & 15;
-            const int gk = k0 + kk;
-            float va = 0.f, vw = 0.f;
-            if (gk < K) {
-                if (m0 + r < M) va = A[(size_t)(m0 + r) * lda + gk];
-                if (n0 + r < N) vw = W[(size_t)(n0 + r) * ldw + gk];
+            for (int c = tid; c < (BM + BN) * PER_ROW; c += THREADS) {
+                const int r = c / PER_ROW, k = k0 + (c % PER_ROW) * 4;
+                const bool is_a = r < BM;
+                const int row = is_a ? m0 + r : n0 + r - BM;
+                const bool ok = row < (is_a ? M : N) && k < K;
+                const float* src = is_a ? A : W;
+                if (ok) src += (size_t)row * (is_a ? lda : ldw) + k;
+                cp_async_16(smem_u32(dst + r * LD + (c % PER_ROW) * 4), src, ok ? 16 : 0);
             }
-            As[kk][r] = va;
-            Ws[kk][r] = vw;
+        } else {
+            for (int c = tid; c < (BM + BN) * BK; c += THREADS) {
+                const int r = c / BK, k = k0 + c % BK;
+                const bool is_a = r < BM;
+                const int row = is_a ? m0 + r : n0 + r - BM;
+                const bool ok = row < (is_a ? M : N) && k < K;
+                const float* src = is_a ? A : W;
+                if (ok) src += (size_t)row * (is_a ? lda : ldw) + k;
+                cp_async_4(smem_u32(dst + r * LD + c % BK), src, ok ? 4 : 0);
+            }
         }
-        __syncthreads();
+    };
+
+    unsigned long long acc[TM][TN];                // (sum over even k, sum over odd k)
 #pragma unroll
-        for (int kk = 0; kk < SG_BK; ++kk) {
-            const float4 a4 = *reinterpret_cast<const float4*>(&As[kk][ty * 4]);
-            const float4 b4 = *reinterpret_cast<const float4*>(&Ws[kk][tx * 4]);
-            const float a[4] = {a4.x, a4.y, a4.z, a4.w};
-            const float b[4] = {b4.x, b4.y, b4.z, b4.w};
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+
+    const int blocks = (K + BK - 1) / BK;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
+    for (int s = 0; s < STAGES - 1; ++s) {
+        if (s < blocks) load_stage(s, s * BK);
+        cp_async_commit();
     }
+    for (int kb = 0; kb < blocks; ++kb) {
+        cp_async_wait<STAGES - 2>();
+        __syncthreads();
+        const int next = kb + STAGES - 1;
+        if (next < blocks) load_stage(next % STAGES, next * BK);
+        cp_async_commit();
+        const float* as = sg_smem + (kb % STAGES) * STAGE + ty * LD;
+        const float* ws = sg_smem + (kb % STAGES) * STAGE + (BM + tx) * LD;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + ty * 4 + i;
+        for (int k = 0; k < BK; k += 4) {
+            ulonglong2 a[TM];
+#pragma unroll
+            for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(as + i * TY * LD + k);
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(ws + j * TX * LD + k);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) {
+                    fma2(acc[i][j], a[i].x, w.x);
+                    fma2(acc[i][j], a[i].y, w.y);
+                }
+            }
+        }
+    }
+    cp_async_wait<0>();
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        const int m = m0 + ty + i * TY;
         if (m >= M) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx * 4 + j;
-            if (n < N) C[(size_t)m * ldc + n] = acc[i][j];
+        for (int j = 0; j < TN; ++j) {
+            const int n = n0 + tx + j * TX;
+            if (n < N)
+                C[(size_t)m * ldc + n] = __uint_as_float((uint32_t)acc[i][j]) +
+                                         __uint_as_float((uint32_t)(acc[i][j] >> 32));
         }
     }
+}
+
+template <int BM, int BN, int TM, int TN, int BK, int STAGES>
+static int launch_sgemm(const float* A, const float* W, float* C, int M, int N, int K, int lda,
+                        int ldw, int ldc, bool vec, cudaStream_t s) {
+    constexpr int smem = STAGES * (BM + BN) * (BK + 4) * (int)sizeof(float);
+    constexpr int threads = (BM / TM) * (BN / TN);
+    auto kernel = vec ? sgemm_nt_kernel<BM, BN, TM, TN, BK, STAGES, true>
+                      : sgemm_nt_kernel<BM, BN, TM, TN, BK, STAGES, false>;
+    static bool configured[2] = {false, false};
+    if (smem > 48 * 1024 && !configured[vec]) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return (int)e;
+        configured[vec] = true;
+    }
+    const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
+    kernel<<<grid, threads, smem, s>>>(A, W, C, M, N, K, lda, ldw, ldc);
+    return launch_status();
 }
 
 MSTAR_API int mstar_sgemm_nt(const float* A, const float* W, float* C, int M, int N, int K,
                              int lda, int ldw, int ldc, void* stream) {
     if (M <= 0 || N <= 0) return 0;
-    dim3 grid((N + SG_BN - 1) / SG_BN, (M + SG_BM - 1) / SG_BM);
-    sgemm_nt_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(A, W, C, M, N, K, lda, ldw, ldc);
-    return launch_status();
+    cudaStream_t s = (cudaStream_t)stream;
+    const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
+                     ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0;
+    const int sms = device_sm_count();
+    auto tiles = [&](int bm, int bn) { return (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
+    // Few rows: the stream of W counts, so narrow tiles (a block an SM or more) with deep stages.
+    // [8, 2048] x [3072, 2048]: 21 us, [8, 3072] x [16384, 3072]: 78 us (64 x 64 tiles of 16 k, no
+    // stages in flight: 248 and 640 us); with 16 rows a tile these two take 25 and 120 us.
+    if (M <= 8) return launch_sgemm<8, 16, 2, 1, 128, 4>(A, W, C, M, N, K, lda, ldw, ldc, vec, s);
+    // up to 32 rows: 30 against 40 to 52 us for tiles of 32 rows at [30, 2048] x [3072, 2048];
+    // twice as wide where that still makes two blocks an SM
+    if (M <= 32) {
+        if (tiles(16, 32) >= 2 * sms)
+            return launch_sgemm<16, 32, 2, 2, 64, 4>(A, W, C, M, N, K, lda, ldw, ldc, vec, s);
+        return launch_sgemm<16, 16, 2, 2, 64, 4>(A, W, C, M, N, K, lda, ldw, ldc, vec, s);
+    }
+    // 64 x 64 tiles with 8 x 4 outputs a thread where they give every SM more than one block (several
+    // share an SM): 46 TFLOP/s at [2048, 4096] x [4096, 4096], 36 at [512, 2048] x [3072, 2048], against
+    // 40 to 42 and 26 to 29 for 128 x 128 and 64 x 128 tiles of 8 x 8.  Below that 32 x 32 tiles: 51
+    // against 75 us at [64, 2048] x [3072, 2048].
+    if (tiles(64, 64) * 2 >= 3 * sms)
+        return launch_sgemm<64, 64, 8, 4, 32, 3>(A, W, C, M, N, K, lda, ldw, ldc, vec, s);
+    return launch_sgemm<32, 32, 4, 4, 32, 4>(A, W, C, M, N, K, lda, ldw, ldc, vec, s);
 }
