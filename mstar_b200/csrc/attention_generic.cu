@@ -11,7 +11,11 @@
 // One block per (token, kv head) handles the whole group of query heads, streaming
 // the keys and values of that head through shared memory in tiles of 32 keys with
 // an online softmax.  The keys of the current step are already in the cache.
+//
+// Float prompt portions with a head_dim of 64 or 128 take the second kernel below, whose
+// blocks share a tile of keys among 64 rows.
 #include "common.cuh"
+#include "mma_util.cuh"
 
 #define ATT_TILE 32
 #define ATT_THREADS 128
@@ -143,20 +147,262 @@ paged_attention_generic_kernel(const A* __restrict__ q, A* __restrict__ out,
     }
 }
 
-// Returns 0, a CUDA error code, or -1 when the shape is refused
-// (group * head_dim > 4096 or head_dim > 256).
+// ------------------------------------------------------------------ float prompt portions
+// The same attention for float tokens that come in runs of one request: a block takes 64 rows
+// (token, head of the group) of one kv head and walks their keys in tiles of 64, so that a key
+// is fetched once for all of them.  Thread (ty, tx) of 16 x 16 owns rows ty + 16 i from the
+// scores to the output: 4 x 4 scores of a tile (packed FMAs over pairs of features), a row's
+// maximum and sum by shuffles among its 16 threads, then 4 rows x HD / 16 output columns
+// (packed FMAs over pairs of columns).  Only the probabilities pass through shared memory; the
+// next tile's keys are fetched under the softmax and the sum, its values under the scores.
+// Tiles start at multiples of 64 keys whatever the block's rows are, and a tile that a row does
+// not see leaves its sums as they are, so a row's result does not depend on what else is in the
+// batch.  Bound by the FMA pipe and the shared loads that feed it (of 16 bytes, no bank met
+// twice): the float attention of 384 prompt tokens with 32 / 8 heads of 64 (requests of 256 and
+// 128) took 435 us with a block per token and takes 41 us.
+#define AR_ROWS 64
+#define AR_KEYS 64
+#define AR_THREADS 256
+
+__device__ __forceinline__ void ar_fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long ar_pack(float lo, float hi) {
+    return (unsigned long long)__float_as_uint(lo) | ((unsigned long long)__float_as_uint(hi) << 32);
+}
+__device__ __forceinline__ float ar_lo(unsigned long long v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float ar_hi(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
+
+// O += P V of one tile.  MASKED: a key past the row's last one is left out (a probability of zero
+// would still make a NaN of a value that is not finite).
+template <int HD, bool MASKED>
+__device__ __forceinline__ void ar_output(unsigned long long (&acc)[4][HD / 32], const float* p_s,
+                                          const float* v_s, int ty, int tx, int key0, const int (&lo_r)[4],
+                                          const int (&hi_r)[4]) {
+    constexpr int PL = AR_KEYS + 4;
+#pragma unroll 2
+    for (int j = 0; j < AR_KEYS; j += 4) {
+        float4 p[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(p_s + (ty + 16 * i) * PL + j);
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {
+            unsigned long long v[HD / 32];
+#pragma unroll
+            for (int c = 0; c < HD / 32; ++c)
+                v[c] = *reinterpret_cast<const unsigned long long*>(v_s + (j + jj) * HD + 2 * tx + 32 * c);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (MASKED && !(key0 + j + jj >= lo_r[i] && key0 + j + jj < hi_r[i])) continue;
+                const float pj = jj == 0 ? p[i].x : jj == 1 ? p[i].y : jj == 2 ? p[i].z : p[i].w;
+                const unsigned long long pp = ar_pack(pj, pj);
+#pragma unroll
+                for (int c = 0; c < HD / 32; ++c) ar_fma2(acc[i][c], pp, v[c]);
+            }
+        }
+    }
+}
+
+template <int HD>
+__global__ void __launch_bounds__(AR_THREADS)
+attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
+                          const float* __restrict__ kv_cache, const int* __restrict__ block_table,
+                          const int* __restrict__ token_req, const int* __restrict__ cache_pos,
+                          AttnArgs a, int num_tokens) {
+    constexpr int QL = HD + 4, PL = AR_KEYS + 4;   // floats between rows: 16-byte reads of 8 rows
+    extern __shared__ __align__(16) float ar_smem[];
+    float* q_s = ar_smem;                          // [ROWS][QL]
+    float* k_s = q_s + AR_ROWS * QL;               // [KEYS][QL]
+    float* v_s = k_s + AR_KEYS * QL;               // [KEYS][HD]
+    float* p_s = v_s + AR_KEYS * HD;               // [ROWS][PL]
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int kvh = blockIdx.x;
+    const int G = a.nq / a.nkv, TPB = AR_ROWS / G;
+    // (the tokens with the most keys first)
+    const int t0 = (int)(gridDim.y - 1 - blockIdx.y) * TPB;
+    const int ntok = min(TPB, num_tokens - t0), nrows = ntok * G;
+    const size_t page_elems = (size_t)2 * a.nkv * a.page_size * HD;
+    const size_t v_off = (size_t)a.nkv * a.page_size * HD;
+    const float* head_base = kv_cache + (size_t)kvh * a.page_size * HD;
+
+    for (int c = tid; c < AR_ROWS * (HD / 4); c += AR_THREADS) {
+        const int r = c / (HD / 4), d = (c % (HD / 4)) * 4;
+        const bool ok = r < nrows;
+        const float* src = q;
+        if (ok) src += (size_t)(t0 + r / G) * a.q_stride + (size_t)(kvh * G + r % G) * HD + d;
+        cp_async_16(smem_u32(q_s + r * QL + d), src, ok ? 16 : 0);
+    }
+    cp_async_commit();
+
+    for (int s0 = 0; s0 < ntok;) {
+        // tokens s0 .. s1-1 of the block belong to one request
+        const int req = token_req[t0 + s0];
+        int s1 = s0, lo_min = 0x7fffffff, hi_max = 0;
+        for (; s1 < ntok && token_req[t0 + s1] == req; ++s1) {
+            const int hi = cache_pos[t0 + s1] + 1;
+            lo_min = min(lo_min, (a.window > 0 && hi > a.window) ? hi - a.window : 0);
+            hi_max = max(hi_max, hi);
+        }
+        const int* bt = block_table + (size_t)req * a.bt_stride;
+        int lo_r[4], hi_r[4];                      // the keys that this thread's rows see
+        int full_lo = 0, full_hi = 0x7fffffff;     // ... and those that every one of them sees
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = ty + 16 * i, tk = r / G;
+            lo_r[i] = hi_r[i] = 0;                 // a row of another request: idle
+            if (r < nrows && tk >= s0 && tk < s1) {
+                hi_r[i] = cache_pos[t0 + tk] + 1;
+                lo_r[i] = (a.window > 0 && hi_r[i] > a.window) ? hi_r[i] - a.window : 0;
+            }
+            full_lo = max(full_lo, lo_r[i]);
+            full_hi = min(full_hi, hi_r[i]);
+        }
+        auto load = [&](bool values, int key0) {
+            for (int c = tid; c < AR_KEYS * (HD / 4); c += AR_THREADS) {
+                const int j = c / (HD / 4), d = (c % (HD / 4)) * 4, key = key0 + j;
+                const bool ok = key >= lo_min && key < hi_max;
+                const float* src = kv_cache;
+                if (ok)
+                    src = head_base + (size_t)bt[key / a.page_size] * page_elems + (values ? v_off : 0) +
+                          (size_t)(key % a.page_size) * HD + d;
+                cp_async_16(smem_u32(values ? v_s + j * HD + d : k_s + j * QL + d), src, ok ? 16 : 0);
+            }
+            cp_async_commit();
+        };
+        float m[4], l[4];
+        unsigned long long acc[4][HD / 32];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            m[i] = -INFINITY;
+            l[i] = 0.f;
+#pragma unroll
+            for (int c = 0; c < HD / 32; ++c) acc[i][c] = 0ull;
+        }
+        const int first = lo_min / AR_KEYS * AR_KEYS;
+        load(false, first);
+        load(true, first);
+        for (int key0 = first; key0 < hi_max; key0 += AR_KEYS) {
+            cp_async_wait<1>();                    // the keys (and the queries) are there
+            __syncthreads();
+            unsigned long long s2[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s2[i][j] = 0ull;
+#pragma unroll 4
+            for (int d = 0; d < HD; d += 4) {
+                ulonglong2 qv[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) qv[i] = *reinterpret_cast<const ulonglong2*>(q_s + (ty + 16 * i) * QL + d);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const ulonglong2 kv = *reinterpret_cast<const ulonglong2*>(k_s + (tx + 16 * j) * QL + d);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        ar_fma2(s2[i][j], qv[i].x, kv.x);
+                        ar_fma2(s2[i][j], qv[i].y, kv.y);
+                    }
+                }
+            }
+            __syncthreads();                       // the keys are done with
+            if (key0 + AR_KEYS < hi_max) load(false, key0 + AR_KEYS);
+            else cp_async_commit();
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float s[4], mx = -INFINITY;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int key = key0 + tx + 16 * j;
+                    s[j] = key >= lo_r[i] && key < hi_r[i] ? (ar_lo(s2[i][j]) + ar_hi(s2[i][j])) * a.scale
+                                                           : -INFINITY;
+                    mx = fmaxf(mx, s[j]);
+                }
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+                const float m_new = fmaxf(m[i], mx);
+                const bool none = m_new == -INFINITY;          // the row has seen no key yet
+                const float alpha = none ? 1.f : expf(m[i] - m_new);
+                m[i] = m_new;
+                float sum = 0.f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float p = none ? 0.f : expf(s[j] - m_new);
+                    sum += p;
+                    p_s[(ty + 16 * i) * PL + tx + 16 * j] = p;
+                }
+                l[i] = l[i] * alpha + sum;
+                const unsigned long long aa = ar_pack(alpha, alpha);
+#pragma unroll
+                for (int c = 0; c < HD / 32; ++c)
+                    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[i][c]) : "l"(aa));
+            }
+            cp_async_wait<1>();                    // the values are there
+            __syncthreads();
+            if (key0 >= full_lo && key0 + AR_KEYS <= full_hi)
+                ar_output<HD, false>(acc, p_s, v_s, ty, tx, key0, lo_r, hi_r);
+            else
+                ar_output<HD, true>(acc, p_s, v_s, ty, tx, key0, lo_r, hi_r);
+            __syncthreads();                       // the values and the probabilities are done with
+            if (key0 + AR_KEYS < hi_max) load(true, key0 + AR_KEYS);
+            else cp_async_commit();
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float sum = l[i];
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            if (hi_r[i] == 0) continue;
+            const int r = ty + 16 * i;
+            float* dst = out + (size_t)(t0 + r / G) * a.nq * HD + (size_t)(kvh * G + r % G) * HD + 2 * tx;
+#pragma unroll
+            for (int c = 0; c < HD / 32; ++c)
+                *reinterpret_cast<float2*>(dst + 32 * c) =
+                    make_float2(ar_lo(acc[i][c]) / sum, ar_hi(acc[i][c]) / sum);
+        }
+        s0 = s1;
+    }
+}
+
+template <int HD>
+static int launch_rows_f32(const float* q, float* out, const float* kv, const int* block_table,
+                           const int* token_req, const int* cache_pos, const AttnArgs& a, int num_tokens,
+                           cudaStream_t s) {
+    constexpr int smem = (int)sizeof(float) *
+                         (2 * AR_ROWS * (HD + 4) + AR_KEYS * HD + AR_ROWS * (AR_KEYS + 4));
+    static bool configured = false;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(attention_rows_f32_kernel<HD>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    const int per_block = AR_ROWS / (a.nq / a.nkv);
+    attention_rows_f32_kernel<HD><<<dim3(a.nkv, (num_tokens + per_block - 1) / per_block), AR_THREADS, smem, s>>>(
+        q, out, kv, block_table, token_req, cache_pos, a, num_tokens);
+    return launch_status();
+}
+
+// `portions`: the tokens come in runs of one request.  Returns 0, a CUDA error code, or -1 when
+// the shape is refused (group * head_dim > 4096 or head_dim > 256).
 MSTAR_API int mstar_paged_attention_generic(const void* q, int q_stride, void* out,
                                             const void* kv_cache, const int* block_table,
                                             int bt_stride, const int* token_req,
                                             const int* cache_pos, int num_tokens, int nq, int nkv,
                                             int hd, int page_size, int window, float scale,
-                                            int act_dtype, void* stream) {
+                                            int act_dtype, int portions, void* stream) {
     if (num_tokens <= 0) return 0;
     if (nkv <= 0 || nq % nkv != 0) return -1;
     const int G = nq / nkv;
     if (G * hd > ATT_MAX_ACC * ATT_THREADS || hd > 256) return -1;
     cudaStream_t s = (cudaStream_t)stream;
     AttnArgs a{nq, nkv, hd, page_size, bt_stride, window, q_stride, scale};
+    if (portions && act_dtype == MSTAR_F32 && (hd == 64 || hd == 128) && G <= AR_ROWS && q_stride % 4 == 0 &&
+        (((uintptr_t)q | (uintptr_t)kv_cache | (uintptr_t)out) & 15) == 0 && num_tokens <= 65535) {
+        return hd == 64 ? launch_rows_f32<64>((const float*)q, (float*)out, (const float*)kv_cache, block_table,
+                                              token_req, cache_pos, a, num_tokens, s)
+                        : launch_rows_f32<128>((const float*)q, (float*)out, (const float*)kv_cache, block_table,
+                                               token_req, cache_pos, a, num_tokens, s);
+    }
     const size_t smem = sizeof(float) * ((size_t)G * hd + (size_t)ATT_TILE * (hd + 1) +
                                          (size_t)G * ATT_TILE + 3 * (size_t)G);
     dim3 grid(num_tokens, nkv);

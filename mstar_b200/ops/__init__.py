@@ -236,16 +236,20 @@ def rope_kv_write(qkv: torch.Tensor, positions, cache_pos, token_req, block_tabl
 def paged_attention_generic(q: torch.Tensor, q_stride: int, out: torch.Tensor, kv_cache,
                             block_table, token_req, cache_pos, num_tokens: int, num_heads: int,
                             num_kv_heads: int, head_dim: int, page_size: int, window: int,
-                            scale: float) -> None:
+                            scale: float, entries: int | None = None) -> None:
     """Attention of ``num_tokens`` query rows (portions and decoded tokens alike)
     over the paged cache; ``q`` may be a view into the fused qkv buffer with
-    ``q_stride`` elements between tokens."""
+    ``q_stride`` elements between tokens.  ``entries``: how many requests the tokens belong to;
+    where they come in runs of one request (four tokens an entry or more), a block of the float
+    kernel takes the rows of several tokens (it walks its requests one after another: a block of
+    single tokens would walk as many caches)."""
     _need_cuda(q, out, kv_cache, block_table, token_req, cache_pos)
     assert out.is_contiguous() and kv_cache.is_contiguous()
     code = lib.get("attention_generic").mstar_paged_attention_generic(
         q.data_ptr(), q_stride, out.data_ptr(), kv_cache.data_ptr(), block_table.data_ptr(),
         block_table.stride(0), token_req.data_ptr(), cache_pos.data_ptr(), num_tokens,
-        num_heads, num_kv_heads, head_dim, page_size, window, float(scale), _dt(out), _stream())
+        num_heads, num_kv_heads, head_dim, page_size, window, float(scale), _dt(out),
+        int(entries is not None and num_tokens >= 4 * max(entries, 1)), _stream())
     if code == -1:
         raise KernelError(
             f"paged attention refuses heads={num_heads}, kv_heads={num_kv_heads}, "

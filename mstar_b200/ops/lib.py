@@ -112,7 +112,7 @@ _SIGNATURES = {
     },
     "attention_generic": {
         "mstar_paged_attention_generic": [_vp, _i, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i,
-                                          _i, _i, _f, _i, _vp],
+                                          _i, _i, _f, _i, _i, _vp],
     },
     "attention_decode": {
         "mstar_make_kv_tensor_map": [_vp, _vp, _ll, _i, _i, _i],

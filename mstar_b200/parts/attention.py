@@ -231,10 +231,15 @@ class Attention:
                     ctx.kv_len, nd, ctx.num_entries - nd, max(ctx.q_lens[nd:]), s.num_heads,
                     s.num_kv_heads, s.head_dim, cache.page_size, s.window or 0, self.scale)
             return
-        ops.paged_attention_generic(
-            qkv, qkv.stride(0), out, cache.kv, cache.block_table, ctx.token_req, ctx.cache_pos,
-            ctx.num_tokens, s.num_heads, s.num_kv_heads, s.head_dim, cache.page_size,
-            s.window or 0, self.scale)
+        # single tokens and portions apart: a block of the float kernel may take the rows of
+        # several tokens of one request
+        nd = ctx.num_decode
+        for t0, t1, entries in ((0, nd, nd), (nd, ctx.num_tokens, ctx.num_entries - nd)):
+            if t1 > t0:
+                ops.paged_attention_generic(
+                    qkv[t0:], qkv.stride(0), out[t0:], cache.kv, cache.block_table,
+                    ctx.token_req[t0:], ctx.cache_pos[t0:], t1 - t0, s.num_heads, s.num_kv_heads,
+                    s.head_dim, cache.page_size, s.window or 0, self.scale, entries=entries)
 
 
 register_part("mixer", "attention", Attention)
