@@ -102,6 +102,16 @@ __device__ __forceinline__ float clamped_swish(float gate, float up, float limit
     return g / (1.f + expf(-alpha * g)) * (u + 1.f);
 }
 
+// The same two gates for results that are rounded to bfloat16 right after: the quotient by
+// __fdividef (2 ulp of a float; a denominator past 2^126 gives 0 where the quotient is under 1e-36).
+// The IEEE division costs some 20 instructions, and several times that where the gate is 0 (rows of
+// a tile past the matrix): the epilogue of a 128-column tile took 6 to 20 us with it.
+__device__ __forceinline__ float silu_bf16(float g) { return __fdividef(g, 1.f + expf(-g)); }
+__device__ __forceinline__ float clamped_swish_bf16(float gate, float up, float limit, float alpha) {
+    const float g = fminf(gate, limit), u = fminf(fmaxf(up, -limit), limit);
+    return __fdividef(g, 1.f + expf(-alpha * g)) * (u + 1.f);
+}
+
 // Sum over a whole block; `scratch` holds at least 32 floats of shared memory.
 // Every thread gets the result.  Safe to call repeatedly with the same scratch.
 __device__ __forceinline__ float block_sum(float v, float* scratch) {

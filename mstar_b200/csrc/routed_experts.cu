@@ -380,9 +380,9 @@ MSTAR_API int mstar_experts_by_row(const void* x, const void* w_gate_up, const v
 
 // ====================================================================== grouped by expert
 // For many rows (prompt portions) the rows are sorted by expert, and every expert's rows go
-// through its matrices as tiles of a tensor-core GEMM (bfloat16 mma.sync, float sums):
+// through its matrices as tiles of a tensor-core GEMM (tcgen05, bfloat16, float sums in TMEM):
 //   1. experts_sort: counting sort of the rows (token x choice) by expert; the list of row
-//      tiles (expert, first sorted row), one per 64 (or 128) rows of a group.
+//      tiles (expert, first sorted row), one per 128 rows of a group.
 //   2. grouped GEMM, gated: act[p] = silu(w G) * (w U), G and U the products of the gathered
 //      token rows with the expert's gate and up rows (bfloat16 out, sorted order).
 //   3. grouped GEMM, plain: y[p] = act[p] W_down[e]^T (float out, sorted order).
@@ -391,201 +391,387 @@ MSTAR_API int mstar_experts_by_row(const void* x, const void* w_gate_up, const v
 // A row's numbers depend on its own inputs only: the position of a row in its tile changes
 // nothing, so the order inside a group need not be stable.
 #include "mma_util.cuh"
+#include "tma_util.cuh"
+#include "tcgen05_util.cuh"
 
-#define GG_BN 64
-#define GG_BK 32
-#define GG_LD 40          // bf16 elements between rows of a shared tile (80 bytes: no bank conflicts)
-#define GG_STAGES 3
+#define GG_BM 128
+#define GG_BN 256                 // accumulator columns of a tile
+#define GG_BK 64
+#define GG_STAGES 4
+// the producer warp, the MMA warp, four epilogue warps and, where token rows are gathered, four more
+__host__ __device__ constexpr int gg_threads(bool gather) { return gather ? 320 : 192; }
+#define GG_STORE_LD 36            // floats between rows of an epilogue warp's 32 x 32 staging tile
+#define GG_A_BYTES (GG_BM * GG_BK * 2)
+#define GG_STAGE_BYTES ((GG_BM + GG_BN) * GG_BK * 2)
 
-// `experts`: all router outputs; tiles are made for the first `real` of them only.
-__global__ void experts_sort_kernel(const int* __restrict__ chosen, int rows, int experts, int real, int tile_rows,
-                                    int* __restrict__ order, int* __restrict__ pos,
-                                    int* __restrict__ offsets, int* __restrict__ tile_expert,
-                                    int* __restrict__ tile_first, int* __restrict__ num_tiles) {
-    extern __shared__ int sh[];               // counts[experts], cursor[experts]
-    int* counts = sh;
-    int* cursor = sh + experts;
+// `experts`: all router outputs; tiles are made for the first `real` of them only.  One block of
+// 1,024 threads, a thread an expert between the two passes over the rows: 7 us for 8,192 rows and 32
+// experts (14 us with one thread making the list and rows asked for one at a time).
+__global__ void __launch_bounds__(1024)
+experts_sort_kernel(const int* __restrict__ chosen, int rows, int experts, int real,
+                    int* __restrict__ order, int* __restrict__ pos, int* __restrict__ offsets,
+                    int* __restrict__ tile_expert, int* __restrict__ tile_first,
+                    int* __restrict__ num_tiles) {
+    __shared__ int cursor[1024];
+    __shared__ int warp_rows[32], warp_tiles[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    cursor[tid] = 0;
     chosen = pdl_after(chosen, pdl_wait());
-    for (int e = threadIdx.x; e < experts; e += blockDim.x) counts[e] = 0;
     __syncthreads();
-    for (int r = threadIdx.x; r < rows; r += blockDim.x) atomicAdd(&counts[chosen[r]], 1);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int at = 0, tiles = 0;
-        for (int e = 0; e < experts; ++e) {
-            offsets[e] = at;
-            cursor[e] = at;
-            for (int p = at; e < real && p < at + counts[e]; p += tile_rows) {
-                tile_expert[tiles] = e;
-                tile_first[tiles] = p;
-                ++tiles;
+    // A row's place in its group is what its expert's counter held before it.  A thread asks for its
+    // rows eight at a time and keeps the first eight for the second pass; further ones leave their
+    // place in pos.  (Lanes counting together by __match_any_sync were slower than the atomics.)
+    int mine[8], place[8];
+    for (int r0 = tid; r0 < rows; r0 += 8 * 1024) {
+        int e[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) e[i] = r0 + i * 1024 < rows ? chosen[r0 + i * 1024] : -1;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int at = e[i] >= 0 ? atomicAdd(&cursor[e[i]], 1) : 0;
+            if (r0 < 1024) {
+                mine[i] = e[i];
+                place[i] = at;
+            } else if (e[i] >= 0) {
+                pos[r0 + i * 1024] = at;
             }
-            at += counts[e];
         }
-        offsets[experts] = at;
-        *num_tiles = tiles;
     }
     __syncthreads();
-    for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-        const int p = atomicAdd(&cursor[chosen[r]], 1);
-        order[p] = r;
-        pos[r] = p;
+    // exclusive sums over the experts of the rows and of the tiles
+    const int n = tid < experts ? cursor[tid] : 0;
+    const int t = tid < real ? (n + GG_BM - 1) / GG_BM : 0;
+    int rows_to = n, tiles_to = t;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, rows_to, o), b = __shfl_up_sync(0xffffffffu, tiles_to, o);
+        if (lane >= o) {
+            rows_to += a;
+            tiles_to += b;
+        }
+    }
+    if (lane == 31) {
+        warp_rows[warp] = rows_to;
+        warp_tiles[warp] = tiles_to;
+    }
+    __syncthreads();
+    for (int w = 0; w < warp; ++w) {
+        rows_to += warp_rows[w];
+        tiles_to += warp_tiles[w];
+    }
+    const int first = rows_to - n, tile0 = tiles_to - t;
+    if (tid < experts) {
+        offsets[tid] = first;
+        cursor[tid] = first;
+        for (int i = 0; i < t; ++i) {
+            tile_expert[tile0 + i] = tid;
+            tile_first[tile0 + i] = first + i * GG_BM;
+        }
+    }
+    if (tid == 1023) {
+        offsets[experts] = rows_to;
+        *num_tiles = tiles_to;
+    }
+    __syncthreads();
+    for (int r0 = tid; r0 < rows; r0 += 8 * 1024) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int r = r0 + i * 1024;
+            if (r >= rows) continue;
+            const int at = r0 < 1024 ? cursor[mine[i]] + place[i] : cursor[chosen[r]] + pos[r];
+            order[at] = r;
+            pos[r] = at;
+        }
     }
 }
 
-// C tile [GG_BM x 64] of one expert's group (a warp per 32 x 32 of it).  GATED: A rows are x[order[p] / top], B rows are
-// the expert's gate rows n0.. and up rows ff + n0..; out = silu(w G) * (w U) as bfloat16.
-// Plain: A rows are act[p], B rows the expert's down rows n0..; out float.
-// MODE 0: plain (down), 1: gated gate/up with SiLU, 2: up alone with relu^2 (A rows gathered
-// like the gated form, one block of B rows, bfloat16 out).
-template <int MODE, int GG_BM>
-__global__ void __launch_bounds__(GG_BM * 2)
-grouped_gemm_kernel(const bf16* __restrict__ a_src, const bf16* __restrict__ w, void* __restrict__ out,
-                    const int* __restrict__ order, const float* __restrict__ weight,
-                    const int* __restrict__ offsets, const int* __restrict__ tile_expert,
-                    const int* __restrict__ tile_first, const int* __restrict__ num_tiles,
-                    int N, int K, int top, int scale_input, int clamped, float limit, float alpha) {
-    constexpr bool GATED = MODE == 1;
-    constexpr bool GATHER = MODE != 0;
-    constexpr int BROWS = GATED ? 2 * GG_BN : GG_BN;
-    constexpr int GG_THREADS = GG_BM * 2;             // a warp per 32 x 32 of the tile
-    extern __shared__ __align__(16) unsigned char gg_smem[];
-    bf16 (*As)[GG_BM * GG_LD] = reinterpret_cast<bf16 (*)[GG_BM * GG_LD]>(gg_smem);
-    bf16 (*Bs)[BROWS * GG_LD] = reinterpret_cast<bf16 (*)[BROWS * GG_LD]>(
-        gg_smem + sizeof(bf16) * GG_STAGES * GG_BM * GG_LD);
-    int* src_row = reinterpret_cast<int*>(gg_smem + sizeof(bf16) * GG_STAGES * (GG_BM + BROWS) * GG_LD);
+struct GroupedArgs {
+    void* out;
+    const int* order;
+    const float* weight;
+    const int* offsets;
+    const int* tile_expert;
+    const int* tile_first;
+    const int* num_tiles;
+    int N, K, top, n_tiles;       // N: output columns, n_tiles: column tiles of an expert
+    int scale_input, clamped;
+    float limit, alpha;
+};
+
+// Persistent CTAs walk over the tiles (row tile, column tile), a row tile's column tiles one after
+// another.  A tile is 128 sorted rows of one expert x 256 rows of its matrix, K in blocks of 64:
+//   warp 0     brings the expert's rows by TMA into a ring of four stages, two boxes of 128, and the
+//              rows of the down product, which lie in order, as a third;
+//   warps 6-9  bring token rows by cp.async (eight lanes a row of 128 bytes, swizzled as TMA would),
+//              and tell a stage's barrier two k-blocks later, when they have landed.  (TMA's gather4
+//              moved four rows in some 70 cycles, 32 of them a k-block: 128 us where this takes
+//              52.)
+//   warp 1     one lane issues tcgen05.mma (M 128, N 256, K 16) into one of two accumulators;
+//   warps 2-5  turn an accumulator into output rows while the next tile's products run; float rows
+//              pass through shared memory so that a store writes whole 128-byte rows.
+// MODE 0: plain (down), A rows are act[p], out float.  1: gated gate/up, A rows are x[order[p] /
+// top], columns 0..127 of the accumulator are gate rows and 128..255 the up rows of the same hidden
+// units, out = act(w G) * (w U) in bfloat16.  2: up alone with relu^2, bfloat16 out.
+// Rows of a tile past the group's last are computed from other rows and not stored.
+//
+// Bound by the operands' way from L2 (48 KB per 512 cycles of MMA and SM) and by the rows that fill
+// up a group's last tile.  2,048 tokens x 4 of 32 experts of 512 at width 2,048: gate/up 52 us, down
+// 31 us (operands alone: 26 and 9 us of MMA); as mma.sync tiles of 128 x 64 fed by cp.async they took
+// 200 and 102 us.
+template <int MODE>
+__global__ void __launch_bounds__(gg_threads(MODE != 0), 1)
+grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                    const bf16* __restrict__ x, GroupedArgs a, int* __restrict__ error_word) {
+    constexpr bool GATED = MODE == 1, GATHER = MODE != 0;
+    constexpr int OUT_COLS = GATED ? GG_BN / 2 : GG_BN;
+    extern __shared__ unsigned char gg_smem[];
+    // the swizzle pattern is a function of the address: stage buffers start on 1024 bytes
+    unsigned char* tiles = reinterpret_cast<unsigned char*>(
+        (reinterpret_cast<uintptr_t>(gg_smem) + 1023) & ~(uintptr_t)1023);
+    __shared__ __align__(8) uint64_t full_bar[GG_STAGES];
+    __shared__ __align__(8) uint64_t empty_bar[GG_STAGES];
+    __shared__ __align__(8) uint64_t acc_full[2];
+    __shared__ __align__(8) uint64_t acc_empty[2];
+    __shared__ uint32_t tmem_base_slot;
+    __shared__ int abort_flag;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < GG_STAGES; ++s) {
+            // the announcement of the TMA bytes, and every thread that gathers
+            mbar_init(tc_smem(&full_bar[s]), GATHER ? 1 + 128 : 1);
+            mbar_init(tc_smem(&empty_bar[s]), 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(tc_smem(&acc_full[b]), 1);
+            mbar_init(tc_smem(&acc_empty[b]), 4);       // the four epilogue warps
+        }
+        abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         tc_smem(&tmem_base_slot)),
+                     "r"(512u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = tmem_base_slot;
 
     const unsigned long long waited = pdl_wait();
-    a_src = pdl_after(a_src, waited);
-    order = pdl_after(order, waited);
-    num_tiles = pdl_after(num_tiles, waited);
-    if ((int)blockIdx.y >= *num_tiles) return;
-    const int e = tile_expert[blockIdx.y], p0 = tile_first[blockIdx.y];
-    const int p_end = offsets[e + 1];
-    const int n0 = blockIdx.x * GG_BN;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+    const int* order = pdl_after(a.order, waited);
+    const int* tile_expert = pdl_after(a.tile_expert, waited);
+    const int* tile_first = pdl_after(a.tile_first, waited);
+    const int* offsets = pdl_after(a.offsets, waited);
+    const int total = *pdl_after(a.num_tiles, waited) * a.n_tiles;
+    const int num_kb = (a.K + GG_BK - 1) / GG_BK;
 
-    if (tid < GG_BM) {
-        const int p = p0 + tid;
-        src_row[tid] = p < p_end ? (GATHER ? order[p] / top : p) : -1;
-    }
-    __syncthreads();
-    const bf16* wbase = w + (size_t)e * (GATED ? 2 : 1) * N * K;
-
-    auto load_stage = [&](int stage, int k0) {
-        // A: 64 rows x 4 chunks of 8
-        for (int c = tid; c < GG_BM * 4; c += GG_THREADS) {
-            const int r = c >> 2, kc = (c & 3) * 8;
-            const int src = src_row[r];
-            const bool ok = src >= 0 && k0 + kc < K;
-            const bf16* g = a_src + (ok ? (size_t)src * K + k0 + kc : 0);
-            cp_async_16(smem_u32(&As[stage][r * GG_LD + kc]), g, ok ? 16 : 0);
-        }
-        for (int c = tid; c < BROWS * 4; c += GG_THREADS) {
-            const int r = c >> 2, kc = (c & 3) * 8;
-            const int n = n0 + (r % GG_BN);
-            const bool ok = n < N && k0 + kc < K;
-            const size_t wrow = (GATED && r >= GG_BN) ? (size_t)N + n : (size_t)n;
-            const bf16* g = wbase + (ok ? wrow * K + k0 + kc : 0);
-            cp_async_16(smem_u32(&Bs[stage][r * GG_LD + kc]), g, ok ? 16 : 0);
-        }
-    };
-
-    float acc[GATED ? 2 : 1][2][4][4];
-#pragma unroll
-    for (int s = 0; s < (GATED ? 2 : 1); ++s)
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) acc[s][i][j][q] = 0.f;
-
-    const int k_tiles = (K + GG_BK - 1) / GG_BK;
-#pragma unroll
-    for (int s = 0; s < GG_STAGES - 1; ++s) {
-        if (s < k_tiles) load_stage(s, s * GG_BK);
-        cp_async_commit();
-    }
-    for (int kt = 0; kt < k_tiles; ++kt) {
-        cp_async_wait<GG_STAGES - 2>();
-        __syncthreads();
-        const int next = kt + GG_STAGES - 1;
-        if (next < k_tiles) load_stage(next % GG_STAGES, next * GG_BK);
-        cp_async_commit();
-        const bf16* At = As[kt % GG_STAGES];
-        const bf16* Bt = Bs[kt % GG_STAGES];
-#pragma unroll
-        for (int kk = 0; kk < GG_BK; kk += 16) {
-            uint32_t af[2][4];
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-                ldmatrix_x4(af[i], smem_u32(&At[(wm + i * 16 + (lane & 15)) * GG_LD + kk + (lane >> 4) * 8]));
-#pragma unroll
-            for (int s = 0; s < (GATED ? 2 : 1); ++s) {
-#pragma unroll
-                for (int jp = 0; jp < 2; ++jp) {
-                    uint32_t bfr[4];
-                    const int brow = s * GG_BN + wn + jp * 16 + (lane & 7) + (lane >> 4) * 8;
-                    ldmatrix_x4(bfr, smem_u32(&Bt[brow * GG_LD + kk + ((lane >> 3) & 1) * 8]));
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        mma_bf16_16816(acc[s][i][jp * 2], af[i], bfr[0], bfr[1]);
-                        mma_bf16_16816(acc[s][i][jp * 2 + 1], af[i], bfr[2], bfr[3]);
+    if (warp == 0) {
+        if (lane == 0) {
+            uint32_t it = 0;                            // k-blocks loaded so far, over all tiles
+            bool ok = true;
+            for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+                const int mt = t / a.n_tiles, n0 = (t - mt * a.n_tiles) * OUT_COLS;
+                const int e = tile_expert[mt], p0 = tile_first[mt];
+                // the expert's rows: gate rows n0.. and up rows N + n0.., or 256 rows from n0 on
+                const int w0 = e * (GATED ? 2 : 1) * a.N + n0, w1 = w0 + (GATED ? a.N : GG_BN / 2);
+                for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                    const int s = it % GG_STAGES;
+                    if (!mbar_wait(tc_smem(&empty_bar[s]), ((it / GG_STAGES) & 1u) ^ 1u)) {
+                        atomicExch(error_word, 19);
+                        abort_flag = 1;
+                        ok = false;
+                        break;
                     }
+                    const uint32_t bar = tc_smem(&full_bar[s]);
+                    const uint32_t at = tc_smem(tiles + (size_t)s * GG_STAGE_BYTES);
+                    mbar_expect_tx(bar, GATHER ? GG_STAGE_BYTES - GG_A_BYTES : GG_STAGE_BYTES);
+                    if (!GATHER) tma_load_2d(at, &map_a, bar, kb * GG_BK, p0);
+                    tma_load_2d(at + GG_A_BYTES, &map_b, bar, kb * GG_BK, w0);
+                    tma_load_2d(at + GG_A_BYTES + GG_BN / 2 * GG_BK * 2, &map_b, bar, kb * GG_BK, w1);
+                }
+                if (*(volatile int*)&abort_flag) break;
+            }
+        }
+    } else if (GATHER && warp >= 6) {
+        constexpr int LAG = 2;                          // k-blocks between asking and telling
+        const int sub = lane >> 3, chunk = lane & 7;    // row of four, 16-byte piece of the row
+        auto tell = [&](uint32_t done) {                // the MMA reads through the asynchronous proxy
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem(&full_bar[done % GG_STAGES])) : "memory");
+        };
+        uint32_t it = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+            const int mt = t / a.n_tiles;
+            const int p0 = tile_first[mt], p_last = offsets[tile_expert[mt] + 1] - 1;
+            const bf16* src[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                src[i] = x + (size_t)(order[min(p0 + (warp - 6) * 32 + i * 4 + sub, p_last)] / a.top) * a.K + chunk * 8;
+            for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                const int s = it % GG_STAGES;
+                ok = __all_sync(0xffffffffu, mbar_wait(tc_smem(&empty_bar[s]), ((it / GG_STAGES) & 1u) ^ 1u) &&
+                                                 !*(volatile int*)&abort_flag);
+                if (!ok) {
+                    if (lane == 0 && !*(volatile int*)&abort_flag) {
+                        atomicExch(error_word, 19);
+                        abort_flag = 1;
+                    }
+                    break;
+                }
+                const uint32_t at = tc_smem(tiles + (size_t)s * GG_STAGE_BYTES);
+                const bool in = kb * GG_BK + chunk * 8 < a.K;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int r = (warp - 6) * 32 + i * 4 + sub;
+                    cp_async_16(at + r * 128 + ((chunk ^ (r & 7)) << 4), in ? src[i] + kb * GG_BK : x, in ? 16 : 0);
+                }
+                cp_async_commit();
+                if (it >= LAG) {
+                    cp_async_wait<LAG>();
+                    tell(it - LAG);
+                }
+            }
+        }
+        cp_async_wait<0>();
+        if (ok)
+            for (uint32_t done = it > LAG ? it - LAG : 0; done < it; ++done) tell(done);
+    } else if (warp == 1) {
+        if (lane == 0) {
+            constexpr uint32_t idesc = instr_desc_bf16(GG_BM, GG_BN);
+            uint32_t it = 0;
+            int j = 0;                                  // tiles done by this CTA
+            bool ok = true;
+            for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++j) {
+                const int b = j & 1;
+                if (!mbar_wait(tc_smem(&acc_empty[b]), (((uint32_t)j >> 1) & 1u) ^ 1u)) {
+                    atomicExch(error_word, 20);
+                    abort_flag = 1;
+                    break;
+                }
+                tc_fence_after_sync();
+                const uint32_t tmem_d = tmem_base + (uint32_t)b * GG_BN;
+                for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                    const int s = it % GG_STAGES;
+                    if (!mbar_wait(tc_smem(&full_bar[s]), (it / GG_STAGES) & 1u)) {
+                        atomicExch(error_word, 20);
+                        abort_flag = 1;
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after_sync();
+                    const uint32_t a_addr = tc_smem(tiles + (size_t)s * GG_STAGE_BYTES);
+                    const uint32_t b_addr = a_addr + GG_A_BYTES;
+#pragma unroll
+                    for (int k4 = 0; k4 < GG_BK / 16; ++k4)
+                        tc_mma(tmem_d, smem_desc_sw128(a_addr + k4 * 32), smem_desc_sw128(b_addr + k4 * 32),
+                               idesc, (kb | k4) != 0 ? 1u : 0u);
+                    tc_commit(tc_smem(&empty_bar[s]));
+                }
+                if (ok) tc_commit(tc_smem(&acc_full[b]));
+            }
+        }
+    } else {
+        const int quarter = warp & 3;                   // the TMEM lanes this warp may touch
+        int j = 0;
+        for (int t = blockIdx.x; t < total; t += gridDim.x, ++j) {
+            const int b = j & 1;
+            const int mt = t / a.n_tiles, n0 = (t - mt * a.n_tiles) * OUT_COLS;
+            const int e = tile_expert[mt], p = tile_first[mt] + quarter * 32 + lane;
+            const int p_end = offsets[e + 1];
+            const bool valid = p < p_end;
+            float wgt = 1.f;
+            if (GATHER && a.scale_input && valid) wgt = a.weight[order[p]];
+            const bool ready = mbar_wait(tc_smem(&acc_full[b]), ((uint32_t)j >> 1) & 1u);
+            // one outcome for the warp: the loads from tensor memory below are warp-wide
+            if (!__all_sync(0xffffffffu, ready && !*(volatile int*)&abort_flag)) {
+                if (!ready && lane == 0) {
+                    atomicExch(error_word, 21);
+                    abort_flag = 1;
+                }
+                break;
+            }
+            tc_fence_after_sync();
+            const uint32_t tbase = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)b * GG_BN;
+#pragma unroll 1
+            for (int c0 = 0; c0 < OUT_COLS; c0 += 32) {
+                uint32_t r[32], u[32];
+                tc_ld32(tbase + (uint32_t)c0, r);
+                if (GATED) tc_ld32(tbase + (uint32_t)(c0 + GG_BN / 2), u);
+                tc_wait_ld();
+                if (c0 + 32 == OUT_COLS) {              // the accumulator is free, the stores follow
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0)
+                        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem(&acc_empty[b])) : "memory");
+                }
+                if (MODE == 0) {
+                    // through shared memory: eight lanes then store a row's 128 bytes (a lane a row
+                    // would touch 32 rows a store: the stores, not the products, set the pace)
+                    float* stage = reinterpret_cast<float*>(tiles + (size_t)GG_STAGES * GG_STAGE_BYTES) +
+                                   quarter * 32 * GG_STORE_LD;
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        *reinterpret_cast<uint4*>(stage + lane * GG_STORE_LD + 4 * i) =
+                            make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+                    __syncwarp();
+                    const int n = n0 + c0 + (lane & 7) * 4;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int row = i * 4 + (lane >> 3);
+                        const float4 v = *reinterpret_cast<const float4*>(stage + row * GG_STORE_LD + (lane & 7) * 4);
+                        if (p - lane + row < p_end && n < a.N)
+                            *reinterpret_cast<float4*>((float*)a.out + (size_t)(p - lane + row) * a.N + n) = v;
+                    }
+                    continue;
+                }
+                if (!valid) continue;
+                // N is a multiple of 8: whole groups of 8 columns are inside or outside
+#pragma unroll
+                for (int c = 0; c < 32; c += 8) {
+                    const int n = n0 + c0 + c;
+                    if (n >= a.N) break;
+                    float v[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const float g = __uint_as_float(r[c + i]) * wgt;
+                        if (GATED) {
+                            const float up = __uint_as_float(u[c + i]) * wgt;
+                            v[i] = a.clamped ? clamped_swish_bf16(g, up, a.limit, a.alpha) : silu_bf16(g) * up;
+                        } else {
+                            const float q = fmaxf(g, 0.f);
+                            v[i] = q * q;
+                        }
+                    }
+                    store8((bf16*)a.out + (size_t)p * a.N + n, v);
                 }
             }
         }
     }
-    cp_async_wait<0>();
-
-    const int g = lane >> 2, t4 = lane & 3;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int r = wm + i * 16 + g + half * 8;
-            const int p = p0 + r;
-            if (p >= p_end) continue;
-            float wgt = 1.f;
-            if (GATHER && scale_input) wgt = weight[order[p]];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int n = n0 + wn + j * 8 + 2 * t4;
-                if (n >= N) continue;
-                if (GATED) {
-                    const float g0 = acc[0][i][j][half * 2] * wgt, g1 = acc[0][i][j][half * 2 + 1] * wgt;
-                    const float u0 = acc[GATED ? 1 : 0][i][j][half * 2] * wgt;
-                    const float u1 = acc[GATED ? 1 : 0][i][j][half * 2 + 1] * wgt;
-                    bf16* o = (bf16*)out + (size_t)p * N + n;
-                    o[0] = __float2bfloat16_rn(clamped ? clamped_swish(g0, u0, limit, alpha)
-                                                       : g0 / (1.f + expf(-g0)) * u0);
-                    if (n + 1 < N)
-                        o[1] = __float2bfloat16_rn(clamped ? clamped_swish(g1, u1, limit, alpha)
-                                                           : g1 / (1.f + expf(-g1)) * u1);
-                } else if (MODE == 2) {
-                    const float r0 = fmaxf(acc[0][i][j][half * 2] * wgt, 0.f);
-                    const float r1 = fmaxf(acc[0][i][j][half * 2 + 1] * wgt, 0.f);
-                    bf16* o = (bf16*)out + (size_t)p * N + n;
-                    o[0] = __float2bfloat16_rn(r0 * r0);
-                    if (n + 1 < N) o[1] = __float2bfloat16_rn(r1 * r1);
-                } else {
-                    float* o = (float*)out + (size_t)p * N + n;
-                    o[0] = acc[0][i][j][half * 2];
-                    if (n + 1 < N) o[1] = acc[0][i][j][half * 2 + 1];
-                }
-            }
-        }
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after_sync();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u)
+                     : "memory");
     }
 }
 
+// A block a token, eight columns a thread: 16 us for 2,048 x 4 rows of 2,048 floats (67 MB, mostly in L2),
+// 36 us a column a thread.  Four rows of y are asked for at once, the sum runs in the
+// order of the choices.
 template <typename A>
-__global__ void experts_combine_kernel(const float* __restrict__ y, const int* __restrict__ pos,
-                                       const float* __restrict__ weight, const A* __restrict__ add,
-                                       A* __restrict__ out, int width, int top, int scale_input,
-                                       const int* __restrict__ chosen, const A* __restrict__ x,
-                                       int real, const float* add_gate, int gate_stride) {
+__global__ void __launch_bounds__(256)
+experts_combine_kernel(const float* __restrict__ y, const int* __restrict__ pos,
+                       const float* __restrict__ weight, const A* __restrict__ add, A* __restrict__ out,
+                       int width, int top, int scale_input, const int* __restrict__ chosen,
+                       const A* __restrict__ x, int real, const float* add_gate, int gate_stride) {
     const unsigned long long waited = pdl_wait();
     y = pdl_after(y, waited);
     pos = pdl_after(pos, waited);
@@ -593,78 +779,113 @@ __global__ void experts_combine_kernel(const float* __restrict__ y, const int* _
     add_gate = pdl_after(add_gate, waited);
     const int t = blockIdx.x;
     const float share = add_gate == nullptr ? 1.f : 1.f / (1.f + expf(-add_gate[(size_t)t * gate_stride]));
-    for (int c = threadIdx.x; c < width; c += blockDim.x) {
-        float total = 0.f;
-        for (int k = 0; k < top; ++k) {
-            if (chosen[(size_t)t * top + k] >= real) {     // identity expert: w x[t]
-                total += weight[(size_t)t * top + k] * to_float(x[(size_t)t * width + c]);
-                continue;
+    for (int c = threadIdx.x * 8; c < width; c += 256 * 8) {
+        float total[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (int k0 = 0; k0 < top; k0 += 4) {
+            float v[4][8];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (k0 + q >= top) continue;
+                const size_t r = (size_t)t * top + k0 + q;
+                // an identity expert: w x[t]
+                if (chosen[r] >= real) load8(x + (size_t)t * width + c, v[q]);
+                else load8(y + (size_t)pos[r] * width + c, v[q]);
             }
-            const float v = y[(size_t)pos[(size_t)t * top + k] * width + c];
-            total += scale_input ? v : v * weight[(size_t)t * top + k];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (k0 + q >= top) continue;
+                const size_t r = (size_t)t * top + k0 + q;
+                const float w = scale_input && chosen[r] < real ? 1.f : weight[r];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) total[i] += v[q][i] * w;
+            }
         }
-        if (add != nullptr) total += share * to_float(add[(size_t)t * width + c]);
-        out[(size_t)t * width + c] = from_float<A>(total);
+        if (add != nullptr) {
+            float s[8];
+            load8(add + (size_t)t * width + c, s);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) total[i] += share * s[i];
+        }
+        store8(out + (size_t)t * width + c, total);
     }
 }
 
-// bfloat16 only.  `ints`: scratch of 2 * rows + experts + 2 + 2 * (rows / 64 + experts) ints;
+// [rows, K] bfloat16 row-major; box = box_rows x 64
+static int gg_make_map(CUtensorMap* map, const void* base, long long rows, int K, int box_rows) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (fn == nullptr) return -3;
+    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
+    const cuuint32_t box[2] = {GG_BK, (cuuint32_t)box_rows};
+    const cuuint32_t elem[2] = {1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -4;
+}
+
+template <int MODE>
+static int launch_grouped(const CUtensorMap& ma, const CUtensorMap& mb, const void* x, GroupedArgs a, int max_row_tiles,
+                          int* error_word, cudaStream_t s) {
+    constexpr size_t smem = (size_t)GG_STAGES * GG_STAGE_BYTES + 1024 +
+                            (MODE == 0 ? 4 * 32 * GG_STORE_LD * sizeof(float) : 0);
+    static bool configured = false;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(grouped_gemm_kernel<MODE>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    const int cols = MODE == 1 ? GG_BN / 2 : GG_BN;
+    a.n_tiles = (a.N + cols - 1) / cols;
+    const long long most = (long long)max_row_tiles * a.n_tiles;
+    const int sms = device_sm_count();
+    mstar_launch((grouped_gemm_kernel<MODE>), dim3((unsigned)(most < sms ? most : sms)), dim3(gg_threads(MODE != 0)),
+                 smem, s, ma, mb, (const bf16*)x, a, error_word);
+    return launch_status();
+}
+
+// bfloat16 only.  `ints`: scratch of 2 * rows + experts + 2 + 2 * (rows / 128 + experts) ints;
 // `act`: bfloat16 [rows, ff]; `y`: float [rows, width] (rows = tokens * top).  Returns 0, a CUDA
-// error code, or -1 when the shape is refused (width or ff no multiple of 8, over 1024 experts).
+// error code, -1 when the shape is refused (width or ff no multiple of 8, over 1024 experts, an
+// operand off 16 bytes), or -3 / -4 when a tensor map cannot be made.  `error_word` receives 19 to 21
+// if a bounded wait ran out.
 MSTAR_API int mstar_experts_grouped(const void* x, const void* w_gate_up, const void* w_down,
                                     const int* chosen, const float* weight, int* ints, void* act,
                                     float* y, const void* add, void* out, int tokens, int width,
                                     int ff, int top, int experts, int scale_input, int gated,
                                     int real, float limit, float alpha, const float* add_gate,
-                                    int gate_stride, void* stream) {
+                                    int gate_stride, int* error_word, void* stream) {
     if (tokens <= 0) return 0;
     if (width % 8 != 0 || ff % 8 != 0 || experts <= 0 || experts > 1024 || top <= 0) return -1;
+    if (((uintptr_t)x | (uintptr_t)w_gate_up | (uintptr_t)w_down | (uintptr_t)act | (uintptr_t)y |
+         (uintptr_t)add | (uintptr_t)out) & 15)
+        return -1;
     cudaStream_t s = (cudaStream_t)stream;
     const int rows = tokens * top;
-    // tiles of 128 rows where an expert's group fills them on average, else of 64
-    const int bm = rows / experts >= 128 ? 128 : 64;
-    const int max_tiles = rows / bm + experts;
+    const int max_tiles = rows / GG_BM + experts;
     int* order = ints;
     int* pos = order + rows;
     int* offsets = pos + rows;
     int* num_tiles = offsets + experts + 1;
     int* tile_expert = num_tiles + 1;
-    int* tile_first = tile_expert + (rows / 64 + experts);
-    mstar_launch(experts_sort_kernel, dim3(1), dim3(1024), sizeof(int) * 2 * experts, s, chosen, rows,
-                 experts, real, bm, order, pos, offsets, tile_expert, tile_first, num_tiles);
-#define GG_SMEM(BM, BROWS) (sizeof(bf16) * GG_STAGES * ((BM) + (BROWS)) * GG_LD + sizeof(int) * (BM))
-#define GG_GO(MODE, BM, BROWS, GRIDX, ...)                                                        \
-    {                                                                                             \
-        static bool configured = false;                                                           \
-        const size_t bytes = GG_SMEM(BM, BROWS);                                                  \
-        if (!configured && bytes > 48 * 1024) {                                                   \
-            cudaFuncSetAttribute(grouped_gemm_kernel<MODE, BM>,                                   \
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);        \
-            configured = true;                                                                    \
-        }                                                                                         \
-        mstar_launch((grouped_gemm_kernel<MODE, BM>), dim3(GRIDX, max_tiles), dim3((BM) * 2), bytes, s, \
-                     __VA_ARGS__);                                                                \
-    }
-    const int gx1 = (ff + GG_BN - 1) / GG_BN, gx2 = (width + GG_BN - 1) / GG_BN;
-#define GG_UP(BM)                                                                                 \
-    if (gated)                                                                                    \
-        GG_GO(1, BM, 2 * GG_BN, gx1, (const bf16*)x, (const bf16*)w_gate_up, act, order, weight,  \
-              offsets, tile_expert, tile_first, num_tiles, ff, width, top, scale_input, (int)(gated == 2), limit, alpha)           \
-    else                                                                                          \
-        GG_GO(2, BM, GG_BN, gx1, (const bf16*)x, (const bf16*)w_gate_up, act, order, weight,      \
-              offsets, tile_expert, tile_first, num_tiles, ff, width, top, scale_input, (int)(gated == 2), limit, alpha)
-    if (bm == 128) {
-        GG_UP(128)
-        GG_GO(0, 128, GG_BN, gx2, (const bf16*)act, (const bf16*)w_down, (void*)y, order, weight,
-              offsets, tile_expert, tile_first, num_tiles, width, ff, top, scale_input, 0, 0.f, 0.f)
-    } else {
-        GG_UP(64)
-        GG_GO(0, 64, GG_BN, gx2, (const bf16*)act, (const bf16*)w_down, (void*)y, order, weight,
-              offsets, tile_expert, tile_first, num_tiles, width, ff, top, scale_input, 0, 0.f, 0.f)
-    }
-#undef GG_UP
-#undef GG_GO
-#undef GG_SMEM
+    int* tile_first = tile_expert + max_tiles;
+    CUtensorMap mgu, mact, mdn;
+    int rc = gg_make_map(&mgu, w_gate_up, (long long)real * (gated ? 2 : 1) * ff, width, GG_BN / 2);
+    if (rc == 0) rc = gg_make_map(&mact, act, rows, ff, GG_BM);
+    if (rc == 0) rc = gg_make_map(&mdn, w_down, (long long)real * width, ff, GG_BN / 2);
+    if (rc != 0) return rc;
+    mstar_launch(experts_sort_kernel, dim3(1), dim3(1024), 0, s, chosen, rows, experts, real, order, pos,
+                 offsets, tile_expert, tile_first, num_tiles);
+    GroupedArgs a{act, order, weight, offsets, tile_expert, tile_first, num_tiles, ff, width, top, 0,
+                  scale_input, (int)(gated == 2), limit, alpha};
+    rc = gated ? launch_grouped<1>(mgu, mgu, x, a, max_tiles, error_word, s)
+               : launch_grouped<2>(mgu, mgu, x, a, max_tiles, error_word, s);
+    if (rc != 0) return rc;
+    a.out = y;
+    a.N = width;
+    a.K = ff;
+    rc = launch_grouped<0>(mact, mdn, nullptr, a, max_tiles, error_word, s);
+    if (rc != 0) return rc;
     mstar_launch((experts_combine_kernel<bf16>), dim3(tokens), dim3(256), 0, s, (const float*)y, pos,
                  weight, (const bf16*)add, (bf16*)out, width, top, scale_input, chosen,
                  (const bf16*)x, real, add_gate, gate_stride);

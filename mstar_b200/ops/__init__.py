@@ -594,7 +594,7 @@ def tcgen05_error_word(device) -> torch.Tensor:
     """Device int32 that a kernel with bounded mbarrier waits sets when one of them ran out:
     1-3 tcgen05 GEMM (producer, MMA issuer, epilogue), 4 decode attention copies, 6-12 tcgen05
     prefill attention, 13-14 bulk-copy small-M GEMM, 15-17 swapped-operand tcgen05 GEMM, 18
-    delta-rule scan in pieces; zero otherwise."""
+    delta-rule scan in pieces, 19-21 grouped expert GEMM; zero otherwise."""
     key = torch.device(device).index or 0
     if key not in _tc_error_words:
         _tc_error_words[key] = torch.zeros(1, dtype=torch.int32, device=device)
@@ -614,6 +614,9 @@ WAIT_CODES.update({15: "swapped-operand tcgen05 GEMM: the producer waited for a 
                    16: "swapped-operand tcgen05 GEMM: the MMA issuer waited for operand tiles",
                    17: "swapped-operand tcgen05 GEMM: the epilogue waited for the accumulator"})
 WAIT_CODES[18] = "delta-rule scan in pieces: a wait for a piece's rows"
+WAIT_CODES.update({19: "grouped expert GEMM: the producer waited for a free stage",
+                   20: "grouped expert GEMM: the MMA issuer waited for operand tiles",
+                   21: "grouped expert GEMM: the epilogue waited for an accumulator"})
 WAIT_CODES.update({c: "tcgen05 prefill attention: a wait on one of its barriers ran out"
                    for c in range(6, 13)})
 
@@ -1283,8 +1286,8 @@ def experts_grouped(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tens
                     experts: int, ff: int, scale_input: bool, add=None, gated: bool = True,
                     real: int | None = None, clamp=None, add_gate=None) -> torch.Tensor:
     """The same sums as ``experts_by_row`` for many bfloat16 rows: rows sorted by expert on
-    the device, each expert's rows through its matrices as 64-row tiles on the tensor cores
-    (float sums), a token's choices added up in their order.  Nothing is read by the host."""
+    the device, each expert's rows through its matrices as 128-row tiles on the tensor cores
+    (tcgen05, float sums), a token's choices added up in their order.  Nothing is read by the host."""
     _need_cuda(x, w_gate_up, w_down, chosen, weight, add)
     tokens, width = x.shape
     top = chosen.shape[1]
@@ -1295,8 +1298,10 @@ def experts_grouped(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tens
     assert tuple(w_gate_up.shape) == (real * (2 if gated else 1) * ff, width)
     assert tuple(w_down.shape) == (real * width, ff)
     assert add is None or (add.shape == x.shape and add.is_contiguous() and add.dtype == x.dtype)
+    if add is not None and add.data_ptr() % 16:    # the kernels read whole 16-byte pieces
+        add = add.clone()
     rows = tokens * top
-    ints = torch.empty(2 * rows + experts + 2 + 2 * (rows // 64 + experts), dtype=torch.int32,
+    ints = torch.empty(2 * rows + experts + 2 + 2 * (rows // 128 + experts), dtype=torch.int32,
                        device=x.device)
     act = torch.empty((rows, ff), dtype=torch.bfloat16, device=x.device)
     y = torch.empty((rows, width), dtype=torch.float32, device=x.device)
@@ -1306,7 +1311,7 @@ def experts_grouped(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tens
         weight.data_ptr(), ints.data_ptr(), act.data_ptr(), y.data_ptr(), _ptr(add),
         out.data_ptr(), tokens, width, ff, top, experts, int(scale_input),
         _gated_code(gated, clamp), int(real), *(clamp or (0.0, 0.0)), *_add_gate(add_gate, tokens),
-        _stream())
+        tcgen05_error_word(x.device).data_ptr(), _stream())
     if code == -1:
         raise KernelError(f"the grouped expert kernels refuse width={width}, ff={ff}, "
                           f"experts={experts} (width and ff multiples of 8, at most 1024 experts)")

@@ -74,7 +74,7 @@ _SIGNATURES = {
         "mstar_experts_by_row": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,
                                  _i, _i, _f, _f, _vp, _i, _vp],
         "mstar_experts_grouped": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i,
-                                  _i, _i, _i, _i, _f, _f, _vp, _i, _vp],
+                                  _i, _i, _i, _i, _f, _f, _vp, _i, _vp, _vp],
     },
     "attention_sink": {
         "mstar_sink_prepare": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp, _vp, _i,

@@ -58,3 +58,50 @@ def test_float_attention_of_portions_leaves_unseen_values_out():
     ops.paged_attention_generic(q, hd, out, kv, i32([[0, 1]]), i32([0] * T), i32(list(range(T))), T, 1,
                                 1, hd, 16, 0, hd ** -0.5, entries=1)
     assert torch.isfinite(out[:-1]).all() and not torch.isfinite(out[-1]).any()
+
+
+@pytest.mark.parametrize("tokens,width,ff,experts,identity,top,form,on_input", [
+    (200, 72, 8, 2, 0, 2, "silu", False),         # k-blocks that end early, one narrow column tile
+    (300, 128, 264, 5, 1, 3, "silu", True),       # column tiles that end inside, identity experts
+    (129, 264, 136, 3, 0, 1, "relu2", False),     # one row past a row tile
+    (2100, 64, 16, 7, 2, 6, "clamped", False),    # more rows than the sort keeps in registers, top > 4
+    (64, 64, 64, 40, 0, 1, "silu", True)])        # experts without rows
+def test_grouped_experts_at_the_borders_of_their_tiles(tokens, width, ff, experts, identity, top, form, on_input):
+    """The grouped tensor-core experts against the sum in double precision from the same bfloat16
+    numbers; the only rounding on the way is that of the hidden units to bfloat16."""
+    from mstar_b200 import ops
+
+    gated, clamp = form != "relu2", (1.5, 1.702) if form == "clamped" else None
+    x = rnd(tokens, width, dtype=torch.bfloat16, seed=1)
+    w_up = rnd(experts * (2 if gated else 1) * ff, width, dtype=torch.bfloat16, seed=2, scale=0.2)
+    w_down = rnd(experts * width, ff, dtype=torch.bfloat16, seed=3, scale=0.2)
+    add = rnd(tokens, width, dtype=torch.bfloat16, seed=4)
+    gate = rnd(tokens, 1, seed=5)
+    chosen, weight = ops.route_topk(rnd(tokens, experts + identity, seed=6), top, softmax=True)
+    got = ops.experts_grouped(x, w_up, w_down, chosen, weight, experts + identity, ff, on_input, add,
+                              gated=gated, real=experts, clamp=clamp, add_gate=gate).double()
+    ops.check_error_word(DEV)
+    xd, ud, dd, w = x.double(), w_up.double().view(experts, -1, width), w_down.double().view(experts, width, ff), weight.double()
+    want = add.double() * torch.sigmoid(gate.double())
+    size = want.abs()
+    for e in range(experts + identity):
+        rows, place = (chosen == e).nonzero(as_tuple=True)
+        a = w[rows, place][:, None]
+        if e >= experts:
+            y = a * xd[rows]
+        else:
+            h = (xd[rows] * a if on_input else xd[rows]) @ ud[e].T
+            if gated:
+                g, u = h.chunk(2, dim=1)
+                if clamp:
+                    g, u = g.clamp(max=clamp[0]), u.clamp(-clamp[0], clamp[0]) + 1
+                    h = g * torch.sigmoid(clamp[1] * g) * u
+                else:
+                    h = g * torch.sigmoid(g) * u
+            else:
+                h = h.clamp(min=0) ** 2
+            b = 1.0 if on_input else a
+            y = b * (h @ dd[e].T)
+            size[rows] += b * (h.abs() @ dd[e].abs().T)      # what the hidden units' rounding can do
+        want[rows] += y
+    assert ((got - want).abs() <= 2 ** -8 * (size + want.abs()) + 1e-5).all()
