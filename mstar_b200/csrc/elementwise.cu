@@ -405,6 +405,34 @@ __global__ void silu_mul_kernel(const A* __restrict__ gate_up, A* __restrict__ o
     }
 }
 
+// The gate for eight numbers that become `A`: float results keep the IEEE division.
+template <typename A>
+__device__ __forceinline__ float gated_product(float g, float u, int kind, float limit, float alpha) {
+    if (kind == 3) return sizeof(A) == 2 ? clamped_swish_bf16(g, u, limit, alpha) : clamped_swish(g, u, limit, alpha);
+    if (sizeof(A) == 2 && kind == 2) return silu_bf16(g) * u;
+    return plain_activation(g, kind) * u;
+}
+
+// The same where rows are whole 16-byte pieces: eight columns a thread, a row's index by blockIdx
+// instead of a division.  [2048, 2 x 2048] in bfloat16: 14.7 us a column a thread, 4.7 us here.
+template <typename A>
+__global__ void __launch_bounds__(256)
+silu_mul_vec_kernel(const A* __restrict__ gate_up, A* __restrict__ out, int inter, int rows, int kind,
+                    float limit, float alpha) {
+    gate_up = pdl_after(gate_up, pdl_wait());
+    const int c = (blockIdx.x * 256 + threadIdx.x) * 8;
+    if (c >= inter) return;
+    for (int row = blockIdx.y; row < rows; row += gridDim.y) {
+        const A* p = gate_up + (size_t)row * 2 * inter + c;
+        float g[8], u[8];
+        load8(p, g);
+        load8(p + inter, u);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) g[i] = gated_product<A>(g[i], u[i], kind, limit, alpha);
+        store8(out + (size_t)row * inter + c, g);
+    }
+}
+
 MSTAR_API int mstar_silu_mul(const void* gate_up, void* out, int act_dtype, int rows, int inter,
                              int kind, float limit, float alpha, void* stream) {
     const size_t total = (size_t)rows * inter;
@@ -412,6 +440,14 @@ MSTAR_API int mstar_silu_mul(const void* gate_up, void* out, int act_dtype, int 
     if (kind < 1 || kind > 3) return -1;
     cudaStream_t s = (cudaStream_t)stream;
     const int threads = 256;
+    if (inter % 8 == 0 && (((uintptr_t)gate_up | (uintptr_t)out) & 15) == 0) {
+        const dim3 grid((inter / 8 + 255) / 256, rows < 65535 ? rows : 65535);
+        if (act_dtype == MSTAR_F32)
+            mstar_launch((silu_mul_vec_kernel<float>), grid, dim3(threads), 0, s, (const float*)gate_up, (float*)out, inter, rows, kind, limit, alpha);
+        else
+            mstar_launch((silu_mul_vec_kernel<bf16>), grid, dim3(threads), 0, s, (const bf16*)gate_up, (bf16*)out, inter, rows, kind, limit, alpha);
+        return launch_status();
+    }
     size_t blocks = (total + threads - 1) / threads;
     const size_t most = (size_t)device_sm_count() * 32;   // a grid-stride loop takes the rest
     if (blocks > most) blocks = most;
@@ -970,6 +1006,28 @@ __global__ void head_gate_mul_kernel(const In* y, Out* out, const G* __restrict_
     }
 }
 
+// The same for bfloat16 results with heads of whole 16-byte pieces: eight features a thread, which
+// share a gate.  [2048, 16 x 512] from float: 60.6 us a feature a thread, 13.2 us here.
+template <typename In, typename G>
+__global__ void __launch_bounds__(256)
+head_gate_mul_vec_kernel(const In* y, bf16* out, const G* __restrict__ gate, int heads, int dim, int ldg,
+                         int rows) {
+    const unsigned long long waited = pdl_wait();
+    y = pdl_after(y, waited);
+    gate = pdl_after(gate, waited);
+    const int cols = heads * dim, c = (blockIdx.x * 256 + threadIdx.x) * 8;
+    if (c >= cols) return;
+    const int h = c / dim;
+    for (int row = blockIdx.y; row < rows; row += gridDim.y) {
+        float v[8];
+        load8(y + (size_t)row * cols + c, v);
+        const float share = 1.f / (1.f + expf(-to_float(gate[(size_t)row * ldg + h])));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] *= share;
+        store8(out + (size_t)row * cols + c, v);
+    }
+}
+
 MSTAR_API int mstar_head_gate_mul(const void* y, int in_dtype, void* out, int out_dtype,
                                   const void* gate, int gate_dtype, int ldg, int rows, int heads,
                                   int dim, void* stream) {
@@ -978,6 +1036,16 @@ MSTAR_API int mstar_head_gate_mul(const void* y, int in_dtype, void* out, int ou
     const size_t total = (size_t)rows * heads * dim;
     const int threads = 256;
     const int blocks = (int)((total + threads - 1) / threads < 4096 ? (total + threads - 1) / threads : 4096);
+    if (out_dtype == MSTAR_BF16 && dim % 8 == 0 && (((uintptr_t)y | (uintptr_t)out) & 15) == 0) {
+        const dim3 grid((heads * dim / 8 + 255) / 256, rows < 65535 ? rows : 65535);
+#define GO(I, G)                                                                                  \
+    mstar_launch((head_gate_mul_vec_kernel<I, G>), grid, dim3(threads), 0, s, (const I*)y,        \
+                 (bf16*)out, (const G*)gate, heads, dim, ldg, rows)
+        if (in_dtype == MSTAR_F32) { if (gate_dtype == MSTAR_F32) { GO(float, float); } else { GO(float, bf16); } }
+        else { if (gate_dtype == MSTAR_F32) { GO(bf16, float); } else { GO(bf16, bf16); } }
+#undef GO
+        return launch_status();
+    }
 #define GO(I, O, G)                                                                               \
     mstar_launch((head_gate_mul_kernel<I, O, G>), dim3(blocks), dim3(threads), 0, s, (const I*)y, \
                  (O*)out, (const G*)gate, heads, dim, ldg, total)

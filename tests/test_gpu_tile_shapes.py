@@ -105,3 +105,28 @@ def test_grouped_experts_at_the_borders_of_their_tiles(tokens, width, ff, expert
             size[rows] += b * (h.abs() @ dd[e].abs().T)      # what the hidden units' rounding can do
         want[rows] += y
     assert ((got - want).abs() <= 2 ** -8 * (size + want.abs()) + 1e-5).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,inter", [(3, 8), (5, 2056), (2, 12)])
+def test_gated_products_by_eight_and_one_by_one(dtype, rows, inter):
+    """Widths of whole 16-byte pieces and others, zeros and large gates among them."""
+    from mstar_b200 import ops
+
+    x = rnd(rows, 2 * inter, dtype=dtype, seed=1, scale=3.0)
+    x[0, :4] = torch.tensor([0.0, -200.0, 200.0, -90.0], dtype=dtype, device=DEV)
+    g, u = x.double().chunk(2, dim=1)
+    clipped = g.clamp(max=2.0)
+    for kind, z, want in (("silu", g, g * torch.sigmoid(g) * u),
+                          ("clamped_swish", 1.75 * clipped, clipped * torch.sigmoid(1.75 * clipped) * (u.clamp(-2, 2) + 1))):
+        got = ops.silu_mul(x, kind=kind, limit=2.0, alpha=1.75).double()
+        # half an ulp of a bfloat16 result; in float the exponent's argument z is rounded (half an
+        # ulp of z, which the exponential makes a relative error), expf, the sum, the quotient and the
+        # product are off by 2 ulp at most each
+        off = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -24 * (z.abs() + 16)
+        assert ((got - want).abs() <= off * want.abs() + 1e-30).all()
+    y = rnd(rows, 2 * inter, dtype=dtype, seed=2)
+    gate = rnd(rows, 2, seed=3)
+    want = (y.double().view(rows, 2, inter) * torch.sigmoid(gate.double())[:, :, None]).view(rows, -1)
+    got = ops.head_gate_mul(y, gate, 2, out_dtype=torch.bfloat16).double()
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-30).all()
