@@ -233,22 +233,30 @@ sample_kernel(const float* __restrict__ logits, int ld, int vocab,
 
 // ------------------------------------------------------------------ cluster variant
 // The same sampling with a thread-block cluster of 8 CTAs per row: each CTA keeps an
-// eighth of the row in shared memory (the penalised logits and their exponentials), so the
-// row is read from global memory once; the thresholds of top-k and top-p are found by radix
-// selection (three rounds of 11, 11 and 10 bits with a histogram per round, summed across
-// the cluster through distributed shared memory) instead of 32 passes of bisection each.
+// eighth of the row in shared memory (the penalised logits), so the row is read from global
+// memory once; the thresholds of top-k and top-p are found by radix selection (three rounds of
+// 11, 11 and 10 bits with a histogram per round, summed across the cluster through distributed
+// shared memory) instead of 32 passes of bisection each.
 // The selection runs on keys that spread the row's range [min, max] linearly over 32 bits
 // (a monotone map of the penalised logits: the bit patterns themselves would put nearly
 // all tokens into the few bins of their common exponents, and the histogram's atomics
 // would serialise); logits closer than range / 2^32 count as tied, and ties with the last
 // kept token are kept, as before.  Probability mass is counted in 64-bit fixed
 // point (exp * 2^40, exact integer sums), so that no sum depends on the order in which it
-// is made: the same (seed, offset) always draws the same token.  With the reference's
-// default options (temperature, top-p and a repetition penalty) a row of 157 k logits takes
-// tens of microseconds instead of three milliseconds.
+// is made: the same (seed, offset) always draws the same token.
+//
+// What a row takes is latencies: passes over a CTA's logits, cluster barriers, histogram atomics.  So
+// two CTAs share an SM (keys and exponentials are made again where they are needed instead of kept:
+// 95 KB a CTA at 157 k logits instead of 189), the first pass over the keys makes the first
+// histogram and the mass as well, histogram entries are two 32-bit words (a 64-bit atomic on shared
+// memory is a loop; the upper word is touched only on a carry or by a large mass), and a histogram is
+// summed over the cluster by all eight CTAs, a slice of the bins each.  157 k logits with temperature,
+// top-p and a repetition penalty: 121 us for 64 rows; with one CTA an SM and
+// the histograms added into rank 0 by remote atomics 61 us for up to 18 and 294 us for 64.
 #define CS_CLUSTER 8
 #define CS_THREADS 512
 #define CS_BINS 2048
+#define CS_SLICE (CS_BINS / CS_CLUSTER)
 #define CS_SCALE 1099511627776.f      // 2^40
 
 namespace cg = cooperative_groups;
@@ -269,7 +277,7 @@ __device__ __forceinline__ unsigned long long cs_block_sum(unsigned long long v,
     return r;
 }
 
-// One value per CTA -> the values of all CTAs of the cluster, in rank order.  `slot`: 8 u64
+// One value per CTA -> the values of all CTAs of the cluster, in rank order.  `slot`: a u64
 // in this CTA's shared memory (the same variable in every CTA).
 __device__ __forceinline__ void cs_gather(cg::cluster_group& cluster, unsigned long long mine,
                                           unsigned long long* slot, unsigned long long (&all)[CS_CLUSTER]) {
@@ -280,77 +288,81 @@ __device__ __forceinline__ void cs_gather(cg::cluster_group& cluster, unsigned l
     cluster.sync();          // nobody overwrites its slot before everybody has read it
 }
 
-// The bin of a radix round.  hist: this CTA's histogram (counts or masses, u64), complete for
-// this CTA's threads only after the barrier inside; ghist: the cluster-wide histogram, kept
-// in rank 0's shared memory and zero between rounds.  Every CTA adds its non-empty bins to it
-// (remote atomics: stores, no round trips); rank 0 walks the bins from the top and finds the
-// bin b where the running sum `above + sum(bins > b)` is still below `need` and `above +
-// sum(bins >= b)` reaches it, and writes (b, above + sum(bins > b)) into every CTA's `result`.
-// Returns b (0 if the need is never reached) and updates `above`.
-__device__ __forceinline__ int cs_pick_bin(cg::cluster_group& cluster, int rank, unsigned long long* hist,
-                                           unsigned long long* ghist, unsigned long long* scratch,
+// hist[0 .. CS_BINS): lower words, hist[CS_BINS ..): upper words of 64-bit sums.
+__device__ __forceinline__ void cs_add(unsigned* hist, unsigned bin, unsigned long long v) {
+    const unsigned lo = (unsigned)v;
+    const unsigned old = atomicAdd(hist + bin, lo);
+    const unsigned hi = (unsigned)(v >> 32) + (old + lo < old ? 1u : 0u);
+    if (hi != 0u) atomicAdd(hist + CS_BINS + bin, hi);
+}
+__device__ __forceinline__ void cs_clear(unsigned* hist) {
+    for (int i = threadIdx.x; i < 2 * CS_BINS; i += CS_THREADS) hist[i] = 0u;
+    __syncthreads();
+}
+
+// The bin of a radix round: with the histograms of all CTAs summed, the bin b where the running sum
+// `above + sum(bins > b)` is still below `need` and `above + sum(bins >= b)` reaches it.  CTA r sums and
+// walks the bins of slice r (from the top; higher slices' totals come before it), and the one that holds
+// b writes (b, above + sum(bins > b)) into every CTA's `result`.  Returns b (0 if the need is never
+// reached) and updates `above`.
+__device__ __forceinline__ int cs_pick_bin(cg::cluster_group& cluster, int rank, unsigned* hist,
+                                           unsigned long long* scratch, unsigned long long* slot,
                                            unsigned long long* result, unsigned long long need,
                                            unsigned long long& above) {
-    constexpr int PER = CS_BINS / CS_THREADS;      // bins per thread: 4
-    const int tid = threadIdx.x;
-    __syncthreads();                                // this CTA's histogram is complete
-    unsigned long long* total = cluster.map_shared_rank(ghist, 0);
-    for (int bin = tid; bin < CS_BINS; bin += CS_THREADS) {
-        const unsigned long long v = hist[bin];
-        if (v != 0ull) atomicAdd(total + bin, v);
-    }
-    cluster.sync();                                 // every CTA's bins have arrived
-    if (rank == 0) {
-        unsigned long long mine[PER];
-        unsigned long long local = 0ull;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    cluster.sync();                                 // every CTA's histogram is complete
+    const int bin = rank * CS_SLICE + tid;
+    unsigned long long mine = 0ull;
+    if (tid < CS_SLICE) {
+        unsigned lo[CS_CLUSTER], hi[CS_CLUSTER];
 #pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            mine[j] = ghist[tid * PER + j];
-            ghist[tid * PER + j] = 0ull;            // ready for the next round
-            local += mine[j];
+        for (int r = 0; r < CS_CLUSTER; ++r) {
+            const unsigned* other = cluster.map_shared_rank(hist, r);
+            lo[r] = other[bin];
+            hi[r] = other[CS_BINS + bin];
         }
-        // suffix sums over the threads' totals: after = sum of the bins of threads > tid
-        const int lane = tid & 31, warp = tid >> 5;
-        unsigned long long incl = local;            // inclusive suffix within the warp
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned long long up = __shfl_down_sync(0xffffffffu, incl, o);
-            if (lane + o < 32) incl += up;
-        }
-        if (lane == 0) scratch[warp] = incl;        // the warp's total
-        __syncthreads();
-        unsigned long long after = incl - local;    // bins of higher lanes of this warp
-        for (int w = warp + 1; w < CS_THREADS / 32; ++w) after += scratch[w];
-        const unsigned long long before = above + after;        // everything in higher bins
-        if (tid == 0) {                             // the answer if nothing reaches the need
-            for (int r = 0; r < CS_CLUSTER; ++r) {
-                unsigned long long* dst = cluster.map_shared_rank(result, r);
-                dst[0] = 0ull;
-                dst[1] = above;
-            }
-        }
-        __syncthreads();
-        if (before < need && before + local >= need) {          // at most one thread
-            unsigned long long run = before;
-            for (int j = PER - 1; j >= 0; --j) {
-                if (run + mine[j] >= need) {
-                    for (int r = 0; r < CS_CLUSTER; ++r) {
-                        unsigned long long* dst = cluster.map_shared_rank(result, r);
-                        dst[0] = (unsigned long long)(tid * PER + j);
-                        dst[1] = run;
-                    }
-                    break;
-                }
-                run += mine[j];
-            }
-        }
+        for (int r = 0; r < CS_CLUSTER; ++r) mine += (unsigned long long)lo[r] + ((unsigned long long)hi[r] << 32);
     }
+    // suffix sums over the slice: after = sum of its bins above this one
+    unsigned long long incl = mine;                 // inclusive suffix within the warp
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long up = __shfl_down_sync(0xffffffffu, incl, o);
+        if (lane + o < 32) incl += up;
+    }
+    if (lane == 0) scratch[warp] = incl;            // the warp's total
+    __syncthreads();
+    unsigned long long after = incl - mine, total = 0ull;
+#pragma unroll
+    for (int w = 0; w < CS_SLICE / 32; ++w) {
+        total += scratch[w];
+        if (w > warp) after += scratch[w];
+    }
+    if (tid == 0) slot[0] = total;
+    cluster.sync();                                 // totals are there, histograms have been read
+    unsigned long long everything = above;
+    after += above;
+#pragma unroll
+    for (int r = 0; r < CS_CLUSTER; ++r) {
+        const unsigned long long t = *cluster.map_shared_rank(slot, r);
+        everything += t;
+        if (r > rank) after += t;
+    }
+    const bool here = tid < CS_SLICE && after < need && after + mine >= need;       // at most one thread
+    const bool nowhere = everything < need && rank == 0 && tid == 0;
+    if (here || nowhere)
+        for (int r = 0; r < CS_CLUSTER; ++r) {
+            unsigned long long* dst = cluster.map_shared_rank(result, r);
+            dst[0] = here ? (unsigned long long)bin : 0ull;
+            dst[1] = here ? after : above;
+        }
     cluster.sync();                                 // the result has been written everywhere
     above = result[1];
     return (int)result[0];
 }
 
-__global__ void __cluster_dims__(CS_CLUSTER, 1, 1) __launch_bounds__(CS_THREADS)
+__global__ void __cluster_dims__(CS_CLUSTER, 1, 1) __launch_bounds__(CS_THREADS, 2)
 sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int chunk,
                       const float* __restrict__ temperature, const int* __restrict__ top_k,
                       const float* __restrict__ top_p, const float* __restrict__ penalty,
@@ -361,11 +373,9 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ __align__(16) unsigned char cs_smem[];
     float* sv = reinterpret_cast<float*>(cs_smem);                  // penalised logits [chunk]
-    float* se = sv + chunk;                                         // exponentials [chunk]
-    unsigned long long* hist = reinterpret_cast<unsigned long long*>(se + chunk);
-    unsigned long long* ghist = hist + CS_BINS;
+    unsigned* hist = reinterpret_cast<unsigned*>(sv + chunk);       // [2][CS_BINS]
     __shared__ unsigned long long scratch[32];
-    __shared__ unsigned long long slot[1];
+    __shared__ unsigned long long slot[2];
     __shared__ unsigned long long result[2];
     __shared__ float best_v[32], low_v[32];
     __shared__ int best_i[32];
@@ -380,17 +390,42 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
     unsigned char* my_seen = srow >= 0 ? seen_mask + (size_t)srow * vocab : nullptr;
     const unsigned char* seen = (my_seen != nullptr && pen != 1.f) ? my_seen : nullptr;
 
-    for (int b = tid; b < CS_BINS; b += CS_THREADS) ghist[b] = 0ull;   // before the first cluster barrier
     // ---- the row, once: penalty, maximum and argmax (smallest index among equal maxima)
     float bv = -INFINITY, lowest = INFINITY;
     int bi = 0x7fffffff;
-    for (int i = tid; i < n; i += CS_THREADS) {
-        float v = x[base + i];
-        if (seen != nullptr && seen[base + i]) v = v > 0.f ? v / pen : v * pen;
+    auto take = [&](int i, float v, bool was_seen) {
+        if (was_seen) v = v > 0.f ? v / pen : v * pen;
         sv[i] = v;
         if (v > bv || (v == bv && base + i < bi)) { bv = v; bi = base + i; }
         if (v > -INFINITY) lowest = fminf(lowest, v);
+    };
+    int done = 0;
+    // (chunks start at multiples of 4)
+    if ((reinterpret_cast<uintptr_t>(x) & 15) == 0 && (seen == nullptr || (reinterpret_cast<uintptr_t>(seen) & 3) == 0)) {
+        constexpr int AHEAD = 4;
+        const int quads = n / 4;
+        for (int q0 = tid; q0 < quads; q0 += AHEAD * CS_THREADS) {
+            float4 v[AHEAD];
+            unsigned s4[AHEAD];
+#pragma unroll
+            for (int k = 0; k < AHEAD; ++k) {
+                const int q = min(q0 + k * CS_THREADS, quads - 1);
+                v[k] = *reinterpret_cast<const float4*>(x + base + 4 * q);
+                s4[k] = seen != nullptr ? *reinterpret_cast<const unsigned*>(seen + base + 4 * q) : 0u;
+            }
+#pragma unroll
+            for (int k = 0; k < AHEAD; ++k) {
+                const int i = 4 * (q0 + k * CS_THREADS);
+                if (i >= 4 * quads) continue;
+                take(i, v[k].x, (s4[k] & 0xffu) != 0u);
+                take(i + 1, v[k].y, (s4[k] & 0xff00u) != 0u);
+                take(i + 2, v[k].z, (s4[k] & 0xff0000u) != 0u);
+                take(i + 3, v[k].w, (s4[k] & 0xff000000u) != 0u);
+            }
+        }
+        done = 4 * quads;
     }
+    for (int i = done + tid; i < n; i += CS_THREADS) take(i, x[base + i], seen != nullptr && seen[base + i]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
@@ -399,7 +434,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
         lowest = fminf(lowest, __shfl_xor_sync(0xffffffffu, lowest, o));
     }
     if (lane == 0) { best_v[warp] = bv; best_i[warp] = bi; low_v[warp] = lowest; }
-    __syncthreads();
+    cs_clear(hist);                                 // (its barrier also ends the writes above)
     if (warp == 0) {
         bv = lane < CS_THREADS / 32 ? best_v[lane] : -INFINITY;
         bi = lane < CS_THREADS / 32 ? best_i[lane] : 0x7fffffff;
@@ -411,19 +446,26 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
             if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
             lowest = fminf(lowest, __shfl_xor_sync(0xffffffffu, lowest, o));
         }
-        if (lane == 0) low_v[0] = lowest;
+        // (value, index) packed: the ordered bits of the value above, the index below (inverted,
+        // so that the larger word is the larger value or, among equals, the smaller index); and the
+        // row's minimum, its ordered bits inverted: the largest word is the smallest value
+        if (lane == 0) {
+            slot[0] = ((unsigned long long)ordered_bits(bv) << 32) | (unsigned)(0x7fffffff - bi);
+            slot[1] = (unsigned long long)(~ordered_bits(lowest));
+        }
     }
-    __syncthreads();
-    lowest = low_v[0];
-    unsigned long long all[CS_CLUSTER];
-    // (value, index) packed: the ordered bits of the value above, the index below (inverted,
-    // so that the larger word is the larger value or, among equals, the smaller index)
-    cs_gather(cluster, ((unsigned long long)ordered_bits(bv) << 32) | (unsigned)(0x7fffffff - bi), slot, all);
-    unsigned long long top = 0ull;
+    cluster.sync();
+    unsigned long long top = 0ull, low_word = 0ull;
 #pragma unroll
-    for (int r = 0; r < CS_CLUSTER; ++r) top = all[r] > top ? all[r] : top;
+    for (int r = 0; r < CS_CLUSTER; ++r) {
+        const unsigned long long* other = cluster.map_shared_rank(slot, r);
+        top = other[0] > top ? other[0] : top;
+        low_word = other[1] > low_word ? other[1] : low_word;
+    }
+    cluster.sync();                                 // nobody overwrites its slot before everybody has read it
     const float vmax = from_ordered_bits((unsigned)(top >> 32));
     const int amax = 0x7fffffff - (int)(unsigned)(top & 0xffffffffu);
+    const float vmin = fminf(from_ordered_bits(~(unsigned)low_word), vmax);
 
     const float temp = temperature[row];
     if (temp <= 0.f) {                      // uniform over the cluster; all reads are done
@@ -434,51 +476,51 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
         return;
     }
     const float inv_temp = 1.f / temp;
-    // the row's minimum over the cluster (ordered bits inverted: the largest word is the smallest value)
-    cs_gather(cluster, (unsigned long long)(~ordered_bits(lowest)), slot, all);
-    unsigned long long low_word = 0ull;
-#pragma unroll
-    for (int r = 0; r < CS_CLUSTER; ++r) low_word = all[r] > low_word ? all[r] : low_word;
-    const float vmin = fminf(from_ordered_bits(~(unsigned)low_word), vmax);
-    // exponentials, and the selection keys in place of the logits
+    // a logit's selection key and its mass, made from it wherever they are needed
     const double spread = vmax > vmin ? 4294967295.0 / ((double)vmax - (double)vmin) : 0.0;
-    unsigned* sq = reinterpret_cast<unsigned*>(sv);
-    for (int i = tid; i < n; i += CS_THREADS) {
-        const float v = sv[i];
-        se[i] = expf((v - vmax) * inv_temp);
+    auto key_of = [&](float v) {
         const double q = v > vmin ? ((double)v - (double)vmin) * spread : 0.0;
-        sq[i] = q >= 4294967295.0 ? 0xffffffffu : (unsigned)q;
-    }
-    __syncthreads();
+        return q >= 4294967295.0 ? 0xffffffffu : (unsigned)q;
+    };
+    auto mass_of = [&](float v) { return cs_fixed(expf((v - vmax) * inv_temp)); };
+    const float p = top_p != nullptr ? top_p[row] : 1.f;
+    const int k = top_k != nullptr ? top_k[row] : 0;
+    const bool choose_k = k > 0 && k < vocab;
+    bool first_made = false;                // the first histogram of top-p is there
 
     // ---- top-k: tau = the k-th largest key, by radix selection on counts
     unsigned tau = 0u;
-    const int k = top_k != nullptr ? top_k[row] : 0;
-    if (k > 0 && k < vocab) {
+    unsigned long long mass = 0ull;         // of the kept tokens
+    if (choose_k) {
         unsigned prefix = 0u;
         unsigned long long above = 0ull;
         int decided = 0;
         for (int round = 0; round < 3; ++round) {
             const int bits = round < 2 ? 11 : 10;
             const int shift = 32 - decided - bits;
-            for (int b = tid; b < CS_BINS; b += CS_THREADS) hist[b] = 0ull;
-            __syncthreads();
+            if (round > 0) cs_clear(hist);
             for (int i = tid; i < n; i += CS_THREADS) {
-                const unsigned key = sq[i];
+                const unsigned key = key_of(sv[i]);
                 if (decided == 0 || (key >> (32 - decided)) == prefix)
-                    atomicAdd(&hist[(key >> shift) & ((1u << bits) - 1u)], 1ull);
+                    cs_add(hist, (key >> shift) & ((1u << bits) - 1u), 1ull);
             }
-            const int bin = cs_pick_bin(cluster, rank, hist, ghist, scratch, result, (unsigned long long)k, above);
+            const int bin = cs_pick_bin(cluster, rank, hist, scratch, slot, result, (unsigned long long)k, above);
             prefix = (prefix << bits) | (unsigned)bin;
             decided += bits;
         }
         tau = prefix;
+        for (int i = tid; i < n; i += CS_THREADS)
+            if (key_of(sv[i]) >= tau) mass += mass_of(sv[i]);
+    } else {
+        first_made = p < 1.f;
+#pragma unroll 2
+        for (int i = tid; i < n; i += CS_THREADS) {
+            const unsigned long long m = mass_of(sv[i]);
+            mass += m;
+            if (first_made) cs_add(hist, key_of(sv[i]) >> 21, m);
+        }
     }
-
-    // ---- mass of the kept tokens
-    unsigned long long mass = 0ull;
-    for (int i = tid; i < n; i += CS_THREADS)
-        if (sq[i] >= tau) mass += cs_fixed(se[i]);
+    unsigned long long all[CS_CLUSTER];
     mass = cs_block_sum(mass, scratch);
     cs_gather(cluster, mass, slot, all);
     unsigned long long total = 0ull;
@@ -486,7 +528,6 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
     for (int r = 0; r < CS_CLUSTER; ++r) total += all[r];
 
     // ---- top-p: the largest tau2 >= tau whose tokens (x >= tau2) hold p of that mass
-    const float p = top_p != nullptr ? top_p[row] : 1.f;
     if (p < 1.f) {
         const unsigned long long need = (unsigned long long)((double)p * (double)total);
         unsigned prefix = 0u;
@@ -495,22 +536,25 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
         for (int round = 0; round < 3; ++round) {
             const int bits = round < 2 ? 11 : 10;
             const int shift = 32 - decided - bits;
-            for (int b = tid; b < CS_BINS; b += CS_THREADS) hist[b] = 0ull;
-            __syncthreads();
-            for (int i = tid; i < n; i += CS_THREADS) {
-                const unsigned key = sq[i];
-                if (key >= tau && (decided == 0 || (key >> (32 - decided)) == prefix))
-                    atomicAdd(&hist[(key >> shift) & ((1u << bits) - 1u)], cs_fixed(se[i]));
+            if (round > 0 || !first_made) {
+                cs_clear(hist);
+#pragma unroll 2
+                for (int i = tid; i < n; i += CS_THREADS) {
+                    const unsigned key = key_of(sv[i]);
+                    if (key >= tau && (decided == 0 || (key >> (32 - decided)) == prefix))
+                        cs_add(hist, (key >> shift) & ((1u << bits) - 1u), mass_of(sv[i]));
+                }
             }
-            const int bin = cs_pick_bin(cluster, rank, hist, ghist, scratch, result, need > 0ull ? need : 1ull, above);
+            const int bin = cs_pick_bin(cluster, rank, hist, scratch, slot, result, need > 0ull ? need : 1ull, above);
             prefix = (prefix << bits) | (unsigned)bin;
             decided += bits;
         }
         if (prefix > tau) {
             tau = prefix;
             mass = 0ull;
+#pragma unroll 2
             for (int i = tid; i < n; i += CS_THREADS)
-                if (sq[i] >= tau) mass += cs_fixed(se[i]);
+                if (key_of(sv[i]) >= tau) mass += mass_of(sv[i]);
             mass = cs_block_sum(mass, scratch);
             cs_gather(cluster, mass, slot, all);
             total = 0ull;
@@ -537,7 +581,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
         const int begin = min(tid * per, n), end = min(begin + per, n);
         unsigned long long mine = 0ull;
         for (int i = begin; i < end; ++i)
-            if (sq[i] >= tau) mine += cs_fixed(se[i]);
+            if (key_of(sv[i]) >= tau) mine += mass_of(sv[i]);
         // exclusive prefix of `mine` over the threads
         unsigned long long incl = mine;
 #pragma unroll
@@ -554,8 +598,8 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
             unsigned long long run = excl;
             int pick = amax;
             for (int i = begin; i < end; ++i) {
-                if (sq[i] >= tau) {
-                    run += cs_fixed(se[i]);
+                if (key_of(sv[i]) >= tau) {
+                    run += mass_of(sv[i]);
                     if (target < run) { pick = base + i; break; }
                 }
             }
@@ -567,7 +611,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
 
 static int cs_chunk(int vocab) { return ((vocab + CS_CLUSTER - 1) / CS_CLUSTER + 3) & ~3; }
 static size_t cs_smem_bytes(int vocab) {
-    return (size_t)cs_chunk(vocab) * 8 + 2 * CS_BINS * sizeof(unsigned long long);
+    return (size_t)cs_chunk(vocab) * sizeof(float) + 2 * CS_BINS * sizeof(unsigned);
 }
 
 MSTAR_API int mstar_sample(const float* logits, int ld, int rows, int vocab,
@@ -576,14 +620,14 @@ MSTAR_API int mstar_sample(const float* logits, int ld, int rows, int vocab,
                            const long long* seed, const long long* offset, int* out,
                            void* stream) {
     if (rows <= 0) return 0;
-    // rows of up to ~200 k logits fit the shared memory of a cluster of 8 CTAs
+    // rows of up to 172,032 logits (two CTAs of a cluster to an SM, half of its shared memory each)
     static int one_block = -1;          // MSTAR_SAMPLER=block: the one-block-per-row kernel
     if (one_block < 0) {
         const char* e = getenv("MSTAR_SAMPLER");
         one_block = (e != nullptr && strcmp(e, "block") == 0) ? 1 : 0;
     }
     const size_t smem = cs_smem_bytes(vocab);
-    if (!one_block && smem <= 200 * 1024 && rows <= 65535 / CS_CLUSTER * CS_CLUSTER) {
+    if (!one_block && cs_chunk(vocab) <= 21504 && rows <= 65535 / CS_CLUSTER * CS_CLUSTER) {
         static size_t configured = 0;
         if (smem > configured) {
             cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel,
