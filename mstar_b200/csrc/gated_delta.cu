@@ -526,358 +526,7 @@ MSTAR_API int mstar_delta_scan(const float* q, const float* k, const float* v, c
     return launch_status();
 }
 
-// ------------------------------------------------------------------ scan in pieces of 16 tokens
-// Within a piece of C tokens that starts from the state S0, with P_t the product of the decays
-// from the piece's first token up to t (per key channel):
-//   r_t = (P_t k_t) . S0 + sum_{j<t} A_tj u_j,        A_tj = sum_d k_t[d] k_j[d] prod_{i=j+1..t} g_i[d]
-//   u_t = beta_t (v_t - r_t)
-//   o_t = (P_t q_t) . S0 + sum_{j<=t} B_tj u_j,       B_tj = sum_d q_t[d] k_j[d] prod_{i=j+1..t} g_i[d]
-//   S_C = P_C S0 + sum_j (k_j prod_{i>j} g_i) u_j
-// A, B and the decayed rows do not depend on the state or on the value column: a first kernel
-// makes them for all pieces side by side (products of decays only, never a quotient).  The scan
-// then walks a piece with one dot product per token against S0 (a lane a token), a chain of C
-// scalar steps for u, and one pass over the rows for the new state.  All float.
-#define GC_TOKENS 16
-#define GC_MAX_ROWS 8        // rows of a column a lane keeps: D <= 256
-
-struct DeltaPieceArgs {
-    const float* q;
-    const float* k;
-    const float* decay;
-    const int* qo_indptr;
-    float* kt;                  // [H][tokens][D]  k_t P_t  (a piece's rows of a head lie together)
-    float* qt;                  // [H][tokens][D]  q_t P_t
-    float* kh;                  // [H][tokens][D]  k_t prod_{i>t} g_i
-    float* pc;                  // [entries][pieces][H][D]  P at the piece's last token
-    float* A;                   // [H][tokens][C]
-    float* B;                   // [H][tokens][C]
-    int H, G, D, max_pieces, tokens;
-};
-
-__global__ void __launch_bounds__(128) delta_pieces_kernel(DeltaPieceArgs a) {
-    extern __shared__ __align__(16) float sm[];          // k, q, g of the piece: [3][C][D]
-    const int piece = blockIdx.x, e = blockIdx.y, h = blockIdx.z;
-    const int D = a.D, g_head = h / (a.H / a.G);
-    const unsigned long long waited = pdl_wait();
-    const float* q = pdl_after(a.q, waited);
-    const float* k = pdl_after(a.k, waited);
-    const float* decay = pdl_after(a.decay, waited);
-    const int start = a.qo_indptr[e], n = a.qo_indptr[e + 1] - start;
-    const int base = piece * GC_TOKENS;
-    if (base >= n) return;
-    const int here = min(GC_TOKENS, n - base);
-    float* ks = sm;
-    float* qs = ks + GC_TOKENS * D;
-    float* gs = qs + GC_TOKENS * D;
-    const int qk = a.G * D, hd = a.H * D;
-    for (int i = threadIdx.x; i < here * D; i += blockDim.x) {
-        const int t = i / D, d = i - t * D;
-        const size_t tok = (size_t)(start + base + t);
-        ks[i] = k[tok * qk + (size_t)g_head * D + d];
-        qs[i] = q[tok * qk + (size_t)g_head * D + d];
-        gs[i] = decay[tok * hd + (size_t)h * D + d];
-    }
-    __syncthreads();
-    for (int d = threadIdx.x; d < D; d += blockDim.x) {
-        float P = 1.f;
-        for (int t = 0; t < here; ++t) {
-            P *= gs[t * D + d];
-            const size_t o = ((size_t)h * a.tokens + start + base + t) * D + d;
-            a.kt[o] = ks[t * D + d] * P;
-            a.qt[o] = qs[t * D + d] * P;
-        }
-        a.pc[(((size_t)e * a.max_pieces + piece) * a.H + h) * D + d] = P;
-        float S = 1.f;
-        for (int t = here - 1; t >= 0; --t) {
-            a.kh[((size_t)h * a.tokens + start + base + t) * D + d] = ks[t * D + d] * S;
-            S *= gs[t * D + d];
-        }
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    for (int j = warp; j < here; j += nwarps) {
-        float w[GC_MAX_ROWS];
-        float b = 0.f;
-#pragma unroll
-        for (int i = 0; i < GC_MAX_ROWS; ++i) {
-            const int d = lane + 32 * i;
-            w[i] = d < D ? ks[j * D + d] : 0.f;
-            if (d < D) b = fmaf(qs[j * D + d], w[i], b);
-        }
-        b = warp_sum(b);
-        if (lane == 0) a.B[((size_t)h * a.tokens + start + base + j) * GC_TOKENS + j] = b;
-        for (int t = j + 1; t < here; ++t) {
-            float av = 0.f, bv = 0.f;
-#pragma unroll
-            for (int i = 0; i < GC_MAX_ROWS; ++i) {
-                const int d = lane + 32 * i;
-                if (d < D) {
-                    w[i] *= gs[t * D + d];
-                    av = fmaf(ks[t * D + d], w[i], av);
-                    bv = fmaf(qs[t * D + d], w[i], bv);
-                }
-            }
-            av = warp_sum(av);
-            bv = warp_sum(bv);
-            if (lane == 0) {
-                const size_t o = ((size_t)h * a.tokens + start + base + t) * GC_TOKENS + j;
-                a.A[o] = av;
-                a.B[o] = bv;
-            }
-        }
-    }
-}
-
-struct DeltaChunkArgs {
-    const float* kt;
-    const float* qt;
-    const float* kh;
-    const float* pc;
-    const float* A;
-    const float* B;
-    const float* v;
-    const float* beta;
-    const int* qo_indptr;
-    const int* slots;
-    float* state;
-    long long state_stride;
-    long long state_offset;
-    float* out;
-    int H, VD, max_pieces, tokens;
-    ConvAdvance conv;
-};
-
-#define GC_THREADS 256
-#define GC_COLS (GC_THREADS / 32)
-
-// R consecutive floats as one access.
-template <int R> struct GcVec;
-template <> struct GcVec<1> { typedef float T; };
-template <> struct GcVec<2> { typedef float2 T; };
-template <> struct GcVec<4> { typedef float4 T; };
-template <int R> __device__ __forceinline__ void gc_load(const float* p, float (&v)[R]) {
-    if constexpr (R == 8) {
-        const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
-        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-    } else if constexpr (R == 4) {
-        const float4 a = *reinterpret_cast<const float4*>(p);
-        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-    } else if constexpr (R == 2) {
-        const float2 a = *reinterpret_cast<const float2*>(p);
-        v[0] = a.x; v[1] = a.y;
-    } else {
-        v[0] = p[0];
-    }
-}
-template <int R> __device__ __forceinline__ void gc_store(float* p, const float (&v)[R]) {
-    if constexpr (R == 8) {
-        reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
-        reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
-    } else if constexpr (R == 4) {
-        *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-    } else if constexpr (R == 2) {
-        *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
-    } else {
-        p[0] = v[0];
-    }
-}
-
-// A warp owns a value column of one head of one entry; its D = 32 R rows lie on the 32 lanes,
-// R consecutive rows a lane.  Per piece: the column goes to shared memory so that lane
-// (t, half) can take token t's two dot products over one half of the rows, four rows an
-// access (each lane starts its walk at another place, so that the lanes read different
-// banks); the scalar chain u_0 .. u_15 goes round by shuffles with every lane's row of A and B
-// in registers; then the new column, R rows an access.
-template <int R>
-__global__ void __launch_bounds__(GC_THREADS) delta_scan_pieces_kernel(DeltaChunkArgs a) {
-    extern __shared__ __align__(16) float sm[];
-    constexpr int C = GC_TOKENS, D = 32 * R, CP = C + 1;
-    constexpr int per_buf = 3 * C * D + 2 * C * CP + C * GC_COLS + C + D;
-    static_assert(per_buf % 4 == 0, "the second buffer starts on a 16-byte boundary");
-    float* col_sm = sm + 2 * per_buf;                    // [GC_COLS][D] the columns at a piece's start
-    const int e = blockIdx.x, h = blockIdx.y;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int col0 = blockIdx.z * GC_COLS, col = col0 + warp;
-    const bool live = col < a.VD;
-    const int ncols = min(GC_COLS, a.VD - col0);
-    const unsigned long long waited = pdl_wait();
-    const float* kt = pdl_after(a.kt, waited);
-    const float* qt = pdl_after(a.qt, waited);
-    const float* kh = pdl_after(a.kh, waited);
-    const float* pc = pdl_after(a.pc, waited);
-    const float* A = pdl_after(a.A, waited);
-    const float* B = pdl_after(a.B, waited);
-    const float* v = pdl_after(a.v, waited);
-    const float* beta = pdl_after(a.beta, waited);
-    float* state = pdl_after(a.state, waited);
-    const int start = a.qo_indptr[e], n = a.qo_indptr[e + 1] - start;
-    if (n <= 0) return;
-    const int vv = a.H * a.VD;
-
-    auto fetch = [&](int buf, int piece) {
-        const int base = piece * C;
-        const int here = min(C, n - base);
-        float* dst = sm + buf * per_buf;
-        const size_t first = (size_t)h * a.tokens + start + base;      // the piece's first row
-        // the decayed rows of the piece's tokens lie together: one run of here * D floats each
-        for (int i = threadIdx.x * 4; i < here * D; i += GC_THREADS * 4) {
-            gd_copy16(dst + i, kt + first * D + i);
-            gd_copy16(dst + C * D + i, qt + first * D + i);
-            gd_copy16(dst + 2 * C * D + i, kh + first * D + i);
-        }
-        for (int i = threadIdx.x; i < here * C; i += GC_THREADS) {
-            const int t = i >> 4, j = i & 15;
-            gd_copy4(dst + 3 * C * D + t * CP + j, A + first * C + i);
-            gd_copy4(dst + 3 * C * D + C * CP + t * CP + j, B + first * C + i);
-        }
-        float* to = dst + 3 * C * D + 2 * C * CP;
-        for (int i = threadIdx.x; i < here * (ncols + 1); i += GC_THREADS) {
-            const int t = i / (ncols + 1), c = i - t * (ncols + 1);
-            const size_t tok = (size_t)(start + base + t);
-            if (c < ncols) gd_copy4(to + t * GC_COLS + c, v + tok * vv + (size_t)h * a.VD + col0 + c);
-            else gd_copy4(to + C * GC_COLS + t, beta + tok * a.H + h);
-        }
-        const float* pcs = pc + (((size_t)e * a.max_pieces + piece) * a.H + h) * D;
-        for (int d = threadIdx.x * 4; d < D; d += GC_THREADS * 4)
-            gd_copy16(to + C * GC_COLS + C + d, pcs + d);
-    };
-
-    const int pieces = (n + C - 1) / C;
-    fetch(0, 0);
-    cp_async_commit();
-    float* s_col = state + (size_t)a.slots[e] * a.state_stride + a.state_offset +
-                   ((size_t)h * a.VD + (live ? col : 0)) * D;
-    float s[R];
-    gc_load<R>(s_col + lane * R, s);
-    float* mycol = col_sm + warp * D;
-    const int t = lane & 15, half = lane >> 4;
-    constexpr int UNITS = D / 8;                         // 16-byte pieces of half a column
-    for (int piece = 0; piece < pieces; ++piece) {
-        const int buf = piece & 1;
-        if (piece + 1 < pieces) fetch(buf ^ 1, piece + 1);
-        cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        const int here = min(C, n - piece * C);
-        const float* bufp = sm + buf * per_buf;
-        const float* kts = bufp;
-        const float* qts = kts + C * D;
-        const float* khs = qts + C * D;
-        const float* As = khs + C * D;
-        const float* Bs = As + C * CP;
-        const float* vs = Bs + C * CP;
-        const float* betas = vs + C * GC_COLS;
-        const float* pcs = betas + C;
-        gc_store<R>(mycol + lane * R, s);                // the column as every lane needs it
-        __syncwarp();
-        float arow[C], brow[C];
-#pragma unroll
-        for (int j = 0; j < C; ++j) {
-            arow[j] = As[t * CP + j];
-            brow[j] = Bs[t * CP + j];
-        }
-        float r0 = 0.f, p0 = 0.f, r1 = 0.f, p1 = 0.f;
-        {
-            const float4* kr = reinterpret_cast<const float4*>(kts + t * D) + half * UNITS;
-            const float4* qr = reinterpret_cast<const float4*>(qts + t * D) + half * UNITS;
-            const float4* sr = reinterpret_cast<const float4*>(mycol) + half * UNITS;
-#pragma unroll
-            for (int i = 0; i < UNITS; ++i) {
-                const int unit = (lane + i) & (UNITS - 1);
-                const float4 k4 = kr[unit], q4 = qr[unit], s4 = sr[unit];
-                r0 = fmaf(k4.x, s4.x, r0); r1 = fmaf(k4.y, s4.y, r1);
-                r0 = fmaf(k4.z, s4.z, r0); r1 = fmaf(k4.w, s4.w, r1);
-                p0 = fmaf(q4.x, s4.x, p0); p1 = fmaf(q4.y, s4.y, p1);
-                p0 = fmaf(q4.z, s4.z, p0); p1 = fmaf(q4.w, s4.w, p1);
-            }
-        }
-        r0 += r1;
-        p0 += p1;
-        r0 += __shfl_xor_sync(0xffffffffu, r0, 16);
-        p0 += __shfl_xor_sync(0xffffffffu, p0, 16);
-        float c = vs[t * GC_COLS + warp] - r0;           // v_t - r_t as far as it is known
-        float o = p0;
-        float u[C];
-#pragma unroll
-        for (int j = 0; j < C; ++j) {
-            // lane j's c is complete here: every earlier u has been taken off it
-            const float uj = betas[j] * __shfl_sync(0xffffffffu, c, j);
-            u[j] = j < here ? uj : 0.f;
-            if (t > j) c = fmaf(-arow[j], u[j], c);
-            if (t >= j) o = fmaf(brow[j], u[j], o);
-        }
-        if (live && half == 0 && t < here)
-            a.out[(size_t)(start + piece * C + t) * vv + (size_t)h * a.VD + col] = o;
-        float pcv[R];
-        gc_load<R>(pcs + lane * R, pcv);
-#pragma unroll
-        for (int i = 0; i < R; ++i) s[i] *= pcv[i];
-#pragma unroll
-        for (int j = 0; j < C; ++j)
-            if (j < here) {                              // (rows past the piece are not staged)
-                float kv[R];
-                gc_load<R>(khs + j * D + lane * R, kv);
-#pragma unroll
-                for (int i = 0; i < R; ++i) s[i] = fmaf(kv[i], u[j], s[i]);
-            }
-        __syncthreads();                       // the buffer is free for the piece after next
-    }
-    cp_async_wait<0>();
-    if (live) gc_store<R>(s_col + lane * R, s);
-    gd_advance_conv(a.conv, waited, state + (size_t)a.slots[e] * a.state_stride, start, n, h, a.H);
-}
-
-// The scan in pieces, for key sizes of 32, 64, 128 or 256 (whole accesses a lane): `work` holds
-// 3 * tokens * H * D + entries * max_pieces * H * D + 2 * tokens * H * 16 floats.  Returns 0, a CUDA
-// error code, or -1 when the shape is refused.
-MSTAR_API int mstar_delta_scan_pieces(const float* q, const float* k, const float* v,
-                                      const float* beta, const float* decay, const int* qo_indptr,
-                                      const int* slots, float* state, long long state_stride,
-                                      long long state_offset, float* out, float* work, int tokens,
-                                      int entries, int max_q_len, int H, int G, int D, int VD,
-                                      const float* conv_raw, int conv_ld, int channels, int taps,
-                                      void* stream) {
-    if (entries <= 0 || tokens <= 0) return 0;
-    if (H <= 0 || G <= 0 || H % G || VD <= 0) return -1;
-    if (D != 32 && D != 64 && D != 128 && D != 256) return -1;
-    if (H > 65535 || entries > 65535 || (state_offset % 4) != 0 || (state_stride % 4) != 0) return -1;
-    const int max_pieces = (max_q_len + GC_TOKENS - 1) / GC_TOKENS;
-    const size_t thd = (size_t)tokens * H * D;
-    DeltaPieceArgs p{q, k, decay, qo_indptr, work, work + thd, work + 2 * thd, work + 3 * thd,
-                     nullptr, nullptr, H, G, D, max_pieces, tokens};
-    p.A = p.pc + (size_t)entries * max_pieces * H * D;
-    p.B = p.A + (size_t)tokens * H * GC_TOKENS;
-    cudaStream_t s = (cudaStream_t)stream;
-    const size_t smem1 = (size_t)3 * GC_TOKENS * D * sizeof(float);
-    mstar_launch(delta_pieces_kernel, dim3(max_pieces, entries, H), dim3(128), smem1, s, p);
-    int code = launch_status();
-    if (code != 0) return code;
-    DeltaChunkArgs c{p.kt, p.qt, p.kh, p.pc, p.A, p.B, v, beta, qo_indptr, slots, state,
-                     state_stride, state_offset, out, H, VD, max_pieces, tokens,
-                     {taps > 1 ? conv_raw : nullptr, conv_ld, channels, taps}};
-    const int per_buf = 3 * GC_TOKENS * D + 2 * GC_TOKENS * (GC_TOKENS + 1) + GC_TOKENS * GC_COLS +
-                        GC_TOKENS + D;
-    const size_t smem2 = ((size_t)2 * per_buf + (size_t)GC_COLS * D) * sizeof(float);
-    dim3 grid(entries, H, (VD + GC_COLS - 1) / GC_COLS);
-    if (grid.z > 65535) return -1;
-#define GO(RR)                                                                                    \
-    do {                                                                                          \
-        static size_t configured = 0;                                                             \
-        if (smem2 > 48 * 1024 && smem2 > configured) {                                            \
-            cudaFuncSetAttribute(delta_scan_pieces_kernel<RR>,                                    \
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);        \
-            configured = smem2;                                                                   \
-        }                                                                                         \
-        mstar_launch((delta_scan_pieces_kernel<RR>), grid, dim3(GC_THREADS), smem2, s, c);        \
-    } while (0)
-    if (D == 32) GO(1);
-    else if (D == 64) GO(2);
-    else if (D == 128) GO(4);
-    else GO(8);
-#undef GO
-    return launch_status();
-}
-
-// ------------------------------------------------------------------ one decay a head, in pieces
+// ------------------------------------------------------------------ scans in pieces of 16 tokens
 // With one decay g_t a head the decayed rows are the rows times a number, and everything inside a
 // piece of C tokens that does not depend on the state is a C x C matrix.  With P_t = g_1 .. g_t
 // (from the piece's first token), dec(t, j) = g_{j+1} .. g_t, the state S0 at the piece's start and
@@ -890,6 +539,12 @@ MSTAR_API int mstar_delta_scan_pieces(const float* q, const float* k, const floa
 // the heads of a group) and lays them, and the piece's k and q rows, down as the scan wants them in
 // its shared memory, so that a piece is two bulk copies.  The scan has no chain from token to token
 // inside a piece.  All float.
+//
+// With a decay per key channel, P_t, dec(t, j) and P_C are vectors over the key channels: the products
+// k_t . k_j become sums of k_t k_j dec(t, j), and the piece's rows are decayed rows, P_t k_t, P_t q_t,
+// dec(C, t) k_t and P_C (CHANNEL below; a first kernel of its own makes them, a block a head); the rest
+// is the same, with P and dec of the matrices' rows at 1.
+#define GC_TOKENS 16
 #define GH_THREADS 128
 #define GH_WAIT_CODE 18             // what the error word gets when a wait for a piece ran out
 #define GH_LD (GC_TOKENS + 4)       // floats between the rows of a C x C matrix in shared memory
@@ -900,10 +555,12 @@ struct DeltaHeadArgs {
     const float* k;
     const float* v;
     const float* beta;
-    const float* decay;         // [tokens][H]
+    const float* decay;         // [tokens][H], CHANNEL: [tokens][H][D]
     const int* qo_indptr;
     const int* slots;
-    float* rows;                // [pieces][G][2 C][D + 4]: the k rows, then the q rows; zeros past the end
+    // [pieces][G][2 C][D + 4]: the k rows, then the q rows; zeros past the end.  CHANNEL: [pieces][H][
+    // 3 C + 1][D + 4]: P_t k_t, P_t q_t, dec(C, t) k_t and P_C
+    float* rows;
     float* mats;                // [pieces][H][C][GH_MROW]
     float* state;
     long long state_stride;
@@ -916,6 +573,40 @@ struct DeltaHeadArgs {
 
 // Pieces are numbered over the batch so that an entry's are consecutive: at most tokens / C + entries.
 __device__ __forceinline__ size_t gh_first_piece(int start, int e) { return (size_t)(start / GC_TOKENS + e); }
+
+// Column j of T and of B T by forward substitution with L and B in shared memory (rows of GH_LD floats);
+// bj: the write strength of token j, m: the piece's matrices.
+__device__ __forceinline__ void gh_solve(const float* L, const float* B, int j, float bj, float* m) {
+    constexpr int C = GC_TOKENS;
+    float col[C];                                 // column j of (I + L)^-1, zero above j
+#pragma unroll
+    for (int t = 0; t < C; ++t) {
+        float s = t == j ? 1.f : 0.f;
+#pragma unroll
+        for (int x = 0; x < t; x += 4) {
+            float l[4];
+            load4(L + t * GH_LD + x, l);
+#pragma unroll
+            for (int w = 0; w < 4; ++w)
+                if (x + w < t) s = fmaf(-l[w], col[x + w], s);
+        }
+        col[t] = s;
+    }
+#pragma unroll
+    for (int t = 0; t < C; ++t) {
+        float s = 0.f;
+#pragma unroll
+        for (int x = 0; x <= t; x += 4) {
+            float bt[4];
+            load4(B + t * GH_LD + x, bt);
+#pragma unroll
+            for (int w = 0; w < 4; ++w)
+                if (x + w <= t) s = fmaf(bt[w], col[x + w], s);
+        }
+        m[t * GH_MROW + j] = col[t] * bj;
+        m[t * GH_MROW + C + j] = s * bj;
+    }
+}
 
 // A block per (piece, entry, group of heads); thread (t, j) of 256 makes k_t . k_j and q_t . k_j,
 // then a warp a head: lane j the column j of T and of B T by forward substitution.
@@ -1000,37 +691,147 @@ __global__ void __launch_bounds__(256) delta_head_pieces_kernel(DeltaHeadArgs a)
             float* m = a.mats + ((gh_first_piece(start, e) + piece) * a.H + h) * C * GH_MROW;
             m[j * GH_MROW + 2 * C] = P;
             m[j * GH_MROW + 2 * C + 1] = dec;            // dec(C, j): a short piece's g are 1 past its end
-            float col[C];                                 // column j of (I + L)^-1, zero above j
-#pragma unroll
-            for (int t = 0; t < C; ++t) {
-                float s = t == j ? 1.f : 0.f;
-#pragma unroll
-                for (int x = 0; x < t; x += 4) {
-                    float l[4];
-                    load4(L + t * GH_LD + x, l);
-#pragma unroll
-                    for (int w = 0; w < 4; ++w)
-                        if (x + w < t) s = fmaf(-l[w], col[x + w], s);
-                }
-                col[t] = s;
-            }
-            const float bj = bs[j];
-#pragma unroll
-            for (int t = 0; t < C; ++t) {
-                float s = 0.f;
-#pragma unroll
-                for (int x = 0; x <= t; x += 4) {
-                    float bt[4];
-                    load4(B + t * GH_LD + x, bt);
-#pragma unroll
-                    for (int w = 0; w < 4; ++w)
-                        if (x + w <= t) s = fmaf(bt[w], col[x + w], s);
-                }
-                m[t * GH_MROW + j] = col[t] * bj;
-                m[t * GH_MROW + C + j] = s * bj;
-            }
+            gh_solve(L, B, j, bs[j], m);
         }
         __syncwarp();
+    }
+}
+
+// The pieces of a decay per key channel: a block per (piece, entry, head).
+//
+// The piece's sums A_tj = sum_d k_t k_j dec(t, j) (and B_tj with q_t) take products of decays only, so
+// dec(t, j) cannot be cut into a factor of t and one of j by a quotient.  It is cut at the start m of
+// token t's four: for j before m it is (g_m .. g_t) (g_{j+1} .. g_{m-1}), which makes the sum a plain product
+// of rows X_t = k_t g_m .. g_t and Y_j = k_j g_{j+1} .. g_{m-1} (24 rows for the three later fours), and within a
+// four the six rows W_tj = k_j g_{j+1} .. g_t are made as they are.  Thread (t, j) then takes its two products
+// by 16-byte loads; the rows are made a thread a channel.  (A warp a token j that walked on over t with
+// two warp sums each took 78 us for 2,048 tokens and 16 heads of 128; 56 us here.)
+#define GK_ROWS(C) (3 * (C) + 1)            // decayed keys, decayed queries, keys on their way to the end, P_C
+__global__ void __launch_bounds__(256) delta_channel_pieces_kernel(DeltaHeadArgs a) {
+    extern __shared__ __align__(16) float sm[];
+    constexpr int C = GC_TOKENS;
+    const int D = a.D, LD = D + 4;
+    float* ks = sm;                              // [C][LD]
+    float* qs = ks + C * LD;                     // [C][LD]
+    float* gs = qs + C * LD;                     // [C][LD]
+    float* Xk = gs + C * LD;                     // [C][LD]
+    float* Xq = Xk + C * LD;                     // [C][LD]
+    float* Y = Xq + C * LD;                      // [24][LD]: of fours 1, 2, 3 (4, 8, 12 rows)
+    float* W = Y + 24 * LD;                      // [24][LD]: six of each four, (1,0) (2,0) (2,1) (3,0) (3,1) (3,2)
+    float* L = W + 24 * LD;                      // [C][GH_LD]
+    float* B = L + C * GH_LD;                    // [C][GH_LD]
+    const int piece = blockIdx.x, e = blockIdx.y, h = blockIdx.z, g_head = h / (a.H / a.G);
+    const int tid = threadIdx.x;
+    const unsigned long long waited = pdl_wait();
+    const float* q = pdl_after(a.q, waited);
+    const float* k = pdl_after(a.k, waited);
+    const float* beta = pdl_after(a.beta, waited);
+    const float* decay = pdl_after(a.decay, waited);
+    const int start = a.qo_indptr[e], n = a.qo_indptr[e + 1] - start;
+    const int base = piece * C;
+    if (base >= n) return;
+    const int here = min(C, n - base);
+    for (int i = tid; i < C * (D / 4); i += 256) {
+        const int t = i / (D / 4), d = (i - t * (D / 4)) * 4;
+        float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), qv = kv, gv = make_float4(1.f, 1.f, 1.f, 1.f);
+        if (t < here) {
+            const size_t tok = (size_t)(start + base + t);
+            kv = *reinterpret_cast<const float4*>(k + tok * a.G * D + (size_t)g_head * D + d);
+            qv = *reinterpret_cast<const float4*>(q + tok * a.G * D + (size_t)g_head * D + d);
+            gv = *reinterpret_cast<const float4*>(decay + tok * a.H * D + (size_t)h * D + d);
+        }
+        *reinterpret_cast<float4*>(ks + t * LD + d) = kv;
+        *reinterpret_cast<float4*>(qs + t * LD + d) = qv;
+        *reinterpret_cast<float4*>(gs + t * LD + d) = gv;
+    }
+    __syncthreads();
+    const size_t at = (gh_first_piece(start, e) + piece) * a.H + h;
+    // a thread a channel: half of the threads the rows for the scan, half those for the sums here
+    for (int i = tid; i < 2 * D; i += 256) {
+        const int d = i % D;
+        float kd[C], gd[C];
+#pragma unroll
+        for (int t = 0; t < C; ++t) {
+            kd[t] = ks[t * LD + d];
+            gd[t] = gs[t * LD + d];
+        }
+        if (i < D) {
+            float* dst = a.rows + at * GK_ROWS(C) * LD + d;
+            float P = 1.f, S = 1.f;
+#pragma unroll
+            for (int t = 0; t < C; ++t) {
+                P *= gd[t];
+                dst[t * LD] = kd[t] * P;
+                dst[(C + t) * LD] = qs[t * LD + d] * P;
+            }
+            dst[3 * C * LD] = P;
+#pragma unroll
+            for (int t = C - 1; t >= 0; --t) {
+                dst[(2 * C + t) * LD] = kd[t] * S;
+                S *= gd[t];
+            }
+        } else {
+            float y[C - 4];                      // Y of the four that comes next
+#pragma unroll
+            for (int f = 0; f < C / 4; ++f) {
+                float P = 1.f;
+#pragma unroll
+                for (int t = 4 * f; t < 4 * f + 4; ++t) {
+                    P *= gd[t];
+                    Xk[t * LD + d] = kd[t] * P;
+                    Xq[t * LD + d] = qs[t * LD + d] * P;
+#pragma unroll
+                    for (int j = 4 * f; j < t; ++j) {
+                        float w = kd[j];
+#pragma unroll
+                        for (int x = j + 1; x <= t; ++x) w *= gd[x];
+                        const int tt = t - 4 * f, jj = j - 4 * f;
+                        W[(6 * f + tt * (tt - 1) / 2 + jj) * LD + d] = w;
+                    }
+                }
+                if (f == C / 4 - 1) break;
+#pragma unroll
+                for (int j = 0; j < 4 * f; ++j) y[j] *= P;
+                float S = 1.f;
+#pragma unroll
+                for (int j = 4 * f + 3; j >= 4 * f; --j) {
+                    y[j] = kd[j] * S;
+                    S *= gd[j];
+                }
+#pragma unroll
+                for (int j = 0; j < 4 * f + 4; ++j) Y[(2 * f * (f + 1) + j) * LD + d] = y[j];
+            }
+        }
+    }
+    __syncthreads();
+    {
+        const int t = tid >> 4, j = tid & 15, f = t >> 2;
+        const bool near = (j >> 2) == f;         // in token t's own four
+        const float* right = j > t ? ks : j == t ? ks + t * LD
+                             : near ? W + (6 * f + (t & 3) * ((t & 3) - 1) / 2 + (j & 3)) * LD
+                                    : Y + (2 * (f - 1) * f + j) * LD;
+        const float* left_k = (near ? ks : Xk) + t * LD;
+        const float* left_q = (near ? qs : Xq) + t * LD;
+        float a0 = 0.f, a1 = 0.f, b0 = 0.f, b1 = 0.f;
+        for (int d = 0; d < D; d += 4) {
+            const float4 kt = *reinterpret_cast<const float4*>(left_k + d);
+            const float4 qt = *reinterpret_cast<const float4*>(left_q + d);
+            const float4 kj = *reinterpret_cast<const float4*>(right + d);
+            a0 = fmaf(kt.x, kj.x, a0); a1 = fmaf(kt.y, kj.y, a1);
+            b0 = fmaf(qt.x, kj.x, b0); b1 = fmaf(qt.y, kj.y, b1);
+            a0 = fmaf(kt.z, kj.z, a0); a1 = fmaf(kt.w, kj.w, a1);
+            b0 = fmaf(qt.z, kj.z, b0); b1 = fmaf(qt.w, kj.w, b1);
+        }
+        const float bt = t < here ? beta[(size_t)(start + base + t) * a.H + h] : 0.f;
+        if (j < t) L[t * GH_LD + j] = bt * (a0 + a1);
+        if (j <= t) B[t * GH_LD + j] = b0 + b1;
+    }
+    __syncthreads();
+    if (tid < C) {
+        float* m = a.mats + at * C * GH_MROW;
+        m[tid * GH_MROW + 2 * C] = 1.f;          // (the rows carry P and dec)
+        m[tid * GH_MROW + 2 * C + 1] = 1.f;
+        gh_solve(L, B, tid, tid < here ? beta[(size_t)(start + base + tid) * a.H + h] : 0.f, m);
     }
 }
 
@@ -1054,11 +855,16 @@ __device__ __forceinline__ void gh_bulk(float* dst, const float* src, uint32_t b
                  ::"r"(tc_smem(dst)), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 
-template <int D, int COLS>
+//
+// CHANNEL: the rows hold the decays (P and dec are 1 in the matrices), the new state takes rows of its own,
+// and P_C is a row.  2,048 tokens, 16 heads of 128 x 128: 173 us (a scan that gave a warp a column and a lane a
+// token's dot products, every warp reading all of the piece's rows, took 430 us: shared loads).
+template <int D, int COLS, bool CHANNEL>
 __global__ void __launch_bounds__(GH_THREADS, 2) delta_head_scan_kernel(DeltaHeadArgs a) {
     extern __shared__ __align__(16) float sm[];
     constexpr int C = GC_TOKENS, LD = D + 4, WARPS = GH_THREADS / 32;
-    constexpr int per_buf = 2 * C * LD + C * GH_MROW;
+    constexpr int ROWS = CHANNEL ? GK_ROWS(C) : 2 * C;
+    constexpr int per_buf = ROWS * LD + C * GH_MROW;
     constexpr int PJ = COLS / 4;                             // columns a thread takes of [r; p]
     constexpr int CT = D >= 96 ? PJ : (D == 64 || PJ < 4 ? PJ / 2 : 1);      // and keeps of S
     constexpr int TN = COLS / 8;                             // and makes of u and o
@@ -1087,8 +893,9 @@ __global__ void __launch_bounds__(GH_THREADS, 2) delta_head_scan_kernel(DeltaHea
         const uint32_t bar = tc_smem(full + buf);
         float* dst = sm + buf * per_buf;
         mbar_expect_tx(bar, (uint32_t)(per_buf * sizeof(float)));
-        gh_bulk(dst, rows + ((first + piece) * a.G + grp) * 2 * C * LD, 2 * C * LD * sizeof(float), bar);
-        gh_bulk(dst + 2 * C * LD, mats + ((first + piece) * a.H + h) * C * GH_MROW, C * GH_MROW * sizeof(float), bar);
+        gh_bulk(dst, rows + (CHANNEL ? (first + piece) * a.H + h : (first + piece) * a.G + grp) * ROWS * LD,
+                ROWS * LD * sizeof(float), bar);
+        gh_bulk(dst + ROWS * LD, mats + ((first + piece) * a.H + h) * C * GH_MROW, C * GH_MROW * sizeof(float), bar);
     };
 
     const int pieces = (n + C - 1) / C;
@@ -1150,7 +957,7 @@ __global__ void __launch_bounds__(GH_THREADS, 2) delta_head_scan_kernel(DeltaHea
         }
         const int here = min(C, n - piece * C);
         const float* ks = sm + buf * per_buf;    // (the q rows follow the k rows)
-        const float* ms = ks + 2 * C * LD;
+        const float* ms = ks + ROWS * LD;
         const float P = ms[t * GH_MROW + 2 * C], dec = ms[t * GH_MROW + 2 * C + 1];
         {
             float acc[4][PJ];
@@ -1238,13 +1045,20 @@ __global__ void __launch_bounds__(GH_THREADS, 2) delta_head_scan_kernel(DeltaHea
         }
         __syncthreads();
         if (keeps) {
-            const float pc = ms[(here - 1) * GH_MROW + 2 * C];
+            const float* news = CHANNEL ? ks + 2 * C * LD : ks;  // the rows that enter the state
 #pragma unroll
-            for (int x = 0; x < DT; ++x)
+            for (int x = 0; x < DT; ++x) {
+                float pc[4];
+                if (CHANNEL) {
+                    load4(ks + 3 * C * LD + (dg + DG * x) * 4, pc);
+                } else {
+                    pc[0] = pc[1] = pc[2] = pc[3] = ms[(here - 1) * GH_MROW + 2 * C];
+                }
 #pragma unroll
                 for (int c = 0; c < CT; ++c)
 #pragma unroll
-                    for (int w = 0; w < 4; ++w) s[x][c][w] *= pc;
+                    for (int w = 0; w < 4; ++w) s[x][c][w] *= pc[w];
+            }
 #pragma unroll
             for (int j = 0; j < C; ++j) {
                 float u[CT];
@@ -1252,7 +1066,7 @@ __global__ void __launch_bounds__(GH_THREADS, 2) delta_head_scan_kernel(DeltaHea
 #pragma unroll
                 for (int x = 0; x < DT; ++x) {
                     float kv[4];
-                    load4(ks + j * LD + (dg + DG * x) * 4, kv);
+                    load4(news + j * LD + (dg + DG * x) * 4, kv);
 #pragma unroll
                     for (int c = 0; c < CT; ++c)
 #pragma unroll
@@ -1276,70 +1090,86 @@ __global__ void __launch_bounds__(GH_THREADS, 2) delta_head_scan_kernel(DeltaHea
     gd_advance_conv(a.conv, waited, state + (size_t)a.slots[e] * a.state_stride, start, n, h, a.H);
 }
 
-// The scan in pieces with one decay a head (`decay` [tokens][H]), for key sizes of 32, 64, 96, 128 or
-// 256: `work` holds (tokens / 16 + entries) * (G * 32 * (D + 4) + H * 16 * 36) floats.  Returns 0, a CUDA error code, or -1 when the
-// shape is refused.
-MSTAR_API int mstar_delta_scan_head_pieces(const float* q, const float* k, const float* v,
-                                           const float* beta, const float* decay,
-                                           const int* qo_indptr, const int* slots, float* state,
-                                           long long state_stride, long long state_offset, float* out,
-                                           float* work, int tokens, int entries, int max_q_len, int H,
-                                           int G, int D, int VD, int* error_word, const float* conv_raw,
-                                           int conv_ld, int channels, int taps, void* stream) {
+template <int D, int COLS, bool CHANNEL>
+static int launch_head_scan(const DeltaHeadArgs& a, int entries, cudaStream_t s) {
+    constexpr int rows = CHANNEL ? GK_ROWS(GC_TOKENS) : 2 * GC_TOKENS;
+    constexpr size_t smem = ((size_t)2 * (rows * (D + 4) + GC_TOKENS * GH_MROW) + COLS * (D + 4) +
+                             (GH_THREADS / 32) * 2 * GC_TOKENS * (COLS + 4) + 2 * GC_TOKENS * COLS) * sizeof(float);
+    static bool configured = false;
+    if (smem > 48 * 1024 && !configured) {
+        const cudaError_t e = cudaFuncSetAttribute(delta_head_scan_kernel<D, COLS, CHANNEL>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    const dim3 grid(entries, a.H, (a.VD + COLS - 1) / COLS);
+    if (grid.z > 65535) return -1;
+    mstar_launch((delta_head_scan_kernel<D, COLS, CHANNEL>), grid, dim3(GH_THREADS), smem, s, a);
+    return launch_status();
+}
+template <int D, bool CHANNEL>
+static int launch_head_scan_cols(const DeltaHeadArgs& a, int entries, cudaStream_t s) {
+    // 16 columns a block where that gives most SMs a block, else 8
+    return (long long)entries * a.H * ((a.VD + 15) / 16) * 4 >= 3LL * device_sm_count()
+               ? launch_head_scan<D, 16, CHANNEL>(a, entries, s)
+               : launch_head_scan<D, 8, CHANNEL>(a, entries, s);
+}
+template <int D> static int launch_head_scan_kind(const DeltaHeadArgs& a, int entries, bool channel, cudaStream_t s) {
+    return channel ? launch_head_scan_cols<D, true>(a, entries, s) : launch_head_scan_cols<D, false>(a, entries, s);
+}
+
+// The scan in pieces, for key sizes of 32, 64, 96, 128 or 256.  head_decay: `decay` is [tokens][H] and `work`
+// holds (tokens / 16 + entries) * (G * 32 * (D + 4) + H * 16 * 36) floats; else `decay` is [tokens][H][D]
+// and `work` holds (tokens / 16 + entries) * H * (49 * (D + 4) + 16 * 36).  Returns 0, a CUDA error code,
+// or -1 when the shape is refused.
+MSTAR_API int mstar_delta_scan_pieces(const float* q, const float* k, const float* v,
+                                      const float* beta, const float* decay,
+                                      const int* qo_indptr, const int* slots, float* state,
+                                      long long state_stride, long long state_offset, float* out,
+                                      float* work, int tokens, int entries, int max_q_len, int H,
+                                      int G, int D, int VD, int head_decay, int* error_word,
+                                      const float* conv_raw, int conv_ld, int channels, int taps,
+                                      void* stream) {
     if (entries <= 0 || tokens <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || VD <= 0) return -1;
     if (D != 32 && D != 64 && D != 96 && D != 128 && D != 256) return -1;
     if (H > 65535 || entries > 65535 || (state_offset % 4) != 0 || (state_stride % 4) != 0) return -1;
-    if ((uintptr_t)q % 16 || (uintptr_t)k % 16 || (uintptr_t)work % 16 || (uintptr_t)state % 16 || !error_word)
+    if ((uintptr_t)q % 16 || (uintptr_t)k % 16 || (uintptr_t)work % 16 || (uintptr_t)state % 16 || !error_word ||
+        (!head_decay && (uintptr_t)decay % 16))
         return -1;
     const int max_pieces = (max_q_len + GC_TOKENS - 1) / GC_TOKENS;
     const size_t most = (size_t)(tokens / GC_TOKENS + entries);
-    DeltaHeadArgs a{q, k, v, beta, decay, qo_indptr, slots, work, work + most * G * 2 * GC_TOKENS * (D + 4), state, state_stride, state_offset, out, H, G, D, VD, tokens,
-                    error_word, {taps > 1 ? conv_raw : nullptr, conv_ld, channels, taps}};
+    const size_t row_floats = head_decay ? most * G * 2 * GC_TOKENS * (D + 4) : most * H * GK_ROWS(GC_TOKENS) * (D + 4);
+    DeltaHeadArgs a{q, k, v, beta, decay, qo_indptr, slots, work, work + row_floats, state, state_stride, state_offset, out,
+                    H, G, D, VD, tokens, error_word, {taps > 1 ? conv_raw : nullptr, conv_ld, channels, taps}};
     cudaStream_t s = (cudaStream_t)stream;
-    // a warp a head in the second half of the first kernel: eight at most, as many as a group has
-    const int per = H / G, warps = per < 8 ? per : 8;
-    const size_t smem1 = (2 * (size_t)GC_TOKENS * (D + 4) + 2 * GC_TOKENS * GH_LD +
-                          warps * (2 * GC_TOKENS * GH_LD + 2 * GC_TOKENS)) * sizeof(float);
-    if (smem1 > 48 * 1024) {
+    if (head_decay) {
+        // a warp a head in the second half of the first kernel: eight at most, as many as a group has
+        const int per = H / G, warps = per < 8 ? per : 8;
+        const size_t smem1 = (2 * (size_t)GC_TOKENS * (D + 4) + 2 * GC_TOKENS * GH_LD +
+                              warps * (2 * GC_TOKENS * GH_LD + 2 * GC_TOKENS)) * sizeof(float);
         static size_t configured = 0;
-        if (smem1 > configured) {
-            cudaFuncSetAttribute(delta_head_pieces_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem1);
+        if (smem1 > 48 * 1024 && smem1 > configured) {
+            cudaFuncSetAttribute(delta_head_pieces_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
             configured = smem1;
         }
+        mstar_launch(delta_head_pieces_kernel, dim3(max_pieces, entries, G), dim3(256), smem1, s, a);
+    } else {
+        const size_t smem1 = ((size_t)128 * (D + 4) + 2 * GC_TOKENS * GH_LD) * sizeof(float);
+        static size_t configured = 0;
+        if (smem1 > 48 * 1024 && smem1 > configured) {
+            cudaFuncSetAttribute(delta_channel_pieces_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
+            configured = smem1;
+        }
+        mstar_launch(delta_channel_pieces_kernel, dim3(max_pieces, entries, H), dim3(256), smem1, s, a);
     }
-    mstar_launch(delta_head_pieces_kernel, dim3(max_pieces, entries, G), dim3(256), smem1, s, a);
-    int code = launch_status();
+    const int code = launch_status();
     if (code != 0) return code;
-    // 16 columns a block where that gives most SMs a block, else 8
-    const int cols = (long long)entries * H * ((VD + 15) / 16) * 4 >= 3LL * device_sm_count() ? 16 : 8;
-    const size_t smem2 = ((size_t)2 * (2 * GC_TOKENS * (D + 4) + GC_TOKENS * GH_MROW) + cols * (D + 4) +
-                          (GH_THREADS / 32) * 2 * GC_TOKENS * (cols + 4) + 2 * GC_TOKENS * cols) * sizeof(float);
-    dim3 grid(entries, H, (VD + cols - 1) / cols);
-    if (grid.z > 65535) return -1;
-#define GO1(DD, CC)                                                                               \
-    do {                                                                                          \
-        static size_t configured = 0;                                                             \
-        if (smem2 > 48 * 1024 && smem2 > configured) {                                            \
-            cudaFuncSetAttribute(delta_head_scan_kernel<DD, CC>,                                  \
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);        \
-            configured = smem2;                                                                   \
-        }                                                                                         \
-        mstar_launch((delta_head_scan_kernel<DD, CC>), grid, dim3(GH_THREADS), smem2, s, a);      \
-    } while (0)
-#define GO(DD)                                                                                    \
-    do {                                                                                          \
-        if (cols == 16) GO1(DD, 16); else GO1(DD, 8);                                             \
-    } while (0)
-    if (D == 32) GO(32);
-    else if (D == 64) GO(64);
-    else if (D == 96) GO(96);
-    else if (D == 128) GO(128);
-    else GO(256);
-#undef GO
-#undef GO1
-    return launch_status();
+    if (D == 32) return launch_head_scan_kind<32>(a, entries, !head_decay, s);
+    if (D == 64) return launch_head_scan_kind<64>(a, entries, !head_decay, s);
+    if (D == 96) return launch_head_scan_kind<96>(a, entries, !head_decay, s);
+    if (D == 128) return launch_head_scan_kind<128>(a, entries, !head_decay, s);
+    return launch_head_scan_kind<256>(a, entries, !head_decay, s);
 }
 
 // ------------------------------------------------------------------ finish

@@ -1818,10 +1818,9 @@ def delta_scan(q, k, v, beta, decay, qo_indptr, slots, state: torch.Tensor, entr
 
     A step with an entry of ``DELTA_PIECES_FROM`` tokens or more (and ``dim`` 32, 64, 128 or 256) is
     scanned in pieces of 16 tokens: what does not depend on the state (decayed keys and
-    queries, the keys' products among themselves) is made for all pieces side by side, and
-    the chain from token to token shrinks to a scalar a token (MSTAR_DELTA_PIECES=0: never;
-    1: always).  ``decay`` [tokens, heads] is one decay a head: the chain inside a piece then
-    becomes a small triangular matrix made ahead.
+    queries, the keys' products among themselves, the inverse of the triangular system that the
+    tokens of a piece form) is made for all pieces side by side (MSTAR_DELTA_PIECES=0: never;
+    1: always).  ``decay``: [tokens, heads * dim], or [tokens, heads] with one decay a head.
 
     ``conv_rows``: the projected rows ``delta_prepare`` read; the slots' convolution inputs then
     move on in the same launch (else ``conv_state_advance`` does that)."""
@@ -1844,33 +1843,18 @@ def delta_scan(q, k, v, beta, decay, qo_indptr, slots, state: torch.Tensor, entr
     longest = int(min(max_q_len, tokens))
     forced = os.environ.get("MSTAR_DELTA_PIECES")
     pieces = (forced == "1" or (forced != "0" and longest >= DELTA_PIECES_FROM))
+    aligned = all(t.data_ptr() % 16 == 0 for t in (q, k, state)) and (head_decay or decay.data_ptr() % 16 == 0)
     if (pieces and dim in (DELTA_HEAD_PIECES_DIMS if head_decay else DELTA_PIECES_DIMS) and tokens > 0 and offset % 4 == 0
-            and state.stride(0) % 4 == 0):
-        max_pieces = -(-longest // DELTA_PIECE)
-        if head_decay:
-            per_piece = (kv_heads * 2 * DELTA_PIECE * (dim + 4)
-                         + heads * DELTA_PIECE * (2 * DELTA_PIECE + 4))
-            work = torch.empty((tokens // DELTA_PIECE + entries) * per_piece, dtype=torch.float32,
-                               device=q.device)
-            code = lib.get("gated_delta").mstar_delta_scan_head_pieces(
-                q.data_ptr(), k.data_ptr(), v.data_ptr(), beta.data_ptr(), decay.data_ptr(),
-                qo_indptr.data_ptr(), slots.data_ptr(), state.data_ptr(), state.stride(0), offset,
-                out.data_ptr(), work.data_ptr(), tokens, entries, longest, heads, kv_heads, dim,
-                vdim, tcgen05_error_word(q.device).data_ptr(), *conv, _stream())
-            if code == -1:
-                raise KernelError(f"delta-rule scan in pieces refuses heads={heads}, "
-                                  f"kv_heads={kv_heads}, dim={dim}")
-            check(code, "delta_scan_head_pieces")
-            lib.add_launches(1)
-            return out
-        floats = (3 * tokens * heads * dim + entries * max_pieces * heads * dim
-                  + 2 * tokens * heads * DELTA_PIECE)
-        work = torch.empty(floats, dtype=torch.float32, device=q.device)
+            and state.stride(0) % 4 == 0 and (aligned or head_decay)):
+        rows = (kv_heads * 2 * DELTA_PIECE if head_decay else heads * (3 * DELTA_PIECE + 1)) * (dim + 4)
+        per_piece = rows + heads * DELTA_PIECE * (2 * DELTA_PIECE + 4)
+        work = torch.empty((tokens // DELTA_PIECE + entries) * per_piece, dtype=torch.float32,
+                           device=q.device)
         code = lib.get("gated_delta").mstar_delta_scan_pieces(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), beta.data_ptr(), decay.data_ptr(),
             qo_indptr.data_ptr(), slots.data_ptr(), state.data_ptr(), state.stride(0), offset,
-            out.data_ptr(), work.data_ptr(), tokens, entries, longest, heads, kv_heads, dim, vdim,
-            *conv, _stream())
+            out.data_ptr(), work.data_ptr(), tokens, entries, longest, heads, kv_heads, dim,
+            vdim, int(head_decay), tcgen05_error_word(q.device).data_ptr(), *conv, _stream())
         if code == -1:
             raise KernelError(f"delta-rule scan in pieces refuses heads={heads}, "
                               f"kv_heads={kv_heads}, dim={dim}")

@@ -63,7 +63,8 @@ def test_float_attention_of_portions_leaves_unseen_values_out():
 @pytest.mark.parametrize("tokens,width,ff,experts,identity,top,form,on_input", [
     (200, 72, 8, 2, 0, 2, "silu", False),         # k-blocks that end early, one narrow column tile
     (300, 128, 264, 5, 1, 3, "silu", True),       # column tiles that end inside, identity experts
-    (129, 264, 136, 3, 0, 1, "relu2", False),     # one row past a row tile
+    (129, 264, 136, 3, 0, 1, "relu2", False),
+    (771, 136, 136, 3, 0, 1, "silu", True),       # groups of a row tile and a few rows more
     (2100, 64, 16, 7, 2, 6, "clamped", False),    # more rows than the sort keeps in registers, top > 4
     (64, 64, 64, 40, 0, 1, "silu", True)])        # experts without rows
 def test_grouped_experts_at_the_borders_of_their_tiles(tokens, width, ff, experts, identity, top, form, on_input):
@@ -130,3 +131,82 @@ def test_gated_products_by_eight_and_one_by_one(dtype, rows, inter):
     want = (y.double().view(rows, 2, inter) * torch.sigmoid(gate.double())[:, :, None]).view(rows, -1)
     got = ops.head_gate_mul(y, gate, 2, out_dtype=torch.bfloat16).double()
     assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-30).all()
+
+
+@pytest.mark.parametrize("lens,heads,kv_heads,dim,vdim", [
+    ([70], 2, 1, 32, 8),                    # a piece of 6 tokens at the end, 8 columns
+    ([64, 1, 33], 2, 2, 64, 20),            # columns that end inside a block, an entry of one token
+    ([100], 1, 1, 256, 16)])
+def test_delta_rule_in_pieces_with_decays_per_channel(lens, heads, kv_heads, dim, vdim):
+    """Against the recurrence in double precision, with decays from 1 down to numbers whose products
+    over a piece underflow, and a state to start from."""
+    from mstar_b200 import ops
+
+    T, taps = sum(lens), 2
+    q, k = (torch.nn.functional.normalize(rnd(T, kv_heads, dim, seed=s), dim=-1).view(T, -1) for s in (1, 2))
+    v, beta = rnd(T, heads * vdim, seed=3), torch.sigmoid(rnd(T, heads, seed=4))
+    decay = torch.exp(-torch.exp(4 * rnd(T, heads * dim, seed=5) - 3))
+    size = ops.gated_delta_state_size(heads, kv_heads, dim, vdim, taps)
+    state = 0.3 * rnd(len(lens), size, seed=6)
+    offset = (taps - 1) * (2 * kv_heads * dim + heads * vdim)
+    S = state[:, offset:offset + heads * vdim * dim].double().view(-1, heads, vdim, dim).transpose(2, 3).clone()
+    starts = [0]
+    for n in lens:
+        starts.append(starts[-1] + n)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    got = ops.delta_scan(q, k, v, beta, decay, i32(starts), i32(list(range(len(lens)))), state, len(lens), heads,
+                         kv_heads, dim, vdim, taps, max_q_len=max(lens)).view(T, heads, vdim)
+    ops.check_error_word(DEV)
+    per = heads // kv_heads
+    qd, kd = (x.double().view(T, kv_heads, dim).repeat_interleave(per, dim=1) for x in (q, k))
+    vd, gd, bd = v.double().view(T, heads, vdim), decay.double().view(T, heads, dim), beta.double()
+    for e in range(len(lens)):
+        for t in range(starts[e], starts[e + 1]):
+            S[e] *= gd[t][:, :, None]
+            u = bd[t][:, None] * (vd[t] - (kd[t][:, None] @ S[e])[:, 0])
+            S[e] += kd[t][:, :, None] * u[:, None]
+            want = (qd[t][:, None] @ S[e])[:, 0]
+            # sums of dim products of numbers of about 1, once a token, over at most 16 tokens' corrections
+            assert (got[t].double() - want).abs().max() < 2 ** -24 * 64 * dim ** 0.5
+    end = state[:, offset:offset + heads * vdim * dim].double().view(-1, heads, vdim, dim).transpose(2, 3)
+    assert (end - S).abs().max() < 2 ** -24 * 64 * dim ** 0.5
+
+
+@pytest.mark.parametrize("lens,inner,piece", [([512, 7, 530], 64, "256"), ([600], 32, "0"), ([513], 96, "16")])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_selective_scan_of_long_portions(lens, inner, piece, dtype, monkeypatch):
+    """The scan for 16 states a channel, whole and in pieces, against the recurrence in double precision."""
+    from mstar_b200 import ops
+
+    monkeypatch.setenv("MSTAR_SCAN_PIECE", piece)
+    T, rank, N, taps = sum(lens), 4, 16, 3
+    xc, xz = rnd(T, inner, dtype=dtype, seed=1), rnd(T, 2 * inner, dtype=dtype, seed=2)
+    proj, w_dt = rnd(T, rank + 2 * N, seed=3), rnd(inner, rank, seed=4)
+    bias, a, d = rnd(inner, seed=5) - 3, -torch.exp(rnd(inner, N, seed=6)), rnd(inner, seed=7)
+    state = rnd(len(lens), ops.selective_scan_state_size(inner, N, taps), seed=8)
+    S = state[:, (taps - 1) * inner:].double().view(-1, inner, N).clone()
+    starts = [0]
+    for n in lens:
+        starts.append(starts[-1] + n)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    got = ops.selective_scan(xc, xz, proj, w_dt, bias, a, d, i32(starts), i32(list(range(len(lens)))), state, len(lens),
+                             inner, N, rank, taps, max_q_len=max(lens)).double()
+    dt = torch.nn.functional.softplus(proj[:, :rank].double() @ w_dt.double().T + bias.double())
+    x, z, p = xc.double(), xz[:, inner:].double(), proj.double()
+    want, size = torch.empty_like(got), torch.empty_like(got)
+    for e in range(len(lens)):
+        for t in range(starts[e], starts[e + 1]):
+            S[e] = torch.exp(dt[t][:, None] * a.double()) * S[e] + (dt[t] * x[t])[:, None] * p[t, rank:rank + N]
+            want[t] = S[e] @ p[t, rank + N:] + d.double() * x[t]
+            size[t] = S[e].abs() @ p[t, rank + N:].abs() + (d.double() * x[t]).abs()
+    gate = z * torch.sigmoid(z)
+    # a state is a sum of decayed inputs whose exponents are rounded (2^-24 of up to 100) and whose exponentials are
+    # off by 2 ulp; the result is rounded to its type
+    off = 2.0 ** -8 if dtype == torch.bfloat16 else 0.0
+    assert ((got - want * gate).abs() <= off * (want * gate).abs() + 2 ** -17 * size * gate.abs() + 1e-6).all()
+    end = state[:, (taps - 1) * inner:].double().view(-1, inner, N)
+    assert ((end - S).abs() <= 2 ** -17 * S.abs() + 1e-5).all()
+    for e in range(len(lens)):                       # the convolution's window moved on
+        for j in range(taps - 1):
+            row = xz[starts[e + 1] - (taps - 1) + j, :inner].float()
+            assert torch.equal(state[e, j * inner:(j + 1) * inner], row)
