@@ -11,6 +11,7 @@
 // Step sizes, decays, their exponentials, the state and its sums are float for both
 // activation types; a channel's arithmetic does not depend on the rest of the batch.
 #include "common.cuh"
+#include "mma_util.cuh"
 
 __device__ __forceinline__ float silu_f(float v) { return v / (1.f + expf(-v)); }
 __device__ __forceinline__ float softplus_f(float v) { return v > 20.f ? v : log1pf(expf(v)); }
@@ -434,6 +435,230 @@ selective_scan_kernel(const A* __restrict__ xc, const A* __restrict__ xz,
     }
 }
 
+// The same for 16 states a channel and step sizes' products made by the caller (long portions). Lane s of a
+// channel's four holds states 4 s .. 4 s + 3 as two pairs, so that B and C come as one 16-byte
+// load each and multiplications run two to an instruction (f32x2); a chunk's [B | C], x, z and
+// step sizes come by 16-byte asynchronous copies, STAGES - 1 chunks ahead, the rest of the projection
+// rows stays where it is.  Tokens past the portion's end get a step size of 0 and leave the
+// state as it is.  The output sums of four tokens meet in one exchange among the lanes, each of which
+// then finishes one token.  Bound by the exponential (one ex2 per state and token: 30 us for 2,048 tokens x
+// 4,096 channels at 16 a cycle and SM) and by one warp a scheduler where channels are few.
+// 2 x 1,024 tokens, 4,096 channels, pieces of 128: 57 + 89 us for the two passes; the kernel above takes 203 us
+// each (a 4-byte copy for every number of the rows, two 4-byte loads of B and C a state, exp2f).
+#define SX_STAGES 3
+
+__device__ __forceinline__ unsigned long long sx_pack(float lo, float hi) {
+    return (unsigned long long)__float_as_uint(lo) | ((unsigned long long)__float_as_uint(hi) << 32);
+}
+__device__ __forceinline__ float sx_lo(unsigned long long v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float sx_hi(unsigned long long v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ unsigned long long sx_mul(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long sx_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+// 2^x for x <= 0 (what underflows is 0)
+__device__ __forceinline__ float sx_ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float sx_silu(float v, bf16) { return silu_bf16(v); }
+__device__ __forceinline__ float sx_silu(float v, float) { return silu_f(v); }
+
+template <typename A> struct ScanStage {
+    float bc[SS_TC][32];            // B then C
+    float d[SS_TC][32];             // W_dt dt_in, then the step size
+    A x[SS_TC][32], z[SS_TC][32];
+};
+
+// PASS as in the kernel above: 0 whole portions, 1 a piece from zero state, 2 a piece from the state
+// that the pieces before it leave.
+template <typename A, int PASS>
+__global__ void __launch_bounds__(128)
+selective_scan16_kernel(const A* __restrict__ xc, const A* __restrict__ xz, const float* __restrict__ proj,
+                        const float* __restrict__ dt_bias, const float* __restrict__ a_neg,
+                        const float* __restrict__ d_skip, const int* __restrict__ qo_indptr,
+                        const int* __restrict__ slots, float* __restrict__ state, A* __restrict__ out, ScanArgs a) {
+    __shared__ __align__(16) ScanStage<A> stage[SX_STAGES];
+    const int e = blockIdx.x, piece = blockIdx.z;
+    const int tid = threadIdx.x, sub = tid & 3, ch = tid >> 2;
+    const int c0 = blockIdx.y * 32, c = c0 + ch;
+    const unsigned long long waited = pdl_wait();
+    xc = pdl_after(xc, waited);
+    xz = pdl_after(xz, waited);
+    proj = pdl_after(proj, waited);
+    const float* dt_pre = pdl_after(a.dt_pre, waited);
+    const int e_start = qo_indptr[e], e_tok = qo_indptr[e + 1] - e_start;
+    const int pieces = PASS != 0 ? max(1, (e_tok + a.piece - 1) / a.piece) : 1;
+    if (piece >= pieces || (PASS == 1 && piece == pieces - 1)) return;
+    const int start = e_start + (PASS != 0 ? piece * a.piece : 0);
+    const int n_tok = PASS != 0 ? min(a.piece, e_tok - piece * a.piece) : e_tok;
+    float* slot = state + (size_t)slots[e] * a.state_stride;
+    float* s_slot = slot + (size_t)(a.taps - 1) * a.inner + (size_t)c * 16 + 4 * sub;
+    const int row = a.rank + 32;
+
+    auto fetch = [&](int t0) {
+        ScanStage<A>& st = stage[(t0 / SS_TC) % SX_STAGES];
+        const int nt = min(SS_TC, n_tok - t0);
+        constexpr int XQ = 32 * (int)sizeof(A) / 16;       // 16-byte pieces of a token's x (or z)
+        for (int i = tid; i < SS_TC * (16 + 2 * XQ); i += 128) {
+            const int k = i / (16 + 2 * XQ), q = i - k * (16 + 2 * XQ);
+            if (k >= nt) break;
+            const size_t t = (size_t)(start + t0 + k);
+            if (q < 8) cp_async_16(smem_u32(&st.bc[k][4 * q]), proj + t * row + a.rank + 4 * q, 16);
+            else if (q < 16) cp_async_16(smem_u32(&st.d[k][4 * (q - 8)]), dt_pre + t * a.inner + c0 + 4 * (q - 8), 16);
+            else if (q < 16 + XQ)
+                cp_async_16(smem_u32(st.x[k]) + 16 * (q - 16),
+                            reinterpret_cast<const char*>(xc + t * a.inner + c0) + 16 * (q - 16), 16);
+            else
+                cp_async_16(smem_u32(st.z[k]) + 16 * (q - 16 - XQ),
+                            reinterpret_cast<const char*>(xz + t * a.ld_xz + a.inner + c0) + 16 * (q - 16 - XQ), 16);
+        }
+    };
+#pragma unroll
+    for (int s = 0; s < SX_STAGES - 1; ++s) {
+        if (s * SS_TC < n_tok) fetch(s * SS_TC);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+
+    // A in units of log2(e): the decays are then 2^(dt A)
+    unsigned long long S[2], An[2];
+    {
+        const float4 an = *reinterpret_cast<const float4*>(a_neg + (size_t)c * 16 + 4 * sub);
+        constexpr float L = 1.4426950408889634f;
+        An[0] = sx_pack(an.x * L, an.y * L);
+        An[1] = sx_pack(an.z * L, an.w * L);
+    }
+    // (the last piece puts the new state into the slot while others may not have started: pass 1
+    // leaves a copy of the old one in the scratch entry of the last piece, which pass 2 reads)
+    float* kept = PASS != 0 ? a.piece_state + (((size_t)e * a.max_pieces + pieces - 1) * a.inner + c) * 16 + 4 * sub : nullptr;
+    if (PASS == 1 && piece == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) kept[i] = s_slot[i];
+    }
+    if (PASS == 1) {
+        S[0] = S[1] = 0ull;
+    } else {
+        const float* from = PASS == 2 && pieces > 1 ? kept : s_slot;
+        S[0] = sx_pack(from[0], from[1]);
+        S[1] = sx_pack(from[2], from[3]);
+    }
+    if (PASS == 2) {
+        for (int j = 0; j < piece; ++j) {
+            const size_t at = (size_t)e * a.max_pieces + j;
+            const float sdt = a.piece_dt[at * a.inner + c];
+            const float4 E = *reinterpret_cast<const float4*>(a.piece_state + (at * a.inner + c) * 16 + 4 * sub);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                S[i] = sx_fma(sx_pack(sx_ex2(sdt * sx_lo(An[i])), sx_ex2(sdt * sx_hi(An[i]))), S[i],
+                              i == 0 ? sx_pack(E.x, E.y) : sx_pack(E.z, E.w));
+        }
+    }
+    float dt_sum = 0.f;
+    const float bias = dt_bias[c], dsk = d_skip[c];
+
+    for (int t0 = 0; t0 < n_tok; t0 += SS_TC) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(SX_STAGES - 2) : "memory");
+        __syncthreads();            // the chunk is there, and the one before it is done with
+        if (t0 + (SX_STAGES - 1) * SS_TC < n_tok) fetch(t0 + (SX_STAGES - 1) * SS_TC);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        ScanStage<A>& st = stage[(t0 / SS_TC) % SX_STAGES];
+        const int nt = min(SS_TC, n_tok - t0);
+        // the softplus of a channel's step sizes is dealt out among its lanes
+#pragma unroll
+        for (int j = 0; j < SS_TC / 4; ++j) {
+            const int k = sub + 4 * j;
+            st.d[k][ch] = k < nt ? softplus_f(st.d[k][ch] + bias) : 0.f;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k0 = 0; k0 < SS_TC; k0 += 4) {
+            unsigned long long da[4][2], db[4][2];
+            float y[4];
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+                const int k = k0 + kk;
+                const float dt = st.d[k][ch], dx = k < nt ? dt * to_float(st.x[k][ch]) : 0.f;
+                if (PASS == 1) dt_sum += dt;
+                const ulonglong2 B = *reinterpret_cast<const ulonglong2*>(&st.bc[k][4 * sub]);
+                const unsigned long long dt2 = sx_pack(dt, dt), dx2 = sx_pack(dx, dx);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const unsigned long long z = sx_mul(dt2, An[i]);
+                    da[kk][i] = sx_pack(sx_ex2(sx_lo(z)), sx_ex2(sx_hi(z)));
+                    db[kk][i] = k < nt ? sx_mul(dx2, i == 0 ? B.x : B.y) : 0ull;
+                }
+            }
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+                S[0] = sx_fma(da[kk][0], S[0], db[kk][0]);
+                S[1] = sx_fma(da[kk][1], S[1], db[kk][1]);
+                if (PASS != 1) {
+                    const ulonglong2 C = *reinterpret_cast<const ulonglong2*>(&st.bc[k0 + kk][16 + 4 * sub]);
+                    const unsigned long long y2 = sx_fma(S[1], C.y, sx_mul(S[0], C.x));
+                    y[kk] = sx_lo(y2) + sx_hi(y2);
+                }
+            }
+            if (PASS != 1) {
+                // lane s ends up with the sum of token k0 + s over the four lanes
+                const bool odd = sub & 1, high = sub & 2;
+                const float r0 = (odd ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, odd ? y[0] : y[1], 1);
+                const float r1 = (odd ? y[3] : y[2]) + __shfl_xor_sync(0xffffffffu, odd ? y[2] : y[3], 1);
+                const float sum = (high ? r1 : r0) + __shfl_xor_sync(0xffffffffu, high ? r0 : r1, 2);
+                const int k = k0 + sub;
+                if (k < nt)
+                    out[(size_t)(start + t0 + k) * a.inner + c] = from_float<A>(
+                        fmaf(dsk, to_float(st.x[k][ch]), sum) * sx_silu(to_float(st.z[k][ch]), A()));
+            }
+        }
+    }
+    if (PASS == 1) {                           // this piece alone, for the pieces after it
+        const size_t at = (size_t)e * a.max_pieces + piece;
+        *reinterpret_cast<float4*>(a.piece_state + (at * a.inner + c) * 16 + 4 * sub) =
+            make_float4(sx_lo(S[0]), sx_hi(S[0]), sx_lo(S[1]), sx_hi(S[1]));
+        if (sub == 0) a.piece_dt[at * a.inner + c] = dt_sum;
+        return;
+    }
+    if (piece != pieces - 1) return;
+    s_slot[0] = sx_lo(S[0]);
+    s_slot[1] = sx_hi(S[0]);
+    s_slot[2] = sx_lo(S[1]);
+    s_slot[3] = sx_hi(S[1]);
+    if (sub == 0 && e_tok > 0) {
+        // the window of the convolution: the last taps-1 inputs of [old window | this portion]
+        for (int j = 0; j < a.taps - 1; ++j) {
+            const int at = e_tok + j;
+            slot[(size_t)j * a.inner + c] =
+                at < a.taps - 1 ? slot[(size_t)at * a.inner + c]
+                                : to_float(xz[(size_t)(e_start + at - (a.taps - 1)) * a.ld_xz + c]);
+        }
+    }
+}
+
+template <typename A>
+static void launch_scan16(const void* xc, const void* xz, const float* proj, const float* dt_bias, const float* a_neg,
+                          const float* d_skip, const int* qo_indptr, const int* slots, float* state, void* out,
+                          ScanArgs a, cudaStream_t s) {
+    const dim3 grid(a.entries, a.inner / 32, a.max_pieces);
+#define GO(PASS)                                                                                  \
+    a.pass = PASS;                                                                                \
+    mstar_launch((selective_scan16_kernel<A, PASS>), grid, dim3(128), 0, s, (const A*)xc, (const A*)xz, proj, \
+                 dt_bias, a_neg, d_skip, qo_indptr, slots, state, (A*)out, a)
+    if (a.piece > 0) {
+        GO(1);
+        GO(2);
+    } else {
+        GO(0);
+    }
+#undef GO
+}
+
 // xc: [tokens, inner] conv outputs; xz: [tokens] rows of ld_xz elements, x then z; proj: float
 // [tokens, rank + 2 n_state]; w_dt float [inner, rank]; a_neg float [inner, n_state] = -exp(A_log);
 // out [tokens, inner].  piece > 0: portions are cut into pieces of that many tokens (a multiple
@@ -455,6 +680,15 @@ MSTAR_API int mstar_selective_scan(const void* xc, const void* xz, int ld_xz, co
     cudaStream_t s = (cudaStream_t)stream;
     ScanArgs a{inner, n_state, rank, taps, ld_xz, entries, state_stride, piece, 0,
                piece > 0 ? max_pieces : 1, piece_state, piece_dt, dt_pre};
+    const int piece16 = act_dtype == MSTAR_F32 ? 4 : 8;          // elements of 16 bytes
+    if (dt_pre != nullptr && n_state == 16 && inner % 32 == 0 && rank % 4 == 0 && ld_xz % piece16 == 0 &&
+        (((uintptr_t)xc | (uintptr_t)xz | (uintptr_t)proj | (uintptr_t)dt_pre | (uintptr_t)a_neg | (uintptr_t)piece_state) & 15) == 0) {
+        if (act_dtype == MSTAR_F32)
+            launch_scan16<float>(xc, xz, proj, dt_bias, a_neg, d_skip, qo_indptr, slots, state, out, a, s);
+        else
+            launch_scan16<bf16>(xc, xz, proj, dt_bias, a_neg, d_skip, qo_indptr, slots, state, out, a, s);
+        return launch_status();
+    }
 #define GO(A, LANES, NPER)                                                                        \
     {                                                                                             \
         constexpr int CH = SS_THREADS / LANES;                                                    \
