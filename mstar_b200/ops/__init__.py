@@ -594,7 +594,8 @@ def tcgen05_error_word(device) -> torch.Tensor:
     """Device int32 that a kernel with bounded mbarrier waits sets when one of them ran out:
     1-3 tcgen05 GEMM (producer, MMA issuer, epilogue), 4 decode attention copies, 6-12 tcgen05
     prefill attention, 13-14 bulk-copy small-M GEMM, 15-17 swapped-operand tcgen05 GEMM, 18
-    delta-rule scan in pieces, 19-21 grouped expert GEMM; zero otherwise."""
+    delta-rule scan in pieces, 19-21 grouped expert GEMM, 22-27 prompt attention with probabilities
+    in two parts; zero otherwise."""
     key = torch.device(device).index or 0
     if key not in _tc_error_words:
         _tc_error_words[key] = torch.zeros(1, dtype=torch.int32, device=device)
@@ -617,6 +618,8 @@ WAIT_CODES[18] = "delta-rule scan in pieces: a wait for a piece's rows"
 WAIT_CODES.update({19: "grouped expert GEMM: the producer waited for a free stage",
                    20: "grouped expert GEMM: the MMA issuer waited for operand tiles",
                    21: "grouped expert GEMM: the epilogue waited for an accumulator"})
+WAIT_CODES.update({c: "prompt attention with probabilities in two parts: a wait on one of its barriers "
+                   "ran out" for c in range(22, 28)})
 WAIT_CODES.update({c: "tcgen05 prefill attention: a wait on one of its barriers ran out"
                    for c in range(6, 13)})
 
@@ -1160,6 +1163,95 @@ def latent_attention(q_abs: torch.Tensor, q_rot: torch.Tensor, cache: torch.Tens
     return out
 
 
+# query-key pairs of a request per key from which on its keys and values are made from the latents
+# (making them costs 13 ns a key for 16 heads of 128 at a rank of 512, 3.5 ns for 8 of 64 at 256; a pair
+# of the folded form 0.9 and 0.22 ns), and the most memory the keys and values made at once take (8
+# bytes a feature as the product's floats, as much again in two parts: 32,768 keys of 16 heads of 128)
+LATENT_PROMPT_PAIRS = 32
+LATENT_PROMPT_BYTES = 1 << 30
+
+
+def latent_prompt_groups(q_lens, kv_lens, window: int, features: int, first_entry: int = 0) -> list:
+    """[(first entry, entries, keys)] of the runs of portions, from ``first_entry`` on, whose keys and
+    values (``features`` each: heads times dim) are made from the latents together; empty where the
+    folded form is the cheaper one or a portion's take more than ``LATENT_PROMPT_BYTES``."""
+    keys, room = [], LATENT_PROMPT_BYTES // (16 * features)
+    for q, n in zip(q_lens[first_entry:], kv_lens[first_entry:]):
+        past = n - q
+        keys.append(n - ((past - window + 1) // PROMPT_KEYS * PROMPT_KEYS if window and past >= window else 0))
+    pairs = sum(q * k for q, k in zip(q_lens[first_entry:], keys))
+    if not keys or pairs < LATENT_PROMPT_PAIRS * sum(keys) or max(keys) > room:
+        return []
+    groups = []
+    for i, k in enumerate(keys, first_entry):
+        if groups and groups[-1][2] + k <= room:
+            first, count, total = groups[-1]
+            groups[-1] = (first, count + 1, total + k)
+        else:
+            groups.append((i, 1, k))
+    return groups
+
+
+def latent_prompt_takes(q: torch.Tensor, cache: torch.Tensor, dim: int, v_dim: int, rank: int,
+                        rot: int) -> bool:
+    """Whether the tcgen05 prompt kernel takes latent attention of these sizes (``q``: [tokens, heads,
+    dim + rot]; MSTAR_LATENT_ATTENTION set to anything: never)."""
+    return (q.dtype == torch.bfloat16 and cache.dtype == torch.bfloat16 and dim == v_dim
+            and dim in (64, 128) and 0 < rot <= 64 and rot % 8 == 0 and rank % 8 == 0
+            and q.stride(2) == 1 and q.stride(0) % 8 == 0 and q.stride(1) % 8 == 0
+            and q.data_ptr() % 16 == 0 and cache.data_ptr() % 16 == 0
+            and os.environ.get("MSTAR_LATENT_ATTENTION") is None)
+
+
+def latent_attention_prompt(q: torch.Tensor, cache: torch.Tensor, block_table, ctx, groups, w_kv,
+                            heads: int, dim: int, rank: int, rot: int, page_size: int, window: int,
+                            scale: float, out: torch.Tensor, gate=None) -> None:
+    """Latent attention of prompt portions on tcgen05: for each of ``groups`` (see
+    ``latent_prompt_groups``) the latent rows its tokens see are gathered, one product with ``w_kv``
+    [2 * heads * dim, rank] (the key rows of all heads, then the value rows) makes every head's keys
+    and values in float, which enter the attention in two bfloat16 parts.  ``q``: [tokens, heads,
+    dim + rot], rotated; writes the groups' rows of ``out`` [tokens, heads * dim], times the sigmoid
+    of ``gate`` (float [tokens, heads]) where given."""
+    _need_cuda(q, cache, block_table, w_kv, out, gate)
+    assert out.is_contiguous() and out.dtype == torch.bfloat16 and cache.is_contiguous()
+    assert tuple(w_kv.shape) == (2 * heads * dim, rank) and w_kv.is_contiguous()
+    assert gate is None or (gate.dtype == torch.float32 and gate.stride(1) == 1)
+    dev, entry = q.device, lib.get("attention_prompt_tc")
+    starts = [0]
+    for n in ctx.q_lens:
+        starts.append(starts[-1] + n)
+    for first, count, keys in groups:
+        q_lens = ctx.q_lens[first:first + count]
+        rows = torch.empty((keys, rank + rot), dtype=torch.bfloat16, device=dev)
+        check(entry.mstar_latent_gather(
+            cache.data_ptr(), block_table.data_ptr(), block_table.stride(0), ctx.qo_indptr.data_ptr(),
+            ctx.kv_len.data_ptr(), rows.data_ptr(), first, count, max(ctx.kv_lens[first:first + count]),
+            window, page_size, rank + rot, _stream()), "latent_gather")
+        made = linear(rows[:, :rank], w_kv, out_dtype=torch.float32)
+        parts = torch.empty((keys, heads, 4 * dim), dtype=torch.bfloat16, device=dev)
+        check(entry.mstar_latent_split(made.data_ptr(), parts.data_ptr(), keys, heads, dim, _stream()),
+              "latent_split")
+        del made
+        ctas = heads * -(-max(q_lens) // PROMPT_ROWS) * count
+        splits = prompt_splits(ctas, min(max(ctx.kv_lens[first:first + count]),
+                                         window + max(q_lens) if window else 1 << 30), num_sms(dev))
+        scratch = None
+        if splits > 1:
+            scratch = torch.empty(q.shape[0] * heads * splits * (dim + 2), dtype=torch.float32, device=dev)
+        code = entry.mstar_latent_attention_prompt(
+            q.data_ptr(), q.stride(0), q.stride(1), q.shape[0], parts.data_ptr(), rows.data_ptr(), keys,
+            out.data_ptr(), ctx.qo_indptr.data_ptr(), ctx.kv_len.data_ptr(), first, count, max(q_lens),
+            starts[first], starts[first + count] - starts[first], heads, dim, rank, rot, window,
+            float(scale), splits, _ptr(scratch), _ptr(gate), gate.stride(0) if gate is not None else 0,
+            tcgen05_error_word(dev).data_ptr(), _stream())
+        if code < 0:
+            raise KernelError(f"latent prompt attention refuses heads={heads}, dim={dim}, rank={rank}, "
+                              f"rot={rot} (code {code})")
+        check(code, "latent_attention_prompt")
+        if splits > 1:
+            lib.add_launches(1)                 # the merge kernel
+
+
 _BMM_INTO_ROWS: dict = {}       # out dtype -> False once the library refused the strided output
 
 
@@ -1465,6 +1557,32 @@ def sink_attention_splits(entries: int, max_q_len: int, num_heads: int, num_kv_h
     return max(1, min(room // ctas, -(-max_keys // 64) // 2, 64))
 
 
+# query rows of an entry (token x head of the group) from which on the tcgen05 prompt kernel takes an
+# attention with options, and its rows a CTA and keys a tile
+PROMPT_MIN_ROWS = 64
+PROMPT_ROWS, PROMPT_KEYS = 128, 64
+
+
+def prompt_splits(ctas: int, max_keys: int, sms: int) -> int:
+    """Among how many CTAs the keys of a row tile of the tcgen05 prompt kernels are shared: one where
+    the row tiles fill half of the GPU, else as many as still give every CTA an SM of its own, a split
+    keeping at least four tiles of keys (the partials and their merge cost some 5 us, four tiles)."""
+    if 2 * ctas > sms:
+        return 1
+    return max(1, min(sms // max(ctas, 1), -(-max_keys // PROMPT_KEYS) // 4, 32))
+
+
+def _sink_prompt_map(q: torch.Tensor, kv_cache: torch.Tensor, ctx, num_heads: int, num_kv_heads: int,
+                     head_dim: int, v_dim: int, page_size: int):
+    """The cache's tensor map where the tcgen05 prompt kernel takes the call, else None."""
+    group = num_heads // num_kv_heads
+    if (head_dim != v_dim or head_dim not in (64, 128) or kv_cache.dim() != 5 or group > PROMPT_ROWS
+            or page_size not in TMA_PAGE_SIZES or ctx.max_q_len * group <= PROMPT_MIN_ROWS
+            or q.data_ptr() % 16 or q.stride(0) % 8 or os.environ.get("MSTAR_SINK_ATTENTION") == "mma"):
+        return None
+    return kv_tensor_map(kv_cache)
+
+
 def sink_attention(q: torch.Tensor, kv_cache: torch.Tensor, block_table, token_req, cache_pos,
                    num_heads: int, num_kv_heads: int, head_dim: int, v_dim: int, page_size: int,
                    window: int, keep_first: int, scale: float, ctx=None, gate=None,
@@ -1482,8 +1600,9 @@ def sink_attention(q: torch.Tensor, kv_cache: torch.Tensor, block_table, token_r
     ``bias``: float [heads], added to the capped scores.  ``sigmoid``: the weight of a visible
     key is the sigmoid of its score, nothing is normalised.  bfloat16 with sizes that are multiples of 8
     up to 256 and a step context (``ctx``: entries, their token ranges and lengths) runs on
-    the tensor cores (MSTAR_SINK_ATTENTION=generic: never); everything else, float32
-    included, on the CUDA cores."""
+    the tensor cores (MSTAR_SINK_ATTENTION=generic: never): prompt portions with keys and values of 64
+    or 128 on tcgen05 (MSTAR_SINK_ATTENTION=mma: never), the rest on mma.sync; everything else,
+    float32 included, on the CUDA cores."""
     _need_cuda(q, kv_cache, block_table, token_req, cache_pos, gate)
     assert q.is_contiguous() and kv_cache.is_contiguous() and kv_cache.dtype == q.dtype
     tokens = q.shape[0]
@@ -1508,6 +1627,29 @@ def sink_attention(q: torch.Tensor, kv_cache: torch.Tensor, block_table, token_r
             max_keys = min(max_keys, window + keep_first + ctx.max_q_len)
         if chunk:
             max_keys = min(max_keys, chunk + ctx.max_q_len)
+        sms = num_sms(q.device)
+        kv_map = _sink_prompt_map(q, kv_cache, ctx, num_heads, num_kv_heads, head_dim, v_dim, page_size)
+        if kv_map is not None:
+            row_tiles = -(-ctx.max_q_len // (PROMPT_ROWS // (num_heads // num_kv_heads)))
+            splits = prompt_splits(row_tiles * num_kv_heads * ctx.num_entries, max_keys, sms)
+            scratch = None
+            if splits > 1:
+                scratch = torch.empty(tokens * num_heads * splits * (v_dim + 2), dtype=torch.float32,
+                                      device=q.device)
+            code = lib.get("attention_prompt_tc").mstar_sink_attention_prompt(
+                kv_map, q.data_ptr(), q.stride(0), out.data_ptr(), block_table.data_ptr(),
+                block_table.stride(0), ctx.qo_indptr.data_ptr(), ctx.kv_len.data_ptr(),
+                ctx.num_entries, tokens, ctx.max_q_len, num_heads, num_kv_heads, head_dim, page_size,
+                int(window or 0), int(keep_first), float(scale), splits, _ptr(scratch), _ptr(gate),
+                gate.stride(0) if gate is not None else 0, int(gate_features), cap, _ptr(sink),
+                int(chunk), int(sigmoid), _ptr(bias), tcgen05_error_word(q.device).data_ptr(), _stream())
+            if code < 0:
+                raise KernelError(f"prompt attention refuses heads={num_heads}, kv_heads={num_kv_heads}, "
+                                  f"head_dim={head_dim} (code {code})")
+            check(code, "sink_attention_prompt")
+            if splits > 1:
+                lib.add_launches(1)             # the merge kernel
+            return out
         splits = sink_attention_splits(ctx.num_entries, ctx.max_q_len, num_heads, num_kv_heads,
                                        max_keys, num_sms(q.device), wide=max(head_dim, v_dim))
         if chunk and splits == 1 and ctx.num_entries == 1 and min(chunk, ctx.max_kv_len) >= 1024:

@@ -46,6 +46,7 @@ LIBRARIES = {
     "routed_experts": ("cuda", ["routed_experts.cu"], []),
     "attention_sink": ("cuda", ["attention_sink.cu"], []),
     "attention_sink_tc": ("cuda", ["attention_sink_tc.cu"], []),
+    "attention_prompt_tc": ("cuda", ["attention_prompt_tc.cu"], []),
     "selective_scan": ("cuda", ["selective_scan.cu"], []),
     "gated_delta": ("cuda", ["gated_delta.cu"], []),
     "hyper": ("cuda", ["hyper.cu"], []),

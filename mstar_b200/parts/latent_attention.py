@@ -9,6 +9,10 @@ attention kernel then reads the same rows for every head, in prompts and in deco
 One product gives the queries, the down-projection and the output gate.  Scores,
 probabilities and the weighted sum are float; the folded query is kept in float as well.
 
+Prompt portions in bfloat16 take the other form where the sizes allow it: with many queries a key it
+costs less to make every head's keys and values from the latents (float, in two bfloat16 parts) than
+to score and sum whole latents a head.
+
 Options of the spec: queries through a normed latent of their own (the first product then
 gives that latent instead of the queries, and a second one the queries), rotary pairs
 interleaved or split in halves, a gate per feature or one a head, and a layer without a
@@ -84,6 +88,10 @@ class LatentAttention:
         # per head: [rank, qk_dim] rows so that a = q @ uk_t[h]^T, and [v_dim, rank]
         self.uk_t = params["uk.weight"].view(h, spec.qk_dim, spec.kv_rank).transpose(1, 2).contiguous()
         self.uv = params["uv.weight"].view(h, spec.v_dim, spec.kv_rank)
+        # all heads' key rows, then their value rows: prompts make both in one product
+        self.w_kv = None
+        if runtime.dtype == torch.bfloat16 and spec.qk_dim == spec.v_dim:
+            self.w_kv = torch.cat([params["uk.weight"], params["uv.weight"]])
         half = p.rotary_dim // 2
         self.freq = torch.tensor([p.theta ** (-(2.0 * i) / p.rotary_dim) for i in range(half)],
                                  dtype=torch.float64, device=runtime.device)
@@ -116,22 +124,41 @@ class LatentAttention:
             ops.latent_fill(q, None, None, self.freq, cache=cache.kv, **fill)
             gate = proj[:, s.q_rank + down:]
         q = q.view(-1, h, per_head)
-        q_abs = ops.linear_per_head(q[:, :, :s.qk_dim], self.uk_t, out_dtype=torch.float32)
-        lat = ops.latent_attention(q_abs, q[:, :, s.qk_dim:], cache.kv, cache.block_table,
-                                   ctx.token_req, ctx.cache_pos, h, s.kv_rank, s.rot_dim,
-                                   cache.page_size, s.window or 0, self.scale,
-                                   max_keys=ctx.max_kv_len, entries=ctx.num_entries)
-        if s.gated and s.gate_per_head:
-            # one gate a head commutes with the head's value up-projection
-            lat = ops.head_gate_mul(lat.view(-1, h * s.kv_rank), gate, h,
-                                    out_dtype=self.runtime.dtype).view(-1, h, s.kv_rank)
+        groups = []
+        if self.w_kv is not None and ops.latent_prompt_takes(q, cache.kv, s.qk_dim, s.v_dim, s.kv_rank,
+                                                             s.rot_dim):
+            groups = ops.latent_prompt_groups(ctx.q_lens, ctx.kv_lens, s.window or 0, h * s.v_dim, ctx.num_decode)
+        if groups:
+            y = q.new_empty((ctx.num_tokens, h * s.v_dim))
+            ops.latent_attention_prompt(q, cache.kv, cache.block_table, ctx, groups, self.w_kv, h, s.qk_dim,
+                                        s.kv_rank, s.rot_dim, cache.page_size, s.window or 0, self.scale, y,
+                                        gate=gate if s.gated and s.gate_per_head else None)
+            if ctx.num_decode:
+                y[:ctx.num_decode] = self._folded(q, gate, ctx, cache, ctx.num_decode, ctx.num_decode)
         else:
-            lat = ops.convert(lat, self.runtime.dtype)
-        y = ops.linear_per_head(lat, self.uv)
-        y = y.view(-1, h * s.v_dim)
+            y = self._folded(q, gate, ctx, cache, ctx.num_tokens, ctx.num_entries)
         if s.gated and not s.gate_per_head:
             ops.sigmoid_gate_mul(y, gate)
         return ops.linear(y, self.w_out, static_weights=True)
+
+    def _folded(self, q, gate, ctx: StepContext, cache: LayerCache, tokens: int, entries: int):
+        """The first ``tokens`` tokens (of the first ``entries`` entries) over the latents themselves,
+        [tokens, heads * v_dim], with the gate a head if there is one."""
+        s = self.spec
+        h = s.num_heads
+        q = q[:tokens]
+        q_abs = ops.linear_per_head(q[:, :, :s.qk_dim], self.uk_t, out_dtype=torch.float32)
+        lat = ops.latent_attention(q_abs, q[:, :, s.qk_dim:], cache.kv, cache.block_table,
+                                   ctx.token_req[:tokens], ctx.cache_pos[:tokens], h, s.kv_rank, s.rot_dim,
+                                   cache.page_size, s.window or 0, self.scale,
+                                   max_keys=ctx.max_kv_len, entries=entries)
+        if s.gated and s.gate_per_head:
+            # one gate a head commutes with the head's value up-projection
+            lat = ops.head_gate_mul(lat.view(-1, h * s.kv_rank), gate[:tokens], h,
+                                    out_dtype=self.runtime.dtype).view(-1, h, s.kv_rank)
+        else:
+            lat = ops.convert(lat, self.runtime.dtype)
+        return ops.linear_per_head(lat, self.uv).view(-1, h * s.v_dim)
 
 
 register_part("mixer", "latent_attention", LatentAttention)

@@ -1,0 +1,185 @@
+"""The tcgen05 prompt attention with probabilities in two bfloat16 parts, paged and latent form, against
+attention in double precision over the same bfloat16 numbers.  Pages that no token sees hold NaN."""
+import math
+
+import pytest
+import torch
+
+from test_gpu_kernels import DEV, rnd
+
+pytestmark = pytest.mark.gpu
+
+
+def i32(values):
+    return torch.tensor(values, dtype=torch.int32, device=DEV)
+
+
+def batch(lens_q, lens_kv):
+    from mstar_b200.parts.base import StepContext
+
+    starts = [0]
+    for n in lens_q:
+        starts.append(starts[-1] + n)
+    pos = i32([k - q + i for q, k in zip(lens_q, lens_kv) for i in range(q)])
+    return StepContext(num_tokens=starts[-1], num_entries=len(lens_q),
+                       token_req=i32([r for r, q in enumerate(lens_q) for _ in range(q)]), positions=pos,
+                       cache_pos=pos, qo_indptr=i32(starts), kv_len=i32(lens_kv), slots=i32(list(range(len(lens_q)))),
+                       q_lens=list(lens_q), kv_lens=list(lens_kv), max_q_len=max(lens_q), max_kv_len=max(lens_kv),
+                       num_decode=0), starts
+
+
+def visible(q, kv, window, keep_first, chunk):
+    i = torch.arange(kv - q, kv, device=DEV)[:, None]
+    j = torch.arange(kv, device=DEV)[None]
+    see = j <= i
+    if chunk:
+        return see & (j >= i // chunk * chunk)
+    return see & ((i - j < window) | (j < keep_first)) if window else see
+
+
+def paged(lens_q, lens_kv, page, lowest, make_row, shape, keep_first=0):
+    """A cache of NaN whose visible rows (keys from lowest[r] on and the first keep_first) are filled;
+    pages without a visible key are -1 in the table."""
+    width = -(-max(lens_kv) // page)
+    order = torch.randperm(len(lens_q) * width + 2, generator=torch.Generator().manual_seed(3)).tolist()
+    cache = torch.full((len(order), *shape), float("nan"), dtype=torch.bfloat16, device=DEV)
+    table = torch.full((len(lens_q), width), -1, dtype=torch.int32)
+    for r, n in enumerate(lens_kv):
+        for key in range(n):
+            if key >= lowest[r] or key < keep_first:
+                table[r, key // page] = pg = order[r * width + key // page]
+                make_row(cache, pg, key % page, r, key)
+    return cache, table.to(DEV)
+
+
+FORMS = {
+    "sink": dict(softcap=30.0, sink=True, gate="feature"),
+    "window": dict(window=70, softcap=20.0),
+    "keep_first": dict(window=70, keep_first=5, gate="head"),
+    "keep_many": dict(window=33, keep_first=66),
+    "chunk": dict(chunk=96, sigmoid=True, softcap=30.0, bias=True, gate="feature"),
+    "sigmoid": dict(sigmoid=True, bias=True),
+    "plain": dict(bias=True),
+    "low_cap": dict(softcap=5.0, sink=True, window=100),        # scores past half of the cap
+    "high_cap": dict(softcap=60.0, bias=True),                  # a cap too high to be the reference maximum
+}
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("lens_q,lens_kv,nq,nkv,hd,page", [
+    ([130, 17], [130, 300], 4, 1, 64, 16),       # a row tile and one row more; keys shared among CTAs
+    ([50], [333], 6, 2, 128, 8),                 # a group of 3: 126 of 128 rows
+    ([300], [300], 1, 1, 128, 64),               # one head a group
+    ([40, 40, 64], [40, 200, 64], 16, 8, 64, 32)])
+def test_prompt_attention_with_options(form, lens_q, lens_kv, nq, nkv, hd, page, monkeypatch):
+    from mstar_b200 import ops
+
+    o = FORMS[form]
+    window, keep, chunk = o.get("window", 0), o.get("keep_first", 0), o.get("chunk", 0)
+    ctx, starts = batch(lens_q, lens_kv)
+    T, G, scale = starts[-1], nq // nkv, hd ** -0.5
+    q = rnd(T, nq * hd, dtype=torch.bfloat16, seed=1, scale=2.0)
+    ks = [rnd(n, nkv, hd, dtype=torch.bfloat16, seed=10 + r) for r, n in enumerate(lens_kv)]
+    vs = [rnd(n, nkv, hd, dtype=torch.bfloat16, seed=20 + r) for r, n in enumerate(lens_kv)]
+    see = [visible(a, n, window, keep, chunk) for a, n in zip(lens_q, lens_kv)]
+
+    def row(cache, pg, slot, r, key):
+        cache[pg, 0, :, slot], cache[pg, 1, :, slot] = ks[r][key], vs[r][key]
+
+    lowest = [max(0, n - a - window + 1) if window else (n - a) // chunk * chunk if chunk else 0
+              for a, n in zip(lens_q, lens_kv)]
+    cache, table = paged(lens_q, lens_kv, page, lowest, row, (2, nkv, page, hd), keep)
+    sink = rnd(nq, seed=5) if o.get("sink") else None
+    bias = rnd(nq, seed=6) if o.get("bias") else None
+    gate = None
+    if o.get("gate"):
+        gate = rnd(T, 8 + nq * (hd if o["gate"] == "feature" else 1), seed=7)[:, 8:]
+    args = (q, cache, table, ctx.token_req, ctx.cache_pos, nq, nkv, hd, hd, page, window, keep, scale)
+    kw = dict(ctx=ctx, gate=gate, softcap=o.get("softcap"), sink=sink, chunk=chunk,
+              sigmoid=bool(o.get("sigmoid")), bias=bias)
+    assert ops._sink_prompt_map(q, cache, ctx, nq, nkv, hd, hd, page) is not None
+    got = ops.sink_attention(*args, **kw)
+    monkeypatch.setattr(ops, "prompt_splits", lambda *a: 1)
+    alone = ops.sink_attention(*args, **kw)
+    monkeypatch.setattr(ops, "prompt_splits", lambda *a: 7)
+    shared = ops.sink_attention(*args, **kw)
+    ops.check_error_word(DEV)
+
+    want = torch.empty(T, nq, hd, dtype=torch.float64, device=DEV)
+    size = torch.empty_like(want)
+    for r, s in enumerate(see):
+        for h in range(nq):
+            at = slice(starts[r], starts[r + 1])
+            z = q.view(T, nq, hd)[at, h].double() @ ks[r][:, h // G].double().T * scale
+            if o.get("softcap"):
+                z = o["softcap"] * torch.tanh(z / o["softcap"])
+            if bias is not None:
+                z = z + bias[h].double()
+            if o.get("sigmoid"):
+                p = torch.sigmoid(z) * s
+            else:
+                z = z.masked_fill(~s, -math.inf)
+                if sink is not None:
+                    z = torch.cat([z, sink[h].double().expand(len(z), 1)], dim=1)
+                p = torch.softmax(z, dim=1)[:, :s.shape[1]]
+            want[at, h] = p @ vs[r][:, h // G].double()
+            size[at, h] = p @ vs[r][:, h // G].double().abs()
+    if gate is not None:
+        g = torch.sigmoid(gate.double()).reshape(T, nq, -1)
+        want, size = want * g, size * g
+    # the result's rounding to bfloat16, and what float scores (sums of hd products, then an
+    # exponential) and probabilities of 16 bits leave of the sum's terms
+    bound = 2 ** -8 * want.abs() + 2 ** -13 * size + 1e-6
+    for y in (got, alone, shared):
+        assert ((y.view(T, nq, hd).double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("window", [0, 70])
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("lens_q,lens_kv,heads,dim,rank,rot,page", [
+    ([130, 33], [130, 300], 3, 64, 32, 32, 16),
+    ([200], [1000], 2, 128, 64, 64, 8),
+    ([64, 64, 65], [64, 64, 200], 1, 128, 40, 8, 4)])
+def test_latent_prompt_attention(window, gated, lens_q, lens_kv, heads, dim, rank, rot, page, monkeypatch):
+    from mstar_b200 import ops
+
+    ctx, starts = batch(lens_q, lens_kv)
+    T, scale = starts[-1], (dim + rot) ** -0.5
+    q = rnd(T, heads, dim + rot, dtype=torch.bfloat16, seed=1)
+    rows = [rnd(n, rank + rot, dtype=torch.bfloat16, seed=10 + r) for r, n in enumerate(lens_kv)]
+    w_kv = rnd(2 * heads * dim, rank, dtype=torch.bfloat16, seed=2, scale=rank ** -0.5)
+    gate = rnd(T, heads + 3, seed=7)[:, 3:] if gated else None
+
+    def row(cache, pg, slot, r, key):
+        cache[pg, 0, 0, slot] = rows[r][key]
+
+    lowest = [max(0, n - a - window + 1) if window else 0 for a, n in zip(lens_q, lens_kv)]
+    cache, table = paged(lens_q, lens_kv, page, lowest, row, (1, 1, page, rank + rot))
+    assert ops.latent_prompt_takes(q, cache, dim, dim, rank, rot)
+    groups = ops.latent_prompt_groups(lens_q, lens_kv, window, heads * dim)
+    assert groups and sum(g[1] for g in groups) == len(lens_q)
+    want = torch.empty(T, heads, dim, dtype=torch.float64, device=DEV)
+    size = torch.empty_like(want)
+    wk, wv = w_kv.double().view(2, heads, dim, rank)
+    for r in range(len(lens_q)):
+        see = visible(lens_q[r], lens_kv[r], window, 0, 0)
+        at = slice(starts[r], starts[r + 1])
+        lat, kr = rows[r][:, :rank].double(), rows[r][:, rank:].double()
+        for h in range(heads):
+            qd = q[at, h].double()
+            z = (qd[:, :dim] @ (lat @ wk[h].T).T + qd[:, dim:] @ kr.T) * scale
+            p = torch.softmax(z.masked_fill(~see, -math.inf), dim=1)
+            want[at, h], size[at, h] = p @ (lat @ wv[h].T), p @ (lat @ wv[h].T).abs()
+    if gated:
+        g = torch.sigmoid(gate.double())[:, :, None]
+        want, size = want * g, size * g
+    bound = 2 ** -8 * want.abs() + 2 ** -13 * size + 1e-6
+    few = [(i, 1, ops.latent_prompt_groups([a], [n], window, heads * dim)[0][2]) for i, (a, n) in enumerate(zip(lens_q, lens_kv))]
+    for parts, splits in ((groups, None), (few, None), (groups, 1), (groups, 5)):
+        if splits:
+            monkeypatch.setattr(ops, "prompt_splits", lambda *a, n=splits: n)
+        out = torch.full((T, heads * dim), float("nan"), dtype=torch.bfloat16, device=DEV)
+        ops.latent_attention_prompt(q, cache, table, ctx, parts, w_kv, heads, dim, rank, rot, page, window, scale,
+                                    out, gate=gate)
+        ops.check_error_word(DEV)
+        assert ((out.view(T, heads, dim).double() - want).abs() <= bound).all()
