@@ -248,11 +248,12 @@ sample_kernel(const float* __restrict__ logits, int ld, int vocab,
 // What a row takes is latencies: passes over a CTA's logits, cluster barriers, histogram atomics.  So
 // two CTAs share an SM (keys and exponentials are made again where they are needed instead of kept:
 // 95 KB a CTA at 157 k logits instead of 189), the first pass over the keys makes the first
-// histogram and the mass as well, histogram entries are two 32-bit words (a 64-bit atomic on shared
+// histogram and the mass as well, later passes make the keys of those logits only that can lie in the
+// bin in question, histogram entries are two 32-bit words (a 64-bit atomic on shared
 // memory is a loop; the upper word is touched only on a carry or by a large mass), and a histogram is
 // summed over the cluster by all eight CTAs, a slice of the bins each.  157 k logits with temperature,
-// top-p and a repetition penalty: 121 us for 64 rows; with one CTA an SM and
-// the histograms added into rank 0 by remote atomics 61 us for up to 18 and 294 us for 64.
+// top-p and a repetition penalty: 108 us for 64 rows (121 with every key made in every pass); with one
+// CTA an SM and the histograms added into rank 0 by remote atomics 61 us for up to 18 and 294 us for 64.
 #define CS_CLUSTER 8
 #define CS_THREADS 512
 #define CS_BINS 2048
@@ -483,6 +484,16 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
         return q >= 4294967295.0 ? 0xffffffffu : (unsigned)q;
     };
     auto mass_of = [&](float v) { return cs_fixed(expf((v - vmax) * inv_temp)); };
+    // Logits that surely have smaller (below lo) or larger (above hi) keys than first .. last, so that
+    // only logits between them need their key: the bounds lie a whole key outside (the products in
+    // double are off by 2^-20 keys at most) and are rounded outwards.
+    float lo = -INFINITY, hi = INFINITY;
+    auto band = [&](unsigned first, unsigned last) {
+        if (spread == 0.0) return;
+        const double step = 1.0 / spread;
+        lo = __double2float_rd((double)vmin + ((double)first - 1.0) * step);
+        hi = __double2float_ru((double)vmin + ((double)last + 2.0) * step);
+    };
     const float p = top_p != nullptr ? top_p[row] : 1.f;
     const int k = top_k != nullptr ? top_k[row] : 0;
     const bool choose_k = k > 0 && k < vocab;
@@ -500,24 +511,31 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
             const int shift = 32 - decided - bits;
             if (round > 0) cs_clear(hist);
             for (int i = tid; i < n; i += CS_THREADS) {
-                const unsigned key = key_of(sv[i]);
+                const float v = sv[i];
+                if (v < lo || v > hi) continue;
+                const unsigned key = key_of(v);
                 if (decided == 0 || (key >> (32 - decided)) == prefix)
                     cs_add(hist, (key >> shift) & ((1u << bits) - 1u), 1ull);
             }
             const int bin = cs_pick_bin(cluster, rank, hist, scratch, slot, result, (unsigned long long)k, above);
             prefix = (prefix << bits) | (unsigned)bin;
             decided += bits;
+            band(prefix << shift, (prefix << shift) + ((1u << shift) - 1u));
         }
         tau = prefix;
-        for (int i = tid; i < n; i += CS_THREADS)
-            if (key_of(sv[i]) >= tau) mass += mass_of(sv[i]);
+        for (int i = tid; i < n; i += CS_THREADS) {
+            const float v = sv[i];
+            if (!(v < lo) && (v > hi || key_of(v) >= tau)) mass += mass_of(v);
+        }
+        lo = -INFINITY;                     // top-p walks the kept ones anew
+        hi = INFINITY;
     } else {
         first_made = p < 1.f;
 #pragma unroll 2
         for (int i = tid; i < n; i += CS_THREADS) {
             const unsigned long long m = mass_of(sv[i]);
             mass += m;
-            if (first_made) cs_add(hist, key_of(sv[i]) >> 21, m);
+            if (first_made && m != 0ull) cs_add(hist, key_of(sv[i]) >> 21, m);
         }
     }
     unsigned long long all[CS_CLUSTER];
@@ -540,21 +558,26 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
                 cs_clear(hist);
 #pragma unroll 2
                 for (int i = tid; i < n; i += CS_THREADS) {
-                    const unsigned key = key_of(sv[i]);
+                    const float v = sv[i];
+                    if (v < lo || v > hi) continue;
+                    const unsigned key = key_of(v);
                     if (key >= tau && (decided == 0 || (key >> (32 - decided)) == prefix))
-                        cs_add(hist, (key >> shift) & ((1u << bits) - 1u), mass_of(sv[i]));
+                        cs_add(hist, (key >> shift) & ((1u << bits) - 1u), mass_of(v));
                 }
             }
             const int bin = cs_pick_bin(cluster, rank, hist, scratch, slot, result, need > 0ull ? need : 1ull, above);
             prefix = (prefix << bits) | (unsigned)bin;
             decided += bits;
+            band(prefix << shift, (prefix << shift) + ((1u << shift) - 1u));
         }
         if (prefix > tau) {
             tau = prefix;
             mass = 0ull;
 #pragma unroll 2
-            for (int i = tid; i < n; i += CS_THREADS)
-                if (key_of(sv[i]) >= tau) mass += mass_of(sv[i]);
+            for (int i = tid; i < n; i += CS_THREADS) {
+                const float v = sv[i];
+                if (!(v < lo) && (v > hi || key_of(v) >= tau)) mass += mass_of(v);
+            }
             mass = cs_block_sum(mass, scratch);
             cs_gather(cluster, mass, slot, all);
             total = 0ull;
@@ -564,6 +587,9 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
     }
 
     // ---- inverse-CDF draw over the kept tokens in index order (exact integer prefix sums)
+    lo = -INFINITY;
+    hi = INFINITY;
+    band(tau, tau);
     unsigned c[4];
     const unsigned long long sd = seed != nullptr ? (unsigned long long)seed[row] : 0ull;
     const unsigned long long of = offset != nullptr ? (unsigned long long)offset[row] : 0ull;
@@ -580,8 +606,9 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
         const int per = (n + CS_THREADS - 1) / CS_THREADS;
         const int begin = min(tid * per, n), end = min(begin + per, n);
         unsigned long long mine = 0ull;
+        auto kept = [&](float v) { return !(v < lo) && (v > hi || key_of(v) >= tau); };
         for (int i = begin; i < end; ++i)
-            if (key_of(sv[i]) >= tau) mine += mass_of(sv[i]);
+            if (kept(sv[i])) mine += mass_of(sv[i]);
         // exclusive prefix of `mine` over the threads
         unsigned long long incl = mine;
 #pragma unroll
@@ -598,7 +625,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
             unsigned long long run = excl;
             int pick = amax;
             for (int i = begin; i < end; ++i) {
-                if (key_of(sv[i]) >= tau) {
+                if (kept(sv[i])) {
                     run += mass_of(sv[i]);
                     if (target < run) { pick = base + i; break; }
                 }
