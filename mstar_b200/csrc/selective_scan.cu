@@ -42,6 +42,10 @@ __global__ void conv_silu_kernel(const A* __restrict__ xz, int ld, const W* __re
     out[idx] = from_float<A>(silu_f(acc));
 }
 
+template <typename A> __device__ __forceinline__ float conv_silu_of(float v);
+template <> __device__ __forceinline__ float conv_silu_of<float>(float v) { return silu_f(v); }
+template <> __device__ __forceinline__ float conv_silu_of<bf16>(float v) { return silu_bf16(v); }
+
 // The same for 8 channels a thread with 16-byte accesses: weights transposed to float
 // [taps][inner], bias float; inner and ld multiples of 8.
 template <typename A>
@@ -68,8 +72,56 @@ __global__ void conv_silu_vec_kernel(const A* __restrict__ xz, int ld, const flo
         for (int i = 0; i < 8; ++i) acc[i] = fmaf(w[i], v[i], acc[i]);
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = silu_f(acc[i]);
+    for (int i = 0; i < 8; ++i) acc[i] = conv_silu_of<A>(acc[i]);
     store8(out + (size_t)t * inner + c, acc);
+}
+
+// For prompts, four taps: CS_RUN tokens a thread, so that the weights (twice the bytes of the rows) and
+// rows are read once for all of them.  Where these are of several entries each is done as above.
+// What counts is instructions: 2 x 1,024 tokens of 4,096 channels take 12.5 us, a token a thread with the
+// quotient in IEEE division 19.
+#define CS_RUN 4
+template <typename A>
+__global__ void __launch_bounds__(128)
+conv_silu_run_kernel(const A* __restrict__ xz, int ld, const float* __restrict__ wt, const float* __restrict__ bias,
+                     const int* __restrict__ token_req, const int* __restrict__ qo_indptr,
+                     const int* __restrict__ slots, const float* __restrict__ state, long long state_stride,
+                     A* __restrict__ out, int t_first, int t_end, int inner) {
+    xz = pdl_after(xz, pdl_wait());
+    const int first = t_first + blockIdx.y * CS_RUN, many = min(CS_RUN, t_end - first);
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+    if (c >= inner) return;
+    float w[4][8], b[8];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) load8(wt + (size_t)k * inner + c, w[k]);
+    load8(bias + c, b);
+    const int e0 = token_req[first];
+    const int step = token_req[first + many - 1] == e0 ? many : 1;
+    for (int t0 = first; t0 < first + many; t0 += step) {
+        const int e = token_req[t0], local = t0 - qo_indptr[e];
+        const float* past = state + (size_t)slots[e] * state_stride;       // [3][inner]
+        const A* row = xz + (size_t)t0 * ld + c;
+        float v[4][8];                           // the rows of the taps, row i of the portion at i % 4
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            if (local >= 3 - i) load8(row - (ptrdiff_t)(3 - i) * ld, v[i]);
+            else load8(past + (size_t)(local + i) * inner + c, v[i]);
+        }
+#pragma unroll
+        for (int t = 0; t < CS_RUN; ++t) {
+            if (t >= step) break;
+            load8(row + (size_t)t * ld, v[(t + 3) % 4]);
+            float acc[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                acc[i] = b[i];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) acc[i] = fmaf(w[k][i], v[(t + k) % 4][i], acc[i]);
+                acc[i] = conv_silu_of<A>(acc[i]);
+            }
+            store8(out + (size_t)(t0 + t) * inner + c, acc);
+        }
+    }
 }
 
 MSTAR_API int mstar_conv_silu_vec(const void* xz, int ld, const float* wt, const float* bias,
@@ -81,8 +133,24 @@ MSTAR_API int mstar_conv_silu_vec(const void* xz, int ld, const float* wt, const
     cudaStream_t s = (cudaStream_t)stream;
     const int lanes = inner / 8;
     const int threads = lanes >= 128 ? 128 : 32;
+    // several tokens a thread where that still gives every SM two blocks (4,096 channels: 512 tokens 12.3 us
+    // against 14.4, 128 tokens 10.2 against 10.3, 64 tokens 10.3 against 8.3)
+    const int columns = (lanes + threads - 1) / threads;
+    if (taps == 4 && (long long)((tokens + CS_RUN - 1) / CS_RUN) * columns >= 2LL * device_sm_count()) {
+        for (int t0 = 0; t0 < tokens; t0 += 65535 * CS_RUN) {
+            const int end = tokens - t0 < 65535 * CS_RUN ? tokens : t0 + 65535 * CS_RUN;
+            const dim3 blocks(columns, (end - t0 + CS_RUN - 1) / CS_RUN);
+            if (act_dtype == MSTAR_F32)
+                mstar_launch((conv_silu_run_kernel<float>), blocks, dim3(threads), 0, s, (const float*)xz, ld, wt,
+                             bias, token_req, qo_indptr, slots, state, state_stride, (float*)out, t0, end, inner);
+            else
+                mstar_launch((conv_silu_run_kernel<bf16>), blocks, dim3(threads), 0, s, (const bf16*)xz, ld, wt,
+                             bias, token_req, qo_indptr, slots, state, state_stride, (bf16*)out, t0, end, inner);
+        }
+        return launch_status();
+    }
     for (int t0 = 0; t0 < tokens; t0 += 65535) {
-        const dim3 blocks((lanes + threads - 1) / threads, tokens - t0 < 65535 ? tokens - t0 : 65535);
+        const dim3 blocks(columns, tokens - t0 < 65535 ? tokens - t0 : 65535);
         if (act_dtype == MSTAR_F32)
             mstar_launch((conv_silu_vec_kernel<float>), blocks, dim3(threads), 0, s, (const float*)xz,
                          ld, wt, bias, token_req, qo_indptr, slots, state, state_stride, (float*)out,

@@ -210,3 +210,33 @@ def test_selective_scan_of_long_portions(lens, inner, piece, dtype, monkeypatch)
         for j in range(taps - 1):
             row = xz[starts[e + 1] - (taps - 1) + j, :inner].float()
             assert torch.equal(state[e, j * inner:(j + 1) * inner], row)
+
+
+@pytest.mark.parametrize("lens,inner", [([1, 2, 3, 1700, 5, 6], 1032), ([2401], 64), ([3] * 800, 64)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_convolution_of_several_tokens_a_thread(lens, inner, dtype):
+    """Portions that begin and end inside a thread's tokens and a number of tokens it does not divide,
+    against the convolution in double precision."""
+    from mstar_b200 import ops
+
+    T, taps, N = sum(lens), 4, 16
+    xz, w, bias = rnd(T, 2 * inner, dtype=dtype, seed=1), rnd(inner, taps, dtype=dtype, seed=2), rnd(inner, dtype=dtype, seed=3)
+    state = rnd(len(lens), ops.selective_scan_state_size(inner, N, taps), seed=4)
+    starts = [0]
+    for n in lens:
+        starts.append(starts[-1] + n)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    req = torch.repeat_interleave(torch.arange(len(lens)), torch.tensor(lens)).to(torch.int32).to(DEV)
+    got = ops.conv_silu(xz, w, bias, req, i32(starts), i32(list(range(len(lens)))), state, inner, taps,
+                        weight_t=w.float().T.contiguous(), bias_f32=bias.float()).double()
+    for e in range(len(lens)):
+        x = torch.cat([state[e, :(taps - 1) * inner].view(taps - 1, inner), xz[starts[e]:starts[e + 1], :inner].float()]).double()
+        y, size = bias.double().expand(lens[e], inner), bias.double().abs().expand(lens[e], inner)
+        for k in range(taps):
+            y = y + w[:, k].double() * x[k:k + lens[e]]
+            size = size + (w[:, k].double() * x[k:k + lens[e]]).abs()
+        want = y * torch.sigmoid(y)
+        # five float sums whose errors the activation's slope (1.1 at most) passes on, an exponential and a quotient
+        # of 2 ulp each, and the result's rounding
+        off = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20
+        assert ((got[starts[e]:starts[e + 1]] - want).abs() <= off * want.abs() + 2 ** -21 * size).all()
