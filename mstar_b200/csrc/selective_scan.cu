@@ -10,6 +10,8 @@
 //
 // Step sizes, decays, their exponentials, the state and its sums are float for both
 // activation types; a channel's arithmetic does not depend on the rest of the batch.
+#include <type_traits>
+
 #include "common.cuh"
 #include "mma_util.cuh"
 
@@ -214,8 +216,9 @@ struct ScanArgs {
     float* piece_state;   // [entries][max_pieces][inner][n_state]
     float* piece_dt;      // [entries][max_pieces][inner]
     // W_dt dt_in of every token and channel, made by a product of its own [tokens][inner]
-    // (long portions), or nullptr: the kernel makes it from the staged rows
-    const float* dt_pre;
+    // (long portions), or nullptr: the kernel makes it from the staged rows.  Pass 1 of the kernel for
+    // 16 states leaves the step sizes made of it in its place.
+    float* dt_pre;
 };
 
 // A block takes one batch entry and SS_THREADS / LANES channels; LANES lanes share a channel:
@@ -307,7 +310,7 @@ selective_scan_kernel(const A* __restrict__ xc, const A* __restrict__ xz,
     float pf_x[(SS_TC * CH + SS_THREADS - 1) / SS_THREADS],
         pf_z[(SS_TC * CH + SS_THREADS - 1) / SS_THREADS],
         pf_d[(SS_TC * CH + SS_THREADS - 1) / SS_THREADS];
-    const float* dt_pre = pdl_after(a.dt_pre, waited);
+    const float* dt_pre = pdl_after((const float*)a.dt_pre, waited);
     auto fetch = [&](float* buf, int t0, int nt) {
         const float* src = proj + (size_t)(start + t0) * row;
         for (int i = tid; i < nt * row; i += SS_THREADS) cp_async_4(buf + i, src + i);
@@ -511,8 +514,10 @@ selective_scan_kernel(const A* __restrict__ xc, const A* __restrict__ xz,
 // state as it is.  The output sums of four tokens meet in one exchange among the lanes, each of which
 // then finishes one token.  Bound by the exponential (one ex2 per state and token: 30 us for 2,048 tokens x
 // 4,096 channels at 16 a cycle and SM) and by one warp a scheduler where channels are few.
-// 2 x 1,024 tokens, 4,096 channels, pieces of 128: 57 + 89 us for the two passes; the kernel above takes 203 us
-// each (a 4-byte copy for every number of the rows, two 4-byte loads of B and C a state, exp2f).
+// 2 x 1,024 tokens, 4,096 channels, pieces of 128: 45 + 63 us for the two passes (57 + 89 with the step sizes made
+// in both, the copies' addresses made anew for every chunk and every token asked for its place in it:
+// instructions took 82 % of the issue slots); the kernel above takes 203 us each (a 4-byte copy for every
+// number of the rows, two 4-byte loads of B and C a state, exp2f).
 #define SX_STAGES 3
 
 __device__ __forceinline__ unsigned long long sx_pack(float lo, float hi) {
@@ -561,7 +566,8 @@ selective_scan16_kernel(const A* __restrict__ xc, const A* __restrict__ xz, cons
     xc = pdl_after(xc, waited);
     xz = pdl_after(xz, waited);
     proj = pdl_after(proj, waited);
-    const float* dt_pre = pdl_after(a.dt_pre, waited);
+    const float* dt_pre = pdl_after((const float*)a.dt_pre, waited);
+    float* dt_made = pdl_after(a.dt_pre, waited);
     const int e_start = qo_indptr[e], e_tok = qo_indptr[e + 1] - e_start;
     const int pieces = PASS != 0 ? max(1, (e_tok + a.piece - 1) / a.piece) : 1;
     if (piece >= pieces || (PASS == 1 && piece == pieces - 1)) return;
@@ -571,22 +577,38 @@ selective_scan16_kernel(const A* __restrict__ xc, const A* __restrict__ xz, cons
     float* s_slot = slot + (size_t)(a.taps - 1) * a.inner + (size_t)c * 16 + 4 * sub;
     const int row = a.rank + 32;
 
-    auto fetch = [&](int t0) {
-        ScanStage<A>& st = stage[(t0 / SS_TC) % SX_STAGES];
-        const int nt = min(SS_TC, n_tok - t0);
-        constexpr int XQ = 32 * (int)sizeof(A) / 16;       // 16-byte pieces of a token's x (or z)
-        for (int i = tid; i < SS_TC * (16 + 2 * XQ); i += 128) {
-            const int k = i / (16 + 2 * XQ), q = i - k * (16 + 2 * XQ);
-            if (k >= nt) break;
-            const size_t t = (size_t)(start + t0 + k);
-            if (q < 8) cp_async_16(smem_u32(&st.bc[k][4 * q]), proj + t * row + a.rank + 4 * q, 16);
-            else if (q < 16) cp_async_16(smem_u32(&st.d[k][4 * (q - 8)]), dt_pre + t * a.inner + c0 + 4 * (q - 8), 16);
-            else if (q < 16 + XQ)
-                cp_async_16(smem_u32(st.x[k]) + 16 * (q - 16),
-                            reinterpret_cast<const char*>(xc + t * a.inner + c0) + 16 * (q - 16), 16);
-            else
-                cp_async_16(smem_u32(st.z[k]) + 16 * (q - 16 - XQ),
-                            reinterpret_cast<const char*>(xz + t * a.ld_xz + a.inner + c0) + 16 * (q - 16 - XQ), 16);
+    // A thread copies the same places of every chunk: 16-byte piece i = tid, tid + 128, .. of the chunk's
+    // tokens (8 pieces of [B | C], 8 of step sizes, XQ of x, XQ of z each); what moves on is the source.
+    constexpr int XQ = 32 * (int)sizeof(A) / 16, PER = 16 + 2 * XQ, ITEMS = SS_TC * PER / 128;
+    const char* from[ITEMS];
+    uint32_t step[ITEMS], to[ITEMS];
+#pragma unroll
+    for (int m = 0; m < ITEMS; ++m) {
+        const int i = tid + 128 * m, k = i / PER, q = i - k * PER;
+        const size_t t = (size_t)(start + k);
+        const ScanStage<A>* st = stage;
+        if (q < 8) {
+            from[m] = reinterpret_cast<const char*>(proj + t * row + a.rank + 4 * q);
+            step[m] = (uint32_t)row * SS_TC * sizeof(float);
+            to[m] = smem_u32(&st->bc[k][4 * q]);
+        } else if (q < 16) {
+            from[m] = reinterpret_cast<const char*>(dt_pre + t * a.inner + c0 + 4 * (q - 8));
+            step[m] = (uint32_t)a.inner * SS_TC * sizeof(float);
+            to[m] = smem_u32(&st->d[k][4 * (q - 8)]);
+        } else {
+            const bool is_x = q < 16 + XQ;
+            const int part = q - (is_x ? 16 : 16 + XQ);
+            from[m] = reinterpret_cast<const char*>(is_x ? xc + t * a.inner + c0 : xz + t * a.ld_xz + a.inner + c0) + 16 * part;
+            step[m] = (uint32_t)(is_x ? a.inner : a.ld_xz) * SS_TC * sizeof(A);
+            to[m] = smem_u32(is_x ? st->x[k] : st->z[k]) + 16 * part;
+        }
+    }
+    auto fetch = [&](int t0) {                    // chunks in order
+        const uint32_t at = (uint32_t)((t0 / SS_TC) % SX_STAGES * sizeof(ScanStage<A>));
+#pragma unroll
+        for (int m = 0; m < ITEMS; ++m) {
+            if (t0 + (tid + 128 * m) / PER < n_tok) cp_async_16(to[m] + at, from[m], 16);
+            from[m] += step[m];
         }
     };
 #pragma unroll
@@ -631,20 +653,26 @@ selective_scan16_kernel(const A* __restrict__ xc, const A* __restrict__ xz, cons
     float dt_sum = 0.f;
     const float bias = dt_bias[c], dsk = d_skip[c];
 
-    for (int t0 = 0; t0 < n_tok; t0 += SS_TC) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(SX_STAGES - 2) : "memory");
-        __syncthreads();            // the chunk is there, and the one before it is done with
-        if (t0 + (SX_STAGES - 1) * SS_TC < n_tok) fetch(t0 + (SX_STAGES - 1) * SS_TC);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        ScanStage<A>& st = stage[(t0 / SS_TC) % SX_STAGES];
-        const int nt = min(SS_TC, n_tok - t0);
-        // the softplus of a channel's step sizes is dealt out among its lanes
+    // The step sizes that pass 1 made lie where it found their products.
+    const bool made = PASS == 2 && piece < pieces - 1;
+
+    auto walk = [&](auto whole, ScanStage<A>& st, int t0, int nt) {
+        constexpr bool WHOLE = decltype(whole)::value;
+        if (!made || !WHOLE) {
+            // the softplus of a channel's step sizes is dealt out among its lanes
 #pragma unroll
-        for (int j = 0; j < SS_TC / 4; ++j) {
-            const int k = sub + 4 * j;
-            st.d[k][ch] = k < nt ? softplus_f(st.d[k][ch] + bias) : 0.f;
+            for (int j = 0; j < SS_TC / 4; ++j) {
+                const int k = sub + 4 * j;
+                float dt = 0.f;
+                if (WHOLE || k < nt) {
+                    dt = st.d[k][ch];
+                    if (!made) dt = softplus_f(dt + bias);
+                    if (PASS == 1) dt_made[(size_t)(start + t0 + k) * a.inner + c] = dt;
+                }
+                st.d[k][ch] = dt;
+            }
+            __syncwarp();
         }
-        __syncwarp();
 #pragma unroll
         for (int k0 = 0; k0 < SS_TC; k0 += 4) {
             unsigned long long da[4][2], db[4][2];
@@ -652,7 +680,8 @@ selective_scan16_kernel(const A* __restrict__ xc, const A* __restrict__ xz, cons
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
                 const int k = k0 + kk;
-                const float dt = st.d[k][ch], dx = k < nt ? dt * to_float(st.x[k][ch]) : 0.f;
+                const bool here = WHOLE || k < nt;
+                const float dt = st.d[k][ch], dx = here ? dt * to_float(st.x[k][ch]) : 0.f;
                 if (PASS == 1) dt_sum += dt;
                 const ulonglong2 B = *reinterpret_cast<const ulonglong2*>(&st.bc[k][4 * sub]);
                 const unsigned long long dt2 = sx_pack(dt, dt), dx2 = sx_pack(dx, dx);
@@ -660,7 +689,7 @@ selective_scan16_kernel(const A* __restrict__ xc, const A* __restrict__ xz, cons
                 for (int i = 0; i < 2; ++i) {
                     const unsigned long long z = sx_mul(dt2, An[i]);
                     da[kk][i] = sx_pack(sx_ex2(sx_lo(z)), sx_ex2(sx_hi(z)));
-                    db[kk][i] = k < nt ? sx_mul(dx2, i == 0 ? B.x : B.y) : 0ull;
+                    db[kk][i] = here ? sx_mul(dx2, i == 0 ? B.x : B.y) : 0ull;
                 }
             }
 #pragma unroll
@@ -680,11 +709,23 @@ selective_scan16_kernel(const A* __restrict__ xc, const A* __restrict__ xz, cons
                 const float r1 = (odd ? y[3] : y[2]) + __shfl_xor_sync(0xffffffffu, odd ? y[2] : y[3], 1);
                 const float sum = (high ? r1 : r0) + __shfl_xor_sync(0xffffffffu, high ? r0 : r1, 2);
                 const int k = k0 + sub;
-                if (k < nt)
+                if (WHOLE || k < nt)
                     out[(size_t)(start + t0 + k) * a.inner + c] = from_float<A>(
                         fmaf(dsk, to_float(st.x[k][ch]), sum) * sx_silu(to_float(st.z[k][ch]), A()));
             }
         }
+    };
+
+    for (int t0 = 0; t0 < n_tok; t0 += SS_TC) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(SX_STAGES - 2) : "memory");
+        __syncthreads();            // the chunk is there, and the one before it is done with
+        if (t0 + (SX_STAGES - 1) * SS_TC < n_tok) fetch(t0 + (SX_STAGES - 1) * SS_TC);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        ScanStage<A>& st = stage[(t0 / SS_TC) % SX_STAGES];
+        const int nt = min(SS_TC, n_tok - t0);
+        // whole chunks ask for no token's place in them
+        if (nt == SS_TC) walk(std::true_type(), st, t0, nt);
+        else walk(std::false_type(), st, t0, nt);
     }
     if (PASS == 1) {                           // this piece alone, for the pieces after it
         const size_t at = (size_t)e * a.max_pieces + piece;
@@ -733,14 +774,14 @@ static void launch_scan16(const void* xc, const void* xz, const float* proj, con
 // of the token chunk) that run side by side in two passes; max_pieces bounds the pieces of any
 // entry, piece_state is float scratch [entries, max_pieces, inner, n_state], piece_dt
 // [entries, max_pieces, inner].  dt_pre: nullptr, or float [tokens, inner] = dt_in W_dt^T made by
-// the caller.  Returns 0, a CUDA error code, or -1 when the shape is refused.
+// the caller (with pieces it may hold step sizes afterwards).  Returns 0, a CUDA error code, or -1 when the shape is refused.
 MSTAR_API int mstar_selective_scan(const void* xc, const void* xz, int ld_xz, const float* proj,
                                    const float* w_dt, const float* dt_bias, const float* a_neg,
                                    const float* d_skip, const int* qo_indptr, const int* slots,
                                    float* state, long long state_stride, void* out, int act_dtype,
                                    int entries, int inner, int n_state, int rank, int taps,
                                    int piece, int max_pieces, float* piece_state, float* piece_dt,
-                                   const float* dt_pre, void* stream) {
+                                   float* dt_pre, void* stream) {
     if (entries <= 0) return 0;
     if (inner <= 0 || n_state <= 0 || rank <= 0 || taps <= 0 || n_state > 256) return -1;
     if (piece < 0 || (piece > 0 && (max_pieces < 1 || piece_state == nullptr || piece_dt == nullptr)))
