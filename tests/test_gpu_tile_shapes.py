@@ -240,3 +240,19 @@ def test_convolution_of_several_tokens_a_thread(lens, inner, dtype):
         # of 2 ulp each, and the result's rounding
         off = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20
         assert ((got[starts[e]:starts[e + 1]] - want).abs() <= off * want.abs() + 2 ** -21 * size).all()
+
+
+@pytest.mark.parametrize("rows,hidden", [(2501, 1024), (1101, 2056), (901, 4096), (5001, 264)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("add", [False, True])
+def test_norm_of_many_rows_has_the_bits_of_the_norm_of_one(rows, hidden, dtype, add):
+    from mstar_b200 import ops
+
+    x, w = rnd(rows, hidden, seed=1), rnd(hidden, dtype=dtype, seed=2)
+    delta = rnd(rows, hidden, dtype=dtype, seed=3) if add else None
+    whole = x.clone()
+    got = ops.add_rmsnorm(whole, delta, w, 1e-6, dtype)
+    for r in list(range(0, rows, 97)) + [rows - 1]:
+        one = x[r:r + 1].clone()
+        y = ops.add_rmsnorm(one, delta[r:r + 1] if add else None, w, 1e-6, dtype)
+        assert torch.equal(y[0], got[r]) and torch.equal(one[0], whole[r])
