@@ -216,6 +216,127 @@ sink_prepare_kernel(const float* __restrict__ qkv, const W* __restrict__ bias,
     }
 }
 
+// The same without a convolution or a norm over all heads, for head sizes of up to 128 features: four
+// neighbouring features a lane (16-byte loads, a head's features in registers, the feature a rotation
+// needs by a shuffle) and the next head's loads on their way while this one is normed and rotated.  What
+// bounds it is the latency of those loads: 2,048 tokens of 16 + 4 + 4 heads of 128 take 16.7 us, a
+// feature at a time through shared memory 26.
+template <typename A, typename W>
+__global__ void __launch_bounds__(256)
+sink_prepare_vec_kernel(const float* __restrict__ qkv, const W* __restrict__ bias,
+                        const W* __restrict__ q_norm, const W* __restrict__ k_norm,
+                        const double* __restrict__ freq, const int* __restrict__ positions,
+                        const int* __restrict__ cache_pos, const int* __restrict__ token_req,
+                        const int* __restrict__ block_table, A* __restrict__ q_out,
+                        A* __restrict__ kv_cache, PrepArgs a) {
+    extern __shared__ __align__(16) float sm[];
+    const int half = a.rot / 2;
+    float* cs = sm;                            // [half] cosines, [half] sines
+    const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nwarps = blockDim.x >> 5, d = 4 * lane;
+    const int nheads = a.v_from_k ? a.nq + a.nkv : a.nq + 2 * a.nkv;
+    const int step = nwarps * gridDim.y;
+    const unsigned long long waited = pdl_wait();
+    qkv = pdl_after(qkv, waited);
+    const float* row = qkv + (size_t)t * a.row_stride;
+    auto load = [&](int h, float (&v)[4]) {    // the lane's features of head h
+        const bool value = h >= a.nq + a.nkv;
+        const int off = value ? (a.nq + a.nkv) * a.hd + (h - a.nq - a.nkv) * a.vd : h * a.hd;
+        v[0] = v[1] = v[2] = v[3] = 0.f;
+        if (h < nheads && d < (value ? a.vd : a.hd)) load4(row + off + d, v);
+    };
+    int h = blockIdx.y * nwarps + warp;
+    float next[4];
+    load(h, next);
+    const double pos = (double)positions[t];
+    for (int i = threadIdx.x; i < half; i += blockDim.x) {     // as above
+        double ang = pos * freq[i];
+        ang -= 6.283185307179586476925 * rint(ang * 0.15915494309189533577);
+        float s, c;
+        sincosf((float)ang, &s, &c);
+        cs[i] = c;
+        cs[half + i] = s;
+    }
+    const int key = cache_pos[t];
+    const int page = block_table[(size_t)token_req[t] * a.bt_stride + key / a.page_size];
+    const int slot = key % a.page_size;
+    A* page_keys = kv_cache + (size_t)page * a.nkv * a.page_size * (a.hd + a.vd);
+    A* page_values = page_keys + (size_t)a.nkv * a.page_size * a.hd;
+    float q_mult = 1.f;
+    if (a.temp_every > 0)
+        q_mult = 1.f + a.temp_coef * logf((float)((positions[t] + 1) / a.temp_every) + 1.f);
+    __syncthreads();
+    for (; h < nheads; h += step) {
+        float v[4] = {next[0], next[1], next[2], next[3]};
+        load(h + step, next);
+        if (h >= a.nq + a.nkv) {               // a value head: bias, then the page
+            const int g = h - a.nq - a.nkv;
+            if (d >= a.vd) continue;
+            if (bias != nullptr) {
+                float b[4];
+                load4(bias + (a.nq + a.nkv) * a.hd + g * a.vd + d, b);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] += b[i];
+            }
+            if (a.v_first != nullptr) {
+                float f[4];
+                load4(pdl_after(a.v_first, waited) + (size_t)t * a.v_first_stride + g * a.vd + d, f);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] = fmaf(a.v_lam, f[i], (1.f - a.v_lam) * v[i]);
+            }
+            store4(page_values + ((size_t)g * a.page_size + slot) * a.vd + d, v);
+            continue;
+        }
+        const bool is_q = h < a.nq, live = d < a.hd;
+        if (bias != nullptr && live) {
+            float b[4];
+            load4(bias + h * a.hd + d, b);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] += b[i];
+        }
+        if (!is_q && a.v_from_k && live)
+            store4(page_values + ((size_t)(h - a.nq) * a.page_size + slot) * a.vd + d, v);
+        const float mult = is_q ? q_mult : 1.f;
+        if (a.norm) {
+            const W* nw = is_q ? q_norm : k_norm;
+            float w[4] = {1.f, 1.f, 1.f, 1.f};
+            if (nw != nullptr && live) load4(nw + d, w);
+            const float ss = warp_sum(fmaf(v[0], v[0], v[1] * v[1]) + fmaf(v[2], v[2], v[3] * v[3]));
+            const float inv = rsqrtf(ss / (float)a.hd + a.eps);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = v[i] * inv * w[i] * mult;
+        } else if (mult != 1.f) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] *= mult;
+        }
+        if (a.interleaved) {
+#pragma unroll
+            for (int i = 0; i < 4; i += 2) {
+                if (d + i >= a.rot) continue;
+                const float c = cs[(d + i) / 2], s = cs[half + (d + i) / 2], x = v[i], y = v[i + 1];
+                v[i] = x * c - y * s;
+                v[i + 1] = y * c + x * s;
+            }
+        } else {
+            // feature d is rotated with d + half; a lane's four lie in one half (half is a multiple of 4)
+            const bool low = d < half, high = !low && d < a.rot;
+            const int with = low ? lane + half / 4 : high ? lane - half / 4 : lane;
+            float p[4], c[4], s[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) p[i] = __shfl_sync(0xffffffffu, v[i], with);
+            if (low || high) {
+                load4(cs + (low ? d : d - half), c);
+                load4(cs + half + (low ? d : d - half), s);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] = low ? v[i] * c[i] - p[i] * s[i] : v[i] * c[i] + p[i] * s[i];
+            }
+        }
+        if (live)
+            store4(is_q ? q_out + (size_t)t * a.q_stride_out + (size_t)h * a.hd + d
+                        : page_keys + ((size_t)(h - a.nq) * a.page_size + slot) * a.hd + d, v);
+    }
+}
+
 MSTAR_API int mstar_sink_prepare(const float* qkv, const void* bias, const void* q_norm,
                                  const void* k_norm, int weight_dtype, const double* freq,
                                  const int* positions, const int* cache_pos, const int* token_req,
@@ -252,11 +373,21 @@ MSTAR_API int mstar_sink_prepare(const float* qkv, const void* bias, const void*
         if (head_blocks > room) head_blocks = room;
         if (head_blocks < 1) head_blocks = 1;
     }
+    // four features a lane where every head and row is whole 16-byte pieces of floats
+    bool vec = taps == 0 && !norm_whole && hd % 4 == 0 && hd <= 128 && vd % 4 == 0 && vd <= 128 &&
+               (interleaved || rot % 8 == 0) && row_stride % 4 == 0 && v_first_stride % 4 == 0;
+    const void* ptrs[] = {qkv, bias, q_norm, k_norm, q_out, kv_cache, v_first};
+    for (const void* p : ptrs) vec = vec && (uintptr_t)p % 16 == 0;
 #define GO(A, W)                                                                                  \
-    mstar_launch((sink_prepare_kernel<A, W>), dim3(tokens, head_blocks), dim3(threads), smem, s, qkv, \
-                 (const W*)bias, (const W*)q_norm, (const W*)k_norm, freq, positions, cache_pos,  \
-                 token_req, block_table, (A*)q_out, (A*)kv_cache, (const W*)conv_q,               \
-                 (const W*)conv_k, qo_indptr, slots, state, a)
+    if (vec)                                                                                      \
+        mstar_launch((sink_prepare_vec_kernel<A, W>), dim3(tokens, head_blocks), dim3(threads),   \
+                     sizeof(float) * rot, s, qkv, (const W*)bias, (const W*)q_norm, (const W*)k_norm, freq, \
+                     positions, cache_pos, token_req, block_table, (A*)q_out, (A*)kv_cache, a);   \
+    else                                                                                          \
+        mstar_launch((sink_prepare_kernel<A, W>), dim3(tokens, head_blocks), dim3(threads), smem, s, qkv, \
+                     (const W*)bias, (const W*)q_norm, (const W*)k_norm, freq, positions, cache_pos, \
+                     token_req, block_table, (A*)q_out, (A*)kv_cache, (const W*)conv_q,           \
+                     (const W*)conv_k, qo_indptr, slots, state, a)
     if (act_dtype == MSTAR_F32) {
         if (weight_dtype == MSTAR_F32) { GO(float, float); } else { GO(float, bf16); }
     } else {

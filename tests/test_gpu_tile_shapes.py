@@ -256,3 +256,62 @@ def test_norm_of_many_rows_has_the_bits_of_the_norm_of_one(rows, hidden, dtype, 
         one = x[r:r + 1].clone()
         y = ops.add_rmsnorm(one, delta[r:r + 1] if add else None, w, 1e-6, dtype)
         assert torch.equal(y[0], got[r]) and torch.equal(one[0], whole[r])
+
+
+# the last one goes a feature at a time, the others four a lane
+@pytest.mark.parametrize("nq,nkv,hd,vd,rot,interleaved,norm,form", [
+    (16, 4, 128, 128, 128, False, True, "bias"), (3, 1, 20, 12, 16, False, True, "first"),
+    (9, 9, 64, 64, 6, True, False, "plain"), (4, 2, 100, 100, 8, False, True, "keys"),
+    (2, 2, 8, 128, 0, False, False, "bias"), (5, 1, 36, 20, 20, False, True, "bias")])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_attention_inputs_by_four_features(nq, nkv, hd, vd, rot, interleaved, norm, form, dtype):
+    """Bias, head norm, temperature, rotation and the cache's pages, against double precision."""
+    from mstar_b200 import ops
+
+    T, page, pages, eps = 37, 4, 12, 1e-6
+    keys = form == "keys"
+    qkv = rnd(T, (nq + nkv) * hd + (0 if keys else nkv * vd) + 4, seed=1)
+    width = qkv.shape[1] - 4
+    bias = rnd(width, seed=2) if form == "bias" else None
+    wq, wk = (rnd(hd, seed=3), rnd(hd, seed=4)) if norm else (None, None)
+    first = (rnd(T, nkv * vd, seed=5), 0.3) if form == "first" else None
+    freq = (10000.0 ** -(torch.arange(rot // 2, dtype=torch.float64) / max(rot // 2, 1))).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    table = torch.randperm(pages, generator=torch.Generator().manual_seed(0)).to(torch.int32).to(DEV)[None]
+    at = list(range(2, 2 + T))
+    cache = torch.zeros(pages, ops.sink_page_elements(nkv, page, hd, vd), dtype=dtype, device=DEV)
+    positions = [1000 + 7 * i for i in range(T)]
+    q = ops.sink_prepare(qkv, bias, wq, wk, freq, i32(positions), i32(at), i32([0] * T), table, cache, nq, nkv, hd, vd,
+                         rot, page, eps, dtype, value_from_key=keys, interleaved=interleaved, q_temp=(0.1, 64),
+                         first_values=first)
+    x = qkv[:, :width].double() + (bias.double() if bias is not None else 0.0)
+    heads, values = x[:, :(nq + nkv) * hd].view(T, nq + nkv, hd), x[:, (nq + nkv) * hd:].view(T, -1, vd)
+    if keys:
+        values = heads[:, nq:]
+    if first is not None:
+        values = 0.3 * first[0].double().view(T, nkv, vd) + 0.7 * values
+    if norm:
+        heads = heads * torch.rsqrt((heads * heads).mean(-1, keepdim=True) + eps)
+        heads = heads * torch.cat([wq.double().expand(nq, hd), wk.double().expand(nkv, hd)])
+    pos = torch.tensor(positions, dtype=torch.float64, device=DEV)
+    temp = 1 + 0.1 * torch.log(torch.floor((pos + 1) / 64) + 1)
+    heads = torch.cat([heads[:, :nq] * temp[:, None, None], heads[:, nq:]], dim=1)
+    want, partner = heads.clone(), torch.zeros_like(heads)
+    if rot:
+        c, s = (f(pos[:, None] * freq)[:, None] for f in (torch.cos, torch.sin))
+        lo = slice(0, rot, 2) if interleaved else slice(0, rot // 2)
+        hi = slice(1, rot, 2) if interleaved else slice(rot // 2, rot)
+        a, b = heads[:, :, lo], heads[:, :, hi]
+        want[:, :, lo], want[:, :, hi] = a * c - b * s, b * c + a * s
+        partner[:, :, lo], partner[:, :, hi] = b, a
+    # a feature and its partner, rounded a few times each on their way, times sines and cosines of angles that are
+    # right to 2e-7; and the result's rounding
+    off = 2.0 ** -8 if dtype == torch.bfloat16 else 0.0
+    bound = off * want.abs() + 2 ** -19 * (heads.abs() + partner.abs()) + 1e-6
+    assert ((q.view(T, nq, hd).double() - want[:, :nq]).abs() <= bound[:, :nq]).all()
+    for t in range(T):
+        row = cache[table[0, at[t] // page]].double()
+        k = row[:nkv * page * hd].view(nkv, page, hd)[:, at[t] % page]
+        v = row[nkv * page * hd:].view(nkv, page, vd)[:, at[t] % page]
+        assert ((k - want[t, nq:]).abs() <= bound[t, nq:]).all()
+        assert ((v - values[t]).abs() <= off * values[t].abs() + 2 ** -20 * (values[t].abs() + 4)).all()
