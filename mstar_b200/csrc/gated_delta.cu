@@ -703,11 +703,12 @@ __global__ void __launch_bounds__(256) delta_head_pieces_kernel(DeltaHeadArgs a)
 // dec(t, j) cannot be cut into a factor of t and one of j by a quotient.  It is cut at the start m of
 // token t's four: for j before m it is (g_m .. g_t) (g_{j+1} .. g_{m-1}), which makes the sum a plain product
 // of rows X_t = k_t g_m .. g_t and Y_j = k_j g_{j+1} .. g_{m-1} (24 rows for the three later fours), and within a
-// four the six rows W_tj = k_j g_{j+1} .. g_t are made as they are.  Thread (t, j) then takes its two products
-// by 16-byte loads; the rows are made a thread a channel.  (A warp a token j that walked on over t with
-// two warp sums each took 78 us for 2,048 tokens and 16 heads of 128; 56 us here.)
+// four the six rows W_tj = k_j g_{j+1} .. g_t are made as they are.  A thread a pair (t, j <= t) then takes its
+// two products by 16-byte loads; the rows are made a thread a channel.  Bound by shared loads and by how few
+// blocks an SM holds: 46 us for 2,048 tokens and 16 heads of 128 (56 with two blocks an SM and a thread
+// for the other pairs too; 78 for a warp a token j that walked on over t with two warp sums each).
 #define GK_ROWS(C) (3 * (C) + 1)            // decayed keys, decayed queries, keys on their way to the end, P_C
-__global__ void __launch_bounds__(256) delta_channel_pieces_kernel(DeltaHeadArgs a) {
+__global__ void __launch_bounds__(256, 3) delta_channel_pieces_kernel(DeltaHeadArgs a) {
     extern __shared__ __align__(16) float sm[];
     constexpr int C = GC_TOKENS;
     const int D = a.D, LD = D + 4;
@@ -804,10 +805,14 @@ __global__ void __launch_bounds__(256) delta_channel_pieces_kernel(DeltaHeadArgs
         }
     }
     __syncthreads();
-    {
-        const int t = tid >> 4, j = tid & 15, f = t >> 2;
+    if (tid < C * (C + 1) / 2) {
+        // pair tid of (0, 0), (1, 0), (1, 1), (2, 0), ..: the largest t with t (t + 1) / 2 <= tid
+        int t = 0;
+#pragma unroll
+        for (int x = 1; x < C; ++x) t += tid >= x * (x + 1) / 2;
+        const int j = tid - t * (t + 1) / 2, f = t >> 2;
         const bool near = (j >> 2) == f;         // in token t's own four
-        const float* right = j > t ? ks : j == t ? ks + t * LD
+        const float* right = j == t ? ks + t * LD
                              : near ? W + (6 * f + (t & 3) * ((t & 3) - 1) / 2 + (j & 3)) * LD
                                     : Y + (2 * (f - 1) * f + j) * LD;
         const float* left_k = (near ? ks : Xk) + t * LD;
@@ -824,7 +829,7 @@ __global__ void __launch_bounds__(256) delta_channel_pieces_kernel(DeltaHeadArgs
         }
         const float bt = t < here ? beta[(size_t)(start + base + t) * a.H + h] : 0.f;
         if (j < t) L[t * GH_LD + j] = bt * (a0 + a1);
-        if (j <= t) B[t * GH_LD + j] = b0 + b1;
+        B[t * GH_LD + j] = b0 + b1;
     }
     __syncthreads();
     if (tid < C) {
@@ -858,7 +863,8 @@ __device__ __forceinline__ void gh_bulk(float* dst, const float* src, uint32_t b
 //
 // CHANNEL: the rows hold the decays (P and dec are 1 in the matrices), the new state takes rows of its own,
 // and P_C is a row.  2,048 tokens, 16 heads of 128 x 128: 173 us (a scan that gave a warp a column and a lane a
-// token's dot products, every warp reading all of the piece's rows, took 430 us: shared loads).
+// token's dot products, every warp reading all of the piece's rows, took 430 us: shared loads, which bound
+// this one too: with eight warps and half the columns of S a thread, 195 us).
 template <int D, int COLS, bool CHANNEL>
 __global__ void __launch_bounds__(GH_THREADS, 2) delta_head_scan_kernel(DeltaHeadArgs a) {
     extern __shared__ __align__(16) float sm[];
