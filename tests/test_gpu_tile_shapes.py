@@ -315,3 +315,54 @@ def test_attention_inputs_by_four_features(nq, nkv, hd, vd, rot, interleaved, no
         v = row[nkv * page * hd:].view(nkv, page, vd)[:, at[t] % page]
         assert ((k - want[t, nq:]).abs() <= bound[t, nq:]).all()
         assert ((v - values[t]).abs() <= off * values[t].abs() + 2 ** -20 * (values[t].abs() + 4)).all()
+
+
+# the last two go a feature at a time (sizes; a view that starts off 16 bytes), the others four a thread
+@pytest.mark.parametrize("rank,rot,rot_dims,q_rank,heads,qk_dim,interleaved,off", [
+    (512, 64, 64, 1024, 16, 128, False, 0), (1024, 8, 8, 2048, 1, 4, True, 0), (20, 12, 8, 1028, 3, 16, True, 0),
+    (64, 40, 16, 4, 5, 20, False, 0), (30, 10, 6, 34, 3, 18, False, 0), (64, 16, 16, 64, 2, 16, True, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_latent_cache_fill_by_four_features(rank, rot, rot_dims, q_rank, heads, qk_dim, interleaved, off, dtype):
+    """Norms, rotation of the shared key part and of the queries, and the cache's rows, against double precision."""
+    from mstar_b200 import ops
+
+    T, page, pages, eps, per = 21, 4, 8, 1e-6, qk_dim + rot
+    proj = rnd(T, q_rank + rank + rot + 4, seed=1)[:, off:]
+    lat_q, dkv = proj[:, :q_rank], proj[:, q_rank:q_rank + rank + rot]
+    q = rnd(T, heads * per, dtype=dtype, seed=2)
+    wq, wk = rnd(q_rank, seed=3), rnd(rank, seed=4)
+    freq = (10000.0 ** -(torch.arange(rot_dims // 2, dtype=torch.float64) / (rot_dims // 2))).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    table = torch.randperm(pages, generator=torch.Generator().manual_seed(0)).to(torch.int32).to(DEV)[None]
+    cache = torch.zeros(pages, 1, 1, page, rank + rot, dtype=dtype, device=DEV)
+    positions = [5000 + 3 * i for i in range(T)]
+    rotated = q.clone()
+    got = ops.latent_fill(rotated, dkv, wk, freq, i32(positions), i32(list(range(3, 3 + T))), i32([0] * T), table, cache,
+                          heads, qk_dim, rot, rot_dims, rank, page, eps, interleaved=interleaved, q_latent=lat_q,
+                          q_latent_weight=wq)
+    angle = torch.tensor(positions, dtype=torch.float64, device=DEV)[:, None] * freq
+
+    def turned(x):
+        """[T, heads, rot], and the size of what its terms were"""
+        lo = slice(0, rot_dims, 2) if interleaved else slice(0, rot_dims // 2)
+        hi = slice(1, rot_dims, 2) if interleaved else slice(rot_dims // 2, rot_dims)
+        y, size, c, s = x.clone(), x.abs(), torch.cos(angle)[:, None], torch.sin(angle)[:, None]
+        y[:, :, lo], y[:, :, hi] = x[:, :, lo] * c - x[:, :, hi] * s, x[:, :, hi] * c + x[:, :, lo] * s
+        size[:, :, lo] = size[:, :, hi] = x[:, :, lo].abs() + x[:, :, hi].abs()
+        return y, size
+
+    # sums of squares and products of some four roundings each; and the result's rounding
+    end = 2.0 ** -8 if dtype == torch.bfloat16 else 0.0
+    close = lambda y, want, size: ((y.double() - want).abs() <= end * want.abs() + 2 ** -20 * size + 1e-9).all()
+    over = lambda x: x * torch.rsqrt((x * x).mean(-1, keepdim=True) + eps)
+    want = over(lat_q.double()) * wq.double()
+    assert close(got, want, want.abs())
+    x = q.double().view(T, heads, per)
+    y, size = turned(x[:, :, qk_dim:])
+    assert close(rotated.view(T, heads, per)[:, :, qk_dim:], y, size)
+    assert torch.equal(rotated.view(T, heads, per)[:, :, :qk_dim], q.view(T, heads, per)[:, :, :qk_dim])
+    lat = over(dkv[:, :rank].double()) * wk.double()
+    key, size = turned(dkv[:, None, rank:].double())
+    for t in range(T):
+        row = cache[table[0, (3 + t) // page], 0, 0, (3 + t) % page]
+        assert close(row[:rank], lat[t], lat[t].abs()) and close(row[rank:], key[t, 0], size[t, 0])
