@@ -251,9 +251,12 @@ sample_kernel(const float* __restrict__ logits, int ld, int vocab,
 // histogram and the mass as well, later passes make the keys of those logits only that can lie in the
 // bin in question, histogram entries are two 32-bit words (a 64-bit atomic on shared
 // memory is a loop; the upper word is touched only on a carry or by a large mass), and a histogram is
-// summed over the cluster by all eight CTAs, a slice of the bins each.  157 k logits with temperature,
-// top-p and a repetition penalty: 108 us for 64 rows (121 with every key made in every pass); with one
-// CTA an SM and the histograms added into rank 0 by remote atomics 61 us for up to 18 and 294 us for 64.
+// summed over the cluster by all eight CTAs, a slice of the bins each.  Where the first round's bin holds
+// few logits they decide by themselves, in a list (cs_pick_few), instead of two more rounds of three
+// cluster barriers; sums have shared words of their own, which spares the barriers behind their reads.
+// 157 k logits with temperature, top-p and a repetition penalty: 85 us for 64 rows (108 with three rounds, 121
+// with every key made in every pass); with one CTA an SM and the histograms added into rank 0 by remote
+// atomics 61 us for up to 18 and 294 us for 64.
 #define CS_CLUSTER 8
 #define CS_THREADS 512
 #define CS_BINS 2048
@@ -279,14 +282,13 @@ __device__ __forceinline__ unsigned long long cs_block_sum(unsigned long long v,
 }
 
 // One value per CTA -> the values of all CTAs of the cluster, in rank order.  `slot`: a u64
-// in this CTA's shared memory (the same variable in every CTA).
+// in this CTA's shared memory (the same variable in every CTA), which nothing else uses.
 __device__ __forceinline__ void cs_gather(cg::cluster_group& cluster, unsigned long long mine,
                                           unsigned long long* slot, unsigned long long (&all)[CS_CLUSTER]) {
     if (threadIdx.x == 0) slot[0] = mine;
     cluster.sync();
 #pragma unroll
     for (int r = 0; r < CS_CLUSTER; ++r) all[r] = *cluster.map_shared_rank(slot, r);
-    cluster.sync();          // nobody overwrites its slot before everybody has read it
 }
 
 // hist[0 .. CS_BINS): lower words, hist[CS_BINS ..): upper words of 64-bit sums.
@@ -363,6 +365,34 @@ __device__ __forceinline__ int cs_pick_bin(cg::cluster_group& cluster, int rank,
     return (int)result[0];
 }
 
+// The end of a search whose remaining candidates are few: CTA 0's list of them (CS_FEW keys, then as many
+// weights, where its histogram was; `count` have been offered, everybody's offers are in) -> the key
+// K with above + sum(weights of keys > K) below `need` and above + sum(weights of keys >= K) not, in every
+// CTA's `result`.  A thread a candidate.  False, for all CTAs alike, where the list was too short.
+#define CS_FEW CS_THREADS
+__device__ __forceinline__ bool cs_pick_few(cg::cluster_group& cluster, int rank, const unsigned* list,
+                                            unsigned* count, unsigned long long* result, unsigned long long need,
+                                            unsigned long long above) {
+    cluster.sync();                                 // all candidates are in the list
+    const unsigned n = *cluster.map_shared_rank(count, 0);
+    if (n > CS_FEW) return false;
+    if (rank == 0 && threadIdx.x < n) {
+        const unsigned long long* weight = reinterpret_cast<const unsigned long long*>(list + CS_FEW);
+        const unsigned key = list[threadIdx.x];
+        unsigned long long more = above, same = 0ull;
+        for (unsigned j = 0; j < n; ++j) {
+            const unsigned k = list[j];
+            const unsigned long long w = weight[j];
+            if (k > key) more += w;
+            else if (k == key) same += w;
+        }
+        if (more < need && more + same >= need)     // (candidates with the same key write the same)
+            for (int r = 0; r < CS_CLUSTER; ++r) *cluster.map_shared_rank(result, r) = (unsigned long long)key;
+    }
+    cluster.sync();                                 // the result has been written everywhere
+    return true;
+}
+
 __global__ void __cluster_dims__(CS_CLUSTER, 1, 1) __launch_bounds__(CS_THREADS, 2)
 sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int chunk,
                       const float* __restrict__ temperature, const int* __restrict__ top_k,
@@ -376,8 +406,9 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
     float* sv = reinterpret_cast<float*>(cs_smem);                  // penalised logits [chunk]
     unsigned* hist = reinterpret_cast<unsigned*>(sv + chunk);       // [2][CS_BINS]
     __shared__ unsigned long long scratch[32];
-    __shared__ unsigned long long slot[2];
+    __shared__ unsigned long long slot[2], sums[2];
     __shared__ unsigned long long result[2];
+    __shared__ unsigned few[2];                     // candidates offered to CTA 0's list: of top-k, of top-p
     __shared__ float best_v[32], low_v[32];
     __shared__ int best_i[32];
 
@@ -435,6 +466,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
         lowest = fminf(lowest, __shfl_xor_sync(0xffffffffu, lowest, o));
     }
     if (lane == 0) { best_v[warp] = bv; best_i[warp] = bi; low_v[warp] = lowest; }
+    if (tid < 2) few[tid] = 0u;
     cs_clear(hist);                                 // (its barrier also ends the writes above)
     if (warp == 0) {
         bv = lane < CS_THREADS / 32 ? best_v[lane] : -INFINITY;
@@ -463,17 +495,17 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
         top = other[0] > top ? other[0] : top;
         low_word = other[1] > low_word ? other[1] : low_word;
     }
-    cluster.sync();                                 // nobody overwrites its slot before everybody has read it
     const float vmax = from_ordered_bits((unsigned)(top >> 32));
     const int amax = 0x7fffffff - (int)(unsigned)(top & 0xffffffffu);
     const float vmin = fminf(from_ordered_bits(~(unsigned)low_word), vmax);
 
     const float temp = temperature[row];
-    if (temp <= 0.f) {                      // uniform over the cluster; all reads are done
+    if (temp <= 0.f) {                      // uniform over the cluster
         if (rank == 0 && tid == 0) {
             out[row] = amax;
             if (my_seen != nullptr) my_seen[amax] = 1;
         }
+        cluster.sync();                     // nobody leaves before everybody has read its slot
         return;
     }
     const float inv_temp = 1.f / temp;
@@ -491,8 +523,31 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
     auto band = [&](unsigned first, unsigned last) {
         if (spread == 0.0) return;
         const double step = 1.0 / spread;
-        lo = __double2float_rd((double)vmin + ((double)first - 1.0) * step);
+        lo = first == 0u ? -INFINITY : __double2float_rd((double)vmin + ((double)first - 1.0) * step);
         hi = __double2float_ru((double)vmin + ((double)last + 2.0) * step);
+    };
+    // After a search's first round: what is left of it among the logits whose keys start with `prefix`
+    // (and are at least tau), weighted by weight_of, by a list of them; false where they are too many.
+    unsigned tau = 0u;                      // selection key threshold: keep key(x) >= tau
+    auto finish_few = [&](unsigned* offered, unsigned prefix, unsigned long long need, unsigned long long above,
+                          auto weight_of) {
+        unsigned* list = cluster.map_shared_rank(hist, 0);
+        unsigned long long* weights = reinterpret_cast<unsigned long long*>(list + CS_FEW);
+        unsigned* place = cluster.map_shared_rank(offered, 0);
+        for (int i = tid; i < n; i += CS_THREADS) {
+            const float v = sv[i];
+            if (v < lo || v > hi) continue;
+            const unsigned key = key_of(v);
+            if (key < tau || (key >> 21) != prefix) continue;
+            const unsigned long long w = weight_of(v);
+            if (w == 0ull) continue;
+            const unsigned at = atomicAdd(place, 1u);
+            if (at < CS_FEW) {
+                list[at] = key;
+                weights[at] = w;
+            }
+        }
+        return cs_pick_few(cluster, rank, hist, offered, result, need, above);
     };
     const float p = top_p != nullptr ? top_p[row] : 1.f;
     const int k = top_k != nullptr ? top_k[row] : 0;
@@ -500,7 +555,6 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
     bool first_made = false;                // the first histogram of top-p is there
 
     // ---- top-k: tau = the k-th largest key, by radix selection on counts
-    unsigned tau = 0u;
     unsigned long long mass = 0ull;         // of the kept tokens
     if (choose_k) {
         unsigned prefix = 0u;
@@ -521,8 +575,13 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
             prefix = (prefix << bits) | (unsigned)bin;
             decided += bits;
             band(prefix << shift, (prefix << shift) + ((1u << shift) - 1u));
+            if (round == 0 && finish_few(few, prefix, (unsigned long long)k, above, [](float) { return 1ull; })) {
+                prefix = (unsigned)result[0];
+                break;
+            }
         }
         tau = prefix;
+        band(tau, tau);
         for (int i = tid; i < n; i += CS_THREADS) {
             const float v = sv[i];
             if (!(v < lo) && (v > hi || key_of(v) >= tau)) mass += mass_of(v);
@@ -540,7 +599,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
     }
     unsigned long long all[CS_CLUSTER];
     mass = cs_block_sum(mass, scratch);
-    cs_gather(cluster, mass, slot, all);
+    cs_gather(cluster, mass, sums, all);
     unsigned long long total = 0ull;
 #pragma unroll
     for (int r = 0; r < CS_CLUSTER; ++r) total += all[r];
@@ -548,6 +607,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
     // ---- top-p: the largest tau2 >= tau whose tokens (x >= tau2) hold p of that mass
     if (p < 1.f) {
         const unsigned long long need = (unsigned long long)((double)p * (double)total);
+        const unsigned long long at_least = need > 0ull ? need : 1ull;
         unsigned prefix = 0u;
         unsigned long long above = 0ull;
         int decided = 0;
@@ -565,13 +625,18 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
                         cs_add(hist, (key >> shift) & ((1u << bits) - 1u), mass_of(v));
                 }
             }
-            const int bin = cs_pick_bin(cluster, rank, hist, scratch, slot, result, need > 0ull ? need : 1ull, above);
+            const int bin = cs_pick_bin(cluster, rank, hist, scratch, slot, result, at_least, above);
             prefix = (prefix << bits) | (unsigned)bin;
             decided += bits;
             band(prefix << shift, (prefix << shift) + ((1u << shift) - 1u));
+            if (round == 0 && finish_few(few + 1, prefix, at_least, above, mass_of)) {
+                prefix = (unsigned)result[0];
+                break;
+            }
         }
         if (prefix > tau) {
             tau = prefix;
+            band(tau, tau);
             mass = 0ull;
 #pragma unroll 2
             for (int i = tid; i < n; i += CS_THREADS) {
@@ -579,12 +644,15 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
                 if (!(v < lo) && (v > hi || key_of(v) >= tau)) mass += mass_of(v);
             }
             mass = cs_block_sum(mass, scratch);
-            cs_gather(cluster, mass, slot, all);
+            cs_gather(cluster, mass, sums + 1, all);
             total = 0ull;
 #pragma unroll
             for (int r = 0; r < CS_CLUSTER; ++r) total += all[r];
         }
     }
+
+    // (no CTA leaves before everybody has read the last sums: the wait is at the end)
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
 
     // ---- inverse-CDF draw over the kept tokens in index order (exact integer prefix sums)
     lo = -INFINITY;
@@ -634,6 +702,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
             if (my_seen != nullptr) my_seen[pick] = 1;
         }
     }
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 
 static int cs_chunk(int vocab) { return ((vocab + CS_CLUSTER - 1) / CS_CLUSTER + 3) & ~3; }

@@ -366,3 +366,29 @@ def test_latent_cache_fill_by_four_features(rank, rot, rot_dims, q_rank, heads, 
     for t in range(T):
         row = cache[table[0, (3 + t) // page], 0, 0, (3 + t) % page]
         assert close(row[:rank], lat[t], lat[t].abs()) and close(row[rank:], key[t, 0], size[t, 0])
+
+
+@pytest.mark.parametrize("kind", ["spread", "crowded", "equal", "masked"])
+@pytest.mark.parametrize("opts", [dict(top_p=0.7), dict(top_k=700), dict(top_k=400, top_p=0.6), dict(top_k=5, top_p=0.99)])
+def test_sampling_thresholds_by_a_list_and_by_rounds(kind, opts):
+    """Few logits in the first round's bin (their list decides) and many (further rounds): a crowd beside one
+    far-off logit, ties, and rows of which little is left."""
+    import plain_llama as P
+    from test_gpu_kernels import draw
+
+    vocab, rows = 20003, 24
+    logits = rnd(1, vocab, seed=31, scale=2.0)
+    if kind == "crowded":
+        logits[0, 7] = -4000.0
+    elif kind == "equal":
+        logits[:] = 1.25
+    elif kind == "masked":
+        logits[0, torch.arange(vocab, device=DEV) % 61 != 0] = -float("inf")
+    seeds, offsets = [17] * rows, list(range(rows))
+    got = draw(logits.repeat(rows, 1).contiguous(), 0.8, seeds, offsets, **opts).tolist()
+    p = P.plain_sampling_distribution(logits[0].cpu(), 0.8, **opts)
+    cdf = torch.cumsum(p.double(), 0)
+    for r, tok in enumerate(got):
+        assert p[tok] > 0, f"row {r}: token {tok} is outside the kept set"
+        u = P.plain_uniform(seeds[r], offsets[r])
+        assert (cdf[tok - 1].item() if tok else 0.0) - 3e-4 <= u <= cdf[tok].item() + 3e-4, (r, tok, u)
