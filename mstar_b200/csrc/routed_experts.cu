@@ -398,6 +398,7 @@ MSTAR_API int mstar_experts_by_row(const void* x, const void* w_gate_up, const v
 #define GG_BN 256                 // accumulator columns of a tile
 #define GG_BK 64
 #define GG_STAGES 4
+#define GG_PART_ROWS 32           // rows of the weight boxes of a tile's part
 // the producer warp, the MMA warp, four epilogue warps and, where token rows are gathered, four more
 __host__ __device__ constexpr int gg_threads(bool gather) { return gather ? 320 : 192; }
 #define GG_STORE_LD 36            // floats between rows of an epilogue warp's 32 x 32 staging tile
@@ -521,7 +522,8 @@ struct GroupedArgs {
 template <int MODE>
 __global__ void __launch_bounds__(gg_threads(MODE != 0), 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                    const bf16* __restrict__ x, GroupedArgs a, int* __restrict__ error_word) {
+                    const __grid_constant__ CUtensorMap map_part, const bf16* __restrict__ x, GroupedArgs a,
+                    int* __restrict__ error_word) {
     constexpr bool GATED = MODE == 1, GATHER = MODE != 0;
     constexpr int OUT_COLS = GATED ? GG_BN / 2 : GG_BN;
     extern __shared__ unsigned char gg_smem[];
@@ -569,16 +571,35 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int* offsets = pdl_after(a.offsets, waited);
     const int total = *pdl_after(a.num_tiles, waited) * a.n_tiles;
     const int num_kb = (a.K + GG_BK - 1) / GG_BK;
+    // Rounds of a tile a CTA; the tiles of a last round that would leave half of the CTAs idle or more are
+    // cut into two or four parts along N (groups of some 256 rows have a third tile of a few rows as often as
+    // not: 320 tiles on 148 SMs, three rounds for 2.2 rounds of work; the layer of 2,048 tokens 183 -> 179 us).
+    // Unit u of this CTA: tile, columns per side and the first of them.
+    const int grid = (int)gridDim.x, rounds = total / grid, rem = total - rounds * grid;
+    const int parts = rem * 4 <= grid ? 4 : rem * 2 <= grid ? 2 : 1;
+    const int units = rounds + ((int)blockIdx.x < rem * parts ? 1 : 0);
+    struct Unit { int mt, n0, cols; };
+    auto unit = [&](int u) {
+        const bool last = u == rounds;
+        const int t = u * grid + (last ? (int)blockIdx.x / parts : (int)blockIdx.x);
+        Unit w;
+        w.mt = t / a.n_tiles;
+        w.cols = last ? OUT_COLS / parts : OUT_COLS;
+        w.n0 = (t - w.mt * a.n_tiles) * OUT_COLS + (last ? (int)blockIdx.x % parts * w.cols : 0);
+        return w;
+    };
 
     if (warp == 0) {
         if (lane == 0) {
             uint32_t it = 0;                            // k-blocks loaded so far, over all tiles
             bool ok = true;
-            for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-                const int mt = t / a.n_tiles, n0 = (t - mt * a.n_tiles) * OUT_COLS;
-                const int e = tile_expert[mt], p0 = tile_first[mt];
+            for (int u = 0; u < units && ok; ++u) {
+                const Unit w = unit(u);
+                const int e = tile_expert[w.mt], p0 = tile_first[w.mt];
                 // the expert's rows: gate rows n0.. and up rows N + n0.., or 256 rows from n0 on
-                const int w0 = e * (GATED ? 2 : 1) * a.N + n0, w1 = w0 + (GATED ? a.N : GG_BN / 2);
+                const int w0 = e * (GATED ? 2 : 1) * a.N + w.n0, w1 = w0 + (GATED ? a.N : GG_BN / 2);
+                const bool whole = w.cols == OUT_COLS;
+                const uint32_t b_bytes = (uint32_t)w.cols * (GATED ? 2 : 1) * GG_BK * 2;
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % GG_STAGES;
                     if (!mbar_wait(tc_smem(&empty_bar[s]), ((it / GG_STAGES) & 1u) ^ 1u)) {
@@ -589,10 +610,18 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     }
                     const uint32_t bar = tc_smem(&full_bar[s]);
                     const uint32_t at = tc_smem(tiles + (size_t)s * GG_STAGE_BYTES);
-                    mbar_expect_tx(bar, GATHER ? GG_STAGE_BYTES - GG_A_BYTES : GG_STAGE_BYTES);
+                    mbar_expect_tx(bar, b_bytes + (GATHER ? 0 : GG_A_BYTES));
                     if (!GATHER) tma_load_2d(at, &map_a, bar, kb * GG_BK, p0);
-                    tma_load_2d(at + GG_A_BYTES, &map_b, bar, kb * GG_BK, w0);
-                    tma_load_2d(at + GG_A_BYTES + GG_BN / 2 * GG_BK * 2, &map_b, bar, kb * GG_BK, w1);
+                    if (whole) {
+                        tma_load_2d(at + GG_A_BYTES, &map_b, bar, kb * GG_BK, w0);
+                        tma_load_2d(at + GG_A_BYTES + GG_BN / 2 * GG_BK * 2, &map_b, bar, kb * GG_BK, w1);
+                        continue;
+                    }
+                    for (int r = 0; r < w.cols; r += GG_PART_ROWS) {
+                        tma_load_2d(at + GG_A_BYTES + r * GG_BK * 2, &map_part, bar, kb * GG_BK, w0 + r);
+                        if (GATED)
+                            tma_load_2d(at + GG_A_BYTES + (w.cols + r) * GG_BK * 2, &map_part, bar, kb * GG_BK, w1 + r);
+                    }
                 }
                 if (*(volatile int*)&abort_flag) break;
             }
@@ -606,8 +635,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         };
         uint32_t it = 0;
         bool ok = true;
-        for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-            const int mt = t / a.n_tiles;
+        for (int u = 0; u < units && ok; ++u) {
+            const int mt = unit(u).mt;
             const int p0 = tile_first[mt], p_last = offsets[tile_expert[mt] + 1] - 1;
             const bf16* src[8];
 #pragma unroll
@@ -643,12 +672,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             for (uint32_t done = it > LAG ? it - LAG : 0; done < it; ++done) tell(done);
     } else if (warp == 1) {
         if (lane == 0) {
-            constexpr uint32_t idesc = instr_desc_bf16(GG_BM, GG_BN);
             uint32_t it = 0;
             int j = 0;                                  // tiles done by this CTA
             bool ok = true;
-            for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++j) {
+            for (int u = 0; u < units && ok; ++u, ++j) {
                 const int b = j & 1;
+                const uint32_t idesc = instr_desc_bf16(GG_BM, unit(u).cols * (GATED ? 2 : 1));
                 if (!mbar_wait(tc_smem(&acc_empty[b]), (((uint32_t)j >> 1) & 1u) ^ 1u)) {
                     atomicExch(error_word, 20);
                     abort_flag = 1;
@@ -679,10 +708,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     } else {
         const int quarter = warp & 3;                   // the TMEM lanes this warp may touch
         int j = 0;
-        for (int t = blockIdx.x; t < total; t += gridDim.x, ++j) {
+        for (int k = 0; k < units; ++k, ++j) {
             const int b = j & 1;
-            const int mt = t / a.n_tiles, n0 = (t - mt * a.n_tiles) * OUT_COLS;
-            const int e = tile_expert[mt], p = tile_first[mt] + quarter * 32 + lane;
+            const Unit w = unit(k);
+            const int n0 = w.n0, e = tile_expert[w.mt], p = tile_first[w.mt] + quarter * 32 + lane;
             const int p_end = offsets[e + 1];
             const bool valid = p < p_end;
             float wgt = 1.f;
@@ -699,12 +728,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             tc_fence_after_sync();
             const uint32_t tbase = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)b * GG_BN;
 #pragma unroll 1
-            for (int c0 = 0; c0 < OUT_COLS; c0 += 32) {
+            for (int c0 = 0; c0 < w.cols; c0 += 32) {
                 uint32_t r[32], u[32];
                 tc_ld32(tbase + (uint32_t)c0, r);
-                if (GATED) tc_ld32(tbase + (uint32_t)(c0 + GG_BN / 2), u);
+                if (GATED) tc_ld32(tbase + (uint32_t)(c0 + w.cols), u);
                 tc_wait_ld();
-                if (c0 + 32 == OUT_COLS) {              // the accumulator is free, the stores follow
+                if (c0 + 32 == w.cols) {              // the accumulator is free, the stores follow
                     tc_fence_before_sync();
                     __syncwarp();
                     if (lane == 0)
@@ -824,8 +853,8 @@ static int gg_make_map(CUtensorMap* map, const void* base, long long rows, int K
 }
 
 template <int MODE>
-static int launch_grouped(const CUtensorMap& ma, const CUtensorMap& mb, const void* x, GroupedArgs a, int max_row_tiles,
-                          int* error_word, cudaStream_t s) {
+static int launch_grouped(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mp, const void* x,
+                          GroupedArgs a, int max_row_tiles, int* error_word, cudaStream_t s) {
     constexpr size_t smem = (size_t)GG_STAGES * GG_STAGE_BYTES + 1024 +
                             (MODE == 0 ? 4 * 32 * GG_STORE_LD * sizeof(float) : 0);
     static bool configured = false;
@@ -837,10 +866,10 @@ static int launch_grouped(const CUtensorMap& ma, const CUtensorMap& mb, const vo
     }
     const int cols = MODE == 1 ? GG_BN / 2 : GG_BN;
     a.n_tiles = (a.N + cols - 1) / cols;
-    const long long most = (long long)max_row_tiles * a.n_tiles;
+    const long long most = (long long)max_row_tiles * a.n_tiles * 4;      // (a tile may be cut into four)
     const int sms = device_sm_count();
     mstar_launch((grouped_gemm_kernel<MODE>), dim3((unsigned)(most < sms ? most : sms)), dim3(gg_threads(MODE != 0)),
-                 smem, s, ma, mb, (const bf16*)x, a, error_word);
+                 smem, s, ma, mb, mp, (const bf16*)x, a, error_word);
     return launch_status();
 }
 
@@ -869,22 +898,24 @@ MSTAR_API int mstar_experts_grouped(const void* x, const void* w_gate_up, const 
     int* num_tiles = offsets + experts + 1;
     int* tile_expert = num_tiles + 1;
     int* tile_first = tile_expert + max_tiles;
-    CUtensorMap mgu, mact, mdn;
+    CUtensorMap mgu, mact, mdn, mgu_part, mdn_part;
     int rc = gg_make_map(&mgu, w_gate_up, (long long)real * (gated ? 2 : 1) * ff, width, GG_BN / 2);
     if (rc == 0) rc = gg_make_map(&mact, act, rows, ff, GG_BM);
     if (rc == 0) rc = gg_make_map(&mdn, w_down, (long long)real * width, ff, GG_BN / 2);
+    if (rc == 0) rc = gg_make_map(&mgu_part, w_gate_up, (long long)real * (gated ? 2 : 1) * ff, width, GG_PART_ROWS);
+    if (rc == 0) rc = gg_make_map(&mdn_part, w_down, (long long)real * width, ff, GG_PART_ROWS);
     if (rc != 0) return rc;
     mstar_launch(experts_sort_kernel, dim3(1), dim3(1024), 0, s, chosen, rows, experts, real, order, pos,
                  offsets, tile_expert, tile_first, num_tiles);
     GroupedArgs a{act, order, weight, offsets, tile_expert, tile_first, num_tiles, ff, width, top, 0,
                   scale_input, (int)(gated == 2), limit, alpha};
-    rc = gated ? launch_grouped<1>(mgu, mgu, x, a, max_tiles, error_word, s)
-               : launch_grouped<2>(mgu, mgu, x, a, max_tiles, error_word, s);
+    rc = gated ? launch_grouped<1>(mgu, mgu, mgu_part, x, a, max_tiles, error_word, s)
+               : launch_grouped<2>(mgu, mgu, mgu_part, x, a, max_tiles, error_word, s);
     if (rc != 0) return rc;
     a.out = y;
     a.N = width;
     a.K = ff;
-    rc = launch_grouped<0>(mact, mdn, nullptr, a, max_tiles, error_word, s);
+    rc = launch_grouped<0>(mact, mdn, mdn_part, nullptr, a, max_tiles, error_word, s);
     if (rc != 0) return rc;
     mstar_launch((experts_combine_kernel<bf16>), dim3(tokens), dim3(256), 0, s, (const float*)y, pos,
                  weight, (const bf16*)add, (bf16*)out, width, top, scale_input, chosen,

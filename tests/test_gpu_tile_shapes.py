@@ -65,6 +65,8 @@ def test_float_attention_of_portions_leaves_unseen_values_out():
     (300, 128, 264, 5, 1, 3, "silu", True),       # column tiles that end inside, identity experts
     (129, 264, 136, 3, 0, 1, "relu2", False),
     (771, 136, 136, 3, 0, 1, "silu", True),       # groups of a row tile and a few rows more
+    (5000, 264, 520, 3, 0, 1, "silu", False),     # a second round of tiles cut in two
+    (4200, 72, 1096, 3, 0, 1, "relu2", True),     # and in four
     (2100, 64, 16, 7, 2, 6, "clamped", False),    # more rows than the sort keeps in registers, top > 4
     (64, 64, 64, 40, 0, 1, "silu", True)])        # experts without rows
 def test_grouped_experts_at_the_borders_of_their_tiles(tokens, width, ff, experts, identity, top, form, on_input):
