@@ -10,17 +10,19 @@
 //            meet in dim + rot features and a probability and a value in dim, instead of the
 //            rank + rot and rank features of the folded form; rows are tokens of one head.
 //
-// Everything that was float in those kernels keeps 16 bits of mantissa or more on its way through
-// the tensor cores: a number is written as the sum of two bfloat16 parts (head and remainder) and the
-// parts' products meet in the float accumulator.  That is the probabilities of both forms (P = P0 +
-// P1, both times V) and, of the latent form, the keys (q K0 + q K1; the rotated key features and the
-// queries are bfloat16 numbers) and the values (P0 V0 + P0 V1 + P1 V0).
+// What is float in those kernels goes through the tensor cores in as many bfloat16 parts (a head and
+// remainders) as there, and the parts' products meet in the float accumulator: the probabilities of both
+// forms in three (24 bits: P = P0 + P1 + P2, all times V), and, of the latent form, the keys in two, as the
+// folded query (q K0 + q K1; the rotated key features and the queries are bfloat16 numbers).  The latent
+// form's values have two as well ((P0 + P1 + P2) V0 + (P0 + P1) V1; the folded form rounds its weighted sum
+// of latents to one).
 //
 // The CTA is that of attention_prefill_tc.cu: 128 rows, tiles of 64 keys, a key and a value producer
 // warp (TMA, two stages each), a warp that issues S = Q K^T a tile ahead into one of two buffers in
 // tensor memory, 128 softmax threads of a row each that write P over S, a warp that issues O += P V.
-// What differs: the two parts of P fill the whole of their S buffer (64 columns), each row masks by
-// its own range, scores pass the cap, and the tiles that hold keys no row of the CTA sees (before a
+// What differs: two parts of P fill the whole of their S buffer (64 columns), the third lies behind them
+// where the CTA's share of tensor memory has room (96 columns a buffer) and in shared memory where not
+// (keys and values of 128 in the paged form: two CTAs an SM), each row masks by its own range, scores pass the cap, and the tiles that hold keys no row of the CTA sees (before a
 // window, past the last key) have those keys' values zeroed in shared memory before the product, so
 // that what lies there, other requests' numbers or none, cannot reach a sum.
 //
@@ -29,10 +31,11 @@
 // in the error word.
 //
 // Bound, in the paged form with a cap, by the softmax warps' arithmetic (2,048 tokens with 16 / 4 heads
-// of 128: 59 us; 68 with tanh from the exponential unit alone instead of its series where scores are
-// small and with running maxima under a low cap; the mma.sync kernel 233), in the latent form by the
-// tensor pipe (26 us of products for 2,048 tokens and 16 heads of 128 + 64 where the kernel takes 52,
-// making the keys and values 28; the folded form on mma.sync, 3.4 times the work, 1,912).
+// of 128: 72 us; 59 with probabilities in two parts, which are 16 bits; the mma.sync kernel 233; tanh from
+// the exponential unit alone instead of its series where scores are small, and running maxima under a low
+// cap, cost 9 us), in the latent form by the tensor pipe (33 us of products for 2,048 tokens and 16 heads of
+// 128 + 64 where the kernel takes 61, and 52 with two parts; making the keys and values 28; the folded form
+// on mma.sync, 3.4 times the work, 1,912).
 #include <string.h>
 
 #include "attention_tc_util.cuh"
@@ -105,6 +108,13 @@ __device__ __forceinline__ pa_f2 pa_tanh2(pa_f2 z) {
     p = pa_fma2(u, p, c(-1.0 / 3.0));
     return pa_fma2(pa_mul2(z, u), p, z);
 }
+// Takes the bfloat16 heads off a pair of floats: returns them packed and leaves the remainders (exact).
+__device__ __forceinline__ uint32_t pa_take_part(pa_f2& x) {
+    const __nv_bfloat162 head2 = __floats2bfloat162_rn(pa_lo(x), pa_hi(x));
+    const uint32_t bits = *reinterpret_cast<const uint32_t*>(&head2);
+    x = pa_fma2(pa_pack(__uint_as_float(bits << 16), __uint_as_float(bits & 0xffff0000u)), pa_pack(-1.f, -1.f), x);
+    return bits;
+}
 __device__ __forceinline__ float pa_sigmoid(float g) { return 1.f / (1.f + expf(-g)); }
 
 // The latent form's keys lie request after request: those of entry e (of the launch) start at row
@@ -126,13 +136,19 @@ template <int HD, bool LATENT> struct PromptShape {
     static constexpr int KB = LATENT ? 2 * NB + 1 : NB;      // ... of a key: heads, remainders, rotated
     static constexpr int VB = LATENT ? 2 * NB : NB;          // ... of a value: heads, remainders
     static constexpr int Q_BYTES = QB * PA_ROWS * 128, K_BYTES = KB * PA_BLOCK, V_BYTES = VB * PA_BLOCK;
-    static constexpr int SMEM = Q_BYTES + 2 * (K_BYTES + V_BYTES) + 128;
-    // no more CTAs on an SM than its 512 TMEM columns serve (256 each)
+    // the third part of P: behind the others in tensor memory, or (one buffer) in shared memory
+    static constexpr bool P2_SMEM = !LATENT && HD == 128;
+    static constexpr int P_COLS = P2_SMEM ? 64 : 96;         // tensor-memory columns of an S / P buffer
+    static constexpr int TMEM_COLS = 2 * P_COLS + HD <= 256 ? 256 : 512;
+    static constexpr int P2_BYTES = P2_SMEM ? PA_ROWS * 128 : 0;
+    static constexpr int SMEM = Q_BYTES + 2 * (K_BYTES + V_BYTES) + P2_BYTES + 128;
+    // no more CTAs on an SM than its 512 TMEM columns serve (two of 256, or one of 512)
     static constexpr int SMEM_LAUNCH = SMEM < 77 * 1024 ? 77 * 1024 : SMEM;
+    static_assert(TMEM_COLS == 256 || SMEM_LAUNCH > 114 * 1024, "two CTAs would want more tensor memory than there is");
 };
 
 template <int HD, bool LATENT, bool CAP, bool SIGMOID>
-__global__ void __launch_bounds__(PA_THREADS)
+__global__ void __launch_bounds__(PA_THREADS, PromptShape<HD, LATENT>::TMEM_COLS == 256 ? 2 : 1)
 prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_constant__ CUtensorMap rot_map,
                         const __grid_constant__ CUtensorMap q_map, PromptArgs a, int* __restrict__ error_word) {
     using Shape = PromptShape<HD, LATENT>;
@@ -141,7 +157,8 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
     unsigned char* q_s = smem_dyn;
     unsigned char* k_s = q_s + Shape::Q_BYTES;          // [2 stages]
     unsigned char* v_s = k_s + 2 * Shape::K_BYTES;      // [2 stages]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(v_s + 2 * Shape::V_BYTES);
+    unsigned char* p2_s = v_s + 2 * Shape::V_BYTES;     // (the third part of P, where it lies here)
+    uint64_t* bars = reinterpret_cast<uint64_t*>(p2_s + Shape::P2_BYTES);
     // k_full[2], v_full[2]: a stage's copies have landed.  k_empty[2]: S of the stage's tile is done.
     // v_empty[2]: O += P V of the stage's tile is done.  s_full[2]: S of a tile is done.  p_ready[2]:
     // P of a tile is written (one arrival per softmax thread).  One phase per two tiles.
@@ -203,7 +220,7 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
     if (warp == 4) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          tc_smem(tmem_slot)),
-                     "r"(256u)
+                     "r"((uint32_t)Shape::TMEM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -211,8 +228,8 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
     __syncthreads();
     pt_fence_after();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t tmem_sp = tmem;                      // S / P: two buffers of 64 columns
-    const uint32_t tmem_o = tmem + 128;                 // O: HD columns
+    const uint32_t tmem_sp = tmem;                      // S / P: two buffers of P_COLS columns
+    const uint32_t tmem_o = tmem + 2 * Shape::P_COLS;   // O: HD columns
 
     if (warp == 5 || warp == 7) {
         // ------------------------------------------- TMA producers: warp 5 the keys, 7 the values
@@ -309,7 +326,7 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
                     const int qb = b < NB ? b : b < 2 * NB ? b - NB : NB;
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
-                        pt_mma(tmem_sp + (uint32_t)s * 64,
+                        pt_mma(tmem_sp + (uint32_t)s * Shape::P_COLS,
                                pt_desc(q_addr + (uint32_t)qb * (PA_ROWS * 128) + (uint32_t)kk * 32, 16, 1024),
                                pt_desc(k_addr + (uint32_t)b * PA_BLOCK + (uint32_t)kk * 32, 16, 1024), idesc_s,
                                (b | kk) != 0);
@@ -349,18 +366,21 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
             }
             if (lane == 0) {
                 pt_fence_after();
-                const uint32_t p0 = tmem_sp + (uint32_t)s * 64;
+                const uint32_t p0 = tmem_sp + (uint32_t)s * Shape::P_COLS;
                 // 4 k-steps of 16 keys (8 columns of packed P); V rows are keys, 8-key groups 1024 bytes
                 // apart, the 64-feature blocks 8192 bytes apart
 #pragma unroll
-                for (int part = 0; part < (LATENT ? 3 : 2); ++part) {   // P0 V0, P1 V0, P0 V1
-                    const uint32_t p = p0 + (part == 1 ? 32u : 0u);
-                    const uint32_t v = v_addr + (part == 2 ? (uint32_t)NB * PA_BLOCK : 0u);
+                for (int part = 0; part < (LATENT ? 5 : 3); ++part) {   // P0 V0, P1 V0, P2 V0, P0 V1, P1 V1
+                    const uint32_t p = p0 + (uint32_t)(part % 3) * 32;
+                    const uint32_t v = v_addr + (part >= 3 ? (uint32_t)NB * PA_BLOCK : 0u);
 #pragma unroll
-                    for (int kk = 0; kk < PA_KEYS / 16; ++kk)
-                        pt_mma_ts(tmem_o, p + (uint32_t)kk * 8,
-                                  pt_desc(v + (uint32_t)kk * 16 * 128, PA_BLOCK, 1024), idesc_o,
-                                  (j | part | kk) != 0);
+                    for (int kk = 0; kk < PA_KEYS / 16; ++kk) {
+                        const uint64_t vd = pt_desc(v + (uint32_t)kk * 16 * 128, PA_BLOCK, 1024);
+                        if (Shape::P2_SMEM && part == 2)
+                            pt_mma(tmem_o, pt_desc(tc_smem(p2_s) + (uint32_t)kk * 32, 16, 1024), vd, idesc_o, 1);
+                        else
+                            pt_mma_ts(tmem_o, p + (uint32_t)kk * 8, vd, idesc_o, (j | part | kk) != 0);
+                    }
                 }
                 pt_commit(v_empty + 8 * s);     // the values are consumed, O holds tiles 0..j
             }
@@ -388,7 +408,7 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
                 break;
             }
             pt_fence_after();
-            const uint32_t sp = tmem_sp + lane_off + (uint32_t)(j & 1) * 64;
+            const uint32_t sp = tmem_sp + lane_off + (uint32_t)(j & 1) * Shape::P_COLS;
             uint32_t s[2][32];
             pt_ld32(sp, s[0]);
             pt_ld32(sp + 32, s[1]);
@@ -458,36 +478,44 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
             }
             const float shift = CAP || SIGMOID ? -m : bias - m;
             pa_f2 sum2 = 0ull;
-            const pa_f2 unit2 = pa_pack(unit, unit), shift2 = pa_pack(shift, shift), minus = pa_pack(-1.f, -1.f);
-            // both parts of P over this row's S: columns 0..31 the heads, 32..63 the remainders; column c
-            // of each holds keys 2 c, 2 c + 1
-            uint32_t p0[32], p1[32];
+            const pa_f2 unit2 = pa_pack(unit, unit), shift2 = pa_pack(shift, shift);
+            // P over this row's S, 16 keys at a time: columns 0..31 the heads, 32..63 the remainders, 64..95 theirs
+            // (or a row of shared memory, below); column c of each holds keys 2 c, 2 c + 1
+            uint32_t p2[4][8];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                pa_f2 x = pa_pack(__uint_as_float(s[i >> 4][(2 * i) & 31]), __uint_as_float(s[i >> 4][(2 * i + 1) & 31]));
-                if (SIGMOID) {
-                    x = pa_pack(pa_rcp(1.f + pt_ex2(-pa_lo(x))), pa_rcp(1.f + pt_ex2(-pa_hi(x))));
-                } else {
-                    x = pa_fma2(x, unit2, shift2);
-                    x = pa_pack(pt_ex2(pa_lo(x)), pt_ex2(pa_hi(x)));
-                    sum2 = pa_add2(sum2, x);
+            for (int h = 0; h < 4; ++h) {
+                uint32_t p0[8], p1[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int k = 16 * (h & 1) + 2 * i;
+                    pa_f2 x = pa_pack(__uint_as_float(s[h >> 1][k]), __uint_as_float(s[h >> 1][k + 1]));
+                    if (SIGMOID) {
+                        x = pa_pack(pa_rcp(1.f + pt_ex2(-pa_lo(x))), pa_rcp(1.f + pt_ex2(-pa_hi(x))));
+                    } else {
+                        x = pa_fma2(x, unit2, shift2);
+                        x = pa_pack(pt_ex2(pa_lo(x)), pt_ex2(pa_hi(x)));
+                        sum2 = pa_add2(sum2, x);
+                    }
+                    p0[i] = pa_take_part(x);
+                    p1[i] = pa_take_part(x);
+                    p2[h][i] = pa_take_part(x);
                 }
-                const __nv_bfloat162 head2 = __floats2bfloat162_rn(pa_lo(x), pa_hi(x));
-                p0[i] = *reinterpret_cast<const uint32_t*>(&head2);
-                const pa_f2 rest = pa_fma2(pa_pack(__uint_as_float(p0[i] << 16), __uint_as_float(p0[i] & 0xffff0000u)),
-                                           minus, x);
-                const __nv_bfloat162 rest2 = __floats2bfloat162_rn(pa_lo(rest), pa_hi(rest));
-                p1[i] = *reinterpret_cast<const uint32_t*>(&rest2);
+                pt_st8(sp + 8 * h, p0);
+                pt_st8(sp + 32 + 8 * h, p1);
+                if (!Shape::P2_SMEM) pt_st8(sp + 64 + 8 * h, p2[h]);
             }
             l = l * alpha + (pa_lo(sum2) + pa_hi(sum2));
-            if (!SIGMOID && j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-                // O += P V of tile j-1 must be done before O is rescaled
+            const bool rescale = !SIGMOID && j > 0 && __any_sync(0xffffffffu, alpha != 1.f);
+            if (rescale || (Shape::P2_SMEM && j > 0)) {
+                // O += P V of tile j-1 must be done before O is rescaled, and has read the third part of its P
                 if (!pt_wait_warp(v_empty + 8 * ((j - 1) & 1), ((uint32_t)(j - 1) >> 1) & 1u)) {
                     if (lane == 0) atomicExch(error_word, 27);
                     ok = false;
                     break;
                 }
                 pt_fence_after();
+            }
+            if (rescale) {
 #pragma unroll 1
                 for (int c0 = 0; c0 < HD; c0 += 32) {
                     uint32_t o[32];
@@ -498,8 +526,15 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
                     pt_st32(tmem_o + lane_off + (uint32_t)c0, o);
                 }
             }
-            pt_st32(sp, p0);
-            pt_st32(sp + 32, p1);
+            if (Shape::P2_SMEM) {
+                // a row of 128 bytes, its 16-byte pieces where the 128-byte swizzle wants them
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    *reinterpret_cast<uint4*>(p2_s + r * 128 + ((c ^ (r & 7)) << 4)) =
+                        make_uint4(p2[c >> 1][4 * (c & 1)], p2[c >> 1][4 * (c & 1) + 1], p2[c >> 1][4 * (c & 1) + 2],
+                                   p2[c >> 1][4 * (c & 1) + 3]);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            }
             pt_wait_st();
             pt_fence_before();
             mbar_arrive(p_ready + 8 * (j & 1));
@@ -579,7 +614,9 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
     __syncthreads();
     if (warp == 4) {
         pt_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                     "r"((uint32_t)Shape::TMEM_COLS)
+                     : "memory");
     }
 }
 
@@ -707,7 +744,8 @@ MSTAR_API int mstar_sink_attention_prompt(const void* kv_map, const void* q, int
     a.cap_in = softcap > 0.f ? 2.f * 1.4426950408889634f * scale / softcap : 0.f;
     a.cap_log2e = softcap * 1.4426950408889634f;
     a.cap_z = softcap > 0.f ? scale / softcap : 0.f;
-    // probabilities then lie within 2^-2 cap of 1: far from what a float, and a remainder 2^-9 below it, hold
+    // probabilities then lie within 2^(-2 cap) of 1: far from what a float, and the remainders 2^-9 and 2^-18 below
+    // it, hold
     a.cap_bounds = softcap > 0.f && a.cap_log2e <= 48.f;
     if ((long long)a.row_tiles * nkv * splits > 2147483647LL) return -1;
     cudaStream_t s = (cudaStream_t)stream;

@@ -595,7 +595,7 @@ def tcgen05_error_word(device) -> torch.Tensor:
     1-3 tcgen05 GEMM (producer, MMA issuer, epilogue), 4 decode attention copies, 6-12 tcgen05
     prefill attention, 13-14 bulk-copy small-M GEMM, 15-17 swapped-operand tcgen05 GEMM, 18
     delta-rule scan in pieces, 19-21 grouped expert GEMM, 22-27 prompt attention with probabilities
-    in two parts; zero otherwise."""
+    in three parts; zero otherwise."""
     key = torch.device(device).index or 0
     if key not in _tc_error_words:
         _tc_error_words[key] = torch.zeros(1, dtype=torch.int32, device=device)
@@ -618,7 +618,7 @@ WAIT_CODES[18] = "delta-rule scan in pieces: a wait for a piece's rows"
 WAIT_CODES.update({19: "grouped expert GEMM: the producer waited for a free stage",
                    20: "grouped expert GEMM: the MMA issuer waited for operand tiles",
                    21: "grouped expert GEMM: the epilogue waited for an accumulator"})
-WAIT_CODES.update({c: "prompt attention with probabilities in two parts: a wait on one of its barriers "
+WAIT_CODES.update({c: "prompt attention with probabilities in three parts: a wait on one of its barriers "
                    "ran out" for c in range(22, 28)})
 WAIT_CODES.update({c: "tcgen05 prefill attention: a wait on one of its barriers ran out"
                    for c in range(6, 13)})

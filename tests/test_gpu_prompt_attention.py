@@ -1,4 +1,4 @@
-"""The tcgen05 prompt attention with probabilities in two bfloat16 parts, paged and latent form, against
+"""The tcgen05 prompt attention with probabilities in three bfloat16 parts, paged and latent form, against
 attention in double precision over the same bfloat16 numbers.  Pages that no token sees hold NaN."""
 import math
 
@@ -183,3 +183,88 @@ def test_latent_prompt_attention(window, gated, lens_q, lens_kv, heads, dim, ran
                                     out, gate=gate)
         ops.check_error_word(DEV)
         assert ((out.view(T, heads, dim).double() - want).abs() <= bound).all()
+
+
+def cancelling(p, seed, reserve=4):
+    """bfloat16 values [keys, probes] whose sums with the weights p [probes, keys] (double) nearly vanish: random
+    ones, then corrections by reserved keys, each of which leaves 2^-9 of what is left.  And the size of a sum
+    whose terms have independent errors: the root of the sum of their squares."""
+    v = rnd(p.shape[1], p.shape[0], dtype=torch.bfloat16, seed=seed)
+    rows = torch.arange(len(p), device=DEV)
+    spare = p.argsort(dim=1, descending=True)[:, 2:2 + reserve]     # keys with much weight
+    for i in range(reserve):
+        v[spare[:, i], rows] = 0
+    for i in range(reserve):
+        left = (p * v.double().T).sum(1)
+        v[spare[:, i], rows] = (-left / p[rows, spare[:, i]]).to(torch.bfloat16)
+    assert ((p * v.double().T).sum(1).abs() < 2 ** -26 * p.sum(1)).all()
+    return v, (p * v.double().T).square().sum(1).sqrt()
+
+
+# What is left of sums that vanish is the error of their terms.  That of a probability: the rounding of a base-2
+# exponent of at most 8 (two roundings of 2^-22 at most, times ln 2), the exponential's 2^-22: some 2^-22 in the
+# mean.  A third bfloat16 part leaves 2^-27 of it; without one the second part's rounding leaves 2^-18.8 in the mean.
+TERM = 2 ** -20.5
+
+
+@pytest.mark.parametrize("form", ["plain", "sink", "cap", "low_cap", "sigmoid"])
+@pytest.mark.parametrize("hd,splits", [(64, 1), (128, 1), (128, 3)])
+def test_probabilities_keep_24_bits(form, hd, splits, monkeypatch):
+    from mstar_b200 import ops
+
+    T, past, page = 40, 150, 16
+    N, scale, nq = T + past, hd ** -0.5, 2
+    ctx, _ = batch([T], [N])
+    q, k = rnd(T, nq * hd, dtype=torch.bfloat16, seed=1), rnd(N, hd, dtype=torch.bfloat16, seed=2)
+    cap = {"cap": 50.0, "low_cap": 10.0}.get(form)
+    sink = rnd(nq, seed=5) if form == "sink" else None
+    z = q.view(T, nq, hd)[:, 0].double() @ k.double().T * scale         # the probes: head 0, a feature a token
+    if cap:
+        z = cap * torch.tanh(z / cap)
+    p = torch.sigmoid(z) if form == "sigmoid" else torch.exp(z)
+    p = p * visible(T, N, 0, 0, 0)
+    v, size = cancelling(p, 3)
+    v = torch.cat([v, rnd(N, hd - T, dtype=torch.bfloat16, seed=4)], dim=1)
+    total = torch.ones_like(size) if form == "sigmoid" else p.sum(1) + (sink[0].double().exp() if sink is not None else 0)
+
+    def row(cache, pg, slot, r, key):
+        cache[pg, 0, 0, slot], cache[pg, 1, 0, slot] = k[key], v[key]
+
+    cache, table = paged([T], [N], page, [0], row, (2, 1, page, hd))
+    assert ops._sink_prompt_map(q, cache, ctx, nq, 1, hd, hd, page) is not None
+    monkeypatch.setattr(ops, "prompt_splits", lambda *a: splits)
+    got = ops.sink_attention(q, cache, table, ctx.token_req, ctx.cache_pos, nq, 1, hd, hd, page, 0, 0, scale, ctx=ctx,
+                             softcap=cap, sink=sink, sigmoid=form == "sigmoid")
+    ops.check_error_word(DEV)
+    left = got.view(T, nq, hd)[:, 0].double().diagonal(dim1=0, dim2=1) * total / size
+    assert left.square().mean().sqrt() < TERM
+
+
+@pytest.mark.parametrize("dim,splits", [(64, 1), (128, 1), (64, 3)])
+def test_latent_probabilities_keep_24_bits(dim, splits, monkeypatch):
+    """With up-projections that pick latents, keys and values are bfloat16 numbers and the probabilities the only
+    ones that are not."""
+    from mstar_b200 import ops
+
+    T, past, page, rank, rot = 40, 150, 16, 2 * dim, 32
+    N, scale = T + past, (dim + rot) ** -0.5
+    ctx, _ = batch([T], [N])
+    q = rnd(T, 1, dim + rot, dtype=torch.bfloat16, seed=1)
+    rows = rnd(N, rank + rot, dtype=torch.bfloat16, seed=2)
+    w_kv = torch.eye(2 * dim, dtype=torch.bfloat16, device=DEV)          # latents: the key's features, the value's
+    z = (q[:, 0, :dim].double() @ rows[:, :dim].double().T + q[:, 0, dim:].double() @ rows[:, rank:].double().T) * scale
+    p = torch.exp(z) * visible(T, N, 0, 0, 0)
+    v, size = cancelling(p, 3)
+    rows[:, dim:dim + T] = v
+
+    def row(cache, pg, slot, r, key):
+        cache[pg, 0, 0, slot] = rows[key]
+
+    cache, table = paged([T], [N], page, [0], row, (1, 1, page, rank + rot))
+    assert ops.latent_prompt_takes(q, cache, dim, dim, rank, rot)
+    monkeypatch.setattr(ops, "prompt_splits", lambda *a: splits)
+    out = torch.empty(T, dim, dtype=torch.bfloat16, device=DEV)
+    ops.latent_attention_prompt(q, cache, table, ctx, [(0, 1, N)], w_kv, 1, dim, rank, rot, page, 0, scale, out)
+    ops.check_error_word(DEV)
+    left = out.double().diagonal(dim1=0, dim2=1) * p.sum(1) / size
+    assert left.square().mean().sqrt() < TERM
