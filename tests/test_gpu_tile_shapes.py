@@ -174,6 +174,32 @@ def test_delta_rule_in_pieces_with_decays_per_channel(lens, heads, kv_heads, dim
     assert (end - S).abs().max() < 2 ** -24 * 64 * dim ** 0.5
 
 
+@pytest.mark.parametrize("head_decay", [False, True])
+@pytest.mark.parametrize("heads,dim,vdim", [(1, 32, 8), (2, 128, 40), (80, 64, 32)])     # 8 and 16 columns a block
+def test_delta_rule_in_pieces_leaves_later_values_out(head_decay, heads, dim, vdim):
+    """A value that is not finite reaches no earlier token's output, wherever it lies in its piece."""
+    from mstar_b200 import ops
+
+    T, taps = 70, 2
+    q, k = (torch.nn.functional.normalize(rnd(T, heads, dim, seed=s), dim=-1).view(T, -1) for s in (1, 2))
+    v, beta = rnd(T, heads * vdim, seed=3), torch.sigmoid(rnd(T, heads, seed=4))
+    decay = torch.sigmoid(rnd(T, heads * (1 if head_decay else dim), seed=5) + 3)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+
+    def run(values):
+        state = 0.3 * rnd(1, ops.gated_delta_state_size(heads, heads, dim, vdim, taps), seed=6)
+        return ops.delta_scan(q, k, values, beta, decay, i32([0, T]), i32([0]), state, 1, heads, heads, dim, vdim, taps,
+                              max_q_len=T)
+
+    want = run(v)
+    for t in (1, 7, 31, 34, 69):
+        bad = v.clone()
+        bad[t] = float("inf")
+        got = run(bad)
+        assert torch.equal(got[:t], want[:t]) and not torch.isfinite(got[t]).any()
+    ops.check_error_word(DEV)
+
+
 @pytest.mark.parametrize("lens,inner,piece", [([512, 7, 530], 64, "256"), ([600], 32, "0"), ([513], 96, "16")])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_selective_scan_of_long_portions(lens, inner, piece, dtype, monkeypatch):
