@@ -9,7 +9,9 @@
 //          y_c = sum_n S[c, n] C_n + D_c xc_c;  out = y * silu(z).
 //
 // Step sizes, decays, their exponentials, the state and its sums are float for both
-// activation types; a channel's arithmetic does not depend on the rest of the batch.
+// activation types.  A channel's arithmetic depends on its own portion and on whether the batch holds a
+// long portion (which has the step sizes' product made ahead and portions cut into pieces), on nothing
+// else of the batch: how a portion is cut follows from its own length.
 #include <type_traits>
 
 #include "common.cuh"
@@ -204,17 +206,27 @@ __device__ __forceinline__ void cp_async_all_done() {
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 }
 
+// Tokens of a piece where the kernel for 16 states cuts a portion of n tokens: some 16 pieces, by the
+// portion's own length alone, so that its sums do not depend on the batch (600 tokens of 2,048 channels:
+// 44 us in pieces of 64, 52 of 128; 2,048 of 4,096: 217 of 128, 223 and 226 of 64 and 256; 8,192: 809 of
+// 256, 832 of 128).
+__host__ __device__ __forceinline__ int scan_piece(int n) {
+    const int p = n / 16 / 64 * 64;
+    return p < 64 ? 64 : p > 256 ? 256 : p;
+}
+
 struct ScanArgs {
     int inner, n_state, rank, taps, ld_xz, entries;
     long long state_stride;
-    // a long portion is cut into pieces of `piece` tokens (0: not cut) that run side by side:
+    // a long portion is cut into pieces of `piece` tokens (0: not cut; below 0, in the kernel for 16 states:
+    // scan_piece of its own length) that run side by side:
     // pass 1 walks every piece but the last from a zero state and leaves its end state and the
     // sum of its step sizes in scratch (the recurrence is linear: the state after a piece is
     // exp(A sum dt) times the state before it, plus that end state); pass 2 starts every piece
     // from the state so joined and writes the outputs
     int piece, pass, max_pieces;
-    float* piece_state;   // [entries][max_pieces][inner][n_state]
-    float* piece_dt;      // [entries][max_pieces][inner]
+    float* piece_state;   // [entries][max_pieces][inner][n_state]; piece < 0: [tokens / 64 + entries][..]
+    float* piece_dt;      // [entries][max_pieces][inner]; likewise
     // W_dt dt_in of every token and channel, made by a product of its own [tokens][inner]
     // (long portions), or nullptr: the kernel makes it from the staged rows.  Pass 1 of the kernel for
     // 16 states leaves the step sizes made of it in its place.
@@ -569,10 +581,14 @@ selective_scan16_kernel(const A* __restrict__ xc, const A* __restrict__ xz, cons
     const float* dt_pre = pdl_after((const float*)a.dt_pre, waited);
     float* dt_made = pdl_after(a.dt_pre, waited);
     const int e_start = qo_indptr[e], e_tok = qo_indptr[e + 1] - e_start;
-    const int pieces = PASS != 0 ? max(1, (e_tok + a.piece - 1) / a.piece) : 1;
+    const int len = a.piece > 0 ? a.piece : scan_piece(e_tok);
+    // the scratch of the entry's first piece: entries take max_pieces each, or, cut by their own lengths, one
+    // for every started 64 tokens
+    const size_t at0 = a.piece > 0 ? (size_t)e * a.max_pieces : (size_t)(e_start / 64 + e);
+    const int pieces = PASS != 0 ? max(1, (e_tok + len - 1) / len) : 1;
     if (piece >= pieces || (PASS == 1 && piece == pieces - 1)) return;
-    const int start = e_start + (PASS != 0 ? piece * a.piece : 0);
-    const int n_tok = PASS != 0 ? min(a.piece, e_tok - piece * a.piece) : e_tok;
+    const int start = e_start + (PASS != 0 ? piece * len : 0);
+    const int n_tok = PASS != 0 ? min(len, e_tok - piece * len) : e_tok;
     float* slot = state + (size_t)slots[e] * a.state_stride;
     float* s_slot = slot + (size_t)(a.taps - 1) * a.inner + (size_t)c * 16 + 4 * sub;
     const int row = a.rank + 32;
@@ -627,7 +643,7 @@ selective_scan16_kernel(const A* __restrict__ xc, const A* __restrict__ xz, cons
     }
     // (the last piece puts the new state into the slot while others may not have started: pass 1
     // leaves a copy of the old one in the scratch entry of the last piece, which pass 2 reads)
-    float* kept = PASS != 0 ? a.piece_state + (((size_t)e * a.max_pieces + pieces - 1) * a.inner + c) * 16 + 4 * sub : nullptr;
+    float* kept = PASS != 0 ? a.piece_state + ((at0 + pieces - 1) * a.inner + c) * 16 + 4 * sub : nullptr;
     if (PASS == 1 && piece == 0) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) kept[i] = s_slot[i];
@@ -641,7 +657,7 @@ selective_scan16_kernel(const A* __restrict__ xc, const A* __restrict__ xz, cons
     }
     if (PASS == 2) {
         for (int j = 0; j < piece; ++j) {
-            const size_t at = (size_t)e * a.max_pieces + j;
+            const size_t at = at0 + j;
             const float sdt = a.piece_dt[at * a.inner + c];
             const float4 E = *reinterpret_cast<const float4*>(a.piece_state + (at * a.inner + c) * 16 + 4 * sub);
 #pragma unroll
@@ -728,7 +744,7 @@ selective_scan16_kernel(const A* __restrict__ xc, const A* __restrict__ xz, cons
         else walk(std::false_type(), st, t0, nt);
     }
     if (PASS == 1) {                           // this piece alone, for the pieces after it
-        const size_t at = (size_t)e * a.max_pieces + piece;
+        const size_t at = at0 + piece;
         *reinterpret_cast<float4*>(a.piece_state + (at * a.inner + c) * 16 + 4 * sub) =
             make_float4(sx_lo(S[0]), sx_hi(S[0]), sx_lo(S[1]), sx_hi(S[1]));
         if (sub == 0) a.piece_dt[at * a.inner + c] = dt_sum;
@@ -759,7 +775,7 @@ static void launch_scan16(const void* xc, const void* xz, const float* proj, con
     a.pass = PASS;                                                                                \
     mstar_launch((selective_scan16_kernel<A, PASS>), grid, dim3(128), 0, s, (const A*)xc, (const A*)xz, proj, \
                  dt_bias, a_neg, d_skip, qo_indptr, slots, state, (A*)out, a)
-    if (a.piece > 0) {
+    if (a.piece != 0) {
         GO(1);
         GO(2);
     } else {
@@ -774,7 +790,9 @@ static void launch_scan16(const void* xc, const void* xz, const float* proj, con
 // of the token chunk) that run side by side in two passes; max_pieces bounds the pieces of any
 // entry, piece_state is float scratch [entries, max_pieces, inner, n_state], piece_dt
 // [entries, max_pieces, inner].  dt_pre: nullptr, or float [tokens, inner] = dt_in W_dt^T made by
-// the caller (with pieces it may hold step sizes afterwards).  Returns 0, a CUDA error code, or -1 when the shape is refused.
+// the caller (with pieces it may hold step sizes afterwards).  piece < 0, where the kernel for 16 states
+// takes the sizes: pieces of scan_piece tokens, max_pieces as with piece > 0, scratch for tokens / 64 +
+// entries pieces.  Returns 0, a CUDA error code, or -1 when the shape is refused.
 MSTAR_API int mstar_selective_scan(const void* xc, const void* xz, int ld_xz, const float* proj,
                                    const float* w_dt, const float* dt_bias, const float* a_neg,
                                    const float* d_skip, const int* qo_indptr, const int* slots,
@@ -784,11 +802,10 @@ MSTAR_API int mstar_selective_scan(const void* xc, const void* xz, int ld_xz, co
                                    float* dt_pre, void* stream) {
     if (entries <= 0) return 0;
     if (inner <= 0 || n_state <= 0 || rank <= 0 || taps <= 0 || n_state > 256) return -1;
-    if (piece < 0 || (piece > 0 && (max_pieces < 1 || piece_state == nullptr || piece_dt == nullptr)))
-        return -1;
+    if (piece != 0 && (max_pieces < 1 || piece_state == nullptr || piece_dt == nullptr)) return -1;
     cudaStream_t s = (cudaStream_t)stream;
     ScanArgs a{inner, n_state, rank, taps, ld_xz, entries, state_stride, piece, 0,
-               piece > 0 ? max_pieces : 1, piece_state, piece_dt, dt_pre};
+               piece != 0 ? max_pieces : 1, piece_state, piece_dt, dt_pre};
     const int piece16 = act_dtype == MSTAR_F32 ? 4 : 8;          // elements of 16 bytes
     if (dt_pre != nullptr && n_state == 16 && inner % 32 == 0 && rank % 4 == 0 && ld_xz % piece16 == 0 &&
         (((uintptr_t)xc | (uintptr_t)xz | (uintptr_t)proj | (uintptr_t)dt_pre | (uintptr_t)a_neg | (uintptr_t)piece_state) & 15) == 0) {
@@ -798,6 +815,7 @@ MSTAR_API int mstar_selective_scan(const void* xc, const void* xz, int ld_xz, co
             launch_scan16<bf16>(xc, xz, proj, dt_bias, a_neg, d_skip, qo_indptr, slots, state, out, a, s);
         return launch_status();
     }
+    if (piece < 0) return -1;
 #define GO(A, LANES, NPER)                                                                        \
     {                                                                                             \
         constexpr int CH = SS_THREADS / LANES;                                                    \

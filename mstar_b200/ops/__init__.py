@@ -1738,6 +1738,13 @@ SCAN_PIECE = 128
 SCAN_PIECES_FROM = 512
 
 
+def scan_most_pieces(longest: int) -> int:
+    """The most pieces that a portion of up to ``longest`` tokens has in the kernel for 16 states, which
+    cuts one of n tokens into pieces of n // 16 tokens, rounded down to a multiple of 64 within 64 and 256:
+    at 2,047 tokens there are 32, more again from 8,192 on."""
+    return max(min(-(-longest // 64), 32), -(-longest // 256))
+
+
 def selective_scan(xc: torch.Tensor, xz: torch.Tensor, proj: torch.Tensor, w_dt, dt_bias, a_neg,
                    d_skip, qo_indptr, slots, state: torch.Tensor, entries: int, inner: int,
                    n_state: int, rank: int, taps: int, max_q_len: int | None = None) -> torch.Tensor:
@@ -1748,7 +1755,8 @@ def selective_scan(xc: torch.Tensor, xz: torch.Tensor, proj: torch.Tensor, w_dt,
     float ``w_dt`` [inner, rank], ``dt_bias`` [inner], ``a_neg`` [inner, n_state] (= -exp(A_log)),
     ``d_skip`` [inner].  Returns y * silu(z) [tokens, inner] in the dtype of ``xc``.
     ``max_q_len`` (the longest portion of the batch) of ``SCAN_PIECES_FROM`` tokens or more
-    cuts every portion into pieces (of ``SCAN_PIECE`` tokens, or by the batch) that run side by side: a first
+    cuts every portion into pieces that run side by side (of ``SCAN_PIECE`` tokens, or, by the kernel
+    for 16 states, of 64 to 256 tokens by the portion's own length): a first
     pass leaves each piece's own end state and summed step sizes, a second starts each piece
     from the state joined over the pieces before it (the recurrence is linear in the state);
     MSTAR_SCAN_PIECE sets another piece size, 0 none."""
@@ -1764,25 +1772,25 @@ def selective_scan(xc: torch.Tensor, xz: torch.Tensor, proj: torch.Tensor, w_dt,
     out = torch.empty_like(xc)
     piece, pieces, piece_state, piece_dt, dt_pre = 0, 1, None, None, None
     if max_q_len is not None and max_q_len >= SCAN_PIECES_FROM:
-        piece = SCAN_PIECE
-        if n_state == 16 and inner % 32 == 0 and rank % 4 == 0:
-            # the kernel for 16 states (blocks of 32 channels): whole portions where these fill every SM
-            # several times (5 x 520 tokens of 4,096 channels: 216 us against 272 to 284 in pieces of 64 to
-            # 256), else some 16 pieces (600 tokens of 2,048 channels: 44 us in pieces of 64, 52 of 128; 2,048 of
-            # 4,096: 217 of 128, 223 and 226 of 64 and 256; 8,192: 809 of 256, 832 of 128)
-            piece = min(max(max_q_len // 16 // 64 * 64, 64), 256)
-            if entries * (inner // 32) >= 4 * num_sms(xc.device):
-                piece = 0
-        piece = int(os.environ.get("MSTAR_SCAN_PIECE", piece)) // 16 * 16
-    if max_q_len is not None and max_q_len >= SCAN_PIECES_FROM:
+        wide = 16 // xz.element_size()
+        sixteen = (n_state == 16 and inner % 32 == 0 and rank % 4 == 0 and xz.stride(0) % wide == 0
+                   and not any(t.data_ptr() % 16 for t in (xc, xz, proj, a_neg)))
+        forced = os.environ.get("MSTAR_SCAN_PIECE")
+        if forced is not None:
+            piece = int(forced) // 16 * 16
+            pieces = -(-max_q_len // piece) if piece else 1
+        elif sixteen:
+            piece, pieces = -1, scan_most_pieces(max_q_len)
+        else:
+            piece, pieces = SCAN_PIECE, -(-max_q_len // SCAN_PIECE)
         # with many tokens the step sizes' product W_dt dt_in is a true-32-bit product of its
         # own (a third of the scan's instructions otherwise)
         dt_pre = sgemm_nt(proj[:, :rank], w_dt)
     if piece:
-        pieces = -(-max_q_len // piece)
-        piece_state = torch.empty((entries, pieces, inner, n_state), dtype=torch.float32,
-                                  device=xc.device)
-        piece_dt = torch.empty((entries, pieces, inner), dtype=torch.float32, device=xc.device)
+        # (cut by their own lengths, portions have a piece for every started 64 tokens at most)
+        places = entries * pieces if piece > 0 else xc.shape[0] // 64 + entries
+        piece_state = torch.empty((places, inner, n_state), dtype=torch.float32, device=xc.device)
+        piece_dt = torch.empty((places, inner), dtype=torch.float32, device=xc.device)
     code = lib.get("selective_scan").mstar_selective_scan(
         xc.data_ptr(), xz.data_ptr(), xz.stride(0), proj.data_ptr(), w_dt.data_ptr(),
         dt_bias.data_ptr(), a_neg.data_ptr(), d_skip.data_ptr(), qo_indptr.data_ptr(),

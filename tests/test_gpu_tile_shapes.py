@@ -240,6 +240,35 @@ def test_selective_scan_of_long_portions(lens, inner, piece, dtype, monkeypatch)
             assert torch.equal(state[e, j * inner:(j + 1) * inner], row)
 
 
+@pytest.mark.parametrize("off", [0, 1])          # rows off 16 bytes: the kernel for any number of states
+@pytest.mark.parametrize("alone,beside", [(600, [4200, 3]), (520, [520] * 9), (2047, [513]), (1024, [1] * 20)])
+def test_selective_scan_of_a_portion_does_not_depend_on_the_batch(alone, beside, off):
+    """A long portion's bits by itself and among others: how it is cut follows from its own length."""
+    from mstar_b200 import ops
+
+    inner, rank, N, taps = 2048, 4, 16, 4
+    lens = beside[:1] + [alone] + beside[1:]
+    T, at = sum(lens), lens[0]
+    xc, xz = rnd(T, inner, dtype=torch.bfloat16, seed=1), rnd(T, 2 * inner + off, dtype=torch.bfloat16, seed=2)[:, :2 * inner]
+    proj, w_dt = rnd(T, rank + 2 * N, seed=3), rnd(inner, rank, seed=4)
+    bias, a, d = rnd(inner, seed=5) - 3, -torch.exp(rnd(inner, N, seed=6)), rnd(inner, seed=7)
+    state = rnd(len(lens), ops.selective_scan_state_size(inner, N, taps), seed=8)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+
+    def run(rows, sizes, slots):
+        starts = [0]
+        for n in sizes:
+            starts.append(starts[-1] + n)
+        moved = state.clone()
+        y = ops.selective_scan(xc[rows].contiguous(), xz[rows], proj[rows].contiguous(), w_dt, bias, a, d, i32(starts),
+                               i32(slots), moved, len(sizes), inner, N, rank, taps, max_q_len=max(sizes))
+        return y, moved[1]
+
+    whole, end = run(slice(0, T), lens, list(range(len(lens))))
+    one, one_end = run(slice(at, at + alone), [alone], [1])
+    assert torch.equal(whole[at:at + alone], one) and torch.equal(end, one_end)
+
+
 @pytest.mark.parametrize("lens,inner", [([1, 2, 3, 1700, 5, 6], 1032), ([2401], 64), ([3] * 800, 64)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_convolution_of_several_tokens_a_thread(lens, inner, dtype):
