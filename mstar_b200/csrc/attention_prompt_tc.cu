@@ -108,6 +108,8 @@ __device__ __forceinline__ pa_f2 pa_tanh2(pa_f2 z) {
     p = pa_fma2(u, p, c(-1.0 / 3.0));
     return pa_fma2(pa_mul2(z, u), p, z);
 }
+// the lowest n bits of 32 (none for n <= 0, all for n >= 32)
+__device__ __forceinline__ uint32_t pa_first(int n) { return n >= 32 ? 0xffffffffu : n <= 0 ? 0u : (1u << n) - 1u; }
 // Takes the bfloat16 heads off a pair of floats: returns them packed and leaves the remainders (exact).
 __device__ __forceinline__ uint32_t pa_take_part(pa_f2& x) {
     const __nv_bfloat162 head2 = __floats2bfloat162_rn(pa_lo(x), pa_hi(x));
@@ -414,16 +416,35 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
             pt_ld32(sp + 32, s[1]);
             pt_wait_ld();
             const int key0 = tile_key(j);
+            // the keys of the tile that the row sees, a bit each (tiles that every row sees whole: not asked)
+            const bool edge = !(key0 + PA_KEYS - 1 <= cp_min && (key0 >= lo_max || key0 + PA_KEYS <= a.keep_first));
+            uint32_t seen[2] = {0xffffffffu, 0xffffffffu};
+            if (edge) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int k0 = key0 + 32 * h;
+                    seen[h] = pa_first(cp + 1 - k0) & (~pa_first(row_lo - k0) | pa_first(a.keep_first - k0));
+                }
+            }
             // scores in base-2 units, capped and biased where the options ask for it:
-            // cap tanh(x / cap) = cap (1 - 2 / (2^(2 log2(e) x / cap) + 1)), or, where all of the warp's scores
-            // lie within half of the cap, by a polynomial, which leaves the exponential unit to the
-            // probabilities (what bounds the kernel otherwise: three operations a score instead of one)
+            // cap tanh(x / cap) = cap (1 - 2 / (2^(2 log2(e) x / cap) + 1)), or, where all of the scores that the
+            // row sees in the tile lie within half of the cap, by a polynomial, which leaves the exponential
+            // unit to the probabilities (what bounds the kernel otherwise: three operations a score instead of
+            // one).  Each row decides for itself by what it sees, so that its bits depend on nothing else.
             if (CAP) {
                 float big = 0.f;
+                if (edge) {
 #pragma unroll
-                for (int i = 0; i < 32; ++i)
-                    big = fmaxf(big, fmaxf(fabsf(__uint_as_float(s[0][i])), fabsf(__uint_as_float(s[1][i]))));
-                if (__all_sync(0xffffffffu, big * a.cap_z <= 0.5f)) {
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            big = fmaxf(big, seen[h] >> i & 1u ? fabsf(__uint_as_float(s[h][i])) : 0.f);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i)
+                        big = fmaxf(big, fmaxf(fabsf(__uint_as_float(s[0][i])), fabsf(__uint_as_float(s[1][i]))));
+                }
+                if (big * a.cap_z <= 0.5f) {
                     const pa_f2 to_z = pa_pack(a.cap_z, a.cap_z), cap2 = pa_pack(a.cap_log2e, a.cap_log2e),
                                 bias2 = pa_pack(bias, bias);
 #pragma unroll
@@ -445,20 +466,19 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
                                 fmaf(pa_rcp(pt_ex2(x * a.cap_in) + 1.f), -2.f * a.cap_log2e, a.cap_log2e) + bias);
                         }
                 }
+                __syncwarp();
             } else if (SIGMOID) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
 #pragma unroll
                     for (int i = 0; i < 32; ++i) s[h][i] = __float_as_uint(fmaf(__uint_as_float(s[h][i]), scale, bias));
             }
-            if (!(key0 + PA_KEYS - 1 <= cp_min && (key0 >= lo_max || key0 + PA_KEYS <= a.keep_first))) {
+            if (edge) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const int key = key0 + 32 * h + i;
-                        if (key > cp || (key < row_lo && key >= a.keep_first)) s[h][i] = 0xff800000u;   // -inf
-                    }
+                    for (int i = 0; i < 32; ++i)
+                        if (!(seen[h] >> i & 1u)) s[h][i] = 0xff800000u;    // -inf
             }
             const float unit = CAP || SIGMOID ? 1.f : scale;
             float alpha = 1.f;

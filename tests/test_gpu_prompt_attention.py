@@ -185,6 +185,39 @@ def test_latent_prompt_attention(window, gated, lens_q, lens_kv, heads, dim, ran
         assert ((out.view(T, heads, dim).double() - want).abs() <= bound).all()
 
 
+@pytest.mark.parametrize("hd,nq,nkv", [(128, 8, 4), (64, 16, 4)])
+def test_capped_rows_have_the_bits_of_what_they_see(hd, nq, nkv):
+    """Later tokens of a request, the next request and what lies on a page behind the last key change no bit of a
+    row, though the two forms of tanh that its scores' sizes choose between differ."""
+    from mstar_b200 import ops
+
+    lens, page, scale = [200, 61], 64, hd ** -0.5
+    ctx, starts = batch(lens, lens)
+    T, half = starts[-1], 130
+    q = rnd(T, nq * hd, dtype=torch.bfloat16, seed=1)
+    kv = rnd(sum(-(-n // page) for n in lens), 2, nkv, page, hd, dtype=torch.bfloat16, seed=2)
+    table = torch.tensor([[3, 1, 2, 0], [4, 0, 0, 0]], dtype=torch.int32, device=DEV)
+
+    def run(queries, cache):
+        out = ops.sink_attention(queries, cache, table, ctx.token_req, ctx.cache_pos, nq, nkv, hd, hd, page, 0, 0,
+                                 scale, ctx=ctx, softcap=30.0)
+        ops.check_error_word(DEV)
+        return out
+
+    want = run(q, kv)
+    q2, kv2 = q.clone(), kv.clone()
+    q2[half:] *= 40                              # from token `half` of the first request on
+    kv2[2, 0, :, half - 128:] *= 40              # ... their keys
+    kv2[0, 0] *= 40
+    kv2[4, 0] *= 40                              # the second request's keys
+    got = run(q2, kv2)
+    assert torch.equal(got[:half], want[:half]) and not torch.equal(got[half:], want[half:])
+    kv3 = kv.clone()
+    kv3[0, 0, :, 200 - 192:] *= 40               # behind the first request's last key
+    kv3[4, 0, :, 61:] *= 40
+    assert torch.equal(run(q, kv3), want)
+
+
 def cancelling(p, seed, reserve=4):
     """bfloat16 values [keys, probes] whose sums with the weights p [probes, keys] (double) nearly vanish: random
     ones, then corrections by reserved keys, each of which leaves 2^-9 of what is left.  And the size of a sum
