@@ -132,7 +132,7 @@ class LatentAttention:
             y = q.new_empty((ctx.num_tokens, h * s.v_dim))
             ops.latent_attention_prompt(q, cache.kv, cache.block_table, ctx, groups, self.w_kv, h, s.qk_dim,
                                         s.kv_rank, s.rot_dim, cache.page_size, s.window or 0, self.scale, y,
-                                        gate=gate if s.gated and s.gate_per_head else None)
+                                        gate=gate.float() if s.gated and s.gate_per_head else None)
             if ctx.num_decode:
                 y[:ctx.num_decode] = self._folded(q, gate, ctx, cache, ctx.num_decode, ctx.num_decode)
         else:

@@ -301,3 +301,56 @@ def test_latent_probabilities_keep_24_bits(dim, splits, monkeypatch):
     ops.check_error_word(DEV)
     left = out.double().diagonal(dim1=0, dim2=1) * p.sum(1) / size
     assert left.square().mean().sqrt() < TERM
+
+
+def latent_layer(seed, heads=4, window=None, gate_per_head=False, q_rank=None, hidden=128, dim=64, rot=32, rank=64):
+    from mstar_b200.config.layout import LatentAttentionSpec, PositionSpec
+    from mstar_b200.parts.base import Runtime
+    from mstar_b200.parts.registry import build_part, part_class
+
+    spec = LatentAttentionSpec(hidden_size=hidden, num_heads=heads, qk_dim=dim, rot_dim=rot, v_dim=dim, kv_rank=rank,
+                               position=PositionSpec(kind="rope", head_dim=rot, rotary_dim=rot, theta=1e4),
+                               window=window, gate_per_head=gate_per_head, q_rank=q_rank)
+    params = {n: rnd(*ps.shape, dtype=torch.bfloat16, seed=seed + i, scale=ps.shape[-1] ** -0.5)
+              if len(ps.shape) > 1 else 1 + rnd(*ps.shape, dtype=torch.bfloat16, seed=seed + i, scale=0.1)
+              for i, (n, ps) in enumerate(part_class("mixer", spec).param_specs(spec).items())}
+    return build_part("mixer", spec, params, Runtime(dtype=torch.bfloat16, device=torch.device(DEV))), rank + rot
+
+
+def latent_forward(part, row, lens_q, lens_kv, x, page=16):
+    """The layer's outputs over requests whose earlier rows are random (the same for a request in every batch:
+    ``lens_kv`` and ``x`` by request name)."""
+    from mstar_b200.parts.base import LayerCache
+
+    names = list(lens_q)
+    ctx, starts = batch([lens_q[n] for n in names], [lens_kv[n] for n in names])
+    ctx.num_decode = next((i for i, n in enumerate(names) if lens_q[n] > 1), len(names))
+    width = max(-(-n // page) for n in lens_kv.values())
+    cache = torch.empty(len(names) * width, 1, 1, page, row, dtype=torch.bfloat16, device=DEV)
+    for i, n in enumerate(names):
+        cache[i * width:(i + 1) * width] = rnd(width, 1, 1, page, row, dtype=torch.bfloat16, seed=100 + n)
+    table = torch.arange(len(names) * width, dtype=torch.int32, device=DEV).view(-1, width)
+    y = part.forward(torch.cat([x[n] for n in names]), ctx, LayerCache(kv=cache, page_size=page, block_table=table))
+    return {n: y[starts[i]:starts[i + 1]].double() for i, n in enumerate(names)}
+
+
+# both forms round to bfloat16 between the layer's products: 0.003 of the result each
+def same(got, want):
+    return (got - want).norm() <= 0.012 * want.norm()
+
+
+@pytest.mark.parametrize("q_rank", [None, 48])
+def test_latent_layer_with_a_gate_a_head(q_rank, monkeypatch):
+    """The first product gives the gate in bfloat16 where the queries come straight from it, else in float."""
+    from mstar_b200 import ops
+
+    part, row = latent_layer(1, heads=8, gate_per_head=True, q_rank=q_rank)
+    x = {0: rnd(130, 128, dtype=torch.bfloat16, seed=50)}
+    calls = []
+    prompt = ops.latent_attention_prompt
+    monkeypatch.setattr(ops, "latent_attention_prompt", lambda *a, **k: (calls.append(1), prompt(*a, **k)))
+    got = latent_forward(part, row, {0: 130}, {0: 200}, x)[0]
+    ops.check_error_word(DEV)
+    assert calls
+    monkeypatch.setattr(ops, "latent_prompt_takes", lambda *a: False)
+    assert same(got, latent_forward(part, row, {0: 130}, {0: 200}, x)[0])
