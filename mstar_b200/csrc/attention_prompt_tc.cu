@@ -68,6 +68,7 @@ struct PromptArgs {
     float cap_z;                        // scale / cap
     int cap_bounds;                     // the cap is low enough to be every row's reference maximum
     int rot_x;                          // latent form: first rotated feature of a latent row
+    int out_heads;                      // heads of a row of `out` (the launch may write some of them)
 };
 
 __device__ __forceinline__ float pa_rcp(float x) {
@@ -570,6 +571,7 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
         // others, the load being a warp's, and not stored)
         if (ok) {
             const size_t row = (size_t)(q_start + tok) * a.nq + head;
+            bf16* out = a.out + ((size_t)(q_start + tok) * a.out_heads + head) * HD;
             const float* gate = nullptr;
             float inv = 1.f;
             if (a.splits == 1 && valid) {
@@ -619,7 +621,7 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
                     }
 #pragma unroll
                     for (int t = 0; t < 8; ++t) f[t] *= __uint_as_float(o[8 * i + t]);
-                    store8(a.out + row * HD + c0 + 8 * i, f);
+                    store8(out + c0 + 8 * i, f);
                 }
             }
             if (a.splits > 1 && valid) {
@@ -671,7 +673,7 @@ prompt_merge_kernel(PromptArgs a, int row0, int rows) {
 #pragma unroll
     for (int i = 0; i < HD / 32; ++i) {
         const float g = gate == nullptr ? 1.f : pa_sigmoid(gate[a.gate_features ? i * 32 + lane : 0]);
-        a.out[(size_t)row * HD + i * 32 + lane] = __float2bfloat16_rn(sum[i] / L * g);
+        a.out[((size_t)tok * a.out_heads + head) * HD + i * 32 + lane] = __float2bfloat16_rn(sum[i] / L * g);
     }
 }
 
@@ -750,6 +752,7 @@ MSTAR_API int mstar_sink_attention_prompt(const void* kv_map, const void* q, int
     a.bt_stride = bt_stride;
     a.nq = nq;
     a.nkv = nkv;
+    a.out_heads = nq;
     a.page_size = page_size;
     a.entries = entries;
     a.window = window;
@@ -799,17 +802,18 @@ latent_gather_kernel(const uint4* __restrict__ cache, const int* __restrict__ bl
     }
 }
 
-// parts[row][head][k head | k remainder | v head | v remainder] from the float product
-// made[row][k | v][head][dim]; eight features a thread.
+// parts[row][head][k head | k remainder | v head | v remainder] from the float products
+// keys[row][head][dim] and values; eight features a thread.
 __global__ void __launch_bounds__(256)
-latent_split_kernel(const float* __restrict__ made, bf16* __restrict__ parts, long long pieces, int heads, int dim) {
+latent_split_kernel(const float* __restrict__ keys, const float* __restrict__ values, bf16* __restrict__ parts,
+                    long long pieces, int heads, int dim) {
     const int per_head = dim / 8, per_row = 2 * heads * per_head;
     for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < pieces; i += (long long)gridDim.x * 256) {
         const long long row = i / per_row;
         const int at = (int)(i - row * per_row), which = at / (heads * per_head);
         const int head = at / per_head - which * heads, d = at % per_head * 8;
         float v[8], rest[8];
-        load8(made + i * 8, v);
+        load8((which ? values : keys) + (row * heads + head) * dim + d, v);
 #pragma unroll
         for (int k = 0; k < 8; ++k) rest[k] = v[k] - __bfloat162float(__float2bfloat16_rn(v[k]));
         bf16* dst = parts + ((row * heads + head) * 4 + 2 * which) * dim + d;
@@ -831,24 +835,25 @@ MSTAR_API int mstar_latent_gather(const void* cache, const int* block_table, int
     return launch_status();
 }
 
-MSTAR_API int mstar_latent_split(const float* made, void* parts, int rows, int heads, int dim, void* stream) {
+MSTAR_API int mstar_latent_split(const float* keys, const float* values, void* parts, int rows, int heads, int dim,
+                                 void* stream) {
     if (rows <= 0) return 0;
-    if (dim % 8 != 0 || (((uintptr_t)made | (uintptr_t)parts) & 15) != 0) return -1;
+    if (dim % 8 != 0 || (((uintptr_t)keys | (uintptr_t)values | (uintptr_t)parts) & 15) != 0) return -1;
     const long long pieces = (long long)rows * 2 * heads * (dim / 8);
     const long long blocks = (pieces + 255) / 256, most = (long long)device_sm_count() * 16;
     latent_split_kernel<<<(unsigned)(blocks < most ? blocks : most), 256, 0, (cudaStream_t)stream>>>(
-        made, (bf16*)parts, pieces, heads, dim);
+        keys, values, (bf16*)parts, pieces, heads, dim);
     return launch_status();
 }
 
 // Entries [first_entry, first_entry + entries), the latent form.  q: `tokens` rows (the whole step's), head
 // h's dim plain and rot rotated features at h * q_head; parts: [key_rows][heads][4 * dim] and latents:
-// [key_rows][rank + rot], made by the two functions above; out: [tokens, heads * dim], of which the
-// entries' rows (rows_from .. + rows) are written; gate: null or one number a head.
+// [key_rows][rank + rot], made by the two functions above; out: [tokens, out_heads * dim], of which the
+// entries' rows (rows_from .. + rows) and the first `heads` heads are written; gate: null or one number a head.
 MSTAR_API int mstar_latent_attention_prompt(const void* q, int q_stride, int q_head, int tokens, const void* parts,
                                             const void* latents, int key_rows, void* out, const int* qo_indptr,
                                             const int* kv_len, int first_entry, int entries, int max_q_len,
-                                            int rows_from, int rows, int heads, int dim, int rank, int rot, int window,
+                                            int rows_from, int rows, int heads, int out_heads, int dim, int rank, int rot, int window,
                                             float scale, int splits, float* scratch, const float* gate,
                                             int gate_stride, int* error_word, void* stream) {
     if (entries <= 0 || max_q_len <= 0) return 0;
@@ -890,6 +895,7 @@ MSTAR_API int mstar_latent_attention_prompt(const void* q, int q_stride, int q_h
     a.scratch = scratch;
     a.gate = gate;
     a.nq = a.nkv = heads;
+    a.out_heads = out_heads;
     a.first_entry = first_entry;
     a.entries = entries;
     a.window = window;

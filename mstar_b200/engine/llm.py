@@ -95,6 +95,7 @@ class LLM:
 
     def _pages_from_memory(self, page_size, fraction: float) -> list:
         free, _ = torch.cuda.mem_get_info(self.device)
+        free = max(free - self.model.workspace_bytes(), 0)
         windows, group_of = plan_groups(self.model.cache_needs)
         if not windows:
             return []

@@ -22,7 +22,7 @@ from ..config.base import ModelConfig
 from ..config.layout import ModelLayout
 from ..config.registry import get_architecture, load_config
 from ..parts.base import CacheNeed, ResidualStream, Runtime, StepContext
-from ..parts.registry import build_part, part_class
+from ..parts.registry import build_part, mixer_workspace_bytes, part_class
 from ..weights.loader import load_parameters
 from ..weights.names import ParamSpec
 
@@ -103,6 +103,11 @@ class Model:
     def max_positions(self) -> Optional[int]:
         """Positions the model was built for (its layout says; None: no limit known)."""
         return self.layout.max_positions
+
+    def workspace_bytes(self) -> int:
+        """What a step may need beside its activations: memory that a cache sized by what is free
+        has to leave."""
+        return max((mixer_workspace_bytes(b.mixer, self.runtime.dtype) for b in self.layout.blocks), default=0)
 
     def parameter_bytes(self) -> int:
         seen, total = set(), 0

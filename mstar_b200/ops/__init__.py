@@ -1163,28 +1163,41 @@ def latent_attention(q_abs: torch.Tensor, q_rot: torch.Tensor, cache: torch.Tens
     return out
 
 
-# query-key pairs of a request per key from which on its keys and values are made from the latents
-# (making them costs 13 ns a key for 16 heads of 128 at a rank of 512, 3.5 ns for 8 of 64 at 256; a pair
-# of the folded form 0.9 and 0.22 ns), and the most memory the keys and values made at once take (8
-# bytes a feature as the product's floats, as much again in two parts: 32,768 keys of 16 heads of 128)
-LATENT_PROMPT_PAIRS = 32
-LATENT_PROMPT_BYTES = 1 << 30
+# tokens of a portion from which on its keys and values are made from the latents (making them costs 13 ns
+# a key for 16 heads of 128 at a rank of 512, 3.5 ns for 8 of 64 at 256; a pair of the folded form 0.9 and
+# 0.22 ns), and the memory that the keys and values made at once may take in any case: what the folded form
+# would take for the same tokens if that is more.  A feature of a key takes 8 bytes as the products' floats
+# and as much again in two parts, a latent feature of a token and head in the folded form 10 (query, sum, and
+# the sum in bfloat16).
+# Shorter portions go along with longer ones where they see few keys: a call of the folded form beside the
+# made one costs some 30 us on the device, as much as making 2,048 keys more (2 tokens beside 1,000 with a
+# window of 1,024: 81 us together, 131 apart; over 16,002 keys 557 together, 236 apart).
+LATENT_PROMPT_TOKENS = 32
+LATENT_PROMPT_SHORT_KEYS = 2048
+LATENT_PROMPT_BYTES = 256 << 20
 
 
-def latent_prompt_groups(q_lens, kv_lens, window: int, features: int, first_entry: int = 0) -> list:
+def latent_prompt_room(q_lens, heads: int, rank: int) -> int:
+    """Bytes that the keys and values made at once for these portions may take."""
+    return max(LATENT_PROMPT_BYTES, 10 * heads * rank * sum(q for q in q_lens if q >= LATENT_PROMPT_TOKENS))
+
+
+def latent_prompt_groups(q_lens, kv_lens, window: int, features: int, first_entry: int = 0, heads: int = 1,
+                         room: int | None = None) -> list:
     """[(first entry, entries, keys)] of the runs of portions, from ``first_entry`` on, whose keys and
-    values (``features`` each: heads times dim) are made from the latents together; empty where the
-    folded form is the cheaper one or a portion's take more than ``LATENT_PROMPT_BYTES``."""
-    keys, room = [], LATENT_PROMPT_BYTES // (16 * features)
-    for q, n in zip(q_lens[first_entry:], kv_lens[first_entry:]):
-        past = n - q
-        keys.append(n - ((past - window + 1) // PROMPT_KEYS * PROMPT_KEYS if window and past >= window else 0))
-    pairs = sum(q * k for q, k in zip(q_lens[first_entry:], keys))
-    if not keys or pairs < LATENT_PROMPT_PAIRS * sum(keys) or max(keys) > room:
-        return []
+    values (``features`` each: heads times dim) are made from the latents together; the other portions
+    (short ones with many keys, for which the folded form is cheaper, and such whose keys and values of one
+    of ``heads`` heads alone take more than ``room`` bytes) lie between the runs."""
+    room = LATENT_PROMPT_BYTES if room is None else room
     groups = []
-    for i, k in enumerate(keys, first_entry):
-        if groups and groups[-1][2] + k <= room:
+    if max(q_lens[first_entry:], default=0) < LATENT_PROMPT_TOKENS:
+        return groups
+    for i, (q, n) in enumerate(zip(q_lens[first_entry:], kv_lens[first_entry:]), first_entry):
+        past = n - q
+        k = n - ((past - window + 1) // PROMPT_KEYS * PROMPT_KEYS if window and past >= window else 0)
+        if (q < LATENT_PROMPT_TOKENS and k > LATENT_PROMPT_SHORT_KEYS) or 16 * (features // heads) * k > room:
+            continue
+        if groups and sum(groups[-1][:2]) == i and 16 * features * (groups[-1][2] + k) <= room:
             first, count, total = groups[-1]
             groups[-1] = (first, count + 1, total + k)
         else:
@@ -1205,16 +1218,20 @@ def latent_prompt_takes(q: torch.Tensor, cache: torch.Tensor, dim: int, v_dim: i
 
 def latent_attention_prompt(q: torch.Tensor, cache: torch.Tensor, block_table, ctx, groups, w_kv,
                             heads: int, dim: int, rank: int, rot: int, page_size: int, window: int,
-                            scale: float, out: torch.Tensor, gate=None) -> None:
+                            scale: float, out: torch.Tensor, gate=None, room: int | None = None) -> None:
     """Latent attention of prompt portions on tcgen05: for each of ``groups`` (see
-    ``latent_prompt_groups``) the latent rows its tokens see are gathered, one product with ``w_kv``
-    [2 * heads * dim, rank] (the key rows of all heads, then the value rows) makes every head's keys
-    and values in float, which enter the attention in two bfloat16 parts.  ``q``: [tokens, heads,
+    ``latent_prompt_groups``) the latent rows its tokens see are gathered, products with ``w_kv`` (the
+    key rows of all heads and the value rows, [heads * dim, rank] each, or both in one matrix) make the
+    keys and values in float, of as many heads at once as ``room`` bytes hold; they enter the attention
+    in two bfloat16 parts.  ``q``: [tokens, heads,
     dim + rot], rotated; writes the groups' rows of ``out`` [tokens, heads * dim], times the sigmoid
     of ``gate`` (float [tokens, heads]) where given."""
-    _need_cuda(q, cache, block_table, w_kv, out, gate)
+    w_k, w_v = w_kv.view(2, -1, rank) if isinstance(w_kv, torch.Tensor) else w_kv
+    room = LATENT_PROMPT_BYTES if room is None else room
+    _need_cuda(q, cache, block_table, w_k, w_v, out, gate)
     assert out.is_contiguous() and out.dtype == torch.bfloat16 and cache.is_contiguous()
-    assert tuple(w_kv.shape) == (2 * heads * dim, rank) and w_kv.is_contiguous()
+    for w in (w_k, w_v):
+        assert tuple(w.shape) == (heads * dim, rank) and w.is_contiguous()
     assert gate is None or (gate.dtype == torch.float32 and gate.stride(1) == 1)
     dev, entry = q.device, lib.get("attention_prompt_tc")
     starts = [0]
@@ -1227,29 +1244,35 @@ def latent_attention_prompt(q: torch.Tensor, cache: torch.Tensor, block_table, c
             cache.data_ptr(), block_table.data_ptr(), block_table.stride(0), ctx.qo_indptr.data_ptr(),
             ctx.kv_len.data_ptr(), rows.data_ptr(), first, count, max(ctx.kv_lens[first:first + count]),
             window, page_size, rank + rot, _stream()), "latent_gather")
-        made = linear(rows[:, :rank], w_kv, out_dtype=torch.float32)
-        parts = torch.empty((keys, heads, 4 * dim), dtype=torch.bfloat16, device=dev)
-        check(entry.mstar_latent_split(made.data_ptr(), parts.data_ptr(), keys, heads, dim, _stream()),
-              "latent_split")
-        del made
-        ctas = heads * -(-max(q_lens) // PROMPT_ROWS) * count
-        splits = prompt_splits(ctas, min(max(ctx.kv_lens[first:first + count]),
-                                         window + max(q_lens) if window else 1 << 30), num_sms(dev))
-        scratch = None
-        if splits > 1:
-            scratch = torch.empty(q.shape[0] * heads * splits * (dim + 2), dtype=torch.float32, device=dev)
-        code = entry.mstar_latent_attention_prompt(
-            q.data_ptr(), q.stride(0), q.stride(1), q.shape[0], parts.data_ptr(), rows.data_ptr(), keys,
-            out.data_ptr(), ctx.qo_indptr.data_ptr(), ctx.kv_len.data_ptr(), first, count, max(q_lens),
-            starts[first], starts[first + count] - starts[first], heads, dim, rank, rot, window,
-            float(scale), splits, _ptr(scratch), _ptr(gate), gate.stride(0) if gate is not None else 0,
-            tcgen05_error_word(dev).data_ptr(), _stream())
-        if code < 0:
-            raise KernelError(f"latent prompt attention refuses heads={heads}, dim={dim}, rank={rank}, "
-                              f"rot={rot} (code {code})")
-        check(code, "latent_attention_prompt")
-        if splits > 1:
-            lib.add_launches(1)                 # the merge kernel
+        passes = -(-heads // max(1, min(heads, room // (16 * dim * keys))))
+        per_pass = -(-heads // passes)
+        for h0 in range(0, heads, per_pass):
+            some = min(per_pass, heads - h0)
+            made_k, made_v = (linear(rows[:, :rank], w if passes == 1 else w[h0 * dim:(h0 + some) * dim],
+                                     out_dtype=torch.float32) for w in (w_k, w_v))
+            parts = torch.empty((keys, some, 4 * dim), dtype=torch.bfloat16, device=dev)
+            check(entry.mstar_latent_split(made_k.data_ptr(), made_v.data_ptr(), parts.data_ptr(), keys, some, dim,
+                                           _stream()), "latent_split")
+            del made_k, made_v
+            ctas = some * -(-max(q_lens) // PROMPT_ROWS) * count
+            splits = prompt_splits(ctas, min(max(ctx.kv_lens[first:first + count]),
+                                             window + max(q_lens) if window else 1 << 30), num_sms(dev))
+            scratch = None
+            if splits > 1:
+                scratch = torch.empty(q.shape[0] * some * splits * (dim + 2), dtype=torch.float32, device=dev)
+            code = entry.mstar_latent_attention_prompt(
+                q.data_ptr() + 2 * h0 * q.stride(1), q.stride(0), q.stride(1), q.shape[0], parts.data_ptr(),
+                rows.data_ptr(), keys, out.data_ptr() + 2 * h0 * dim, ctx.qo_indptr.data_ptr(),
+                ctx.kv_len.data_ptr(), first, count, max(q_lens), starts[first], starts[first + count] - starts[first], some, heads, dim, rank, rot, window,
+                float(scale), splits, _ptr(scratch), gate.data_ptr() + 4 * h0 if gate is not None else 0,
+                gate.stride(0) if gate is not None else 0, tcgen05_error_word(dev).data_ptr(), _stream())
+            if code < 0:
+                raise KernelError(f"latent prompt attention refuses heads={heads}, dim={dim}, rank={rank}, "
+                                  f"rot={rot} (code {code})")
+            check(code, "latent_attention_prompt")
+            if splits > 1:
+                lib.add_launches(1)             # the merge kernel
+            del parts, scratch                  # (before the next ones are made)
 
 
 _BMM_INTO_ROWS: dict = {}       # out dtype -> False once the library refused the strided output

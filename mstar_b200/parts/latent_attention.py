@@ -11,7 +11,8 @@ probabilities and the weighted sum are float; the folded query is kept in float 
 
 Prompt portions in bfloat16 take the other form where the sizes allow it: with many queries a key it
 costs less to make every head's keys and values from the latents (float, in two bfloat16 parts) than
-to score and sum whole latents a head.
+to score and sum whole latents a head.  They take no more memory than the folded form does for the same
+tokens, or ``LATENT_PROMPT_BYTES``, which ``workspace_bytes`` asks the engine to keep free.
 
 Options of the spec: queries through a normed latent of their own (the first product then
 gives that latent instead of the queries, and a second one the queries), rotary pairs
@@ -29,7 +30,8 @@ from .registry import register_part
 
 
 class LatentAttention:
-    graph_safe = True       # nothing per-step is read from the host
+    # the lengths of prompt portions are read on the host; a captured decode step has none
+    graph_safe = True
 
     @staticmethod
     def _gate_rows(spec) -> int:
@@ -64,6 +66,11 @@ class LatentAttention:
         return CacheNeed(kv=KVNeed(num_kv_heads=1, head_dim=spec.kv_rank + spec.rot_dim,
                                    window=spec.window, planes=1))
 
+    @classmethod
+    def workspace_bytes(cls, spec, dtype: torch.dtype) -> int:
+        """What a step may need beside its activations (made keys and values of prompts)."""
+        return ops.LATENT_PROMPT_BYTES if dtype == torch.bfloat16 and spec.qk_dim == spec.v_dim else 0
+
     def __init__(self, spec, params: dict, runtime: Runtime):
         p = spec.position
         if p.kind != "rope":
@@ -88,10 +95,8 @@ class LatentAttention:
         # per head: [rank, qk_dim] rows so that a = q @ uk_t[h]^T, and [v_dim, rank]
         self.uk_t = params["uk.weight"].view(h, spec.qk_dim, spec.kv_rank).transpose(1, 2).contiguous()
         self.uv = params["uv.weight"].view(h, spec.v_dim, spec.kv_rank)
-        # all heads' key rows, then their value rows: prompts make both in one product
-        self.w_kv = None
-        if runtime.dtype == torch.bfloat16 and spec.qk_dim == spec.v_dim:
-            self.w_kv = torch.cat([params["uk.weight"], params["uv.weight"]])
+        # prompts make keys and values from the latents (the parameters as they are, no copies)
+        self.w_kv = (params["uk.weight"].contiguous(), params["uv.weight"].contiguous())
         half = p.rotary_dim // 2
         self.freq = torch.tensor([p.theta ** (-(2.0 * i) / p.rotary_dim) for i in range(half)],
                                  dtype=torch.float64, device=runtime.device)
@@ -124,37 +129,43 @@ class LatentAttention:
             ops.latent_fill(q, None, None, self.freq, cache=cache.kv, **fill)
             gate = proj[:, s.q_rank + down:]
         q = q.view(-1, h, per_head)
-        groups = []
-        if self.w_kv is not None and ops.latent_prompt_takes(q, cache.kv, s.qk_dim, s.v_dim, s.kv_rank,
-                                                             s.rot_dim):
-            groups = ops.latent_prompt_groups(ctx.q_lens, ctx.kv_lens, s.window or 0, h * s.v_dim, ctx.num_decode)
+        groups, room = [], 0
+        if ctx.max_q_len > 1 and ops.latent_prompt_takes(q, cache.kv, s.qk_dim, s.v_dim, s.kv_rank, s.rot_dim):
+            room = ops.latent_prompt_room(ctx.q_lens, h, s.kv_rank)
+            groups = ops.latent_prompt_groups(ctx.q_lens, ctx.kv_lens, s.window or 0, h * s.v_dim,
+                                              ctx.num_decode, h, room)
         if groups:
             y = q.new_empty((ctx.num_tokens, h * s.v_dim))
             ops.latent_attention_prompt(q, cache.kv, cache.block_table, ctx, groups, self.w_kv, h, s.qk_dim,
                                         s.kv_rank, s.rot_dim, cache.page_size, s.window or 0, self.scale, y,
-                                        gate=gate.float() if s.gated and s.gate_per_head else None)
-            if ctx.num_decode:
-                y[:ctx.num_decode] = self._folded(q, gate, ctx, cache, ctx.num_decode, ctx.num_decode)
+                                        gate=gate.float() if s.gated and s.gate_per_head else None, room=room)
+            # the runs between the groups: single tokens, short portions
+            e = t = 0
+            for first, count, _ in groups + [(ctx.num_entries, 0, 0)]:
+                t1 = t + sum(ctx.q_lens[e:first])
+                if first > e:
+                    y[t:t1] = self._folded(q, gate, ctx, cache, t, t1, first - e)
+                e, t = first + count, t1 + sum(ctx.q_lens[first:first + count])
         else:
-            y = self._folded(q, gate, ctx, cache, ctx.num_tokens, ctx.num_entries)
+            y = self._folded(q, gate, ctx, cache, 0, ctx.num_tokens, ctx.num_entries)
         if s.gated and not s.gate_per_head:
             ops.sigmoid_gate_mul(y, gate)
         return ops.linear(y, self.w_out, static_weights=True)
 
-    def _folded(self, q, gate, ctx: StepContext, cache: LayerCache, tokens: int, entries: int):
-        """The first ``tokens`` tokens (of the first ``entries`` entries) over the latents themselves,
-        [tokens, heads * v_dim], with the gate a head if there is one."""
+    def _folded(self, q, gate, ctx: StepContext, cache: LayerCache, t0: int, t1: int, entries: int):
+        """Tokens t0 .. t1-1 (of ``entries`` entries) over the latents themselves, [t1 - t0, heads *
+        v_dim], with the gate a head if there is one."""
         s = self.spec
         h = s.num_heads
-        q = q[:tokens]
+        q = q[t0:t1]
         q_abs = ops.linear_per_head(q[:, :, :s.qk_dim], self.uk_t, out_dtype=torch.float32)
         lat = ops.latent_attention(q_abs, q[:, :, s.qk_dim:], cache.kv, cache.block_table,
-                                   ctx.token_req[:tokens], ctx.cache_pos[:tokens], h, s.kv_rank, s.rot_dim,
+                                   ctx.token_req[t0:t1], ctx.cache_pos[t0:t1], h, s.kv_rank, s.rot_dim,
                                    cache.page_size, s.window or 0, self.scale,
                                    max_keys=ctx.max_kv_len, entries=entries)
         if s.gated and s.gate_per_head:
             # one gate a head commutes with the head's value up-projection
-            lat = ops.head_gate_mul(lat.view(-1, h * s.kv_rank), gate[:tokens], h,
+            lat = ops.head_gate_mul(lat.view(-1, h * s.kv_rank), gate[t0:t1], h,
                                     out_dtype=self.runtime.dtype).view(-1, h, s.kv_rank)
         else:
             lat = ops.convert(lat, self.runtime.dtype)

@@ -19,7 +19,7 @@ import torch
 from .. import ops
 from ..weights.names import ParamSpec
 from .base import CacheNeed, LayerCache, Runtime, SideStream, StepContext
-from .registry import build_part, part_class, register_part
+from .registry import build_part, mixer_workspace_bytes, part_class, register_part
 
 
 def _sub(params: dict, prefix: str) -> dict:
@@ -54,6 +54,10 @@ class ParallelMixer:
                     raise ValueError("two branches of a parallel mixer ask for a state slot")
                 state = need.state
         return CacheNeed(kv=kv, state=state)
+
+    @classmethod
+    def workspace_bytes(cls, spec, dtype) -> int:
+        return sum(mixer_workspace_bytes(branch, dtype) for branch in spec.branches)
 
     def __init__(self, spec, params: dict, runtime: Runtime):
         if not 1 <= len(spec.branches) <= 4:

@@ -13,6 +13,8 @@ and, by category,
     ffn       forward(x, ctx) -> y
     mixer     cache_need(spec) -> CacheNeed              (classmethod)
               forward(x, ctx, cache) -> y
+              workspace_bytes(spec, dtype) -> int          (classmethod, optional: what a step may
+                                                           need beside its activations)
     block     sub-parts named by the spec; forward(stream, ctx, cache)
     embedding forward(token_ids, ctx) -> float residual [tokens, hidden]
     head      forward(normed rows) -> float logits [rows, vocab]
@@ -60,6 +62,11 @@ def part_class(category: str, spec):
 
 def build_part(category: str, spec, params: dict, runtime):
     return part_class(category, spec)(spec, params, runtime)
+
+
+def mixer_workspace_bytes(spec, dtype) -> int:
+    need = getattr(part_class("mixer", spec), "workspace_bytes", None)
+    return need(spec, dtype) if need is not None else 0
 
 
 _done = False

@@ -354,3 +354,28 @@ def test_latent_layer_with_a_gate_a_head(q_rank, monkeypatch):
     assert calls
     monkeypatch.setattr(ops, "latent_prompt_takes", lambda *a: False)
     assert same(got, latent_forward(part, row, {0: 130}, {0: 200}, x)[0])
+
+
+@pytest.mark.parametrize("window", [None, 70])
+@pytest.mark.parametrize("gate_per_head", [False, True])
+def test_latent_layer_in_mixed_steps(window, gate_per_head, monkeypatch):
+    """Single tokens, long portions and a short one between them, each as by itself in the folded form; with the
+    keys and values of all heads made at once and of three at a time."""
+    from mstar_b200 import ops
+
+    part, row = latent_layer(1, heads=8, window=window, gate_per_head=gate_per_head)
+    lens_q, lens_kv = {0: 1, 1: 1, 2: 100, 3: 20, 4: 70}, {0: 50, 1: 300, 2: 100, 3: 220, 4: 400}
+    x = {n: rnd(q, 128, dtype=torch.bfloat16, seed=50 + n) for n, q in lens_q.items()}
+    seen = []
+    monkeypatch.setattr(ops, "LATENT_PROMPT_SHORT_KEYS", 50)
+    prompt = ops.latent_attention_prompt
+    monkeypatch.setattr(ops, "latent_attention_prompt", lambda *a, **k: (seen.append(a[4]), prompt(*a, **k)))
+    got = latent_forward(part, row, lens_q, lens_kv, x)
+    monkeypatch.setattr(ops, "latent_prompt_room", lambda *a: 3 * 16 * 64 * 400)
+    three = latent_forward(part, row, lens_q, lens_kv, x)
+    ops.check_error_word(DEV)
+    assert [[g[:2] for g in groups] for groups in seen] == [[(2, 1), (4, 1)]] * 2
+    monkeypatch.setattr(ops, "latent_prompt_takes", lambda *a: False)
+    for n in lens_q:
+        alone = latent_forward(part, row, {n: lens_q[n]}, lens_kv, x)[n]
+        assert same(got[n], alone) and same(three[n], alone)
