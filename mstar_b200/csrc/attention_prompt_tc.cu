@@ -614,7 +614,7 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
                             for (int t = 0; t < 8; ++t) f[t] = gate[c0 + 8 * i + t];
                         }
 #pragma unroll
-                        for (int t = 0; t < 8; ++t) f[t] = __fdividef(inv, 1.f + expf(-f[t]));
+                        for (int t = 0; t < 8; ++t) f[t] = over_one_plus_bf16(inv, expf(-f[t]));
                     } else {
 #pragma unroll
                         for (int t = 0; t < 8; ++t) f[t] = inv;

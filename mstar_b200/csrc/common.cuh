@@ -102,14 +102,19 @@ __device__ __forceinline__ float clamped_swish(float gate, float up, float limit
     return g / (1.f + expf(-alpha * g)) * (u + 1.f);
 }
 
-// The same two gates for results that are rounded to bfloat16 right after: the quotient by
-// __fdividef (2 ulp of a float; a denominator past 2^126 gives 0 where the quotient is under 1e-36).
-// The IEEE division costs some 20 instructions, and several times that where the gate is 0 (rows of
-// a tile past the matrix): the epilogue of a 128-column tile took 6 to 20 us with it.
-__device__ __forceinline__ float silu_bf16(float g) { return __fdividef(g, 1.f + expf(-g)); }
+// x / (1 + e), e an exponential, for results that are rounded to bfloat16 right after: __fdividef (2 ulp of a
+// float), both sides by 1/4, since it gives 0 for a denominator from 2^126 on.  The IEEE division costs
+// some 20 instructions, and several times that where x is 0 (rows of a tile past the matrix): the epilogue
+// of a 128-column tile took 6 to 20 us with it.  (x times rcp.approx, which also holds up to 2^128, took the
+// gate and up product of [2048, 512] x [16384, 512] from 69 to 77 us.)
+__device__ __forceinline__ float over_one_plus_bf16(float x, float e) {
+    return __fdividef(0.25f * x, fmaf(0.25f, e, 0.25f));
+}
+// The same two gates for such results.
+__device__ __forceinline__ float silu_bf16(float g) { return over_one_plus_bf16(g, expf(-g)); }
 __device__ __forceinline__ float clamped_swish_bf16(float gate, float up, float limit, float alpha) {
     const float g = fminf(gate, limit), u = fminf(fmaxf(up, -limit), limit);
-    return __fdividef(g, 1.f + expf(-alpha * g)) * (u + 1.f);
+    return over_one_plus_bf16(g, expf(-alpha * g)) * (u + 1.f);
 }
 
 // Sum over a whole block; `scratch` holds at least 32 floats of shared memory.

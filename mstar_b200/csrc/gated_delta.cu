@@ -1188,9 +1188,9 @@ MSTAR_API int mstar_delta_scan_pieces(const float* q, const float* k, const floa
 // sigmoid or the SiLU; a warp per (token, head).  V: elements an access; a lane keeps up to four
 // accesses' worth of its head in registers.  Results that are rounded to bfloat16 take the quotient of
 // 2 ulp, as the other gates do: 12.0 us for 2,048 tokens of 16 heads of 128, 13.8 with the IEEE division.
-template <typename A> __device__ __forceinline__ float gd_quotient(float x, float y) {
-    if constexpr (sizeof(A) == 2) return __fdividef(x, y);
-    else return x / y;
+template <typename A> __device__ __forceinline__ float gd_over_one_plus(float x, float e) {
+    if constexpr (sizeof(A) == 2) return over_one_plus_bf16(x, e);
+    else return x / (1.f + e);
 }
 template <typename A, typename T, int V>
 __global__ void delta_finish_kernel(const float* o, const T* gate, int gate_stride,
@@ -1227,7 +1227,7 @@ __global__ void delta_finish_kernel(const float* o, const T* gate, int gate_stri
                 load_v<V>(weight + j, w);
 #pragma unroll
                 for (int e = 0; e < V; ++e)
-                    v[i][e] = gd_quotient<A>(v[i][e] * inv * w[e], 1.f + expf(-z[i][e])) * (silu ? z[i][e] : 1.f);
+                    v[i][e] = gd_over_one_plus<A>(v[i][e] * inv * w[e], expf(-z[i][e])) * (silu ? z[i][e] : 1.f);
                 store_v<V>(dst + j, v[i]);
             }
         }
@@ -1237,7 +1237,7 @@ __global__ void delta_finish_kernel(const float* o, const T* gate, int gate_stri
     const float inv = rsqrtf(warp_sum(ss) / (float)vdim + eps) * scale;
     for (int j = lane; j < vdim; j += 32) {
         const float z = to_float(g[j]);
-        dst[j] = from_float<A>(gd_quotient<A>(row[j] * inv * weight[j], 1.f + expf(-z)) * (silu ? z : 1.f));
+        dst[j] = from_float<A>(gd_over_one_plus<A>(row[j] * inv * weight[j], expf(-z)) * (silu ? z : 1.f));
     }
 }
 

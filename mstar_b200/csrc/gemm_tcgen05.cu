@@ -597,7 +597,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
                         // 2: the clamped swish.  (Not the IEEE division, as in silu_bf16: tiles of
                         // [1500, 3072] x [16384, 3072] took 141 us with it and take 120)
                         r[i] = __float_as_uint(gate_act == 2 ? clamped_swish_bf16(g, v, limit, alpha)
-                                                             : __fdividef(g, 1.f + expf(-z)) * v);
+                                                             : over_one_plus_bf16(g, expf(-z)) * v);
                     }
                     const int col = n0 + c0;
                     if (row < M && col < N)

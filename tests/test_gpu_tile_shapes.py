@@ -135,6 +135,18 @@ def test_gated_products_by_eight_and_one_by_one(dtype, rows, inter):
     assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-30).all()
 
 
+@pytest.mark.parametrize("g", [-86.0, -87.5, -88.0, -88.5])
+def test_gates_whose_exponential_nears_the_largest_float(g):
+    """The denominator 1 + exp(-g) lies around 2^126 and above, the product within bfloat16's range."""
+    from mstar_b200 import ops
+
+    x = torch.full((1, 16), g, dtype=torch.bfloat16, device=DEV)
+    x[0, 8:] = 2.0 ** 20
+    want = g / (1 + torch.tensor(-g, dtype=torch.float64).exp()) * 2.0 ** 20
+    got = ops.silu_mul(x).double()
+    assert ((got - want).abs() <= 2.0 ** -8 * abs(want)).all()
+
+
 @pytest.mark.parametrize("lens,heads,kv_heads,dim,vdim", [
     ([70], 2, 1, 32, 8),                    # a piece of 6 tokens at the end, 8 columns
     ([64, 1, 33], 2, 2, 64, 20),            # columns that end inside a block, an entry of one token
