@@ -1129,7 +1129,7 @@ template <int D> static int launch_head_scan_kind(const DeltaHeadArgs& a, int en
     return channel ? launch_head_scan_cols<D, true>(a, entries, s) : launch_head_scan_cols<D, false>(a, entries, s);
 }
 
-// The scan in pieces, for key sizes of 32, 64, 96, 128 or 256.  head_decay: `decay` is [tokens][H] and `work`
+// The scan in pieces, for key sizes of 32, 64, 128 or 256, with one decay a head 96 as well.  head_decay: `decay` is [tokens][H] and `work`
 // holds (tokens / 16 + entries) * (G * 32 * (D + 4) + H * 16 * 36) floats; else `decay` is [tokens][H][D]
 // and `work` holds (tokens / 16 + entries) * H * (49 * (D + 4) + 16 * 36).  Returns 0, a CUDA error code,
 // or -1 when the shape is refused.
@@ -1143,7 +1143,7 @@ MSTAR_API int mstar_delta_scan_pieces(const float* q, const float* k, const floa
                                       void* stream) {
     if (entries <= 0 || tokens <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || VD <= 0) return -1;
-    if (D != 32 && D != 64 && D != 96 && D != 128 && D != 256) return -1;
+    if (D != 32 && D != 64 && D != 128 && D != 256 && !(D == 96 && head_decay)) return -1;
     if (H > 65535 || entries > 65535 || (state_offset % 4) != 0 || (state_stride % 4) != 0) return -1;
     if ((uintptr_t)q % 16 || (uintptr_t)k % 16 || (uintptr_t)work % 16 || (uintptr_t)state % 16 || !error_word ||
         (!head_decay && (uintptr_t)decay % 16))
@@ -1178,7 +1178,7 @@ MSTAR_API int mstar_delta_scan_pieces(const float* q, const float* k, const floa
     if (code != 0) return code;
     if (D == 32) return launch_head_scan_kind<32>(a, entries, !head_decay, s);
     if (D == 64) return launch_head_scan_kind<64>(a, entries, !head_decay, s);
-    if (D == 96) return launch_head_scan_kind<96>(a, entries, !head_decay, s);
+    if (D == 96) return launch_head_scan_cols<96, false>(a, entries, s);
     if (D == 128) return launch_head_scan_kind<128>(a, entries, !head_decay, s);
     return launch_head_scan_kind<256>(a, entries, !head_decay, s);
 }
