@@ -170,7 +170,8 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
                    q_ready = tc_smem(bars + 12);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
 
-    // grid: x (split, kv head, row tile), the row tiles with the most keys first; z the entry.  `fold`: all
+    // grid: x (split, kv head, row tile), the last row tile first (the most keys, where there are no chunks); z
+    // the entry.  `fold`: all
     // CTAs run at once, two an SM: from this rank on the order is turned round, so that the CTA that
     // shares its SM with the longest is the shortest.
     int rank = blockIdx.x;
@@ -803,17 +804,17 @@ latent_gather_kernel(const uint4* __restrict__ cache, const int* __restrict__ bl
 }
 
 // parts[row][head][k head | k remainder | v head | v remainder] from the float products
-// keys[row][head][dim] and values; eight features a thread.
+// keys[row][head][dim] and values, rows `ld` floats apart; eight features a thread.
 __global__ void __launch_bounds__(256)
 latent_split_kernel(const float* __restrict__ keys, const float* __restrict__ values, bf16* __restrict__ parts,
-                    long long pieces, int heads, int dim) {
+                    int ld, long long pieces, int heads, int dim) {
     const int per_head = dim / 8, per_row = 2 * heads * per_head;
     for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < pieces; i += (long long)gridDim.x * 256) {
         const long long row = i / per_row;
         const int at = (int)(i - row * per_row), which = at / (heads * per_head);
         const int head = at / per_head - which * heads, d = at % per_head * 8;
         float v[8], rest[8];
-        load8((which ? values : keys) + (row * heads + head) * dim + d, v);
+        load8((which ? values : keys) + row * ld + head * dim + d, v);
 #pragma unroll
         for (int k = 0; k < 8; ++k) rest[k] = v[k] - __bfloat162float(__float2bfloat16_rn(v[k]));
         bf16* dst = parts + ((row * heads + head) * 4 + 2 * which) * dim + d;
@@ -835,14 +836,14 @@ MSTAR_API int mstar_latent_gather(const void* cache, const int* block_table, int
     return launch_status();
 }
 
-MSTAR_API int mstar_latent_split(const float* keys, const float* values, void* parts, int rows, int heads, int dim,
-                                 void* stream) {
+MSTAR_API int mstar_latent_split(const float* keys, const float* values, int ld, void* parts, int rows, int heads,
+                                 int dim, void* stream) {
     if (rows <= 0) return 0;
-    if (dim % 8 != 0 || (((uintptr_t)keys | (uintptr_t)values | (uintptr_t)parts) & 15) != 0) return -1;
+    if (dim % 8 != 0 || ld % 4 != 0 || (((uintptr_t)keys | (uintptr_t)values | (uintptr_t)parts) & 15) != 0) return -1;
     const long long pieces = (long long)rows * 2 * heads * (dim / 8);
     const long long blocks = (pieces + 255) / 256, most = (long long)device_sm_count() * 16;
     latent_split_kernel<<<(unsigned)(blocks < most ? blocks : most), 256, 0, (cudaStream_t)stream>>>(
-        keys, values, (bf16*)parts, pieces, heads, dim);
+        keys, values, (bf16*)parts, ld, pieces, heads, dim);
     return launch_status();
 }
 

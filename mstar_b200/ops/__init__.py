@@ -1220,18 +1220,16 @@ def latent_attention_prompt(q: torch.Tensor, cache: torch.Tensor, block_table, c
                             heads: int, dim: int, rank: int, rot: int, page_size: int, window: int,
                             scale: float, out: torch.Tensor, gate=None, room: int | None = None) -> None:
     """Latent attention of prompt portions on tcgen05: for each of ``groups`` (see
-    ``latent_prompt_groups``) the latent rows its tokens see are gathered, products with ``w_kv`` (the
-    key rows of all heads and the value rows, [heads * dim, rank] each, or both in one matrix) make the
-    keys and values in float, of as many heads at once as ``room`` bytes hold; they enter the attention
-    in two bfloat16 parts.  ``q``: [tokens, heads,
-    dim + rot], rotated; writes the groups' rows of ``out`` [tokens, heads * dim], times the sigmoid
+    ``latent_prompt_groups``) the latent rows its tokens see are gathered, and products with ``w_kv``
+    [2 * heads * dim, rank] (the key rows of all heads, then the value rows) make the keys and values in
+    float, of as many heads at once as ``room`` bytes hold; they enter the attention in two bfloat16
+    parts.  ``q``: [tokens, heads, dim + rot], rotated; writes the groups' rows of ``out`` [tokens,
+    heads * dim], times the sigmoid
     of ``gate`` (float [tokens, heads]) where given."""
-    w_k, w_v = w_kv.view(2, -1, rank) if isinstance(w_kv, torch.Tensor) else w_kv
     room = LATENT_PROMPT_BYTES if room is None else room
-    _need_cuda(q, cache, block_table, w_k, w_v, out, gate)
+    _need_cuda(q, cache, block_table, w_kv, out, gate)
     assert out.is_contiguous() and out.dtype == torch.bfloat16 and cache.is_contiguous()
-    for w in (w_k, w_v):
-        assert tuple(w.shape) == (heads * dim, rank) and w.is_contiguous()
+    assert tuple(w_kv.shape) == (2 * heads * dim, rank) and w_kv.is_contiguous()
     assert gate is None or (gate.dtype == torch.float32 and gate.stride(1) == 1)
     dev, entry = q.device, lib.get("attention_prompt_tc")
     starts = [0]
@@ -1248,12 +1246,17 @@ def latent_attention_prompt(q: torch.Tensor, cache: torch.Tensor, block_table, c
         per_pass = -(-heads // passes)
         for h0 in range(0, heads, per_pass):
             some = min(per_pass, heads - h0)
-            made_k, made_v = (linear(rows[:, :rank], w if passes == 1 else w[h0 * dim:(h0 + some) * dim],
-                                     out_dtype=torch.float32) for w in (w_k, w_v))
+            if passes == 1:
+                made = linear(rows[:, :rank], w_kv, out_dtype=torch.float32)
+                made_k, made_v, ld = made.data_ptr(), made.data_ptr() + 4 * heads * dim, 2 * heads * dim
+            else:
+                made = [linear(rows[:, :rank], w_kv[at:at + some * dim], out_dtype=torch.float32)
+                        for at in (h0 * dim, (heads + h0) * dim)]
+                made_k, made_v, ld = made[0].data_ptr(), made[1].data_ptr(), some * dim
             parts = torch.empty((keys, some, 4 * dim), dtype=torch.bfloat16, device=dev)
-            check(entry.mstar_latent_split(made_k.data_ptr(), made_v.data_ptr(), parts.data_ptr(), keys, some, dim,
-                                           _stream()), "latent_split")
-            del made_k, made_v
+            check(entry.mstar_latent_split(made_k, made_v, ld, parts.data_ptr(), keys, some, dim, _stream()),
+                  "latent_split")
+            del made
             ctas = some * -(-max(q_lens) // PROMPT_ROWS) * count
             splits = prompt_splits(ctas, min(max(ctx.kv_lens[first:first + count]),
                                              window + max(q_lens) if window else 1 << 30), num_sms(dev))

@@ -86,7 +86,7 @@ _SIGNATURES = {
         "mstar_sink_attention_prompt": [_vp, _vp, _i, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i,
                                         _i, _i, _f, _i, _vp, _vp, _i, _i, _f, _vp, _i, _i, _vp, _vp, _vp],
         "mstar_latent_gather": [_vp, _vp, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp],
-        "mstar_latent_split": [_vp, _vp, _vp, _i, _i, _i, _vp],
+        "mstar_latent_split": [_vp, _vp, _i, _vp, _i, _i, _i, _vp],
         "mstar_latent_attention_prompt": [_vp, _i, _i, _i, _vp, _vp, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i,
                                           _i, _i, _i, _i, _i, _i, _f, _i, _vp, _vp, _i, _vp, _vp],
     },

@@ -69,7 +69,13 @@ class LatentAttention:
     @classmethod
     def workspace_bytes(cls, spec, dtype: torch.dtype) -> int:
         """What a step may need beside its activations (made keys and values of prompts)."""
-        return ops.LATENT_PROMPT_BYTES if dtype == torch.bfloat16 and spec.qk_dim == spec.v_dim else 0
+        return ops.LATENT_PROMPT_BYTES if cls._makes_keys(spec, dtype) else 0
+
+    @staticmethod
+    def _makes_keys(spec, dtype: torch.dtype) -> bool:
+        """Whether prompts may take the form with made keys and values (sizes that its kernel takes)."""
+        return (dtype == torch.bfloat16 and spec.qk_dim == spec.v_dim and spec.qk_dim in (64, 128)
+                and spec.kv_rank % 8 == 0)
 
     def __init__(self, spec, params: dict, runtime: Runtime):
         p = spec.position
@@ -92,11 +98,15 @@ class LatentAttention:
         if spec.q_rank is not None:
             self.w_uq = params["uq.weight"]
             self.q_norm_weight = params["q_norm.weight"].float().contiguous()
+        # all heads' key rows, then their value rows: prompts make both in one product.  The parameters become
+        # the two halves of this matrix, so that neither lies in memory twice.
+        self.w_kv = None
+        if self._makes_keys(spec, runtime.dtype):
+            self.w_kv = torch.cat([params["uk.weight"], params["uv.weight"]])
+            params["uk.weight"].data, params["uv.weight"].data = self.w_kv.chunk(2)
         # per head: [rank, qk_dim] rows so that a = q @ uk_t[h]^T, and [v_dim, rank]
         self.uk_t = params["uk.weight"].view(h, spec.qk_dim, spec.kv_rank).transpose(1, 2).contiguous()
         self.uv = params["uv.weight"].view(h, spec.v_dim, spec.kv_rank)
-        # prompts make keys and values from the latents (the parameters as they are, no copies)
-        self.w_kv = (params["uk.weight"].contiguous(), params["uv.weight"].contiguous())
         half = p.rotary_dim // 2
         self.freq = torch.tensor([p.theta ** (-(2.0 * i) / p.rotary_dim) for i in range(half)],
                                  dtype=torch.float64, device=runtime.device)
@@ -130,7 +140,8 @@ class LatentAttention:
             gate = proj[:, s.q_rank + down:]
         q = q.view(-1, h, per_head)
         groups, room = [], 0
-        if ctx.max_q_len > 1 and ops.latent_prompt_takes(q, cache.kv, s.qk_dim, s.v_dim, s.kv_rank, s.rot_dim):
+        if (ctx.max_q_len > 1 and self.w_kv is not None
+                and ops.latent_prompt_takes(q, cache.kv, s.qk_dim, s.v_dim, s.kv_rank, s.rot_dim)):
             room = ops.latent_prompt_room(ctx.q_lens, h, s.kv_rank)
             groups = ops.latent_prompt_groups(ctx.q_lens, ctx.kv_lens, s.window or 0, h * s.v_dim,
                                               ctx.num_decode, h, room)

@@ -364,6 +364,7 @@ def test_latent_layer_in_mixed_steps(window, gate_per_head, monkeypatch):
     from mstar_b200 import ops
 
     part, row = latent_layer(1, heads=8, window=window, gate_per_head=gate_per_head)
+    assert part.uv.data_ptr() == part.w_kv[8 * 64:].data_ptr()       # no second copy
     lens_q, lens_kv = {0: 1, 1: 1, 2: 100, 3: 20, 4: 70}, {0: 50, 1: 300, 2: 100, 3: 220, 4: 400}
     x = {n: rnd(q, 128, dtype=torch.bfloat16, seed=50 + n) for n, q in lens_q.items()}
     seen = []
