@@ -248,12 +248,14 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
                 pt_tma_load_4d(tc_smem(q_s + b * (PA_ROWS * 128)), &q_map, q_ready, b * 64, 0, kvh, q_start + tok0);
         }
         bool ok = true;
+        int asked = 0;                                  // tiles whose copies have been asked for
         if (LATENT) {
             const int row0 = pa_latent_base(a.qo_indptr, a.kv_len, a.first_entry, blockIdx.z, a.window) -
                              pa_latent_first(past, a.window);
             const int blocks = which ? VB : KB;
             for (int j = 0; j < ntiles; ++j) {
                 const int s = j & 1;
+                asked = j + 1;
                 if (lane < blocks) {
                     if (!mbar_wait(empty0 + 8 * s, (((uint32_t)j >> 1) & 1u) ^ 1u)) {
                         atomicExch(error_word, 23);
@@ -284,6 +286,7 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
             int mine = 0, have_from = -1;               // lanes hold pages have_from .. +31
             for (int j = 0; j < ntiles; ++j) {
                 const int s = j & 1;
+                asked = j + 1;
                 const int key0 = tile_key(j);
                 const int base_page = key0 >> ps_log;
                 if (have_from < 0 || base_page + per_tile > have_from + 32) {
@@ -306,6 +309,11 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
                 if (!__all_sync(0xffffffffu, ok)) break;
             }
         }
+        // no copy outlives the CTA, whatever became of its reader
+        if (lane == 0) {
+            if (which == 0 && ntiles > 0) mbar_wait(q_ready, 0);
+            for (int j = max(0, asked - 2); j < asked; ++j) mbar_wait(full0 + 8 * (j & 1), ((uint32_t)j >> 1) & 1u);
+        }
     } else if (warp == 4) {
         // ------------------------------------------------ S = Q K^T, a tile ahead of the softmax
         if (lane == 0 && ntiles > 0) {
@@ -313,7 +321,8 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
             const uint32_t q_addr = tc_smem(q_s);
             bool q_there = mbar_wait(q_ready, 0);
             if (!q_there) atomicExch(error_word, 24);
-            for (int j = 0; j < ntiles && q_there; ++j) {
+            int j = 0;
+            for (; j < ntiles && q_there; ++j) {
                 const int s = j & 1;
                 const uint32_t parity = ((uint32_t)j >> 1) & 1u;
                 // the buffer is free once O += P V of tile j-2, which read P from it, is done
@@ -338,11 +347,14 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
                 pt_commit(s_full + 8 * s);
                 pt_commit(k_empty + 8 * s);
             }
+            // ... nor a product
+            if (j > 0) mbar_wait(k_empty + 8 * ((j - 1) & 1), ((uint32_t)(j - 1) >> 1) & 1u);
         }
     } else if (warp == 6) {
         // ------------------------------------------------ O += P V, V the N-major operand
         constexpr uint32_t idesc_o = pt_idesc(PA_ROWS, HD, 1);
-        for (int j = 0; j < ntiles; ++j) {
+        int j = 0;
+        for (; j < ntiles; ++j) {
             const int s = j & 1;
             const uint32_t parity = ((uint32_t)j >> 1) & 1u;
             if (!pt_wait_warp(v_full + 8 * s, parity)) {
@@ -390,6 +402,7 @@ prompt_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid
             }
             __syncwarp();
         }
+        if (lane == 0 && j > 0) mbar_wait(v_empty + 8 * ((j - 1) & 1), ((uint32_t)(j - 1) >> 1) & 1u);
     } else if (warp < 4) {
         // ------------------------------------------------------ softmax, one row per thread
         const int r = tid;                              // row of the tile = TMEM lane

@@ -625,6 +625,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 }
                 if (*(volatile int*)&abort_flag) break;
             }
+            // no copy outlives the CTA, whatever became of its reader
+            for (uint32_t k = it > GG_STAGES ? it - GG_STAGES : 0; k < it; ++k)
+                mbar_wait(tc_smem(&full_bar[k % GG_STAGES]), (k / GG_STAGES) & 1u);
         }
     } else if (GATHER && warp >= 6) {
         constexpr int LAG = 2;                          // k-blocks between asking and telling
@@ -704,6 +707,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 }
                 if (ok) tc_commit(tc_smem(&acc_full[b]));
             }
+            // ... nor a product
+            if (it > 0) mbar_wait(tc_smem(&empty_bar[(it - 1) % GG_STAGES]), ((it - 1) / GG_STAGES) & 1u);
         }
     } else {
         const int quarter = warp & 3;                   // the TMEM lanes this warp may touch
