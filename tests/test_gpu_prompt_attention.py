@@ -70,7 +70,9 @@ FORMS = {
     ([130, 17], [130, 300], 4, 1, 64, 16),       # a row tile and one row more; keys shared among CTAs
     ([50], [333], 6, 2, 128, 8),                 # a group of 3: 126 of 128 rows
     ([300], [300], 1, 1, 128, 64),               # one head a group
-    ([40, 40, 64], [40, 200, 64], 16, 8, 64, 32)])
+    ([40, 40, 64], [40, 200, 64], 16, 8, 64, 32),
+    ([1, 130, 1], [290, 300, 33], 4, 1, 64, 128),    # pages of several tiles; single tokens beside a portion
+    ([70, 1], [600, 257], 4, 2, 128, 256)])
 def test_prompt_attention_with_options(form, lens_q, lens_kv, nq, nkv, hd, page, monkeypatch):
     from mstar_b200 import ops
 
