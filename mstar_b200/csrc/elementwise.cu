@@ -515,7 +515,10 @@ MSTAR_API int mstar_silu_mul(const void* gate_up, void* out, int act_dtype, int 
     if (kind < 1 || kind > 3) return -1;
     cudaStream_t s = (cudaStream_t)stream;
     const int threads = 256;
-    if (inter % 8 == 0 && (((uintptr_t)gate_up | (uintptr_t)out) & 15) == 0) {
+    // eight columns a thread where there are enough of them: [64, 2048] in bfloat16 1.57 us against 1.64 a column
+    // a thread, [8, 8192] 1.54 against 1.42; float [33, 8192] 1.90 against 2.14, [64, 2048] 1.86 against 1.61
+    const size_t many = act_dtype == MSTAR_F32 ? 1u << 18 : 1u << 17;
+    if (inter % 8 == 0 && total >= many && (((uintptr_t)gate_up | (uintptr_t)out) & 15) == 0) {
         const dim3 grid((inter / 8 + 255) / 256, rows < 65535 ? rows : 65535);
         if (act_dtype == MSTAR_F32)
             mstar_launch((silu_mul_vec_kernel<float>), grid, dim3(threads), 0, s, (const float*)gate_up, (float*)out, inter, rows, kind, limit, alpha);

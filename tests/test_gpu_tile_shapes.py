@@ -111,7 +111,7 @@ def test_grouped_experts_at_the_borders_of_their_tiles(tokens, width, ff, expert
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("rows,inter", [(3, 8), (5, 2056), (2, 12)])
+@pytest.mark.parametrize("rows,inter", [(3, 8), (5, 2056), (2, 12), (70, 4104), (17000, 16)])
 def test_gated_products_by_eight_and_one_by_one(dtype, rows, inter):
     """Widths of whole 16-byte pieces and others, zeros and large gates among them."""
     from mstar_b200 import ops
@@ -140,8 +140,8 @@ def test_gates_whose_exponential_nears_the_largest_float(g):
     """The denominator 1 + exp(-g) lies around 2^126 and above, the product within bfloat16's range."""
     from mstar_b200 import ops
 
-    x = torch.full((1, 16), g, dtype=torch.bfloat16, device=DEV)
-    x[0, 8:] = 2.0 ** 20
+    x = torch.full((17000, 16), g, dtype=torch.bfloat16, device=DEV)      # (enough for eight columns a thread)
+    x[:, 8:] = 2.0 ** 20
     want = g / (1 + torch.tensor(-g, dtype=torch.float64).exp()) * 2.0 ** 20
     got = ops.silu_mul(x).double()
     assert ((got - want).abs() <= 2.0 ** -8 * abs(want)).all()
