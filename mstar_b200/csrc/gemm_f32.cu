@@ -52,6 +52,25 @@ sgemm_nt_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
                 if (ok) src += (size_t)row * (is_a ? lda : ldw) + k;
                 cp_async_16(smem_u32(dst + r * LD + (c % PER_ROW) * 4), src, ok ? 16 : 0);
             }
+        } else if (THREADS % BK == 0) {
+            // a thread keeps its place in k and walks down the rows, of A, then of W
+            constexpr int STEP = THREADS / BK > 0 ? THREADS / BK : 1;
+            const int k = k0 + tid % BK, r0 = tid / BK;
+            const bool in = k < K;
+            const float* src = A + (size_t)(m0 + r0) * lda + k;
+            uint32_t to = smem_u32(dst + r0 * LD + tid % BK);
+#pragma unroll 8
+            for (int r = r0; r < BM; r += STEP, src += (size_t)STEP * lda, to += STEP * LD * 4) {
+                const bool ok = in && m0 + r < M;
+                cp_async_4(to, ok ? src : A, ok ? 4 : 0);
+            }
+            src = W + (size_t)(n0 + r0) * ldw + k;
+            to = smem_u32(dst + (BM + r0) * LD + tid % BK);
+#pragma unroll 8
+            for (int r = r0; r < BN; r += STEP, src += (size_t)STEP * ldw, to += STEP * LD * 4) {
+                const bool ok = in && n0 + r < N;
+                cp_async_4(to, ok ? src : W, ok ? 4 : 0);
+            }
         } else {
             for (int c = tid; c < (BM + BN) * BK; c += THREADS) {
                 const int r = c / BK, k = k0 + c % BK;
