@@ -526,9 +526,9 @@ selective_scan_kernel(const A* __restrict__ xc, const A* __restrict__ xz,
 // state as it is.  The output sums of four tokens meet in one exchange among the lanes, each of which
 // then finishes one token.  Bound by the exponential (one ex2 per state and token: 30 us for 2,048 tokens x
 // 4,096 channels at 16 a cycle and SM) and by one warp a scheduler where channels are few.
-// 2 x 1,024 tokens, 4,096 channels, pieces of 128: 45 + 63 us for the two passes (57 + 89 with the step sizes made
-// in both, the copies' addresses made anew for every chunk and every token asked for its place in it:
-// instructions took 82 % of the issue slots); the kernel above takes 203 us each (a 4-byte copy for every
+// 2 x 1,024 tokens, 4,096 channels, pieces of 64: 49 + 69 us for the two passes one at a time with cold caches (64
+// + 94 with the step sizes made in both, the copies' addresses made anew for every chunk and every token asked
+// for its place in it: instructions took 82 % of the issue slots); the kernel above takes 203 us each (a 4-byte copy for every
 // number of the rows, two 4-byte loads of B and C a state, exp2f).
 #define SX_STAGES 3
 

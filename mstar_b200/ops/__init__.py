@@ -1266,8 +1266,9 @@ def latent_attention_prompt(q: torch.Tensor, cache: torch.Tensor, block_table, c
             code = entry.mstar_latent_attention_prompt(
                 q.data_ptr() + 2 * h0 * q.stride(1), q.stride(0), q.stride(1), q.shape[0], parts.data_ptr(),
                 rows.data_ptr(), keys, out.data_ptr() + 2 * h0 * dim, ctx.qo_indptr.data_ptr(),
-                ctx.kv_len.data_ptr(), first, count, max(q_lens), starts[first], starts[first + count] - starts[first], some, heads, dim, rank, rot, window,
-                float(scale), splits, _ptr(scratch), gate.data_ptr() + 4 * h0 if gate is not None else 0,
+                ctx.kv_len.data_ptr(), first, count, max(q_lens), starts[first],
+                starts[first + count] - starts[first], some, heads, dim, rank, rot, window, float(scale), splits,
+                _ptr(scratch), gate.data_ptr() + 4 * h0 if gate is not None else 0,
                 gate.stride(0) if gate is not None else 0, tcgen05_error_word(dev).data_ptr(), _stream())
             if code < 0:
                 raise KernelError(f"latent prompt attention refuses heads={heads}, dim={dim}, rank={rank}, "
@@ -1583,8 +1584,13 @@ def sink_attention_splits(entries: int, max_q_len: int, num_heads: int, num_kv_h
     return max(1, min(room // ctas, -(-max_keys // 64) // 2, 64))
 
 
-# query rows of an entry (token x head of the group) from which on the tcgen05 prompt kernel takes an
-# attention with options, and its rows a CTA and keys a tile
+# query rows of an entry (token x head of the group) beyond which the tcgen05 prompt kernel takes an
+# attention with options, and its rows a CTA and keys a tile.  Under a cap, one entry / eight entries of 68
+# rows over 300 and 2,048 keys, 16 / 4 heads of 128: 18 and 26 / 20 and 32 us (mma.sync 36 and 38 / 38 and 79),
+# 8 / 2 heads of 64: 18 and 22 / 18 and 24 (28 and 26 / 28 and 38).  It is ahead from 32 rows on (16 to 32
+# against 24 to 67 us); fewer than a tile of the other kernel's rows stay with what decoding takes.
+# Whole prompts, 2,048 tokens of 16 / 4 heads of 128: cap 70 us (226), chunks of 1,024 with sigmoid weights 52
+# (127), window of 512 with and without 4 kept keys 31 (115, 109); 1,024 tokens in one chunk 41 (93).
 PROMPT_MIN_ROWS = 64
 PROMPT_ROWS, PROMPT_KEYS = 128, 64
 
