@@ -255,8 +255,8 @@ sample_kernel(const float* __restrict__ logits, int ld, int vocab,
 // few logits they decide by themselves, in a list (cs_pick_few), instead of two more rounds of three
 // cluster barriers; sums have shared words of their own, which spares the barriers behind their reads.
 // 157 k logits with temperature, top-p and a repetition penalty: 85 us for 64 rows (108 with three rounds, 121
-// with every key made in every pass); with one CTA an SM and the histograms added into rank 0 by remote
-// atomics 61 us for up to 18 and 294 us for 64.
+// with every key made in every pass); with cold caches 39, 41, 47 and 90 us for 1, 8, 18 and 64 rows, where one
+// CTA an SM and the histograms added into rank 0 by remote atomics took 66, 66, 123 and 292.
 #define CS_CLUSTER 8
 #define CS_THREADS 512
 #define CS_BINS 2048
