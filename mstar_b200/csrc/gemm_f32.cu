@@ -1,5 +1,6 @@
 // C[M,N] = A[M,K] * W[N,K]^T in true 32-bit: float inputs, float FMA accumulation on
-// CUDA cores, no tensor-core mode of reduced precision.  This is the matrix product
+// CUDA cores, no tensor-core mode of reduced precision (gemm_f32_tc.cu: the same by parts on the tensor cores
+// for wide matrices, chosen at the end of this file).  This is the matrix product
 // of the float32 path of the whole model (the reference has no such path: it lets
 // float matmuls run as TF32, mstar/engine/__init__.py:6).
 //
@@ -15,6 +16,7 @@
 // row-major order; rows are BK + 4 floats apart in shared memory, so that eight threads reading
 // 16 bytes of eight neighbouring rows meet no bank twice, and nothing has to be transposed.
 #include "common.cuh"
+#include "gemm_f32.h"
 #include "mma_util.cuh"
 
 __device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
@@ -154,9 +156,14 @@ static int launch_sgemm(const float* A, const float* W, float* C, int M, int N, 
 }
 
 MSTAR_API int mstar_sgemm_nt(const float* A, const float* W, float* C, int M, int N, int K,
-                             int lda, int ldw, int ldc, void* stream) {
+                             int lda, int ldw, int ldc, int* error, void* stream) {
     if (M <= 0 || N <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
+    // Wide matrices of aligned rows go to the tensor cores, three bfloat16 parts a float (gemm_f32_tc.cu, with both
+    // sides measured; no error word: never).  From K = 512 on: the start and end of a tile there take some
+    // 8 us, as long as the FMAs of a shorter row ([1536, 128] x [4096, 128]: 47 to 49 against 50 us).
+    if (error != nullptr && sgemm_parts_takes(A, W, N, K, lda, ldw))
+        return sgemm_parts(A, W, C, M, N, K, lda, ldw, ldc, 0, 0, error, s);
     const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
                      ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0;
     const int sms = device_sm_count();

@@ -449,7 +449,7 @@ def sgemm_nt(a: torch.Tensor, w: torch.Tensor, out=None):
     assert out.stride(1) == 1
     check(lib.get("gemm_f32").mstar_sgemm_nt(
         a.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, a.stride(0), w.stride(0),
-        out.stride(0), _stream()), "sgemm_nt")
+        out.stride(0), tcgen05_error_word(a.device).data_ptr(), _stream()), "sgemm_nt")
     return out
 
 
@@ -595,7 +595,7 @@ def tcgen05_error_word(device) -> torch.Tensor:
     1-3 tcgen05 GEMM (producer, MMA issuer, epilogue), 4 decode attention copies, 6-12 tcgen05
     prefill attention, 13-14 bulk-copy small-M GEMM, 15-17 swapped-operand tcgen05 GEMM, 18
     delta-rule scan in pieces, 19-21 grouped expert GEMM, 22-27 prompt attention with probabilities
-    in three parts; zero otherwise."""
+    in three parts, 28-29 float product by bfloat16 parts; zero otherwise."""
     key = torch.device(device).index or 0
     if key not in _tc_error_words:
         _tc_error_words[key] = torch.zeros(1, dtype=torch.int32, device=device)
@@ -620,6 +620,8 @@ WAIT_CODES.update({19: "grouped expert GEMM: the producer waited for a free stag
                    21: "grouped expert GEMM: the epilogue waited for an accumulator"})
 WAIT_CODES.update({c: "prompt attention with probabilities in three parts: a wait on one of its barriers "
                    "ran out" for c in range(22, 28)})
+WAIT_CODES.update({28: "float product by bfloat16 parts: a worker waited for a stage or a sum",
+                   29: "float product by bfloat16 parts: the MMA issuer waited for operands"})
 WAIT_CODES.update({c: "tcgen05 prefill attention: a wait on one of its barriers ran out"
                    for c in range(6, 13)})
 

@@ -136,7 +136,8 @@ _SIGNATURES = {
                                              _i, _i, _i, _i, _f, _vp, _vp],
     },
     "gemm_f32": {
-        "mstar_sgemm_nt": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp],
+        "mstar_sgemm_nt": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp],
+        "mstar_sgemm_parts": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp],
     },
     "gemm_smallm_bulk": {
         "mstar_gemm_smallm_bulk_bf16": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _f, _f,

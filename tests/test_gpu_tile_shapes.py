@@ -27,6 +27,59 @@ def test_sgemm_at_the_borders_of_its_tiles(m, n, k, off):
     assert torch.equal(ops.sgemm_nt(a[m - 1:], w), got[m - 1:])
 
 
+def _sgemm(a, w, *tile):
+    """The FMA kernel, or with (bn, cluster) the tensor-core kernel with that tile; None: refused."""
+    from mstar_b200 import ops
+    from mstar_b200.ops import lib
+
+    out = torch.full((a.shape[0], w.shape[0]), float("nan"), device=DEV)
+    args = (a.data_ptr(), w.data_ptr(), out.data_ptr(), a.shape[0], w.shape[0], a.shape[1], a.stride(0),
+            w.stride(0), out.stride(0)) + tile
+    word = ops.tcgen05_error_word(DEV).data_ptr() if tile else 0
+    fn = lib.get("gemm_f32").mstar_sgemm_parts if tile else lib.get("gemm_f32").mstar_sgemm_nt
+    code = fn(*args, word, torch.cuda.current_stream().cuda_stream)
+    assert code in (0, -1)
+    return out if code == 0 else None
+
+
+# one row, a row past every tile width, the last tile of W shifted back by all but one row, K that ends inside
+# a block, inside a slice and on its border, longer slices
+@pytest.mark.parametrize("m,n,k,pad", [(1, 128, 512, 0), (17, 129, 516, 4), (80, 300, 1000, 0), (81, 255, 2112, 0),
+                                       (33, 256, 4100, 8), (200, 640, 1024, 0)])
+def test_sgemm_by_parts(m, n, k, pad):
+    """Three bfloat16 parts a float: no further from 64 bits than the FMA kernel, the same bits from every
+    tile, however K is shared, and for a row alone."""
+    from mstar_b200 import ops
+
+    a, w = rnd(m, k + pad, seed=5)[:, :k], rnd(n, k + pad, seed=6)[:, :k]
+    want = a.double() @ w.double().T
+    got = ops.sgemm_nt(a, w)
+    far = lambda c: ((c.double() - want).norm() / want.norm()).item()
+    assert far(got) <= far(_sgemm(a, w))
+    # every sum into an accumulator cuts off at most a last place (2^-23) of what is there, every sum of
+    # slices rounds: at most K / 16 + 16 of them
+    assert ((got.double() - want).abs() <= 2 ** -23 * (k / 16 + 16) * (a.double().abs() @ w.double().abs().T)).all()
+    assert torch.equal(ops.sgemm_nt(a[m - 1:], w), got[m - 1:])
+    tiles = [_sgemm(a, w, bn, cluster) for bn in (16, 32, 48, 64, 80) for cluster in (1, 2, 4, 8)]
+    assert all(torch.equal(t, got) for t in tiles if t is not None) and sum(t is not None for t in tiles) >= 6
+    ops.check_error_word(DEV)
+
+
+@pytest.mark.parametrize("m,k", [(5, 512), (100, 2048)])
+def test_sgemm_by_parts_keeps_infinities(m, k):
+    from mstar_b200 import ops
+
+    a, w = rnd(m, k, seed=7), rnd(256, k, seed=8).bfloat16().float()     # parts of w that are zero
+    a[1, 3], a[2, 100], a[3, 40], a[3, 300] = float("inf"), float("nan"), float("inf"), -float("inf")
+    a[4, 7], w[9, 7] = 3.4e38, 0.5               # its first part would round to an infinity
+    w[11, 5], w[12, 6] = -float("inf"), float("nan")
+    got, want = ops.sgemm_nt(a, w), _sgemm(a, w)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    both = want.isfinite()
+    assert torch.equal(got[want.isinf()], want[want.isinf()]) and both[0].sum() == 254 and both[4].any()
+    torch.testing.assert_close(got[both], want[both], rtol=1e-5, atol=1e-3)
+
+
 @pytest.mark.parametrize("lens_q,lens_kv,nq,nkv,hd,page,window", [
     ([70, 9], [70, 200], 4, 1, 64, 16, 0),          # several blocks, a border between requests in one
     ([33, 4, 64], [100, 4, 129], 6, 2, 128, 8, 0),  # a group of 3: 63 of 64 rows
