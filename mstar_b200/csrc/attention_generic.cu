@@ -12,8 +12,8 @@
 // the keys and values of that head through shared memory in tiles of 32 keys with
 // an online softmax.  The keys of the current step are already in the cache.
 //
-// Float prompt portions with a head_dim of 64 or 128 take the second kernel below, whose
-// blocks share a tile of keys among 64 rows.
+// Floats with a head_dim of 64 or 128 take the kernels below: prompt portions one whose blocks share a tile of
+// keys among 64 rows, single tokens one whose warps read their keys straight from the cache.
 #include "common.cuh"
 #include "mma_util.cuh"
 
@@ -363,6 +363,162 @@ attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
     }
 }
 
+// ------------------------------------------------------------------ float single tokens
+// One token's attention, a block for four query heads of a kv head (blockIdx.z: which four of its
+// group): scores of up to 512 keys into shared memory, their softmax statistics, then the values.  HD / 16
+// lanes share a key, HD / 4 a value, each 16 bytes at a time, so a warp has 8 to 16 rows in flight
+// and nothing is staged; warps take the keys in turn and their sums are added at the end in a fixed
+// order: a row's result does not depend on what else is in the batch.  Bound by the latency of three
+// dependent rounds of loads (table, keys, values).  20 tokens on 100 to 200 keys with 32 / 8 heads of
+// 64: 156 us with the kernel above (keys of 32 staged by one load a thread at a time), 13 us here.
+#define AT_THREADS 256
+#define AT_KEYS 512
+
+template <int HD>
+__global__ void __launch_bounds__(AT_THREADS)
+attention_token_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
+                           const float* __restrict__ kv_cache, const int* __restrict__ block_table,
+                           const int* __restrict__ token_req, const int* __restrict__ cache_pos, AttnArgs a) {
+    constexpr int WARPS = AT_THREADS / 32;
+    constexpr int KL = HD / 16, KEYS = 32 / KL;    // lanes a key, keys a warp at a time
+    constexpr int VL = HD / 4, VALS = 32 / VL;     // lanes a value row
+    constexpr int U = 4;                           // rows a lane has in flight
+    __shared__ float4 s_s[AT_KEYS];                // scores, then probabilities, of the four heads
+    __shared__ size_t at_s[AT_KEYS];               // where a key's row begins
+    __shared__ float4 stat_s[2];                   // per head: the factor for older sums, the sum
+    __shared__ float4 acc_s[WARPS][4][HD / 4];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int t = blockIdx.x, kvh = blockIdx.y, G = a.nq / a.nkv, g0 = blockIdx.z * 4, heads = min(4, G - g0);
+    const int hi = cache_pos[t] + 1;
+    const int lo = (a.window > 0 && hi > a.window) ? hi - a.window : 0;
+    const int* bt = block_table + (size_t)token_req[t] * a.bt_stride;
+    const size_t page_elems = (size_t)2 * a.nkv * a.page_size * HD;
+    const size_t v_off = (size_t)a.nkv * a.page_size * HD;
+    const float* head_base = kv_cache + (size_t)kvh * a.page_size * HD;
+
+    // this lane's part of the queries: floats 4 (KL i + lane % KL) ..
+    const int kl = lane % KL, vl = lane % VL;
+    ulonglong2 qv[4][4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            qv[h][i] = *reinterpret_cast<const ulonglong2*>(
+                q + (size_t)t * a.q_stride + (size_t)(kvh * G + g0 + min(h, heads - 1)) * HD + (i * KL + kl) * 4);
+
+    float m = -INFINITY, l = 0.f;                  // of head `warp`, in the first four warps
+    unsigned long long acc[4][2];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) acc[h][0] = acc[h][1] = 0ull;
+
+    for (int base = lo; base < hi; base += AT_KEYS) {
+        const int n = min(AT_KEYS, hi - base);
+        for (int j = tid; j < n; j += AT_THREADS) {
+            const int key = base + j, page = key / a.page_size;
+            at_s[j] = (size_t)bt[page] * page_elems + (size_t)(key - page * a.page_size) * HD;
+        }
+        __syncthreads();
+        for (int j0 = warp * KEYS + lane / KL; j0 < n; j0 += WARPS * KEYS * 2) {
+            ulonglong2 kv[2][4];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float* row = head_base + at_s[min(j0 + u * WARPS * KEYS, n - 1)];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) kv[u][i] = *reinterpret_cast<const ulonglong2*>(row + (i * KL + kl) * 4);
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                float dot[4];
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    unsigned long long d = 0ull;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        ar_fma2(d, qv[h][i].x, kv[u][i].x);
+                        ar_fma2(d, qv[h][i].y, kv[u][i].y);
+                    }
+                    dot[h] = ar_lo(d) + ar_hi(d);
+                }
+                // (lanes of a key leave the loop together, those of one warp may not)
+                const unsigned mask = ((KL == 32 ? 0u : 1u << KL) - 1u) << (lane & ~(KL - 1));
+#pragma unroll
+                for (int h = 0; h < 4; ++h)
+#pragma unroll
+                    for (int o = KL / 2; o > 0; o >>= 1) dot[h] += __shfl_xor_sync(mask, dot[h], o);
+                if (kl == 0 && j0 + u * WARPS * KEYS < n)
+                    s_s[j0 + u * WARPS * KEYS] =
+                        make_float4(dot[0] * a.scale, dot[1] * a.scale, dot[2] * a.scale, dot[3] * a.scale);
+            }
+        }
+        __syncthreads();
+        if (warp < 4) {
+            float* s = reinterpret_cast<float*>(s_s) + warp;
+            float mx = -INFINITY;
+            for (int j = lane; j < n; j += 32) mx = fmaxf(mx, s[4 * j]);
+            const float m_new = fmaxf(m, warp_max(mx));
+            float sum = 0.f;
+            for (int j = lane; j < n; j += 32) {
+                const float p = expf(s[4 * j] - m_new);
+                sum += p;
+                s[4 * j] = p;
+            }
+            const float alpha = expf(m - m_new);   // 0 on the first round
+            l = l * alpha + warp_sum(sum);
+            m = m_new;
+            if (lane == 0) {
+                reinterpret_cast<float*>(stat_s)[warp] = alpha;
+                reinterpret_cast<float*>(stat_s)[4 + warp] = l;
+            }
+        }
+        __syncthreads();
+        const float4 al = stat_s[0];
+        const float alpha[4] = {al.x, al.y, al.z, al.w};
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const unsigned long long f = ar_pack(alpha[h], alpha[h]);
+            asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[h][0]) : "l"(f));
+            asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[h][1]) : "l"(f));
+        }
+        for (int j0 = warp * VALS + lane / VL; j0 < n; j0 += WARPS * VALS * U) {
+            ulonglong2 v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                v[u] = *reinterpret_cast<const ulonglong2*>(head_base + v_off + at_s[min(j0 + u * WARPS * VALS, n - 1)] +
+                                                            vl * 4);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (j0 + u * WARPS * VALS >= n) break;
+                const float4 p4 = s_s[j0 + u * WARPS * VALS];
+                const float p[4] = {p4.x, p4.y, p4.z, p4.w};
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    const unsigned long long pp = ar_pack(p[h], p[h]);
+                    ar_fma2(acc[h][0], pp, v[u].x);
+                    ar_fma2(acc[h][1], pp, v[u].y);
+                }
+            }
+        }
+        __syncthreads();                           // scores and places are done with
+    }
+    // the two value rows of a warp (HD 64), then the warps, in order
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        float r[4] = {ar_lo(acc[h][0]), ar_hi(acc[h][0]), ar_lo(acc[h][1]), ar_hi(acc[h][1])};
+        if (VALS == 2)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) r[i] += __shfl_xor_sync(0xffffffffu, r[i], 16);
+        if (lane < VL) acc_s[warp][h][vl] = make_float4(r[0], r[1], r[2], r[3]);
+    }
+    __syncthreads();
+    for (int i = tid; i < heads * HD; i += AT_THREADS) {
+        float sum = 0.f;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) sum += reinterpret_cast<const float*>(acc_s[w])[i];
+        out[(size_t)t * a.nq * HD + (size_t)(kvh * G + g0) * HD + i] =
+            sum / reinterpret_cast<const float*>(stat_s)[4 + i / HD];
+    }
+}
+
 template <int HD>
 static int launch_rows_f32(const float* q, float* out, const float* kv, const int* block_table,
                            const int* token_req, const int* cache_pos, const AttnArgs& a, int num_tokens,
@@ -396,12 +552,20 @@ MSTAR_API int mstar_paged_attention_generic(const void* q, int q_stride, void* o
     if (G * hd > ATT_MAX_ACC * ATT_THREADS || hd > 256) return -1;
     cudaStream_t s = (cudaStream_t)stream;
     AttnArgs a{nq, nkv, hd, page_size, bt_stride, window, q_stride, scale};
-    if (portions && act_dtype == MSTAR_F32 && (hd == 64 || hd == 128) && G <= AR_ROWS && q_stride % 4 == 0 &&
-        (((uintptr_t)q | (uintptr_t)kv_cache | (uintptr_t)out) & 15) == 0 && num_tokens <= 65535) {
+    const bool rows_of_16 = act_dtype == MSTAR_F32 && (hd == 64 || hd == 128) && q_stride % 4 == 0 &&
+                            (((uintptr_t)q | (uintptr_t)kv_cache | (uintptr_t)out) & 15) == 0;
+    if (portions && rows_of_16 && G <= AR_ROWS && num_tokens <= 65535) {
         return hd == 64 ? launch_rows_f32<64>((const float*)q, (float*)out, (const float*)kv_cache, block_table,
                                               token_req, cache_pos, a, num_tokens, s)
                         : launch_rows_f32<128>((const float*)q, (float*)out, (const float*)kv_cache, block_table,
                                                token_req, cache_pos, a, num_tokens, s);
+    }
+    if (rows_of_16 && nkv <= 65535) {
+        const dim3 grid(num_tokens, nkv, (G + 3) / 4);
+        auto kernel = hd == 64 ? attention_token_f32_kernel<64> : attention_token_f32_kernel<128>;
+        kernel<<<grid, AT_THREADS, 0, s>>>((const float*)q, (float*)out, (const float*)kv_cache, block_table, token_req,
+                                           cache_pos, a);
+        return launch_status();
     }
     const size_t smem = sizeof(float) * ((size_t)G * hd + (size_t)ATT_TILE * (hd + 1) +
                                          (size_t)G * ATT_TILE + 3 * (size_t)G);

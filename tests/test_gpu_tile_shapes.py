@@ -98,6 +98,18 @@ def test_float_attention_of_portions(lens_q, lens_kv, nq, nkv, hd, page, window,
     assert (got - one_token).abs().max() < 2e-6
 
 
+# one key, a warp's keys and one more, a round of 512 keys and one more, several rounds; groups of one to nine
+# heads; a window that begins inside a page
+@pytest.mark.parametrize("lens_kv,nq,nkv,hd,page,window", [
+    ([1, 65, 64], 8, 2, 64, 16, 0), ([513, 512, 33], 3, 1, 128, 16, 0), ([1300, 7], 9, 1, 64, 8, 0),
+    ([700, 40], 4, 4, 128, 64, 37), ([1200], 10, 2, 64, 4, 600)])
+def test_float_attention_of_single_tokens(lens_kv, nq, nkv, hd, page, window):
+    ones = [1] * len(lens_kv)
+    got, want, _ = paged_case(ones, lens_kv, nq, nkv, hd, page, torch.float32, 6, window)
+    # products of some 8 rounded to 24 bits in the scores, weights that add up to one
+    assert (got - want).abs().max() < 4e-6
+
+
 def test_float_attention_of_portions_leaves_unseen_values_out():
     """A later token's value that is not finite reaches no earlier token of the same block."""
     from mstar_b200 import ops
