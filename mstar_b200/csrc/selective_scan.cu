@@ -15,6 +15,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "gemm_f32.h"
 #include "mma_util.cuh"
 
 __device__ __forceinline__ float silu_f(float v) { return v / (1.f + expf(-v)); }
@@ -210,7 +211,12 @@ __device__ __forceinline__ void cp_async_all_done() {
 // portion's own length alone, so that its sums do not depend on the batch (600 tokens of 2,048 channels:
 // 44 us in pieces of 64, 52 of 128; 2,048 of 4,096: 217 of 128, 223 and 226 of 64 and 256; 8,192: 809 of
 // 256, 832 of 128).
+// Shorter portions stay whole: one of 130 tokens of 4,096 channels takes 32 us either way, one of 100 28 us
+// against 30 in two pieces, one of 333 58 against 46; with several of them the SMs are full and whole is
+// faster (three of 333: 85 against 97).
+#define SCAN_CUT_FROM 192
 __host__ __device__ __forceinline__ int scan_piece(int n) {
+    if (n < SCAN_CUT_FROM) return SCAN_CUT_FROM;
     const int p = n / 16 / 64 * 64;
     return p < 64 ? 64 : p > 256 ? 256 : p;
 }
@@ -227,8 +233,7 @@ struct ScanArgs {
     int piece, pass, max_pieces;
     float* piece_state;   // [entries][max_pieces][inner][n_state]; piece < 0: [tokens / 64 + entries][..]
     float* piece_dt;      // [entries][max_pieces][inner]; likewise
-    // W_dt dt_in of every token and channel, made by a product of its own [tokens][inner]
-    // (long portions), or nullptr: the kernel makes it from the staged rows.  Pass 1 of the kernel for
+    // W_dt dt_in of every token and channel, made by a product of its own [tokens][inner], or nullptr: the kernel makes it from the staged rows.  Pass 1 of the kernel for
     // 16 states leaves the step sizes made of it in its place.
     float* dt_pre;
 };
@@ -766,11 +771,156 @@ selective_scan16_kernel(const A* __restrict__ xc, const A* __restrict__ xz, cons
     }
 }
 
+// Portions of a few tokens (decode steps): nothing is staged, a lane reads its tokens' numbers itself, two tokens
+// at a time, all loads in flight at once; the arithmetic is the kernel's above, number by number.  MAKE: the
+// block makes its own step sizes' products, the rows of W_dt of its channels in shared memory, a lane a
+// token, summed in the order of the product for many tokens (gemm_f32.cu: even and odd places apart), so that a
+// token's bits do not depend on which of the two made them.  Every entry reads W_dt again then, which
+// costs less than a launch up to some 32 tokens.  Bound by the stream of the states and by two dependent
+// rounds of loads: 20 entries of one token, 4,096 channels: 18 us (34 in the kernel for any state, whose lanes read
+// W_dt from global memory, 28 in the kernel above, 10 of them the product's launch); 64: 30 (84, 56).
+#define SCAN_FEW 8
+#define SCAN_FEW_RANK 256           // rows of W_dt that a block can hold
+template <typename A, bool MAKE>
+__global__ void __launch_bounds__(128)
+selective_scan16_few_kernel(const A* __restrict__ xc, const A* __restrict__ xz, const float* __restrict__ proj,
+                            const float* __restrict__ w_dt, const float* __restrict__ dt_bias, const float* __restrict__ a_neg,
+                            const float* __restrict__ d_skip, const int* __restrict__ qo_indptr,
+                            const int* __restrict__ slots, float* __restrict__ state, A* __restrict__ out, ScanArgs a) {
+    constexpr int FEW = 2;
+    extern __shared__ __align__(16) float sf_smem[];             // MAKE: [32][rank + 4] of W_dt, [SCAN_FEW][rank]
+    const int e = blockIdx.x, sub = threadIdx.x & 3, ch = threadIdx.x >> 2, c = blockIdx.y * 32 + ch;
+    const int ld = a.rank + 4, quads = a.rank / 4;
+    if (MAKE) {                                                  // (no kernel writes W_dt)
+        for (int i = threadIdx.x; i < 32 * quads; i += 128)
+            cp_async_16(smem_u32(sf_smem + i / quads * ld + i % quads * 4),
+                        w_dt + (size_t)(blockIdx.y * 32 + i / quads) * a.rank + i % quads * 4, 16);
+    }
+    const unsigned long long waited = pdl_wait();
+    xc = pdl_after(xc, waited);
+    xz = pdl_after(xz, waited);
+    proj = pdl_after(proj, waited);
+    const float* dt_pre = pdl_after((const float*)a.dt_pre, waited);
+    const int start = qo_indptr[e], n_tok = qo_indptr[e + 1] - start;
+    const int row = a.rank + 32;
+    float* dt_in = sf_smem + 32 * ld;
+    if (MAKE) {
+        for (int i = threadIdx.x; i < n_tok * quads; i += 128)
+            cp_async_16(smem_u32(dt_in + i * 4), proj + (size_t)(start + i / quads) * row + i % quads * 4, 16);
+        asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+    }
+    if (n_tok <= 0) return;
+    float made[SCAN_FEW / 4];                                    // of tokens sub and sub + 4
+    if (MAKE) {
+#pragma unroll
+        for (int m = 0; m < SCAN_FEW / 4; ++m) {
+            unsigned long long acc = 0ull;
+            if (sub + 4 * m < n_tok) {
+                const float* w = sf_smem + ch * ld;
+                const float* d = dt_in + (sub + 4 * m) * a.rank;
+#pragma unroll 8
+                for (int k = 0; k < a.rank; k += 4) {
+                    const ulonglong2 x2 = *reinterpret_cast<const ulonglong2*>(d + k), w2 = *reinterpret_cast<const ulonglong2*>(w + k);
+                    acc = sx_fma(x2.x, w2.x, acc);
+                    acc = sx_fma(x2.y, w2.y, acc);
+                }
+            }
+            made[m] = sx_lo(acc) + sx_hi(acc);
+        }
+    }
+    float* slot = state + (size_t)slots[e] * a.state_stride;
+    float* s_slot = slot + (size_t)(a.taps - 1) * a.inner + (size_t)c * 16 + 4 * sub;
+    const float4 an = *reinterpret_cast<const float4*>(a_neg + (size_t)c * 16 + 4 * sub);
+    constexpr float L = 1.4426950408889634f;
+    const unsigned long long An[2] = {sx_pack(an.x * L, an.y * L), sx_pack(an.z * L, an.w * L)};
+    const float bias = dt_bias[c], dsk = d_skip[c];
+    const bool wide = (reinterpret_cast<uintptr_t>(s_slot) & 15) == 0;
+    unsigned long long S[2];
+    if (wide) {
+        const float4 s4 = *reinterpret_cast<const float4*>(s_slot);
+        S[0] = sx_pack(s4.x, s4.y);
+        S[1] = sx_pack(s4.z, s4.w);
+    } else {
+        S[0] = sx_pack(s_slot[0], s_slot[1]);
+        S[1] = sx_pack(s_slot[2], s_slot[3]);
+    }
+    // the window of the convolution: the last taps - 1 inputs of [old window | this portion]
+    if (a.taps <= 5) {
+        float w = 0.f;
+        const int at = n_tok + sub;
+        if (sub < a.taps - 1)
+            w = at < a.taps - 1 ? slot[(size_t)at * a.inner + c]
+                                : to_float(xz[(size_t)(start + at - (a.taps - 1)) * a.ld_xz + c]);
+        __syncwarp();
+        if (sub < a.taps - 1) slot[(size_t)sub * a.inner + c] = w;
+    } else if (sub == 0) {
+        for (int j = 0; j < a.taps - 1; ++j) {
+            const int at = n_tok + j;
+            slot[(size_t)j * a.inner + c] =
+                at < a.taps - 1 ? slot[(size_t)at * a.inner + c]
+                                : to_float(xz[(size_t)(start + at - (a.taps - 1)) * a.ld_xz + c]);
+        }
+    }
+    for (int t0 = 0; t0 < n_tok; t0 += FEW) {
+        float dt[FEW], x[FEW], z[FEW];
+        ulonglong2 B[FEW], C[FEW];
+#pragma unroll
+        for (int k = 0; k < FEW; ++k) {
+            const size_t t = (size_t)(start + min(t0 + k, n_tok - 1));
+            const float* bc = proj + t * row + a.rank + 4 * sub;
+            B[k] = *reinterpret_cast<const ulonglong2*>(bc);
+            C[k] = *reinterpret_cast<const ulonglong2*>(bc + 16);
+            if (MAKE) {
+                const int j = min(t0 + k, n_tok - 1);
+                dt[k] = __shfl_sync(0xffffffffu, j < 4 ? made[0] : made[1], j & 3, 4);
+            } else {
+                dt[k] = dt_pre[t * a.inner + c];
+            }
+            x[k] = to_float(xc[t * a.inner + c]);
+            z[k] = to_float(xz[t * a.ld_xz + a.inner + c]);
+        }
+#pragma unroll
+        for (int k = 0; k < FEW; ++k) {
+            if (t0 + k >= n_tok) break;
+            const float d = softplus_f(dt[k] + bias), dx = d * x[k];
+            const unsigned long long d2 = sx_pack(d, d), dx2 = sx_pack(dx, dx);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const unsigned long long p = sx_mul(d2, An[i]);
+                S[i] = sx_fma(sx_pack(sx_ex2(sx_lo(p)), sx_ex2(sx_hi(p))), S[i], sx_mul(dx2, i == 0 ? B[k].x : B[k].y));
+            }
+            const unsigned long long y2 = sx_fma(S[1], C[k].y, sx_mul(S[0], C[k].x));
+            float y = sx_lo(y2) + sx_hi(y2);
+            y += __shfl_xor_sync(0xffffffffu, y, 1);
+            y += __shfl_xor_sync(0xffffffffu, y, 2);
+            if (sub == 0)
+                out[(size_t)(start + t0 + k) * a.inner + c] = from_float<A>(fmaf(dsk, x[k], y) * sx_silu(z[k], A()));
+        }
+    }
+    if (wide) {
+        *reinterpret_cast<float4*>(s_slot) = make_float4(sx_lo(S[0]), sx_hi(S[0]), sx_lo(S[1]), sx_hi(S[1]));
+    } else {
+        s_slot[0] = sx_lo(S[0]);
+        s_slot[1] = sx_hi(S[0]);
+        s_slot[2] = sx_lo(S[1]);
+        s_slot[3] = sx_hi(S[1]);
+    }
+}
+
 template <typename A>
-static void launch_scan16(const void* xc, const void* xz, const float* proj, const float* dt_bias, const float* a_neg,
+static int launch_scan16(const void* xc, const void* xz, const float* proj, const float* w_dt, const float* dt_bias, const float* a_neg,
                           const float* d_skip, const int* qo_indptr, const int* slots, float* state, void* out,
-                          ScanArgs a, cudaStream_t s) {
+                          ScanArgs a, bool few, cudaStream_t s) {
     const dim3 grid(a.entries, a.inner / 32, a.max_pieces);
+    if (few) {
+        const bool make = a.dt_pre == nullptr;
+        const size_t smem = make ? sizeof(float) * (32 * (a.rank + 4) + SCAN_FEW * a.rank) : 0;
+        mstar_launch(make ? selective_scan16_few_kernel<A, true> : selective_scan16_few_kernel<A, false>, grid, dim3(128),
+                     smem, s, (const A*)xc, (const A*)xz, proj, w_dt, dt_bias, a_neg, d_skip, qo_indptr, slots, state,
+                     (A*)out, a);
+        return launch_status();
+    }
 #define GO(PASS)                                                                                  \
     a.pass = PASS;                                                                                \
     mstar_launch((selective_scan16_kernel<A, PASS>), grid, dim3(128), 0, s, (const A*)xc, (const A*)xz, proj, \
@@ -782,6 +932,7 @@ static void launch_scan16(const void* xc, const void* xz, const float* proj, con
         GO(0);
     }
 #undef GO
+    return launch_status();
 }
 
 // xc: [tokens, inner] conv outputs; xz: [tokens] rows of ld_xz elements, x then z; proj: float
@@ -789,31 +940,38 @@ static void launch_scan16(const void* xc, const void* xz, const float* proj, con
 // out [tokens, inner].  piece > 0: portions are cut into pieces of that many tokens (a multiple
 // of the token chunk) that run side by side in two passes; max_pieces bounds the pieces of any
 // entry, piece_state is float scratch [entries, max_pieces, inner, n_state], piece_dt
-// [entries, max_pieces, inner].  dt_pre: nullptr, or float [tokens, inner] = dt_in W_dt^T made by
-// the caller (with pieces it may hold step sizes afterwards).  piece < 0, where the kernel for 16 states
+// [entries, max_pieces, inner].  dt_pre: nullptr, or float scratch [dt_tokens, inner], all tokens', for a
+// product dt_in W_dt^T of its own (with pieces it may hold step sizes afterwards).  piece < 0, where the kernel for 16 states
 // takes the sizes: pieces of scan_piece tokens, max_pieces as with piece > 0, scratch for tokens / 64 +
-// entries pieces.  Returns 0, a CUDA error code, or -1 when the shape is refused.
+// entries pieces.  max_tokens: no entry has more (0: not known).  Returns 0, a CUDA error code, or -1 when the shape is refused.
 MSTAR_API int mstar_selective_scan(const void* xc, const void* xz, int ld_xz, const float* proj,
                                    const float* w_dt, const float* dt_bias, const float* a_neg,
                                    const float* d_skip, const int* qo_indptr, const int* slots,
                                    float* state, long long state_stride, void* out, int act_dtype,
                                    int entries, int inner, int n_state, int rank, int taps,
                                    int piece, int max_pieces, float* piece_state, float* piece_dt,
-                                   float* dt_pre, void* stream) {
+                                   float* dt_pre, int dt_tokens, int max_tokens, int* error, void* stream) {
     if (entries <= 0) return 0;
     if (inner <= 0 || n_state <= 0 || rank <= 0 || taps <= 0 || n_state > 256) return -1;
     if (piece != 0 && (max_pieces < 1 || piece_state == nullptr || piece_dt == nullptr)) return -1;
     cudaStream_t s = (cudaStream_t)stream;
     ScanArgs a{inner, n_state, rank, taps, ld_xz, entries, state_stride, piece, 0,
                piece != 0 ? max_pieces : 1, piece_state, piece_dt, dt_pre};
+    if (dt_pre != nullptr) {
+        const int code = mstar_sgemm_nt(proj, w_dt, dt_pre, dt_tokens, inner, rank, rank + 2 * n_state, rank, inner,
+                                        error, stream);
+        if (code != 0) return code;
+    }
     const int piece16 = act_dtype == MSTAR_F32 ? 4 : 8;          // elements of 16 bytes
-    if (dt_pre != nullptr && n_state == 16 && inner % 32 == 0 && rank % 4 == 0 && ld_xz % piece16 == 0 &&
+    // (without a product of its own the kernel for a few tokens makes it; the row of W_dt must fit)
+    const bool few = piece == 0 && max_tokens > 0 && max_tokens <= SCAN_FEW &&
+                     (dt_pre != nullptr || (rank <= SCAN_FEW_RANK && ((uintptr_t)w_dt & 15) == 0));
+    if ((dt_pre != nullptr || few) && n_state == 16 && inner % 32 == 0 && rank % 4 == 0 && ld_xz % piece16 == 0 &&
         (((uintptr_t)xc | (uintptr_t)xz | (uintptr_t)proj | (uintptr_t)dt_pre | (uintptr_t)a_neg | (uintptr_t)piece_state) & 15) == 0) {
-        if (act_dtype == MSTAR_F32)
-            launch_scan16<float>(xc, xz, proj, dt_bias, a_neg, d_skip, qo_indptr, slots, state, out, a, s);
-        else
-            launch_scan16<bf16>(xc, xz, proj, dt_bias, a_neg, d_skip, qo_indptr, slots, state, out, a, s);
-        return launch_status();
+        return act_dtype == MSTAR_F32 ? launch_scan16<float>(xc, xz, proj, w_dt, dt_bias, a_neg, d_skip, qo_indptr, slots,
+                                                             state, out, a, few, s)
+                                      : launch_scan16<bf16>(xc, xz, proj, w_dt, dt_bias, a_neg, d_skip, qo_indptr, slots,
+                                                            state, out, a, few, s);
     }
     if (piece < 0) return -1;
 #define GO(A, LANES, NPER)                                                                        \

@@ -1770,6 +1770,12 @@ def conv_silu(xz: torch.Tensor, weight, bias, token_req, qo_indptr, slots, state
 # (a multiple of the kernel's chunk of 16), and the portion length from which on it is cut.
 SCAN_PIECE = 128
 SCAN_PIECES_FROM = 512
+# The same for the kernels for 16 states (the csrc constant of this name says what was measured).
+SCAN_CUT_FROM = 192
+# Portions of at most so many tokens go to a kernel that stages nothing, and a step of at most so many
+# tokens in all needs no launch of its own for the step sizes' product there.
+SCAN_FEW = 8
+SCAN_FEW_TOKENS = 32
 
 
 def scan_most_pieces(longest: int) -> int:
@@ -1789,11 +1795,13 @@ def selective_scan(xc: torch.Tensor, xz: torch.Tensor, proj: torch.Tensor, w_dt,
     float ``w_dt`` [inner, rank], ``dt_bias`` [inner], ``a_neg`` [inner, n_state] (= -exp(A_log)),
     ``d_skip`` [inner].  Returns y * silu(z) [tokens, inner] in the dtype of ``xc``.
     ``max_q_len`` (the longest portion of the batch) of ``SCAN_PIECES_FROM`` tokens or more
-    cuts every portion into pieces that run side by side (of ``SCAN_PIECE`` tokens, or, by the kernel
-    for 16 states, of 64 to 256 tokens by the portion's own length): a first
+    cuts every portion into pieces of ``SCAN_PIECE`` tokens that run side by side; the kernel
+    for 16 states cuts portions of ``SCAN_CUT_FROM`` tokens or more, by their own length, into pieces
+    of 64 to 256: a first
     pass leaves each piece's own end state and summed step sizes, a second starts each piece
     from the state joined over the pieces before it (the recurrence is linear in the state);
-    MSTAR_SCAN_PIECE sets another piece size, 0 none."""
+    MSTAR_SCAN_PIECE sets another piece size for portions of ``SCAN_PIECES_FROM`` tokens or more, 0
+    none."""
     _need_cuda(xc, xz, proj, w_dt, dt_bias, a_neg, d_skip, qo_indptr, slots, state)
     assert xc.is_contiguous() and xz.stride(1) == 1 and xz.dtype == xc.dtype
     assert proj.dtype == torch.float32 and proj.is_contiguous()
@@ -1804,35 +1812,45 @@ def selective_scan(xc: torch.Tensor, xz: torch.Tensor, proj: torch.Tensor, w_dt,
     assert state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1
     assert state.shape[1] == selective_scan_state_size(inner, n_state, taps)
     out = torch.empty_like(xc)
-    piece, pieces, piece_state, piece_dt, dt_pre = 0, 1, None, None, None
-    if max_q_len is not None and max_q_len >= SCAN_PIECES_FROM:
-        wide = 16 // xz.element_size()
-        sixteen = (n_state == 16 and inner % 32 == 0 and rank % 4 == 0 and xz.stride(0) % wide == 0
-                   and not any(t.data_ptr() % 16 for t in (xc, xz, proj, a_neg)))
+    tokens = xc.shape[0]
+    piece, pieces, places, dt_tokens = 0, 1, 0, 0
+    sixteen = (max_q_len is not None and n_state == 16 and inner % 32 == 0 and rank % 4 == 0
+               and xz.stride(0) * xz.element_size() % 16 == 0
+               and (xc.data_ptr() | xz.data_ptr() | proj.data_ptr() | a_neg.data_ptr()) % 16 == 0)
+    if sixteen or (max_q_len is not None and max_q_len >= SCAN_PIECES_FROM):
         forced = os.environ.get("MSTAR_SCAN_PIECE")
-        if forced is not None:
+        if forced is not None and max_q_len >= SCAN_PIECES_FROM:
             piece = int(forced) // 16 * 16
             pieces = -(-max_q_len // piece) if piece else 1
         elif sixteen:
-            piece, pieces = -1, scan_most_pieces(max_q_len)
+            if max_q_len >= SCAN_CUT_FROM:
+                piece, pieces = -1, scan_most_pieces(max_q_len)
         else:
             piece, pieces = SCAN_PIECE, -(-max_q_len // SCAN_PIECE)
-        # with many tokens the step sizes' product W_dt dt_in is a true-32-bit product of its
-        # own (a third of the scan's instructions otherwise)
-        dt_pre = sgemm_nt(proj[:, :rank], w_dt)
+        # with many tokens, and by the kernels for 16 states, the step sizes' product W_dt dt_in is a
+        # true-32-bit product of its own (a third of the scan's instructions otherwise, and W_dt read
+        # again for every entry)
+        # (portions of a few tokens: the scan makes its own, in the same order, up to so many of them)
+        if not (sixteen and max_q_len <= SCAN_FEW and tokens <= SCAN_FEW_TOKENS and rank <= 256
+                and w_dt.data_ptr() % 16 == 0):
+            dt_tokens = tokens
     if piece:
         # (cut by their own lengths, portions have a piece for every started 64 tokens at most)
-        places = entries * pieces if piece > 0 else xc.shape[0] // 64 + entries
-        piece_state = torch.empty((places, inner, n_state), dtype=torch.float32, device=xc.device)
-        piece_dt = torch.empty((places, inner), dtype=torch.float32, device=xc.device)
+        places = entries * pieces if piece > 0 else tokens // 64 + entries
+    # one piece of scratch: the product, the pieces' states, their summed step sizes
+    scratch = (torch.empty(inner * (dt_tokens + places * (n_state + 1)), dtype=torch.float32, device=xc.device)
+               if dt_tokens or places else None)
+    work = _ptr(scratch)
+    piece_state = work + 4 * inner * dt_tokens if places else 0
+    piece_dt = piece_state + 4 * inner * places * n_state if places else 0
     code = lib.get("selective_scan").mstar_selective_scan(
         xc.data_ptr(), xz.data_ptr(), xz.stride(0), proj.data_ptr(), w_dt.data_ptr(),
         dt_bias.data_ptr(), a_neg.data_ptr(), d_skip.data_ptr(), qo_indptr.data_ptr(),
         slots.data_ptr(), state.data_ptr(), state.stride(0), out.data_ptr(), _dt(xc), entries,
-        inner, n_state, rank, taps, piece, pieces, _ptr(piece_state), _ptr(piece_dt), _ptr(dt_pre),
-        _stream())
-    if piece:
-        lib.add_launches(1)                     # two passes behind one call
+        inner, n_state, rank, taps, piece, pieces, piece_state, piece_dt,
+        work if dt_tokens else 0, dt_tokens,
+        max_q_len or 0, tcgen05_error_word(xc.device).data_ptr() if rank >= 512 else 0, _stream())
+    lib.add_launches(bool(piece) + bool(dt_tokens))     # several behind one call
     if code == -1:
         raise KernelError(f"selective scan refuses inner={inner}, state={n_state}, rank={rank} "
                           "(at most 256 states a channel)")

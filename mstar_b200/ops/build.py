@@ -47,7 +47,7 @@ LIBRARIES = {
     "attention_sink": ("cuda", ["attention_sink.cu"], []),
     "attention_sink_tc": ("cuda", ["attention_sink_tc.cu"], []),
     "attention_prompt_tc": ("cuda", ["attention_prompt_tc.cu"], []),
-    "selective_scan": ("cuda", ["selective_scan.cu"], []),
+    "selective_scan": ("cuda", ["selective_scan.cu", "gemm_f32.cu", "gemm_f32_tc.cu"], []),
     "gated_delta": ("cuda", ["gated_delta.cu"], []),
     "hyper": ("cuda", ["hyper.cu"], []),
     "side_by_side": ("cuda", ["side_by_side.cu"], []),

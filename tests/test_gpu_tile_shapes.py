@@ -277,19 +277,23 @@ def test_delta_rule_in_pieces_leaves_later_values_out(head_decay, heads, dim, vd
     ops.check_error_word(DEV)
 
 
-@pytest.mark.parametrize("lens,inner,piece", [([512, 7, 530], 64, "256"), ([600], 32, "0"), ([513], 96, "16")])
+# pieces of a given size; then a few tokens (8 at most), whole portions, portions cut by their own length
+@pytest.mark.parametrize("lens,inner,piece", [([512, 7, 530], 64, "256"), ([600], 32, "0"), ([513], 96, "16"),
+                                              ([1, 8, 2, 1], 64, None), ([9, 1], 32, None), ([192, 191, 1], 64, None)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_selective_scan_of_long_portions(lens, inner, piece, dtype, monkeypatch):
     """The scan for 16 states a channel, whole and in pieces, against the recurrence in double precision."""
     from mstar_b200 import ops
 
-    monkeypatch.setenv("MSTAR_SCAN_PIECE", piece)
+    if piece is not None:
+        monkeypatch.setenv("MSTAR_SCAN_PIECE", piece)
     T, rank, N, taps = sum(lens), 4, 16, 3
     xc, xz = rnd(T, inner, dtype=dtype, seed=1), rnd(T, 2 * inner, dtype=dtype, seed=2)
     proj, w_dt = rnd(T, rank + 2 * N, seed=3), rnd(inner, rank, seed=4)
     bias, a, d = rnd(inner, seed=5) - 3, -torch.exp(rnd(inner, N, seed=6)), rnd(inner, seed=7)
     state = rnd(len(lens), ops.selective_scan_state_size(inner, N, taps), seed=8)
     S = state[:, (taps - 1) * inner:].double().view(-1, inner, N).clone()
+    window = state[:, :(taps - 1) * inner].view(-1, taps - 1, inner).clone()
     starts = [0]
     for n in lens:
         starts.append(starts[-1] + n)
@@ -312,15 +316,16 @@ def test_selective_scan_of_long_portions(lens, inner, piece, dtype, monkeypatch)
     end = state[:, (taps - 1) * inner:].double().view(-1, inner, N)
     assert ((end - S).abs() <= 2 ** -17 * S.abs() + 1e-5).all()
     for e in range(len(lens)):                       # the convolution's window moved on
-        for j in range(taps - 1):
-            row = xz[starts[e + 1] - (taps - 1) + j, :inner].float()
-            assert torch.equal(state[e, j * inner:(j + 1) * inner], row)
+        seen = torch.cat([window[e], xz[starts[e]:starts[e + 1], :inner].float()])
+        assert torch.equal(state[e, :(taps - 1) * inner].view(taps - 1, inner), seen[-(taps - 1):])
 
 
-@pytest.mark.parametrize("off", [0, 1])          # rows off 16 bytes: the kernel for any number of states
-@pytest.mark.parametrize("alone,beside", [(600, [4200, 3]), (520, [520] * 9), (2047, [513]), (1024, [1] * 20)])
+# off 1: rows off 16 bytes, the kernel for any number of states, which cuts where the batch's longest is long
+@pytest.mark.parametrize("alone,beside,off", [
+    (alone, beside, off) for alone, beside in ((600, [4200, 3]), (520, [520] * 9), (2047, [513]), (1024, [1] * 20))
+    for off in (0, 1)] + [(1, [9], 0), (5, [300], 0), (150, [700], 0)])
 def test_selective_scan_of_a_portion_does_not_depend_on_the_batch(alone, beside, off):
-    """A long portion's bits by itself and among others: how it is cut follows from its own length."""
+    """A portion's bits by itself and among others: how it is cut follows from its own length."""
     from mstar_b200 import ops
 
     inner, rank, N, taps = 2048, 4, 16, 4
