@@ -607,6 +607,30 @@ __global__ void convert_kernel(const S* __restrict__ src, D* __restrict__ dst, s
         dst[i] = from_float<D>(to_float(src[i]));
 }
 
+// the same for rows of `cols` elements that lie `ld` apart
+template <typename S, typename D>
+__global__ void convert_rows_kernel(const S* __restrict__ src, D* __restrict__ dst, size_t n, int cols, int ld) {
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const size_t row = i / cols;
+        dst[i] = from_float<D>(to_float(src[row * ld + (i - row * cols)]));
+    }
+}
+
+MSTAR_API int mstar_convert_rows(const void* src, int src_dtype, void* dst, int dst_dtype, long long rows, int cols,
+                                 int ld, void* stream) {
+    if (rows <= 0 || cols <= 0) return 0;
+    cudaStream_t s = (cudaStream_t)stream;
+    const size_t n = (size_t)rows * cols, most = (size_t)device_sm_count() * 32;
+    const int blocks = (int)((n + 255) / 256 < most ? (n + 255) / 256 : most);
+    if (src_dtype == MSTAR_F32 && dst_dtype == MSTAR_BF16)
+        convert_rows_kernel<<<blocks, 256, 0, s>>>((const float*)src, (bf16*)dst, n, cols, ld);
+    else if (src_dtype == MSTAR_BF16 && dst_dtype == MSTAR_F32)
+        convert_rows_kernel<<<blocks, 256, 0, s>>>((const bf16*)src, (float*)dst, n, cols, ld);
+    else
+        return -1;
+    return launch_status();
+}
+
 MSTAR_API int mstar_convert(const void* src, int src_dtype, void* dst, int dst_dtype, long long n,
                             void* stream) {
     if (n <= 0) return 0;

@@ -201,8 +201,13 @@ def convert(src: torch.Tensor, dtype: torch.dtype):
     _need_cuda(src)
     if src.dtype == dtype:
         return src
-    assert src.is_contiguous()
     out = torch.empty(src.shape, dtype=dtype, device=src.device)
+    if src.dim() == 2 and src.stride(1) == 1 and src.shape[1] < src.stride(0) < 1 << 31:    # columns of wider rows
+        check(lib.get("elementwise").mstar_convert_rows(
+            src.data_ptr(), _dt(src), out.data_ptr(), _dt(out), src.shape[0], src.shape[1], src.stride(0),
+            _stream()), "convert_rows")
+        return out
+    assert src.is_contiguous()
     check(lib.get("elementwise").mstar_convert(
         src.data_ptr(), _dt(src), out.data_ptr(), _dt(out), src.numel(), _stream()), "convert")
     return out
@@ -2018,6 +2023,7 @@ def delta_prepare(proj: torch.Tensor, conv_w: torch.Tensor, a_proj: torch.Tensor
 DELTA_PIECE = 16            # tokens of a piece of the delta-rule scan
 DELTA_PIECES_FROM = 64      # entries of this many tokens or more are scanned in pieces
 DELTA_PIECES_DIMS = (32, 64, 128, 256)     # key sizes the scan in pieces takes
+DELTA_PARTS_DIMS = (64, 128, 256)   # ... and takes on the tensor cores
 DELTA_HEAD_PIECES_DIMS = (32, 64, 96, 128, 256)    # with one decay a head
 
 
@@ -2058,8 +2064,13 @@ def delta_scan(q, k, v, beta, decay, qo_indptr, slots, state: torch.Tensor, entr
     aligned = all(t.data_ptr() % 16 == 0 for t in (q, k, state)) and (head_decay or decay.data_ptr() % 16 == 0)
     if (pieces and dim in (DELTA_HEAD_PIECES_DIMS if head_decay else DELTA_PIECES_DIMS) and tokens > 0 and offset % 4 == 0
             and state.stride(0) % 4 == 0 and (aligned or head_decay)):
-        rows = (kv_heads * 2 * DELTA_PIECE if head_decay else heads * (3 * DELTA_PIECE + 1)) * (dim + 4)
-        per_piece = rows + heads * DELTA_PIECE * (2 * DELTA_PIECE + 4)
+        # a piece's rows as the scan wants them: floats, or three bfloat16 parts of each
+        kinds = 2 if head_decay else 3
+        if dim in DELTA_PARTS_DIMS:
+            row = kinds * DELTA_PIECE * (dim + 8) * 3 // 2 + (0 if head_decay else dim)
+        else:
+            row = (kinds * DELTA_PIECE + (0 if head_decay else 1)) * (dim + 4)
+        per_piece = (kv_heads if head_decay else heads) * row + heads * DELTA_PIECE * (2 * DELTA_PIECE + 4)
         work = torch.empty((tokens // DELTA_PIECE + entries) * per_piece, dtype=torch.float32,
                            device=q.device)
         code = lib.get("gated_delta").mstar_delta_scan_pieces(

@@ -98,15 +98,16 @@ class GatedDelta:
         a_proj = None if s.head_decay else proj[:, at:at + a_cols]
         gate = proj[:, at + a_cols:at + a_cols + (s.num_heads * s.v_dim if s.full_gate
                                                   else s.gate_rank)]
-        if a_proj is not None and not s.full_gate and self.runtime.dtype != torch.float32:
-            low = ops.convert(proj[:, at:].contiguous(), self.runtime.dtype)
-            a_proj, gate = low[:, :a_cols], low[:, a_cols:a_cols + s.gate_rank]
+        narrow = self.runtime.dtype != torch.float32
+        if a_proj is not None and not s.full_gate and narrow:
+            low = ops.convert(proj[:, at:at + a_cols + s.gate_rank], self.runtime.dtype)
+            a_proj, gate = low[:, :a_cols], low[:, a_cols:]
         if a_proj is not None:
-            a_proj = ops.linear(ops.convert(a_proj.contiguous(), self.runtime.dtype), self.w_a2,
-                                out_dtype=torch.float32, static_weights=True)
+            a_proj = ops.linear(ops.convert(a_proj, self.runtime.dtype) if narrow else a_proj.contiguous(),
+                                self.w_a2, out_dtype=torch.float32, static_weights=True)
         if not s.full_gate:
-            gate = ops.linear(ops.convert(gate.contiguous(), self.runtime.dtype), self.w_g2,
-                              static_weights=True)
+            gate = ops.linear(ops.convert(gate, self.runtime.dtype) if narrow else gate.contiguous(),
+                              self.w_g2, static_weights=True)
         return a_proj, gate
 
 
