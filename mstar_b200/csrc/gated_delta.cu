@@ -1544,7 +1544,8 @@ static int launch_parts_scan(const DeltaHeadArgs& a, int entries, cudaStream_t s
     if (grid.z > 65535) return -1;
     // as many pieces on their way as the blocks that an SM gets leave room for
     const long long blocks = (long long)grid.x * grid.y * grid.z, sms = device_sm_count();
-    const size_t share = most / (size_t)((blocks + sms - 1) / sms) - 1024, room = share > rest ? (share - rest) / buf : 0;
+    const long long share = (long long)most / ((blocks + sms - 1) / sms) - 1024 - (long long)rest;
+    const long long room = share / (long long)buf;       // (2 or fewer where there are more blocks than fit at once)
     const int bufs = room >= GP_BUFS ? GP_BUFS : room >= 2 ? (int)room : 2;
     mstar_launch((delta_parts_scan_kernel<D, CHANNEL>), grid, dim3(GH_THREADS), bufs * buf + rest, s, a, bufs);
     return launch_status();

@@ -277,6 +277,25 @@ def test_delta_rule_in_pieces_leaves_later_values_out(head_decay, heads, dim, vd
     ops.check_error_word(DEV)
 
 
+def test_delta_rule_in_pieces_with_more_blocks_than_fit():
+    """So many blocks an SM (34,816 in all) that a share of its shared memory holds no piece."""
+    from mstar_b200 import ops
+
+    entries, heads, dim, taps = 34, 64, 256, 1
+    T = 64 + entries - 1
+    starts = torch.tensor([0] + list(range(64, T + 1)), dtype=torch.int32, device=DEV)
+    q, k = (torch.nn.functional.normalize(rnd(T, dim, seed=s), dim=-1) for s in (1, 2))
+    v, beta = rnd(T, heads * dim, seed=3), torch.sigmoid(rnd(T, heads, seed=4))
+    decay = torch.sigmoid(rnd(T, heads, seed=5) + 3)
+    state = torch.zeros(entries, ops.gated_delta_state_size(heads, 1, dim, dim, taps), device=DEV)
+    slots = torch.arange(entries, dtype=torch.int32, device=DEV)
+    got = ops.delta_scan(q, k, v, beta, decay, starts, slots, state, entries, heads, 1, dim, dim, taps, max_q_len=64)
+    ops.check_error_word(DEV)
+    # an entry of one token from an empty state: o = (q . k) beta v
+    want = (q * k).sum(1)[64:, None, None] * (beta[:, :, None] * v.view(T, heads, dim))[64:]
+    assert (got.view(T, heads, dim)[64:] - want).abs().max() < 2 ** -24 * 64 * dim ** 0.5
+
+
 # pieces of a given size; then a few tokens (8 at most), whole portions, portions cut by their own length
 @pytest.mark.parametrize("lens,inner,piece", [([512, 7, 530], 64, "256"), ([600], 32, "0"), ([513], 96, "16"),
                                               ([1, 8, 2, 1], 64, None), ([9, 1], 32, None), ([192, 191, 1], 64, None)])
