@@ -234,29 +234,28 @@ sample_kernel(const float* __restrict__ logits, int ld, int vocab,
 // ------------------------------------------------------------------ cluster variant
 // The same sampling with a thread-block cluster of 8 CTAs per row: each CTA keeps an
 // eighth of the row in shared memory (the penalised logits), so the row is read from global
-// memory once; the thresholds of top-k and top-p are found by radix selection (three rounds of
-// 11, 11 and 10 bits with a histogram per round, summed across the cluster through distributed
-// shared memory) instead of 32 passes of bisection each.
-// The selection runs on keys that spread the row's range [min, max] linearly over 32 bits
-// (a monotone map of the penalised logits: the bit patterns themselves would put nearly
-// all tokens into the few bins of their common exponents, and the histogram's atomics
-// would serialise); logits closer than range / 2^32 count as tied, and ties with the last
-// kept token are kept, as before.  Probability mass is counted in 64-bit fixed
+// memory once; the thresholds of top-k and top-p are found by a histogram of 2,048 bins, summed across the
+// cluster through distributed shared memory, and a list of what lies in the threshold's bin (or three radix
+// rounds of 11, 11 and 10 bits over it) instead of 32 passes of bisection each.
+// The first round's bins cut the logits' range linearly (the bit patterns themselves would put nearly all tokens
+// into the few bins of their common exponents, and the histogram's atomics would serialise), of top-p only the part
+// that can hold the threshold; what is left goes by the logits' ordered bits, so that equal logits alone tie
+// (ties with the last kept token are kept).  Probability mass is counted in 64-bit fixed
 // point (exp * 2^40, exact integer sums), so that no sum depends on the order in which it
 // is made: the same (seed, offset) always draws the same token.
 //
 // What a row takes is latencies: passes over a CTA's logits, cluster barriers, histogram atomics.  So
 // two CTAs share an SM (keys and exponentials are made again where they are needed instead of kept:
-// 95 KB a CTA at 157 k logits instead of 189), the first pass over the keys makes the first
-// histogram and the mass as well, later passes make the keys of those logits only that can lie in the
-// bin in question, histogram entries are two 32-bit words (a 64-bit atomic on shared
-// memory is a loop; the upper word is touched only on a carry or by a large mass), and a histogram is
-// summed over the cluster by all eight CTAs, a slice of the bins each.  Where the first round's bin holds
-// few logits they decide by themselves, in a list (cs_pick_few), instead of two more rounds of three
+// 95 KB a CTA at 157 k logits instead of 189), the pass that makes the mass makes the first histogram of
+// top-p as well, of the logits that can matter only, histogram entries are two 32-bit words (a 64-bit
+// atomic on shared memory is a loop; the upper word is touched only on a carry or by a large mass), and a
+// histogram is summed over the cluster by all eight CTAs, a slice of the bins each.  Where the first round's bin
+// holds few logits they decide by themselves, in a list (cs_pick_few), instead of three more rounds of three
 // cluster barriers; sums have shared words of their own, which spares the barriers behind their reads.
-// 157 k logits with temperature, top-p and a repetition penalty: 85 us for 64 rows (108 with three rounds, 121
-// with every key made in every pass); with cold caches 39, 41, 47 and 90 us for 1, 8, 18 and 64 rows, where one
-// CTA an SM and the histograms added into rank 0 by remote atomics took 66, 66, 123 and 292.
+// 157 k logits with temperature, top-p and a repetition penalty, the head's product before it: 31, 33, 44 and 79 us
+// for 1, 8, 18 and 64 rows (33, 35, 47 and 88 with every logit in the first histogram and keys made in double
+// precision).  Entering the histogram's logits behind the pass was no faster at 64 rows and slower (51 us) at 18
+// of a flatter distribution.
 #define CS_CLUSTER 8
 #define CS_THREADS 512
 #define CS_BINS 2048
@@ -265,7 +264,10 @@ sample_kernel(const float* __restrict__ logits, int ld, int vocab,
 
 namespace cg = cooperative_groups;
 
-__device__ __forceinline__ unsigned long long cs_fixed(float e) { return __float2ull_rz(e * CS_SCALE); }
+// (conversions to 64 bits are many instructions: only numbers of 2^-8 and more, the few at a row's top, take one)
+__device__ __forceinline__ unsigned long long cs_fixed(float e) {
+    return e < 0.00390625f ? (unsigned long long)__float2uint_rz(e * CS_SCALE) : __float2ull_rz(e * CS_SCALE);
+}
 
 // Sum of one u64 per thread over the block; every thread gets it.  `scratch`: 32 u64.
 __device__ __forceinline__ unsigned long long cs_block_sum(unsigned long long v, unsigned long long* scratch) {
@@ -307,13 +309,15 @@ __device__ __forceinline__ void cs_clear(unsigned* hist) {
 // `above + sum(bins > b)` is still below `need` and `above + sum(bins >= b)` reaches it.  CTA r sums and
 // walks the bins of slice r (from the top; higher slices' totals come before it), and the one that holds
 // b writes (b, above + sum(bins > b)) into every CTA's `result`.  Returns b (0 if the need is never
-// reached) and updates `above`.
+// reached) and updates `above`.  need_of is asked once everybody's shared words can be read.
+template <typename Need>
 __device__ __forceinline__ int cs_pick_bin(cg::cluster_group& cluster, int rank, unsigned* hist,
                                            unsigned long long* scratch, unsigned long long* slot,
-                                           unsigned long long* result, unsigned long long need,
+                                           unsigned long long* result, Need need_of,
                                            unsigned long long& above) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     cluster.sync();                                 // every CTA's histogram is complete
+    const unsigned long long need = need_of();
     const int bin = rank * CS_SLICE + tid;
     unsigned long long mine = 0ull;
     if (tid < CS_SLICE) {
@@ -419,6 +423,12 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
     const float* x = logits + (size_t)row * ld;
     const float pen = penalty != nullptr ? penalty[row] : 1.f;
     const int srow = (seen_mask != nullptr && seen_rows != nullptr) ? seen_rows[row] : -1;
+    // (asked for here, with the first logits: each would be a round trip of its own behind the barriers)
+    const float temp = temperature[row];
+    const float p = top_p != nullptr ? top_p[row] : 1.f;
+    const int k = top_k != nullptr ? top_k[row] : 0;
+    const unsigned long long sd = seed != nullptr ? (unsigned long long)seed[row] : 0ull;
+    const unsigned long long of = offset != nullptr ? (unsigned long long)offset[row] : 0ull;
     unsigned char* my_seen = srow >= 0 ? seen_mask + (size_t)srow * vocab : nullptr;
     const unsigned char* seen = (my_seen != nullptr && pen != 1.f) ? my_seen : nullptr;
 
@@ -499,7 +509,6 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
     const int amax = 0x7fffffff - (int)(unsigned)(top & 0xffffffffu);
     const float vmin = fminf(from_ordered_bits(~(unsigned)low_word), vmax);
 
-    const float temp = temperature[row];
     if (temp <= 0.f) {                      // uniform over the cluster
         if (rank == 0 && tid == 0) {
             out[row] = amax;
@@ -509,158 +518,137 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
         return;
     }
     const float inv_temp = 1.f / temp;
-    // a logit's selection key and its mass, made from it wherever they are needed
-    const double spread = vmax > vmin ? 4294967295.0 / ((double)vmax - (double)vmin) : 0.0;
-    auto key_of = [&](float v) {
-        const double q = v > vmin ? ((double)v - (double)vmin) * spread : 0.0;
-        return q >= 4294967295.0 ? 0xffffffffu : (unsigned)q;
+    // f(logit) over this CTA's part of the row
+    auto each = [&](auto f) {
+        const float4* sv4 = reinterpret_cast<const float4*>(sv);
+#pragma unroll 2
+        for (int q = tid; q < n / 4; q += CS_THREADS) {
+            const float4 v = sv4[q];
+            f(v.x);
+            f(v.y);
+            f(v.z);
+            f(v.w);
+        }
+        if (tid < n % 4) f(sv[n / 4 * 4 + tid]);
     };
     auto mass_of = [&](float v) { return cs_fixed(expf((v - vmax) * inv_temp)); };
-    // Logits that surely have smaller (below lo) or larger (above hi) keys than first .. last, so that
-    // only logits between them need their key: the bounds lie a whole key outside (the products in
-    // double are off by 2^-20 keys at most) and are rounded outwards.
-    float lo = -INFINITY, hi = INFINITY;
-    auto band = [&](unsigned first, unsigned last) {
-        if (spread == 0.0) return;
-        const double step = 1.0 / spread;
-        lo = first == 0u ? -INFINITY : __double2float_rd((double)vmin + ((double)first - 1.0) * step);
-        hi = __double2float_ru((double)vmin + ((double)last + 2.0) * step);
+    // a logit's key: its ordered bits, and 0 for the row's smallest ones
+    auto key_of = [&](float v) { return v > vmin ? ordered_bits(v) : 0u; };
+    // The first round's bins cut [base, vmax] evenly: rounded differences and products keep the logits' order.
+    float base_v = vmin, per_bin = 0.f;
+    auto bins_from = [&](float from) {
+        base_v = from;
+        per_bin = vmax > from ? (float)CS_BINS / (vmax - from) : 0.f;   // (an infinite range: one bin)
     };
-    // After a search's first round: what is left of it among the logits whose keys start with `prefix`
-    // (and are at least tau), weighted by weight_of, by a list of them; false where they are too many.
-    unsigned tau = 0u;                      // selection key threshold: keep key(x) >= tau
-    auto finish_few = [&](unsigned* offered, unsigned prefix, unsigned long long need, unsigned long long above,
-                          auto weight_of) {
+    auto bin_of = [&](float v) {
+        return v > base_v ? min(__float2uint_rz((v - base_v) * per_bin), (unsigned)CS_BINS - 1u) : 0u;
+    };
+    unsigned tau = 0u;                      // keep key(x) >= tau
+    float tau_v = -INFINITY;
+    auto set_tau = [&](unsigned key) {
+        tau = key;
+        tau_v = key != 0u ? from_ordered_bits(key) : -INFINITY;
+    };
+    auto kept = [&](float v) { return tau == 0u || v >= tau_v; };
+    // What is left of a search after its first round, among the logits of one bin (that `among` lets in): by a
+    // list of them, or where they are too many by radix rounds over their keys.
+    auto finish = [&](unsigned* offered, unsigned bin, auto need, unsigned long long above, auto among,
+                      auto weight_of) {
         unsigned* list = cluster.map_shared_rank(hist, 0);
         unsigned long long* weights = reinterpret_cast<unsigned long long*>(list + CS_FEW);
         unsigned* place = cluster.map_shared_rank(offered, 0);
-        for (int i = tid; i < n; i += CS_THREADS) {
-            const float v = sv[i];
-            if (v < lo || v > hi) continue;
-            const unsigned key = key_of(v);
-            if (key < tau || (key >> 21) != prefix) continue;
+        each([&](float v) {
+            if (!among(v) || bin_of(v) != bin) return;
             const unsigned long long w = weight_of(v);
-            if (w == 0ull) continue;
+            if (w == 0ull) return;
             const unsigned at = atomicAdd(place, 1u);
             if (at < CS_FEW) {
-                list[at] = key;
+                list[at] = key_of(v);
                 weights[at] = w;
             }
-        }
-        return cs_pick_few(cluster, rank, hist, offered, result, need, above);
-    };
-    const float p = top_p != nullptr ? top_p[row] : 1.f;
-    const int k = top_k != nullptr ? top_k[row] : 0;
-    const bool choose_k = k > 0 && k < vocab;
-    bool first_made = false;                // the first histogram of top-p is there
-
-    // ---- top-k: tau = the k-th largest key, by radix selection on counts
-    unsigned long long mass = 0ull;         // of the kept tokens
-    if (choose_k) {
+        });
+        if (cs_pick_few(cluster, rank, hist, offered, result, need(), above)) return (unsigned)result[0];
         unsigned prefix = 0u;
-        unsigned long long above = 0ull;
         int decided = 0;
         for (int round = 0; round < 3; ++round) {
             const int bits = round < 2 ? 11 : 10;
             const int shift = 32 - decided - bits;
-            if (round > 0) cs_clear(hist);
-            for (int i = tid; i < n; i += CS_THREADS) {
-                const float v = sv[i];
-                if (v < lo || v > hi) continue;
+            cs_clear(hist);
+            each([&](float v) {
+                if (!among(v) || bin_of(v) != bin) return;
                 const unsigned key = key_of(v);
                 if (decided == 0 || (key >> (32 - decided)) == prefix)
-                    cs_add(hist, (key >> shift) & ((1u << bits) - 1u), 1ull);
-            }
-            const int bin = cs_pick_bin(cluster, rank, hist, scratch, slot, result, (unsigned long long)k, above);
-            prefix = (prefix << bits) | (unsigned)bin;
+                    cs_add(hist, (key >> shift) & ((1u << bits) - 1u), weight_of(v));
+            });
+            prefix = (prefix << bits) | (unsigned)cs_pick_bin(cluster, rank, hist, scratch, slot, result, need, above);
             decided += bits;
-            band(prefix << shift, (prefix << shift) + ((1u << shift) - 1u));
-            if (round == 0 && finish_few(few, prefix, (unsigned long long)k, above, [](float) { return 1ull; })) {
-                prefix = (unsigned)result[0];
-                break;
-            }
         }
-        tau = prefix;
-        band(tau, tau);
-        for (int i = tid; i < n; i += CS_THREADS) {
-            const float v = sv[i];
-            if (!(v < lo) && (v > hi || key_of(v) >= tau)) mass += mass_of(v);
-        }
-        lo = -INFINITY;                     // top-p walks the kept ones anew
-        hi = INFINITY;
-    } else {
-        first_made = p < 1.f;
-#pragma unroll 2
-        for (int i = tid; i < n; i += CS_THREADS) {
-            const unsigned long long m = mass_of(sv[i]);
-            mass += m;
-            if (first_made && m != 0ull) cs_add(hist, key_of(sv[i]) >> 21, m);
-        }
-    }
-    unsigned long long all[CS_CLUSTER];
-    mass = cs_block_sum(mass, scratch);
-    cs_gather(cluster, mass, sums, all);
-    unsigned long long total = 0ull;
-#pragma unroll
-    for (int r = 0; r < CS_CLUSTER; ++r) total += all[r];
+        return prefix;
+    };
+    const bool choose_k = k > 0 && k < vocab;
 
-    // ---- top-p: the largest tau2 >= tau whose tokens (x >= tau2) hold p of that mass
-    if (p < 1.f) {
-        const unsigned long long need = (unsigned long long)((double)p * (double)total);
-        const unsigned long long at_least = need > 0ull ? need : 1ull;
-        unsigned prefix = 0u;
-        unsigned long long above = 0ull;
-        int decided = 0;
-        for (int round = 0; round < 3; ++round) {
-            const int bits = round < 2 ? 11 : 10;
-            const int shift = 32 - decided - bits;
-            if (round > 0 || !first_made) {
-                cs_clear(hist);
-#pragma unroll 2
-                for (int i = tid; i < n; i += CS_THREADS) {
-                    const float v = sv[i];
-                    if (v < lo || v > hi) continue;
-                    const unsigned key = key_of(v);
-                    if (key >= tau && (decided == 0 || (key >> (32 - decided)) == prefix))
-                        cs_add(hist, (key >> shift) & ((1u << bits) - 1u), mass_of(v));
-                }
-            }
-            const int bin = cs_pick_bin(cluster, rank, hist, scratch, slot, result, at_least, above);
-            prefix = (prefix << bits) | (unsigned)bin;
-            decided += bits;
-            band(prefix << shift, (prefix << shift) + ((1u << shift) - 1u));
-            if (round == 0 && finish_few(few + 1, prefix, at_least, above, mass_of)) {
-                prefix = (unsigned)result[0];
-                break;
-            }
-        }
-        if (prefix > tau) {
-            tau = prefix;
-            band(tau, tau);
-            mass = 0ull;
-#pragma unroll 2
-            for (int i = tid; i < n; i += CS_THREADS) {
-                const float v = sv[i];
-                if (!(v < lo) && (v > hi || key_of(v) >= tau)) mass += mass_of(v);
-            }
-            mass = cs_block_sum(mass, scratch);
-            cs_gather(cluster, mass, sums + 1, all);
-            total = 0ull;
+    // ---- top-k: tau = the k-th largest key, by counts
+    unsigned long long mass = 0ull, above = 0ull;         // mass: of the kept tokens
+    if (choose_k) {
+        auto need = [&] { return (unsigned long long)k; };
+        bins_from(vmin);
+        each([&](float v) { atomicAdd(hist + bin_of(v), 1u); });
+        const int bin = cs_pick_bin(cluster, rank, hist, scratch, slot, result, need, above);
+        set_tau(finish(few, (unsigned)bin, need, above, [](float) { return true; }, [](float) { return 1ull; }));
+        if (p < 1.f) cs_clear(hist);
+    }
+    // ---- the kept tokens' mass, and the first round of top-p: the largest tau2 >= tau whose tokens (x >= tau2)
+    // hold p of it.  Logits far enough below the maximum hold less than (1 - p) of its mass, 1, all together, and
+    // so of the whole: the threshold lies above them, and the search does without them (half a unit of room
+    // for the rounding of the exponentials; a bound that is no number holds nothing back).
+    const bool choose_p = p < 1.f;
+    const float aside = choose_p ? fminf(vmax - temp * (logf((float)vocab / (1.f - p)) + 0.5f), vmax) : 0.f;
+    if (choose_p) bins_from(fmaxf(vmin, aside));
+    each([&](float v) {
+        if (!kept(v)) return;
+        const unsigned long long m = mass_of(v);
+        mass += m;
+        if (choose_p && !(v < aside) && m != 0ull) cs_add(hist, bin_of(v), m);
+    });
+    unsigned long long all[CS_CLUSTER];
+    unsigned long long total = 0ull;
+    mass = cs_block_sum(mass, scratch);
+    if (!choose_p) {
+        cs_gather(cluster, mass, sums, all);
 #pragma unroll
-            for (int r = 0; r < CS_CLUSTER; ++r) total += all[r];
+        for (int r = 0; r < CS_CLUSTER; ++r) total += all[r];
+    } else {
+        if (tid == 0) sums[0] = mass;               // (read behind the next barrier of the cluster)
+        unsigned long long at_least = 0ull;
+        auto need = [&] {
+#pragma unroll
+            for (int r = 0; r < CS_CLUSTER; ++r) total += *cluster.map_shared_rank(sums, r);
+            at_least = (unsigned long long)((double)p * (double)total);
+            return at_least > 0ull ? at_least : at_least = 1ull;
+        };
+        above = 0ull;
+        const int bin = cs_pick_bin(cluster, rank, hist, scratch, slot, result, need, above);
+        const unsigned tau2 = finish(few + 1, (unsigned)bin, [&] { return at_least; }, above,
+                                     [&](float v) { return kept(v) && !(v < aside); }, mass_of);
+        if (tau2 > tau) {
+            set_tau(tau2);
+            mass = 0ull;
+            each([&](float v) {
+                if (kept(v)) mass += mass_of(v);
+            });
+            mass = cs_block_sum(mass, scratch);
         }
+        cs_gather(cluster, mass, sums + 1, all);
+        total = 0ull;
+#pragma unroll
+        for (int r = 0; r < CS_CLUSTER; ++r) total += all[r];
     }
 
     // (no CTA leaves before everybody has read the last sums: the wait is at the end)
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
 
     // ---- inverse-CDF draw over the kept tokens in index order (exact integer prefix sums)
-    lo = -INFINITY;
-    hi = INFINITY;
-    band(tau, tau);
     unsigned c[4];
-    const unsigned long long sd = seed != nullptr ? (unsigned long long)seed[row] : 0ull;
-    const unsigned long long of = offset != nullptr ? (unsigned long long)offset[row] : 0ull;
     c[0] = (unsigned)of; c[1] = (unsigned)(of >> 32); c[2] = 0u; c[3] = 0u;
     philox4x32_10((unsigned)sd, (unsigned)(sd >> 32), c);
     const double u = (double)(c[0] >> 8) * (1.0 / 16777216.0);   // [0, 1)
@@ -674,7 +662,6 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
         const int per = (n + CS_THREADS - 1) / CS_THREADS;
         const int begin = min(tid * per, n), end = min(begin + per, n);
         unsigned long long mine = 0ull;
-        auto kept = [&](float v) { return !(v < lo) && (v > hi || key_of(v) >= tau); };
         for (int i = begin; i < end; ++i)
             if (kept(sv[i])) mine += mass_of(sv[i]);
         // exclusive prefix of `mine` over the threads

@@ -277,6 +277,35 @@ def test_delta_rule_in_pieces_leaves_later_values_out(head_decay, heads, dim, vd
     ops.check_error_word(DEV)
 
 
+@pytest.mark.parametrize("temperature,opts", [(0.6, {"top_p": 0.8}), (3.0, {"top_p": 0.95}), (0.05, {"top_p": 0.999}),
+                                              (1.0, {"top_p": 1e-6}), (1.5, {"top_k": 3000, "top_p": 0.9}),
+                                              (1.0, {"top_k": 700})])
+def test_sampling_where_the_threshold_is_hard_to_find(temperature, opts):
+    """The kept set and the draw where the first round's bins tell little: equal logits, two values, one logit far
+    above the others, a range past the largest float, minus infinities, many logits in a bin, few logits in all."""
+    import plain_llama as P
+    from mstar_b200 import ops
+
+    vocab = 20011
+    x = rnd(8, vocab, seed=3, scale=2.0)
+    x[0] = 1.5
+    x[1] = (x[1] > 0).float()
+    x[2, 77] = 1e30
+    x[3, 5], x[3, 6] = 3e38, -3e38
+    x[4, ::2] = -float("inf")
+    x[5] = 10 + x[5] * 1e-4
+    x[6] = torch.round(x[6] * 8) / 8
+    seeds, offsets = torch.arange(50, 58, device=DEV), torch.arange(8, device=DEV)
+    full = lambda v, dt: torch.full((8,), v, dtype=dt, device=DEV)
+    extra = {k: full(v, torch.int32 if k == "top_k" else torch.float32) for k, v in opts.items()}
+    got = ops.sample(x, full(temperature, torch.float32), seed=seeds, offset=offsets, **extra).tolist()
+    for r, tok in enumerate(got):
+        p = P.plain_sampling_distribution(x[r].cpu(), temperature, **opts)
+        assert p[tok] > 0, f"row {r}: token {tok} is outside the kept set"
+        cdf, u = torch.cumsum(p, 0), P.plain_uniform(50 + r, r)
+        assert (cdf[tok - 1].item() if tok else 0.0) - 1e-4 <= u <= cdf[tok].item() + 1e-4, (r, tok, u)
+
+
 def test_delta_rule_in_pieces_with_more_blocks_than_fit():
     """So many blocks an SM (34,816 in all) that a share of its shared memory holds no piece."""
     from mstar_b200 import ops
