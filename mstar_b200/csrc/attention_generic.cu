@@ -155,14 +155,20 @@ paged_attention_generic_kernel(const A* __restrict__ q, A* __restrict__ out,
 // maximum and sum by shuffles among its 16 threads, then 4 rows x HD / 16 output columns
 // (packed FMAs over pairs of columns).  Only the probabilities pass through shared memory; the
 // next tile's keys are fetched under the softmax and the sum, its values under the scores.
+// Two groups of 256 threads take the even and the odd tiles, each with stages of its own, and are added up at
+// the end: a block alone on its SM, as most are in a batch of short prompts, is a chain of loads, scores, softmax
+// and sums a tile.  Of a tile, scores are made for the sixteens of keys that a row of the block sees, and only
+// the few keys that some rows see and others don't are taken one by one (the last tile of every row is such a one).
 // Tiles start at multiples of 64 keys whatever the block's rows are, and a tile that a row does
 // not see leaves its sums as they are, so a row's result does not depend on what else is in the
-// batch.  Bound by the FMA pipe and the shared loads that feed it (of 16 bytes, no bank met
-// twice): the float attention of 384 prompt tokens with 32 / 8 heads of 64 (requests of 256 and
-// 128) took 435 us with a block per token and takes 41 us.
+// batch.  Bound by the shared loads that feed the FMA pipe (of 16 bytes, no bank met
+// twice).  448 prompt tokens with 32 / 8 heads of 64 (requests of 256 and 192): 33 us, 41 with one group and
+// whole tiles; one of 250 tokens on 250 cached keys, 24 / 8 heads of 128: 89 and 121 us; 2,000 tokens: 876 and 1,258.
+// 32 rows a block, two blocks an SM: 31 us for the first, 291 instead of 283 for 1,500 tokens with heads of 64.
 #define AR_ROWS 64
 #define AR_KEYS 64
-#define AR_THREADS 256
+#define AR_THREADS 256                         // of a group
+#define AR_GROUPS 2
 
 __device__ __forceinline__ void ar_fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
@@ -173,38 +179,35 @@ __device__ __forceinline__ unsigned long long ar_pack(float lo, float hi) {
 __device__ __forceinline__ float ar_lo(unsigned long long v) { return __uint_as_float((uint32_t)v); }
 __device__ __forceinline__ float ar_hi(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
 
-// O += P V of one tile.  MASKED: a key past the row's last one is left out (a probability of zero
+// O += P V of four keys of a tile.  MASKED: a key that a row does not see is left out (a probability of zero
 // would still make a NaN of a value that is not finite).
 template <int HD, bool MASKED>
 __device__ __forceinline__ void ar_output(unsigned long long (&acc)[4][HD / 32], const float* p_s,
-                                          const float* v_s, int ty, int tx, int key0, const int (&lo_r)[4],
+                                          const float* v_s, int ty, int tx, int j, int key0, const int (&lo_r)[4],
                                           const int (&hi_r)[4]) {
     constexpr int PL = AR_KEYS + 4;
-#pragma unroll 2
-    for (int j = 0; j < AR_KEYS; j += 4) {
-        float4 p[4];
+    float4 p[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(p_s + (ty + 16 * i) * PL + j);
+    for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(p_s + (ty + 16 * i) * PL + j);
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-            unsigned long long v[HD / 32];
+    for (int jj = 0; jj < 4; ++jj) {
+        unsigned long long v[HD / 32];
 #pragma unroll
-            for (int c = 0; c < HD / 32; ++c)
-                v[c] = *reinterpret_cast<const unsigned long long*>(v_s + (j + jj) * HD + 2 * tx + 32 * c);
+        for (int c = 0; c < HD / 32; ++c)
+            v[c] = *reinterpret_cast<const unsigned long long*>(v_s + (j + jj) * HD + 2 * tx + 32 * c);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                if (MASKED && !(key0 + j + jj >= lo_r[i] && key0 + j + jj < hi_r[i])) continue;
-                const float pj = jj == 0 ? p[i].x : jj == 1 ? p[i].y : jj == 2 ? p[i].z : p[i].w;
-                const unsigned long long pp = ar_pack(pj, pj);
+        for (int i = 0; i < 4; ++i) {
+            if (MASKED && !(key0 + j + jj >= lo_r[i] && key0 + j + jj < hi_r[i])) continue;
+            const float pj = jj == 0 ? p[i].x : jj == 1 ? p[i].y : jj == 2 ? p[i].z : p[i].w;
+            const unsigned long long pp = ar_pack(pj, pj);
 #pragma unroll
-                for (int c = 0; c < HD / 32; ++c) ar_fma2(acc[i][c], pp, v[c]);
-            }
+            for (int c = 0; c < HD / 32; ++c) ar_fma2(acc[i][c], pp, v[c]);
         }
     }
 }
 
 template <int HD>
-__global__ void __launch_bounds__(AR_THREADS)
+__global__ void __launch_bounds__(AR_GROUPS * AR_THREADS)
 attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
                           const float* __restrict__ kv_cache, const int* __restrict__ block_table,
                           const int* __restrict__ token_req, const int* __restrict__ cache_pos,
@@ -212,10 +215,13 @@ attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
     constexpr int QL = HD + 4, PL = AR_KEYS + 4;   // floats between rows: 16-byte reads of 8 rows
     extern __shared__ __align__(16) float ar_smem[];
     float* q_s = ar_smem;                          // [ROWS][QL]
-    float* k_s = q_s + AR_ROWS * QL;               // [KEYS][QL]
+    constexpr int BUFS = AR_KEYS * QL + AR_KEYS * HD + AR_ROWS * PL;   // floats of a group
+    const int group = threadIdx.x / AR_THREADS;
+    float* k_s = q_s + AR_ROWS * QL + group * BUFS;    // [KEYS][QL]
     float* v_s = k_s + AR_KEYS * QL;               // [KEYS][HD]
     float* p_s = v_s + AR_KEYS * HD;               // [ROWS][PL]
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int tid = threadIdx.x % AR_THREADS, tx = tid & 15, ty = tid >> 4;
+    auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(AR_THREADS) : "memory"); };
     const int kvh = blockIdx.x;
     const int G = a.nq / a.nkv, TPB = AR_ROWS / G;
     // (the tokens with the most keys first)
@@ -225,7 +231,7 @@ attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
     const size_t v_off = (size_t)a.nkv * a.page_size * HD;
     const float* head_base = kv_cache + (size_t)kvh * a.page_size * HD;
 
-    for (int c = tid; c < AR_ROWS * (HD / 4); c += AR_THREADS) {
+    for (int c = threadIdx.x; c < AR_ROWS * (HD / 4); c += AR_GROUPS * AR_THREADS) {
         const int r = c / (HD / 4), d = (c % (HD / 4)) * 4;
         const bool ok = r < nrows;
         const float* src = q;
@@ -237,15 +243,18 @@ attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
     for (int s0 = 0; s0 < ntok;) {
         // tokens s0 .. s1-1 of the block belong to one request
         const int req = token_req[t0 + s0];
-        int s1 = s0, lo_min = 0x7fffffff, hi_max = 0;
+        int s1 = s0, lo_min = 0x7fffffff, hi_max = 0;      // the keys that any of them sees
+        int full_lo = 0, full_hi = 0x7fffffff;             // ... and those that all of them see
         for (; s1 < ntok && token_req[t0 + s1] == req; ++s1) {
             const int hi = cache_pos[t0 + s1] + 1;
-            lo_min = min(lo_min, (a.window > 0 && hi > a.window) ? hi - a.window : 0);
+            const int lo = (a.window > 0 && hi > a.window) ? hi - a.window : 0;
+            lo_min = min(lo_min, lo);
             hi_max = max(hi_max, hi);
+            full_lo = max(full_lo, lo);
+            full_hi = min(full_hi, hi);
         }
         const int* bt = block_table + (size_t)req * a.bt_stride;
         int lo_r[4], hi_r[4];                      // the keys that this thread's rows see
-        int full_lo = 0, full_hi = 0x7fffffff;     // ... and those that every one of them sees
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int r = ty + 16 * i, tk = r / G;
@@ -254,10 +263,9 @@ attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
                 hi_r[i] = cache_pos[t0 + tk] + 1;
                 lo_r[i] = (a.window > 0 && hi_r[i] > a.window) ? hi_r[i] - a.window : 0;
             }
-            full_lo = max(full_lo, lo_r[i]);
-            full_hi = min(full_hi, hi_r[i]);
         }
         auto load = [&](bool values, int key0) {
+#pragma unroll
             for (int c = tid; c < AR_KEYS * (HD / 4); c += AR_THREADS) {
                 const int j = c / (HD / 4), d = (c % (HD / 4)) * 4, key = key0 + j;
                 const bool ok = key >= lo_min && key < hi_max;
@@ -278,17 +286,23 @@ attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
 #pragma unroll
             for (int c = 0; c < HD / 32; ++c) acc[i][c] = 0ull;
         }
-        const int first = lo_min / AR_KEYS * AR_KEYS;
-        load(false, first);
-        load(true, first);
-        for (int key0 = first; key0 < hi_max; key0 += AR_KEYS) {
-            cp_async_wait<1>();                    // the keys (and the queries) are there
-            __syncthreads();
+        const int tile0 = lo_min / AR_KEYS;
+        const int first = (tile0 + ((tile0 ^ group) & 1)) * AR_KEYS;       // even tiles: group 0
+        if (first < hi_max) load(false, first);
+        else cp_async_commit();
+        if (first < hi_max) load(true, first);
+        else cp_async_commit();
+        cp_async_wait<1>();
+        __syncthreads();                           // the queries are there
+        for (int key0 = first; key0 < hi_max; key0 += AR_GROUPS * AR_KEYS) {
+            cp_async_wait<1>();                    // the keys are there
+            group_sync();
             unsigned long long s2[4][4];
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) s2[i][j] = 0ull;
+            const int sixteens = (min(AR_KEYS, hi_max - key0) + 15) / 16;      // of keys that anyone sees
 #pragma unroll 4
             for (int d = 0; d < HD; d += 4) {
                 ulonglong2 qv[4];
@@ -296,6 +310,7 @@ attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
                 for (int i = 0; i < 4; ++i) qv[i] = *reinterpret_cast<const ulonglong2*>(q_s + (ty + 16 * i) * QL + d);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
+                    if (j >= sixteens) break;
                     const ulonglong2 kv = *reinterpret_cast<const ulonglong2*>(k_s + (tx + 16 * j) * QL + d);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
@@ -304,8 +319,8 @@ attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
                     }
                 }
             }
-            __syncthreads();                       // the keys are done with
-            if (key0 + AR_KEYS < hi_max) load(false, key0 + AR_KEYS);
+            group_sync();                          // the keys are done with
+            if (key0 + AR_GROUPS * AR_KEYS < hi_max) load(false, key0 + AR_GROUPS * AR_KEYS);
             else cp_async_commit();
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -337,28 +352,52 @@ attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
                     asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[i][c]) : "l"(aa));
             }
             cp_async_wait<1>();                    // the values are there
-            __syncthreads();
-            if (key0 >= full_lo && key0 + AR_KEYS <= full_hi)
-                ar_output<HD, false>(acc, p_s, v_s, ty, tx, key0, lo_r, hi_r);
-            else
-                ar_output<HD, true>(acc, p_s, v_s, ty, tx, key0, lo_r, hi_r);
-            __syncthreads();                       // the values and the probabilities are done with
-            if (key0 + AR_KEYS < hi_max) load(true, key0 + AR_KEYS);
+            group_sync();
+            // four keys at a time, of which all are seen by all rows but at the ends
+            const int j1 = min(AR_KEYS, hi_max - key0), j0 = max(0, lo_min - key0) & ~3;
+            const int m0 = min(j1, max(j0, (max(0, full_lo - key0) + 3) & ~3));
+            const int m1 = max(m0, min(j1, full_hi - key0) & ~3);
+            for (int j = j0; j < m0; j += 4) ar_output<HD, true>(acc, p_s, v_s, ty, tx, j, key0, lo_r, hi_r);
+#pragma unroll 2
+            for (int j = m0; j < m1; j += 4) ar_output<HD, false>(acc, p_s, v_s, ty, tx, j, key0, lo_r, hi_r);
+            for (int j = m1; j < j1; j += 4) ar_output<HD, true>(acc, p_s, v_s, ty, tx, j, key0, lo_r, hi_r);
+            group_sync();                          // the values and the probabilities are done with
+            if (key0 + AR_GROUPS * AR_KEYS < hi_max) load(true, key0 + AR_GROUPS * AR_KEYS);
             else cp_async_commit();
         }
+        // the odd tiles' sums pass through the place of their values, the rows' statistics through that of
+        // their probabilities; the even ones' group adds them up
+        float* other_v = q_s + AR_ROWS * QL + BUFS + AR_KEYS * QL;
+        float2* other_ml = reinterpret_cast<float2*>(other_v + AR_KEYS * HD);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            float sum = l[i];
 #pragma unroll
-            for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-            if (hi_r[i] == 0) continue;
+            for (int o = 8; o > 0; o >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], o);
+            if (group == 0) continue;
             const int r = ty + 16 * i;
-            float* dst = out + (size_t)(t0 + r / G) * a.nq * HD + (size_t)(kvh * G + r % G) * HD + 2 * tx;
+            if (tx == 0) other_ml[r] = make_float2(m[i], l[i]);
 #pragma unroll
             for (int c = 0; c < HD / 32; ++c)
-                *reinterpret_cast<float2*>(dst + 32 * c) =
-                    make_float2(ar_lo(acc[i][c]) / sum, ar_hi(acc[i][c]) / sum);
+                *reinterpret_cast<unsigned long long*>(other_v + r * HD + 2 * tx + 32 * c) = acc[i][c];
         }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (group != 0 || hi_r[i] == 0) continue;
+            const int r = ty + 16 * i;
+            const float2 ml = other_ml[r];
+            const float top = fmaxf(m[i], ml.x);
+            const float w0 = expf(m[i] - top), w1 = expf(ml.x - top);      // (a group that saw no key: 0)
+            const float sum = fmaf(l[i], w0, ml.y * w1);
+            float* dst = out + (size_t)(t0 + r / G) * a.nq * HD + (size_t)(kvh * G + r % G) * HD + 2 * tx;
+#pragma unroll
+            for (int c = 0; c < HD / 32; ++c) {
+                const float2 v = *reinterpret_cast<const float2*>(other_v + r * HD + 2 * tx + 32 * c);
+                *reinterpret_cast<float2*>(dst + 32 * c) =
+                    make_float2(fmaf(ar_lo(acc[i][c]), w0, v.x * w1) / sum, fmaf(ar_hi(acc[i][c]), w0, v.y * w1) / sum);
+            }
+        }
+        __syncthreads();                           // the sums have been read
         s0 = s1;
     }
 }
@@ -524,7 +563,8 @@ static int launch_rows_f32(const float* q, float* out, const float* kv, const in
                            const int* token_req, const int* cache_pos, const AttnArgs& a, int num_tokens,
                            cudaStream_t s) {
     constexpr int smem = (int)sizeof(float) *
-                         (2 * AR_ROWS * (HD + 4) + AR_KEYS * HD + AR_ROWS * (AR_KEYS + 4));
+                         (AR_ROWS * (HD + 4) +
+                          AR_GROUPS * (AR_KEYS * (HD + 4) + AR_KEYS * HD + AR_ROWS * (AR_KEYS + 4)));
     static bool configured = false;
     if (!configured) {
         const cudaError_t e = cudaFuncSetAttribute(attention_rows_f32_kernel<HD>,
@@ -533,7 +573,8 @@ static int launch_rows_f32(const float* q, float* out, const float* kv, const in
         configured = true;
     }
     const int per_block = AR_ROWS / (a.nq / a.nkv);
-    attention_rows_f32_kernel<HD><<<dim3(a.nkv, (num_tokens + per_block - 1) / per_block), AR_THREADS, smem, s>>>(
+    attention_rows_f32_kernel<HD><<<dim3(a.nkv, (num_tokens + per_block - 1) / per_block),
+                                     AR_GROUPS * AR_THREADS, smem, s>>>(
         q, out, kv, block_table, token_req, cache_pos, a, num_tokens);
     return launch_status();
 }

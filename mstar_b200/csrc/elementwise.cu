@@ -818,8 +818,9 @@ __global__ void rope_kv_write_vec_kernel(A* __restrict__ qkv, const int* __restr
             const int it = item - rot_items;
             const int per = tail >> 3;
             const int h = it / per, d = a.rotary_dim + (it - h * per) * 8;
-            *reinterpret_cast<uint4*>(kdst + (size_t)h * a.page_size * hd + d) =
-                *reinterpret_cast<const uint4*>(row + (size_t)(a.nq + h) * hd + d);
+            float v[8];
+            load8(row + (size_t)(a.nq + h) * hd + d, v);
+            store8(kdst + (size_t)h * a.page_size * hd + d, v);
         } else {
             const int it = item - rot_items - tail_items;
             const int per = hd >> 3;
@@ -844,16 +845,19 @@ MSTAR_API int mstar_rope_kv_write(void* qkv, int act_dtype, const int* positions
     // table aligned: the vector kernel; else one pair per item
     const bool vec = !interleaved && rotary_dim > 0 && rotary_dim <= 256 && (rotary_dim / 2) % 8 == 0 && hd % 8 == 0 &&
                      (hd - rotary_dim) % 8 == 0 && ((uintptr_t)qkv % 32 == 0) &&
-                     ((uintptr_t)inv_freq % 32 == 0) && (kv_cache == nullptr || (uintptr_t)kv_cache % 32 == 0) &&
-                     act_dtype == MSTAR_BF16;
+                     ((uintptr_t)inv_freq % 32 == 0) && (kv_cache == nullptr || (uintptr_t)kv_cache % 32 == 0);
     if (vec) {
         const int items = (nq + nkv) * (rotary_dim / 16) + nkv * ((hd - rotary_dim) / 8) + nkv * (hd / 8);
         int slices = (items + threads - 1) / threads;
         if (num_tokens >= 256 && slices > 1) slices = 1;
         if (slices < 1) slices = 1;
         dim3 grid(num_tokens, slices);
-        mstar_launch((rope_kv_write_vec_kernel<bf16>), dim3(grid), dim3(threads), 0, s, 
-            (bf16*)qkv, positions, cache_pos, token_req, block_table, inv_freq, (bf16*)kv_cache, a);
+        if (act_dtype == MSTAR_F32)
+            mstar_launch((rope_kv_write_vec_kernel<float>), dim3(grid), dim3(threads), 0, s, (float*)qkv, positions,
+                         cache_pos, token_req, block_table, inv_freq, (float*)kv_cache, a);
+        else
+            mstar_launch((rope_kv_write_vec_kernel<bf16>), dim3(grid), dim3(threads), 0, s, (bf16*)qkv, positions,
+                         cache_pos, token_req, block_table, inv_freq, (bf16*)kv_cache, a);
         return launch_status();
     }
     const int items = (nq + nkv) * (rotary_dim / 2) + nkv * (hd - rotary_dim) + nkv * hd;

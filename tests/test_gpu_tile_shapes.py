@@ -98,6 +98,22 @@ def test_float_attention_of_portions(lens_q, lens_kv, nq, nkv, hd, page, window,
     assert (got - one_token).abs().max() < 2e-6
 
 
+# windows that leave a group of threads no tile, or begin and end inside tiles of both; rows of many tiles; requests
+# that meet inside a block
+@pytest.mark.parametrize("lens_q,lens_kv,nq,nkv,hd,page,window", [
+    ([30], [190], 4, 1, 64, 16, 20), ([70, 3, 50], [500, 67, 300], 4, 2, 128, 16, 130), ([260], [260], 8, 2, 64, 16, 0),
+    ([5, 6, 7, 9, 4], [5, 70, 64, 137, 4], 2, 1, 128, 4, 0)])
+def test_float_attention_of_tiles_in_two_groups(lens_q, lens_kv, nq, nkv, hd, page, window, monkeypatch):
+    from mstar_b200 import ops
+
+    one_token, want, _ = paged_case(lens_q, lens_kv, nq, nkv, hd, page, torch.float32, 7, window)
+    monkeypatch.setattr(ops, "paged_attention_generic",
+                        functools.partial(ops.paged_attention_generic, entries=len(lens_q)))
+    got, want, _ = paged_case(lens_q, lens_kv, nq, nkv, hd, page, torch.float32, 7, window)
+    # products of some 8 rounded to 24 bits in the scores, weights that add up to one
+    assert (got - want).abs().max() < 4e-6
+
+
 # one key, a warp's keys and one more, a round of 512 keys and one more, several rounds; groups of one to nine
 # heads; a window that begins inside a page
 @pytest.mark.parametrize("lens_kv,nq,nkv,hd,page,window", [
