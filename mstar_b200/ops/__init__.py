@@ -54,7 +54,7 @@ def embed_rows(table: torch.Tensor, ids: torch.Tensor, out: torch.Tensor | None 
     assert ids.dtype == torch.int32 and table.dim() == 2 and table.is_contiguous()
     n, (vocab, hidden) = ids.numel(), table.shape
     if out is None:
-        out = torch.empty((n, hidden), dtype=torch.float32, device=table.device)
+        out = table.new_empty((n, hidden), dtype=torch.float32)
     src = prev = None
     if source is not None:
         src, prev = source
@@ -81,7 +81,7 @@ def embed_tanh(table: torch.Tensor, ids: torch.Tensor, norm, source=None, scale:
     _need_cuda(table, ids)
     assert ids.dtype == torch.int32 and table.dim() == 2 and table.is_contiguous()
     n, (vocab, hidden) = ids.numel(), table.shape
-    out = torch.empty((n, hidden), dtype=torch.float32, device=table.device)
+    out = table.new_empty((n, hidden), dtype=torch.float32)
     src = prev = None
     if source is not None:
         src, prev = source
@@ -102,7 +102,7 @@ def add_tanh(resid: torch.Tensor, delta, norm, out_dtype: torch.dtype):
     rows, hidden = resid.shape
     if delta is not None:
         assert delta.shape == resid.shape and delta.dtype == out_dtype and delta.is_contiguous()
-    out = torch.empty((rows, hidden), dtype=out_dtype, device=resid.device)
+    out = resid.new_empty((rows, hidden), dtype=out_dtype)
     w, b, wd, alpha = _tanh_norm_args(norm, hidden)
     check(lib.get("elementwise").mstar_add_tanh(
         resid.data_ptr(), _ptr(delta), w, b, wd, alpha, out.data_ptr(), _dt(out), rows, hidden,
@@ -132,7 +132,7 @@ def add_rmsnorm(resid: torch.Tensor, delta, weight: torch.Tensor, eps: float,
     if delta is not None:
         assert delta.shape == resid.shape and delta.dtype == out_dtype and delta.is_contiguous()
     if out is None:
-        out = torch.empty((rows, hidden), dtype=out_dtype, device=resid.device)
+        out = resid.new_empty((rows, hidden), dtype=out_dtype)
     check(lib.get("elementwise").mstar_add_rmsnorm(
         resid.data_ptr(), _ptr(delta), weight.data_ptr(), _dt(weight), out.data_ptr(), _dt(out),
         rows, hidden, float(eps), float(weight_offset), int(resid_static), _stream()),
@@ -145,7 +145,7 @@ def gather_add_rows(resid: torch.Tensor, delta, rows: torch.Tensor):
     _need_cuda(resid, delta, rows)
     assert resid.dtype == torch.float32 and resid.is_contiguous() and rows.dtype == torch.int32
     hidden = resid.shape[1]
-    out = torch.empty((rows.numel(), hidden), dtype=torch.float32, device=resid.device)
+    out = resid.new_empty((rows.numel(), hidden), dtype=torch.float32)
     act = _dt(delta) if delta is not None else F32
     if delta is not None:
         assert delta.shape == resid.shape and delta.is_contiguous()
@@ -172,7 +172,7 @@ def silu_mul(gate_up: torch.Tensor, out=None, kind: str = "silu", limit: float =
     assert gate_up.dim() == 2 and gate_up.is_contiguous() and gate_up.shape[1] % 2 == 0
     rows, inter = gate_up.shape[0], gate_up.shape[1] // 2
     if out is None:
-        out = torch.empty((rows, inter), dtype=gate_up.dtype, device=gate_up.device)
+        out = gate_up.new_empty((rows, inter), dtype=gate_up.dtype)
     check(lib.get("elementwise").mstar_silu_mul(
         gate_up.data_ptr(), out.data_ptr(), _dt(gate_up), rows, inter, GATED_PRODUCTS[kind],
         float(limit), float(alpha), _stream()), "silu_mul")
@@ -190,7 +190,7 @@ def bias_act_mul(gate_up: torch.Tensor, bias: torch.Tensor, out_dtype: torch.dty
     assert gate_up.dtype == torch.float32 and gate_up.dim() == 2 and gate_up.is_contiguous()
     assert gate_up.shape[1] % 2 == 0 and bias.numel() == gate_up.shape[1] and bias.is_contiguous()
     rows, inter = gate_up.shape[0], gate_up.shape[1] // 2
-    out = torch.empty((rows, inter), dtype=out_dtype, device=gate_up.device)
+    out = gate_up.new_empty((rows, inter), dtype=out_dtype)
     check(lib.get("elementwise").mstar_bias_act_mul(
         gate_up.data_ptr(), bias.data_ptr(), _dt(bias), out.data_ptr(), _DT[out_dtype], rows,
         inter, GATE_ACTIVATIONS[kind], _stream()), "bias_act_mul")
@@ -201,7 +201,7 @@ def convert(src: torch.Tensor, dtype: torch.dtype):
     _need_cuda(src)
     if src.dtype == dtype:
         return src
-    out = torch.empty(src.shape, dtype=dtype, device=src.device)
+    out = src.new_empty(src.shape, dtype=dtype)
     if src.dim() == 2 and src.stride(1) == 1 and src.shape[1] < src.stride(0) < 1 << 31:    # columns of wider rows
         check(lib.get("elementwise").mstar_convert_rows(
             src.data_ptr(), _dt(src), out.data_ptr(), _dt(out), src.shape[0], src.shape[1], src.stride(0),
@@ -366,15 +366,14 @@ def paged_decode_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, kv
                                  sms=num_sms(q.device))
     scratch = None
     if splits > 1:
-        scratch = torch.empty(tokens * num_heads * splits * (head_dim + 2), dtype=torch.float32,
-                              device=q.device)
+        scratch = q.new_empty(tokens * num_heads * splits * (head_dim + 2), dtype=torch.float32)
     if kv_map is not None:
         code = lib.get("attention_decode").mstar_paged_decode_attention_bf16_tma(
             kv_map, q.data_ptr(), q_stride, out.data_ptr(), kv_cache.data_ptr(),
             block_table.data_ptr(), block_table.stride(0), token_req.data_ptr(),
             cache_pos.data_ptr(), tokens, num_heads, num_kv_heads, head_dim, page_size,
             float(scale), chunk, splits, int(static_keys), _ptr(scratch),
-            tcgen05_error_word(q.device).data_ptr(), _stream())
+            _error_ptr(q), _stream())
         if code == -1:
             raise KernelError("TMA decode attention refuses this shape")
         check(code, "paged_decode_attention_tma")
@@ -425,7 +424,7 @@ def paged_prefill_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, k
             kv_map, q.data_ptr(), q_stride, q.shape[0], out.data_ptr(), block_table.data_ptr(),
             block_table.stride(0), qo_indptr.data_ptr(), kv_len.data_ptr(), first_entry, entries,
             max_q_len, num_heads, num_kv_heads, head_dim, page_size, float(scale),
-            tcgen05_error_word(q.device).data_ptr(), _stream())
+            _error_ptr(q), _stream())
         if code == -1:
             raise KernelError("tcgen05 prefill attention refuses this shape")
         check(code, "paged_prefill_attention_tc")
@@ -434,7 +433,7 @@ def paged_prefill_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, k
         kv_map or 0, q.data_ptr(), q_stride, out.data_ptr(), kv_cache.data_ptr(),
         block_table.data_ptr(), block_table.stride(0), qo_indptr.data_ptr(), kv_len.data_ptr(),
         first_entry, entries, max_q_len, num_heads, num_kv_heads, head_dim, page_size, window,
-        float(scale), tcgen05_error_word(q.device).data_ptr(), _stream())
+        float(scale), _error_ptr(q), _stream())
     if code == -1:
         raise KernelError(f"prefill attention refuses heads={num_heads}, kv_heads={num_kv_heads}, "
                           f"head_dim={head_dim} (head_dim in {FAST_ATTENTION_HEAD_DIMS})")
@@ -450,11 +449,11 @@ def sgemm_nt(a: torch.Tensor, w: torch.Tensor, out=None):
     m, k = a.shape
     n = w.shape[0]
     if out is None:
-        out = torch.empty((m, n), dtype=torch.float32, device=a.device)
+        out = a.new_empty((m, n), dtype=torch.float32)
     assert out.stride(1) == 1
     check(lib.get("gemm_f32").mstar_sgemm_nt(
         a.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, a.stride(0), w.stride(0),
-        out.stride(0), tcgen05_error_word(a.device).data_ptr(), _stream()), "sgemm_nt")
+        out.stride(0), _error_ptr(a), _stream()), "sgemm_nt")
     return out
 
 
@@ -464,10 +463,11 @@ SMALL_M = 16
 
 
 def _smallm_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
-    return (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and 0 < x.shape[0] <= SMALL_M
-            and x.shape[1] % 32 == 0 and x.stride(1) == 1 and w.stride(1) == 1
-            and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
-            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+    if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or not 0 < x.shape[0] <= SMALL_M:
+        return False
+    (ldx, sx), (ldw, sw) = x.stride(), w.stride()
+    return (x.shape[1] % 32 == 0 and sx == 1 and sw == 1 and (ldx | ldw) % 8 == 0
+            and (x.data_ptr() | w.data_ptr()) % 16 == 0)
 
 
 def _gemm_smallm(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype, gated,
@@ -476,11 +476,11 @@ def _gemm_smallm(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype, gated
     form of gelu, 3 by the clamped swish with ``limit`` and ``alpha``."""
     m, k = x.shape
     n = w.shape[0]
-    out = torch.empty((m, n // 2 if gated else n), dtype=out_dtype, device=x.device)
+    cols = n // 2 if gated else n
+    out = x.new_empty((m, cols), dtype=out_dtype)
     code = lib.get("gemm_smallm_bulk").mstar_gemm_smallm_bulk_bf16(
-        x.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, x.stride(0), w.stride(0),
-        out.stride(0), int(gated), _dt(out), int(static_weights),
-        tcgen05_error_word(x.device).data_ptr(), float(limit), float(alpha), _stream())
+        x.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, x.stride(0), w.stride(0), cols, gated,
+        _DT[out_dtype], static_weights, _error_ptr(x), limit, alpha, _stream())
     if code == -1:
         raise KernelError(f"small-M GEMM refuses M={m}, N={n}, K={k}")
     check(code, "gemm_smallm_bulk")
@@ -500,10 +500,10 @@ def linear_planes(x: torch.Tensor, w: torch.Tensor, plane_rows: int,
     n, full = w.shape[0], planes - 1
     assert planes > 1 and n > full * plane_rows
     if _smallm_ok(x[0], w) and plane_rows % 8 == 0 and os.environ.get("MSTAR_PLANES") != "0":
-        out = torch.empty((m, n), dtype=torch.float32, device=x.device)
+        out = x.new_empty((m, n), dtype=torch.float32)
         code = lib.get("gemm_smallm_bulk").mstar_gemm_smallm_bulk_planes(
             x.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, k, k, n, plane_rows, planes, m * k,
-            int(static_weights), tcgen05_error_word(x.device).data_ptr(), _stream())
+            int(static_weights), _error_ptr(x), _stream())
         if code == -1:
             raise KernelError(f"small-M GEMM refuses M={m}, N={n}, K={k}, planes of {plane_rows} rows")
         check(code, "gemm_smallm_bulk_planes")
@@ -546,11 +546,11 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None 
     m, k = x.shape
     n = w.shape[0]
     out_dtype = out_dtype or torch.bfloat16
-    out = torch.empty((m, n), dtype=out_dtype, device=x.device)
+    out = x.new_empty((m, n), dtype=out_dtype)
     code = lib.get("gemm_skinny").mstar_gemm_skinny_bf16(
         x.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, x.stride(0), w.stride(0),
         out.stride(0), _dt(out), int(static_weights),
-        tcgen05_error_word(x.device).data_ptr(), _stream())
+        _error_ptr(x), _stream())
     if code == -1:
         raise KernelError(f"skinny GEMM refuses M={m}, N={n}, K={k} (at most {SKINNY_MAX} rows, "
                           "K and row strides multiples of 8, operands 16-byte aligned)")
@@ -578,13 +578,13 @@ def qkv_rope_write(x: torch.Tensor, w_qkv: torch.Tensor, positions, cache_pos, t
     assert kv_cache.is_contiguous() and inv_freq.dtype == torch.float32
     assert tuple(kv_cache.shape[1:]) == (2, num_kv_heads, page_size, head_dim)
     m, k = x.shape
-    q = torch.empty((m, num_heads * head_dim), dtype=torch.bfloat16, device=x.device)
+    q = x.new_empty((m, num_heads * head_dim), dtype=torch.bfloat16)
     code = lib.get("gemm_smallm_bulk").mstar_qkv_rope_write_bulk_bf16(
         x.data_ptr(), w_qkv.data_ptr(), q.data_ptr(), m, k, x.stride(0), w_qkv.stride(0),
         q.stride(0), positions.data_ptr(), cache_pos.data_ptr(), token_req.data_ptr(),
         block_table.data_ptr(), block_table.stride(0), inv_freq.data_ptr(), kv_cache.data_ptr(),
         num_heads, num_kv_heads, head_dim, page_size, int(static_weights),
-        tcgen05_error_word(x.device).data_ptr(), _stream())
+        _error_ptr(x), _stream())
     if code == -1:
         raise KernelError(f"fused qkv/rotary product refuses M={m}, K={k}, heads={num_heads}, "
                           f"kv_heads={num_kv_heads}, head_dim={head_dim}")
@@ -605,6 +605,12 @@ def tcgen05_error_word(device) -> torch.Tensor:
     if key not in _tc_error_words:
         _tc_error_words[key] = torch.zeros(1, dtype=torch.int32, device=device)
     return _tc_error_words[key]
+
+
+def _error_ptr(t: torch.Tensor) -> int:
+    """Address of the error word of the device that ``t`` lies on."""
+    word = _tc_error_words.get(t.get_device())
+    return (tcgen05_error_word(t.device) if word is None else word).data_ptr()
 
 
 WAIT_CODES = {
@@ -665,10 +671,10 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None
     assert x.stride(1) == 1 and w.stride(1) == 1
     m, k = x.shape
     n = w.shape[0]
-    out = torch.empty((m, n), dtype=out_dtype, device=x.device)
+    out = x.new_empty((m, n), dtype=out_dtype)
     code = lib.get("gemm_tcgen05").mstar_gemm_tcgen05_bf16(
         x.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, x.stride(0), w.stride(0),
-        out.stride(0), _dt(out), bn, tcgen05_error_word(x.device).data_ptr(), _stream())
+        out.stride(0), _dt(out), bn, _error_ptr(x), _stream())
     if code == -1:
         raise KernelError(f"tcgen05 GEMM refuses M={m}, N={n}, K={k} (K and row strides must be "
                           "multiples of 8, operands 16-byte aligned)")
@@ -690,10 +696,10 @@ def gemm_tcgen05_gated(x: torch.Tensor, w_gate_up: torch.Tensor, kind: str = "si
     assert x.stride(1) == 1 and w_gate_up.stride(1) == 1 and x.shape[1] == w_gate_up.shape[1]
     m, k = x.shape
     n = w_gate_up.shape[0]
-    out = torch.empty((m, n // 2), dtype=torch.bfloat16, device=x.device)
+    out = x.new_empty((m, n // 2), dtype=torch.bfloat16)
     code = lib.get("gemm_tcgen05").mstar_gemm_tcgen05_gated_bf16(
         x.data_ptr(), w_gate_up.data_ptr(), out.data_ptr(), m, n, k, x.stride(0),
-        w_gate_up.stride(0), out.stride(0), tcgen05_error_word(x.device).data_ptr(),
+        w_gate_up.stride(0), out.stride(0), _error_ptr(x),
         code_of[kind], float(limit), float(alpha), _stream())
     if code == -1:
         raise KernelError(f"gated tcgen05 GEMM refuses M={m}, N={n}, K={k}")
@@ -743,14 +749,16 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = Non
     then start their weight copies while the kernel before them is still draining."""
     bf16 = x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.is_cuda and w.is_cuda
     m, n = x.shape[0], w.shape[0]
-    if bf16 and out_dtype is None and m > SKINNY_MAX and tcgen05_tile(m, n) is None:
-        # the common case of a prompt portion on a narrow projection, decided first: this
-        # function runs a hundred times in a step that the host has to get launched
-        return torch.mm(x, w.t())
+    # the common cases of a decode step and of a prompt portion on a narrow projection, decided first: this
+    # function runs a hundred times in a step that the host has to get launched
+    if bf16:
+        if m <= SMALL_M:
+            if out_dtype in (None, torch.bfloat16, torch.float32) and _smallm_ok(x, w):
+                return _gemm_smallm(x, w, out_dtype or torch.bfloat16, 0, static_weights)
+        elif out_dtype is None and m > SKINNY_MAX and tcgen05_tile(m, n) is None:
+            return torch.mm(x, w.t())
     _need_cuda(x, w)
     out_dtype = out_dtype or x.dtype
-    if out_dtype in (torch.bfloat16, torch.float32) and _smallm_ok(x, w):
-        return _gemm_smallm(x, w, out_dtype, gated=False, static_weights=static_weights)
     if out_dtype in (torch.bfloat16, torch.float32) and _skinny_ok(x, w):
         return gemm_skinny(x, w, out_dtype, static_weights=static_weights)
     if out_dtype in (torch.bfloat16, torch.float32) and _tc_ok(x, w):
@@ -778,10 +786,10 @@ def linear_act(x: torch.Tensor, w: torch.Tensor, kind: str, static_weights: bool
     if (kind == "relu2" and _smallm_ok(x, w) and os.environ.get("MSTAR_FUSED_ACT") != "0"):
         m, k = x.shape
         n = w.shape[0]
-        out = torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
+        out = x.new_empty((m, n), dtype=torch.bfloat16)
         code = lib.get("gemm_smallm_bulk").mstar_gemm_smallm_bulk_relu2_bf16(
             x.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, x.stride(0), w.stride(0),
-            out.stride(0), int(static_weights), tcgen05_error_word(x.device).data_ptr(), _stream())
+            out.stride(0), int(static_weights), _error_ptr(x), _stream())
         if code == -1:
             raise KernelError(f"small-M GEMM refuses M={m}, N={n}, K={k}")
         check(code, "gemm_smallm_bulk_relu2")
@@ -827,7 +835,7 @@ def argmax(logits: torch.Tensor):
     _need_cuda(logits)
     assert logits.dtype == torch.float32 and logits.dim() == 2 and logits.stride(1) == 1
     rows, vocab = logits.shape
-    out = torch.empty((rows,), dtype=torch.int32, device=logits.device)
+    out = logits.new_empty((rows,), dtype=torch.int32)
     best, arrived = _argmax_buffers(logits.device, rows)
     check(lib.get("sampling").mstar_argmax(
         logits.data_ptr(), logits.stride(0), rows, vocab, out.data_ptr(), best.data_ptr(),
@@ -850,7 +858,7 @@ def sample(logits: torch.Tensor, temperature, top_k=None, top_p=None, penalty=No
     if seen_mask is not None:
         assert seen_mask.dtype == torch.uint8 and seen_mask.shape[1] == vocab
         assert seen_mask.is_contiguous()
-    out = torch.empty((rows,), dtype=torch.int32, device=logits.device)
+    out = logits.new_empty((rows,), dtype=torch.int32)
     check(lib.get("sampling").mstar_sample(
         logits.data_ptr(), logits.stride(0), rows, vocab, temperature.data_ptr(), _ptr(top_k),
         _ptr(top_p), _ptr(penalty), _ptr(seen_mask), _ptr(seen_rows), _ptr(seed), _ptr(offset),
@@ -886,9 +894,9 @@ def add_postnorm_rmsnorm(resid: torch.Tensor, delta: torch.Tensor, post_weight: 
     assert delta.dtype in (out_dtype, torch.float32)
     if weight is not None:
         assert weight.numel() == hidden and weight.is_contiguous()
-        out = torch.empty((rows, hidden), dtype=out_dtype, device=resid.device)
+        out = resid.new_empty((rows, hidden), dtype=out_dtype)
     elif plain_out and out_dtype != torch.float32:
-        out = torch.empty((rows, hidden), dtype=out_dtype, device=resid.device)
+        out = resid.new_empty((rows, hidden), dtype=out_dtype)
     code = lib.get("elementwise").mstar_add_postnorm_rmsnorm(
         resid.data_ptr(), delta.data_ptr(), _dt(delta), post_weight.data_ptr(), float(post_eps),
         float(post_offset), float(post_scale), _ptr(weight),
@@ -912,7 +920,7 @@ def mean_of_norms(branches, weights, eps: float) -> torch.Tensor:
     for x, w in zip(branches, weights):
         assert x.shape == (rows, hidden) and x.is_contiguous() and x.dtype == branches[0].dtype
         assert w.dtype == torch.float32 and w.numel() == hidden
-    out = torch.empty((rows, hidden), dtype=torch.float32, device=branches[0].device)
+    out = branches[0].new_empty((rows, hidden), dtype=torch.float32)
     xs = [b.data_ptr() for b in branches] + [0] * (4 - n)
     ws = [w.data_ptr() for w in weights] + [0] * (4 - n)
     check(lib.get("elementwise").mstar_mean_of_norms(
@@ -951,7 +959,7 @@ class MeanOfNorms:
             assert w.dtype == torch.float32 and w.numel() == hidden
         out = None
         if plain_out and out_dtype != torch.float32:
-            out = torch.empty(resid.shape, dtype=out_dtype, device=resid.device)
+            out = resid.new_empty(resid.shape, dtype=out_dtype)
         check(lib.get("elementwise").mstar_mean2_postnorm(
             resid.data_ptr(), x0.data_ptr(), self.branches[1].data_ptr(),
             self.weights[0].data_ptr(), self.weights[1].data_ptr(), self.eps,
@@ -998,7 +1006,7 @@ def head_gate_mul(y: torch.Tensor, gate: torch.Tensor, heads: int,
     assert y.dim() == 2 and y.is_contiguous() and y.shape[1] % heads == 0
     assert tuple(gate.shape) == (y.shape[0], heads) and gate.stride(1) == 1
     out_dtype = out_dtype or y.dtype
-    out = y if out_dtype == y.dtype else torch.empty(y.shape, dtype=out_dtype, device=y.device)
+    out = y if out_dtype == y.dtype else y.new_empty(y.shape, dtype=out_dtype)
     check(lib.get("elementwise").mstar_head_gate_mul(
         y.data_ptr(), _dt(y), out.data_ptr(), _dt(out), gate.data_ptr(), _dt(gate), gate.stride(0),
         y.shape[0], heads, y.shape[1] // heads, _stream()), "head_gate_mul")
@@ -1024,7 +1032,7 @@ def matrix_memory_scan(proj: torch.Tensor, gates: torch.Tensor, bias: torch.Tens
     assert bias.dtype == torch.float32 and bias.numel() == 2 * heads
     assert state.dtype == torch.float32 and state.dim() == 2 and state.is_contiguous()
     tokens = proj.shape[0]
-    out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=proj.device)
+    out = proj.new_empty((tokens, heads * vdim), dtype=torch.float32)
     code = lib.get("matrix_memory").mstar_matrix_memory_scan(
         proj.data_ptr(), _dt(proj), proj.stride(0), heads * dim, 2 * heads * dim, gates.data_ptr(),
         bias.data_ptr(), qo_indptr.data_ptr(), slots.data_ptr(), state.data_ptr(),
@@ -1047,7 +1055,7 @@ def head_norm_gate(o: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, he
     assert kind in ("sigmoid", "silu")
     assert o.dtype == torch.float32 and o.is_contiguous() and weight.dtype == torch.float32
     assert gate.dtype in (out_dtype, torch.float32) and gate.stride(1) == 1 and gate.shape == o.shape
-    out = torch.empty(o.shape, dtype=out_dtype, device=o.device)
+    out = o.new_empty(o.shape, dtype=out_dtype)
     check(lib.get("matrix_memory").mstar_head_norm_gate(
         o.data_ptr(), gate.data_ptr(), _dt(gate), gate.stride(0), weight.data_ptr(), out.data_ptr(),
         _dt(out), o.shape[0], heads, vdim, float(eps), int(kind == "silu"), int(gate_first),
@@ -1091,7 +1099,7 @@ def latent_fill(q, dkv, norm_weight, freq: torch.Tensor, positions, cache_pos, t
     if q_latent is not None:
         q_rank = q_latent.shape[1]
         assert q_latent_weight.dtype == torch.float32 and q_latent_weight.numel() == q_rank
-        out = torch.empty((tokens, q_rank), dtype=act, device=q_latent.device)
+        out = q_latent.new_empty((tokens, q_rank), dtype=act)
     code = lib.get("attention_latent").mstar_latent_fill(
         _ptr(q), q.stride(0) if q is not None else 0, _ptr(dkv),
         dkv.stride(0) if dkv is not None else 0, _DT[in_dtype], _DT[act], _ptr(norm_weight),
@@ -1150,11 +1158,10 @@ def latent_attention(q_abs: torch.Tensor, q_rot: torch.Tensor, cache: torch.Tens
     if window:
         max_keys = min(max_keys, window)
     group, splits = latent_attention_plan(tokens, heads, rank, max_keys, num_sms(q_abs.device))
-    out = torch.empty((tokens, heads, rank), dtype=torch.float32, device=q_abs.device)
+    out = q_abs.new_empty((tokens, heads, rank), dtype=torch.float32)
     scratch = None
     if splits > 1:
-        scratch = torch.empty(tokens * heads * splits * (rank + 2), dtype=torch.float32,
-                              device=q_abs.device)
+        scratch = q_abs.new_empty(tokens * heads * splits * (rank + 2), dtype=torch.float32)
     code = lib.get("attention_latent").mstar_latent_attention(
         q_abs.data_ptr(), q_rot.data_ptr(), q_rot.stride(0), q_rot.stride(1), out.data_ptr(),
         cache.data_ptr(), block_table.data_ptr(), block_table.stride(0), token_req.data_ptr(),
@@ -1302,7 +1309,7 @@ def linear_per_head(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | N
         a, b = x.transpose(0, 1), w.transpose(1, 2)
         # the library writes [heads, tokens, n] straight into the rows of [tokens, heads, n]
         # (a row stride of heads * n), so no copy follows the product
-        out = torch.empty((tokens, heads, n), dtype=out_dtype, device=x.device)
+        out = x.new_empty((tokens, heads, n), dtype=out_dtype)
         if _BMM_INTO_ROWS.get(out_dtype, True):
             try:
                 if out_dtype == torch.float32:
@@ -1320,7 +1327,7 @@ def linear_per_head(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | N
         return torch.bmm(a, b).transpose(0, 1).contiguous()
     xf = x if x.dtype == torch.float32 else x.float()
     wf = w if w.dtype == torch.float32 else w.float()
-    out = torch.empty((tokens, heads, n), dtype=torch.float32, device=x.device)
+    out = x.new_empty((tokens, heads, n), dtype=torch.float32)
     for h in range(heads):
         sgemm_nt(xf[:, h], wf[h], out[:, h])
     return out if out_dtype == torch.float32 else convert(out, out_dtype)
@@ -1340,8 +1347,8 @@ def route_topk(logits: torch.Tensor, top: int, softmax: bool = False, renormaliz
     tokens, experts = logits.shape
     assert choice_bias is None or (choice_bias.dtype == torch.float32
                                    and choice_bias.numel() == experts)
-    chosen = torch.empty((tokens, top), dtype=torch.int32, device=logits.device)
-    weight = torch.empty((tokens, top), dtype=torch.float32, device=logits.device)
+    chosen = logits.new_empty((tokens, top), dtype=torch.int32)
+    weight = logits.new_empty((tokens, top), dtype=torch.float32)
     code = lib.get("routed_experts").mstar_route_topk(
         logits.data_ptr(), _ptr(choice_bias), chosen.data_ptr(), weight.data_ptr(), tokens, experts, top,
         int(softmax), int(renormalize), logits.stride(0), *(groups or (0, 0)), float(renorm_eps),
@@ -1373,7 +1380,7 @@ def experts_by_row(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tenso
     assert w_gate_up.dtype == x.dtype and w_down.dtype == x.dtype
     assert w_gate_up.shape[1] == width and w_down.shape[1] == ff
     assert add is None or (add.shape == x.shape and add.is_contiguous() and add.dtype == x.dtype)
-    act = torch.empty((tokens * top, ff), dtype=torch.float32, device=x.device)
+    act = x.new_empty((tokens * top, ff), dtype=torch.float32)
     out = torch.empty_like(x)
     code = lib.get("routed_experts").mstar_experts_by_row(
         x.data_ptr(), w_gate_up.data_ptr(), w_down.data_ptr(), chosen.data_ptr(),
@@ -1427,17 +1434,16 @@ def experts_grouped(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tens
     if add is not None and add.data_ptr() % 16:    # the kernels read whole 16-byte pieces
         add = add.clone()
     rows = tokens * top
-    ints = torch.empty(2 * rows + experts + 2 + 2 * (rows // 128 + experts), dtype=torch.int32,
-                       device=x.device)
-    act = torch.empty((rows, ff), dtype=torch.bfloat16, device=x.device)
-    y = torch.empty((rows, width), dtype=torch.float32, device=x.device)
+    ints = x.new_empty(2 * rows + experts + 2 + 2 * (rows // 128 + experts), dtype=torch.int32)
+    act = x.new_empty((rows, ff), dtype=torch.bfloat16)
+    y = x.new_empty((rows, width), dtype=torch.float32)
     out = torch.empty_like(x)
     code = lib.get("routed_experts").mstar_experts_grouped(
         x.data_ptr(), w_gate_up.data_ptr(), w_down.data_ptr(), chosen.data_ptr(),
         weight.data_ptr(), ints.data_ptr(), act.data_ptr(), y.data_ptr(), _ptr(add),
         out.data_ptr(), tokens, width, ff, top, experts, int(scale_input),
         _gated_code(gated, clamp), int(real), *(clamp or (0.0, 0.0)), *_add_gate(add_gate, tokens),
-        tcgen05_error_word(x.device).data_ptr(), _stream())
+        _error_ptr(x), _stream())
     if code == -1:
         raise KernelError(f"the grouped expert kernels refuse width={width}, ff={ff}, "
                           f"experts={experts} (width and ff multiples of 8, at most 1024 experts)")
@@ -1534,7 +1540,7 @@ def sink_prepare(qkv: torch.Tensor, bias, q_norm, k_norm, freq, positions, cache
         assert w is None or (_dt(w) == wd and w.is_contiguous())
     if rot:
         assert freq is not None and freq.dtype == torch.float64 and freq.numel() == rot // 2
-    q = torch.empty((tokens, num_heads * head_dim), dtype=out_dtype, device=qkv.device)
+    q = qkv.new_empty((tokens, num_heads * head_dim), dtype=out_dtype)
     code = lib.get("attention_sink").mstar_sink_prepare(
         qkv.data_ptr(), _ptr(bias), _ptr(q_norm), _ptr(k_norm), wd, _ptr(freq),
         positions.data_ptr(), cache_pos.data_ptr(), token_req.data_ptr(), block_table.data_ptr(),
@@ -1658,7 +1664,7 @@ def sink_attention(q: torch.Tensor, kv_cache: torch.Tensor, block_table, token_r
         assert bias.dtype == torch.float32 and bias.numel() == num_heads and bias.is_contiguous()
     assert not (sigmoid and sink is not None) and not (chunk and window)
     cap = float(softcap or 0.0)
-    out = torch.empty((tokens, num_heads * v_dim), dtype=q.dtype, device=q.device)
+    out = q.new_empty((tokens, num_heads * v_dim), dtype=q.dtype)
     if (ctx is not None and q.dtype == torch.bfloat16 and head_dim % 8 == 0 and v_dim % 8 == 0
             and max(head_dim, v_dim) <= 256 and os.environ.get("MSTAR_SINK_ATTENTION") != "generic"):
         max_keys = ctx.max_kv_len
@@ -1673,15 +1679,14 @@ def sink_attention(q: torch.Tensor, kv_cache: torch.Tensor, block_table, token_r
             splits = prompt_splits(row_tiles * num_kv_heads * ctx.num_entries, max_keys, sms)
             scratch = None
             if splits > 1:
-                scratch = torch.empty(tokens * num_heads * splits * (v_dim + 2), dtype=torch.float32,
-                                      device=q.device)
+                scratch = q.new_empty(tokens * num_heads * splits * (v_dim + 2), dtype=torch.float32)
             code = lib.get("attention_prompt_tc").mstar_sink_attention_prompt(
                 kv_map, q.data_ptr(), q.stride(0), out.data_ptr(), block_table.data_ptr(),
                 block_table.stride(0), ctx.qo_indptr.data_ptr(), ctx.kv_len.data_ptr(),
                 ctx.num_entries, tokens, ctx.max_q_len, num_heads, num_kv_heads, head_dim, page_size,
                 int(window or 0), int(keep_first), float(scale), splits, _ptr(scratch), _ptr(gate),
                 gate.stride(0) if gate is not None else 0, int(gate_features), cap, _ptr(sink),
-                int(chunk), int(sigmoid), _ptr(bias), tcgen05_error_word(q.device).data_ptr(), _stream())
+                int(chunk), int(sigmoid), _ptr(bias), _error_ptr(q), _stream())
             if code < 0:
                 raise KernelError(f"prompt attention refuses heads={num_heads}, kv_heads={num_kv_heads}, "
                                   f"head_dim={head_dim} (code {code})")
@@ -1700,8 +1705,7 @@ def sink_attention(q: torch.Tensor, kv_cache: torch.Tensor, block_table, token_r
                 splits = 2
         scratch = None
         if splits > 1:
-            scratch = torch.empty(tokens * num_heads * splits * (v_dim + 2), dtype=torch.float32,
-                                  device=q.device)
+            scratch = q.new_empty(tokens * num_heads * splits * (v_dim + 2), dtype=torch.float32)
         code = lib.get("attention_sink_tc").mstar_sink_attention_tc(
             q.data_ptr(), q.stride(0), out.data_ptr(), kv_cache.data_ptr(), block_table.data_ptr(),
             block_table.stride(0), ctx.qo_indptr.data_ptr(), ctx.kv_len.data_ptr(),
@@ -1751,7 +1755,7 @@ def conv_silu(xz: torch.Tensor, weight, bias, token_req, qo_indptr, slots, state
     assert weight.dtype == bias.dtype
     assert state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1
     tokens = xz.shape[0]
-    out = torch.empty((tokens, inner), dtype=xz.dtype, device=xz.device)
+    out = xz.new_empty((tokens, inner), dtype=xz.dtype)
     if (weight_t is not None and bias_f32 is not None and inner % 8 == 0 and xz.stride(0) % 8 == 0
             and state.stride(0) % 4 == 0 and xz.data_ptr() % 16 == 0
             and os.environ.get("MSTAR_CONV") != "scalar"):
@@ -1843,7 +1847,7 @@ def selective_scan(xc: torch.Tensor, xz: torch.Tensor, proj: torch.Tensor, w_dt,
         # (cut by their own lengths, portions have a piece for every started 64 tokens at most)
         places = entries * pieces if piece > 0 else tokens // 64 + entries
     # one piece of scratch: the product, the pieces' states, their summed step sizes
-    scratch = (torch.empty(inner * (dt_tokens + places * (n_state + 1)), dtype=torch.float32, device=xc.device)
+    scratch = (xc.new_empty(inner * (dt_tokens + places * (n_state + 1)), dtype=torch.float32)
                if dt_tokens or places else None)
     work = _ptr(scratch)
     piece_state = work + 4 * inner * dt_tokens if places else 0
@@ -1854,7 +1858,7 @@ def selective_scan(xc: torch.Tensor, xz: torch.Tensor, proj: torch.Tensor, w_dt,
         slots.data_ptr(), state.data_ptr(), state.stride(0), out.data_ptr(), _dt(xc), entries,
         inner, n_state, rank, taps, piece, pieces, piece_state, piece_dt,
         work if dt_tokens else 0, dt_tokens,
-        max_q_len or 0, tcgen05_error_word(xc.device).data_ptr() if rank >= 512 else 0, _stream())
+        max_q_len or 0, _error_ptr(xc) if rank >= 512 else 0, _stream())
     lib.add_launches(bool(piece) + bool(dt_tokens))     # several behind one call
     if code == -1:
         raise KernelError(f"selective scan refuses inner={inner}, state={n_state}, rank={rank} "
@@ -1911,7 +1915,7 @@ def hyper_step(x: torch.Tensor, *, init=None, y=None, y2=None, y_scales=(1.0, 1.
         blocks = tokens if rows is None else rows.numel()
         w, b, td, alpha = _tanh_norm_args(tanh_norm, width)
         assert y_bias is None or td == wd
-        normed = torch.empty((blocks, width), dtype=out_dtype, device=x.device)
+        normed = x.new_empty((blocks, width), dtype=out_dtype)
         code = lib.get("hyper").mstar_hyper_step_tanh(
             x.data_ptr(), _ptr(init), _ptr(y), _ptr(y2), _ptr(y_bias), float(y_scales[0]),
             float(y_scales[1]), mix.data_ptr(), out.data_ptr(), _ptr(read), w, b, alpha,
@@ -1924,12 +1928,12 @@ def hyper_step(x: torch.Tensor, *, init=None, y=None, y2=None, y_scales=(1.0, 1.
     if read is not None:
         assert read.dtype == torch.float32 and read.numel() == streams
         assert norm_weight is not None and out_dtype is not None
-        normed = torch.empty((tokens, width), dtype=out_dtype, device=x.device)
+        normed = x.new_empty((tokens, width), dtype=out_dtype)
         blocks = tokens
     else:
         assert rows.dtype == torch.int32 and rows.is_contiguous()
         blocks = rows.numel()
-        sums = torch.empty((blocks, width), dtype=torch.float32, device=x.device)
+        sums = x.new_empty((blocks, width), dtype=torch.float32)
     code = lib.get("hyper").mstar_hyper_step(
         x.data_ptr(), _ptr(init), _ptr(y), _ptr(y2), _ptr(y_bias), float(y_scales[0]),
         float(y_scales[1]), mix.data_ptr(), out.data_ptr(), _ptr(read), _ptr(norm_weight),
@@ -2049,7 +2053,7 @@ def delta_scan(q, k, v, beta, decay, qo_indptr, slots, state: torch.Tensor, entr
     tokens = q.shape[0]
     head_decay = tuple(decay.shape) == (tokens, heads) and dim > 1
     assert head_decay or tuple(decay.shape) == (tokens, heads * dim)
-    out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=q.device)
+    out = q.new_empty((tokens, heads * vdim), dtype=torch.float32)
     channels = 2 * kv_heads * dim + heads * vdim
     offset = (taps - 1) * channels
     conv = (0, 0, 0, 0)
@@ -2071,13 +2075,12 @@ def delta_scan(q, k, v, beta, decay, qo_indptr, slots, state: torch.Tensor, entr
         else:
             row = (kinds * DELTA_PIECE + (0 if head_decay else 1)) * (dim + 4)
         per_piece = (kv_heads if head_decay else heads) * row + heads * DELTA_PIECE * (2 * DELTA_PIECE + 4)
-        work = torch.empty((tokens // DELTA_PIECE + entries) * per_piece, dtype=torch.float32,
-                           device=q.device)
+        work = q.new_empty((tokens // DELTA_PIECE + entries) * per_piece, dtype=torch.float32)
         code = lib.get("gated_delta").mstar_delta_scan_pieces(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), beta.data_ptr(), decay.data_ptr(),
             qo_indptr.data_ptr(), slots.data_ptr(), state.data_ptr(), state.stride(0), offset,
             out.data_ptr(), work.data_ptr(), tokens, entries, longest, heads, kv_heads, dim,
-            vdim, int(head_decay), tcgen05_error_word(q.device).data_ptr(), *conv, _stream())
+            vdim, int(head_decay), _error_ptr(q), *conv, _stream())
         if code == -1:
             raise KernelError(f"delta-rule scan in pieces refuses heads={heads}, "
                               f"kv_heads={kv_heads}, dim={dim}")
@@ -2108,7 +2111,7 @@ def delta_finish(o: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, head
     assert o.dtype == torch.float32 and o.is_contiguous()
     assert weight.dtype == torch.float32 and weight.numel() == vdim
     assert gate.dtype in (out_dtype, torch.float32) and gate.stride(1) == 1 and gate.shape == o.shape
-    out = torch.empty(o.shape, dtype=out_dtype, device=o.device)
+    out = o.new_empty(o.shape, dtype=out_dtype)
     check(lib.get("gated_delta").mstar_delta_finish(
         o.data_ptr(), gate.data_ptr(), gate.stride(0), weight.data_ptr(), out.data_ptr(),
         _DT[out_dtype], o.shape[0], heads, vdim, float(eps), float(scale), _dt(gate),
@@ -2235,7 +2238,7 @@ def time_mix(x: torch.Tensor, mu: torch.Tensor, ctx, state: torch.Tensor) -> tor
     tokens, width = x.shape
     assert x.stride(1) == 1 and mu.dtype == torch.float32 and mu.numel() == 5 * width
     assert state.dtype == torch.float32 and state.stride(1) == 1 and state.shape[1] >= width
-    out = torch.empty((5, tokens, width), dtype=x.dtype, device=x.device)
+    out = x.new_empty((5, tokens, width), dtype=x.dtype)
     check(lib.get("linear_recurrence").mstar_time_mix(
         x.data_ptr(), x.stride(0), mu.data_ptr(), out.data_ptr(), ctx.token_req.data_ptr(),
         ctx.qo_indptr.data_ptr(), ctx.slots.data_ptr(), state.data_ptr(), state.stride(0), _dt(x),
@@ -2247,7 +2250,7 @@ def tanh_rows(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     """tanh of float rows (a column view will do), in ``dtype``."""
     _need_cuda(x)
     assert x.dtype == torch.float32 and x.dim() == 2 and x.stride(1) == 1
-    out = torch.empty(tuple(x.shape), dtype=dtype, device=x.device)
+    out = x.new_empty(tuple(x.shape), dtype=dtype)
     check(lib.get("linear_recurrence").mstar_tanh_rows(
         x.data_ptr(), x.stride(0), out.data_ptr(), _DT[dtype], x.shape[0], x.shape[1], _stream()),
         "tanh_rows")
@@ -2274,8 +2277,8 @@ def mix_prepare(rows: torch.Tensor, low: torch.Tensor, w2: torch.Tensor, w0: tor
     z = None
     if tokens > MIX_FUSED_TOKENS or rank > 8192:
         z = linear(tanh_rows(low, dtype), w2, out_dtype=torch.float32, static_weights=True)
-    decay = torch.empty((tokens, hd), dtype=torch.float32, device=rows.device)
-    direct = torch.empty((tokens, heads), dtype=torch.float32, device=rows.device)
+    decay = rows.new_empty((tokens, hd), dtype=torch.float32)
+    direct = rows.new_empty((tokens, heads), dtype=torch.float32)
     check(lib.get("linear_recurrence").mstar_mix_prepare(
         rows.data_ptr(), rows.stride(0), _ptr(z), hd, low.data_ptr(), low.stride(0), rank,
         w2.data_ptr(), _dt(w2), w0.data_ptr(), u.data_ptr(), decay.data_ptr(), direct.data_ptr(),
@@ -2354,15 +2357,13 @@ def linear_scan(r, k, v, decay, direct, ctx, state: torch.Tensor, offset: int, h
     assert state.shape[1] >= offset + heads * dim * vdim
     if taps > 1:
         assert raw.dtype == torch.float32 and raw.stride(1) == 1 and raw.shape[1] >= channels
-    out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=v.device)
+    out = v.new_empty((tokens, heads * vdim), dtype=torch.float32)
     entries = ctx.num_entries
     piece, pieces = linear_scan_pieces(entries, heads, ctx.max_q_len, num_sms(v.device))
     piece_state = piece_decay = None
     if piece:
-        piece_state = torch.empty(entries * pieces * heads * vdim * dim, dtype=torch.float32,
-                                  device=v.device)
-        piece_decay = torch.empty(entries * pieces * heads * (dim if vector_decay else 1),
-                                  dtype=torch.float32, device=v.device)
+        piece_state = v.new_empty(entries * pieces * heads * vdim * dim, dtype=torch.float32)
+        piece_decay = v.new_empty(entries * pieces * heads * (dim if vector_decay else 1), dtype=torch.float32)
     code = lib.get("linear_recurrence").mstar_linear_scan(
         r.data_ptr(), k.data_ptr(), v.data_ptr(), r.stride(0), k.stride(0), v.stride(0), rk_share,
         decay.data_ptr(), int(vector_decay), direct.data_ptr(), _ptr(dt), ctx.qo_indptr.data_ptr(),
