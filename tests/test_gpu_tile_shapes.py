@@ -141,6 +141,32 @@ def test_float_attention_of_portions_leaves_unseen_values_out():
     assert torch.isfinite(out[:-1]).all() and not torch.isfinite(out[-1]).any()
 
 
+# a key a token, a tile and one more, a block a tile; heads that fill a block and that don't; no rotated features
+@pytest.mark.parametrize("kv,heads,rank,rot", [([1, 33, 32], 5, 64, 16), ([400, 7], 16, 512, 64), ([90], 17, 96, 32),
+                                               ([65], 3, 256, 0)])
+def test_latent_attention_of_single_tokens(kv, heads, rank, rot):
+    """Against double precision; queries whose rows lie off 16 bytes give the same bits."""
+    from mstar_b200 import ops
+
+    T, page, D = len(kv), 16, rank + rot
+    width = -(-max(kv) // page)
+    cache = rnd(T * width, 1, 1, page, D, dtype=torch.bfloat16, seed=1)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    table = torch.randperm(T * width, device=DEV).to(torch.int32).view(T, width)
+    q_abs, wide = 0.3 * rnd(T, heads, rank, seed=2), 0.3 * rnd(T, heads, rot + 9, dtype=torch.bfloat16, seed=3)
+    run = lambda q_rot: ops.latent_attention(q_abs, q_rot, cache, table, i32(list(range(T))), i32([n - 1 for n in kv]),
+                                             heads, rank, rot, page, 0, 0.1, max_keys=max(kv))
+    off = wide[:, :, 1:1 + rot]                      # rows of an odd number of elements
+    got = run(off.contiguous())
+    assert torch.equal(run(off), got)
+    for t, n in enumerate(kv):
+        rows = cache[table[t].long()].view(-1, D)[:n].double()
+        q = torch.cat([q_abs[t].double(), off[t].double()], 1)
+        want = torch.softmax(q @ rows.T * 0.1, -1) @ rows[:, :rank]
+        # queries in two bfloat16 parts (2^-16), scores of about 2, weights that add up to one, values of up to 5
+        assert (got[t].double() - want).abs().max() < 2 ** -16 * 2 * 5
+
+
 @pytest.mark.parametrize("tokens,width,ff,experts,identity,top,form,on_input", [
     (200, 72, 8, 2, 0, 2, "silu", False),         # k-blocks that end early, one narrow column tile
     (300, 128, 264, 5, 1, 3, "silu", True),       # column tiles that end inside, identity experts
