@@ -161,10 +161,8 @@ paged_attention_generic_kernel(const A* __restrict__ q, A* __restrict__ out,
 // the few keys that some rows see and others don't are taken one by one (the last tile of every row is such a one).
 // Tiles start at multiples of 64 keys whatever the block's rows are, and a tile that a row does
 // not see leaves its sums as they are, so a row's result does not depend on what else is in the
-// batch.  Bound by the shared loads that feed the FMA pipe (of 16 bytes, no bank met
-// twice).  448 prompt tokens with 32 / 8 heads of 64 (requests of 256 and 192): 33 us, 41 with one group and
-// whole tiles; one of 250 tokens on 250 cached keys, 24 / 8 heads of 128: 89 and 121 us; 2,000 tokens: 876 and 1,258.
-// 32 rows a block, two blocks an SM: 31 us for the first, 291 instead of 283 for 1,500 tokens with heads of 64.
+// batch.  Bound by the shared loads that feed the FMA pipe (of 16 bytes, no bank met twice).  It makes the blocks
+// whose operands are not finite; the others go to the tensor cores (below, both sides measured).
 #define AR_ROWS 64
 #define AR_KEYS 64
 #define AR_THREADS 256                         // of a group
@@ -207,11 +205,10 @@ __device__ __forceinline__ void ar_output(unsigned long long (&acc)[4][HD / 32],
 }
 
 template <int HD>
-__global__ void __launch_bounds__(AR_GROUPS * AR_THREADS)
-attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
-                          const float* __restrict__ kv_cache, const int* __restrict__ block_table,
-                          const int* __restrict__ token_req, const int* __restrict__ cache_pos,
-                          AttnArgs a, int num_tokens) {
+__device__ __noinline__ void ar_block_fma(const float* __restrict__ q, float* __restrict__ out,
+                                          const float* __restrict__ kv_cache, const int* __restrict__ block_table,
+                                          const int* __restrict__ token_req, const int* __restrict__ cache_pos,
+                                          const AttnArgs& a, int num_tokens) {
     constexpr int QL = HD + 4, PL = AR_KEYS + 4;   // floats between rows: 16-byte reads of 8 rows
     extern __shared__ __align__(16) float ar_smem[];
     float* q_s = ar_smem;                          // [ROWS][QL]
@@ -402,6 +399,280 @@ attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
     }
 }
 
+// ------------------------------------------------------------------ the same on the tensor cores
+// A float is the sum of three bfloat16 numbers, its 24 bits eight at a time; of the nine products of such parts the
+// six of 2^-16 or more of the whole are made by mma.sync m16n8k16, the leading one into a sum of its own, since
+// the tensor core cuts its sums off instead of rounding them; a tile's P V is summed by itself and then added.
+// A block takes the same 64 rows.  Its two groups of eight warps take the even and the odd tiles, in a group a
+// warp takes 16 rows and one half of a tile's keys, and keeps maxima, sums and output of its own; the four
+// shares of a row are added up at the end in their order.  A tile's keys and values are fetched into registers under
+// the products of the tile before it, cut into their parts and put into shared memory by the whole group;
+// probabilities go from the scores' registers into the products' without passing through memory.
+// Operands that are not finite leave no sum behind in their parts (infinity less infinity): a block that met one
+// makes its rows again with plain FMAs.
+// Bound by latencies where prompts are short (of a block's 10 us with one tile the queries take 1.2, the first
+// keys 2, the tile 3, the shares 2) and by the warp-level tensor path and the splitting where they are long.  448
+// prompt tokens with 32 / 8 heads of 64 (requests of 256 and 192): 26.5 us, with FMAs 33, and 41 in one group with
+// whole tiles; 1,500 tokens: 211, 283, 283; one of 250 tokens on 250 cached keys, 24 / 8 heads of 128: 72, 89, 121;
+// 2,000 tokens: 695, 876, 1,258.  Error against 64 bits as with FMAs (the layer: 5.0e-7, 4.9e-7).
+template <int HD> __host__ __device__ constexpr int ap_keys() { return HD == 64 ? 64 : 32; }     // of a tile
+template <int HD> __host__ __device__ constexpr int ap_smem() {
+    return 3 * 2 * (HD + 8) * (AR_ROWS + AR_GROUPS * 2 * ap_keys<HD>());
+}
+
+// Two floats as three pairs of bfloat16 numbers; false if one of them is not finite (or too large for its part).
+__device__ __forceinline__ bool ap_split(float x, float y, uint32_t (&p)[3]) {
+    p[0] = pack_bf16(x, y);
+    const float rx = x - __uint_as_float(p[0] << 16), ry = y - __uint_as_float(p[0] & 0xffff0000u);
+    p[1] = pack_bf16(rx, ry);
+    const float sx = rx - __uint_as_float(p[1] << 16), sy = ry - __uint_as_float(p[1] & 0xffff0000u);
+    p[2] = pack_bf16(sx, sy);
+    return isfinite(sx + sy);
+}
+
+template <int HD>
+__global__ void __launch_bounds__(AR_GROUPS * AR_THREADS)
+attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
+                          const float* __restrict__ kv_cache, const int* __restrict__ block_table,
+                          const int* __restrict__ token_req, const int* __restrict__ cache_pos,
+                          AttnArgs a, int num_tokens) {
+    constexpr int KEYS = ap_keys<HD>(), HALF = KEYS / 2, LD = HD + 8;
+    constexpr int NT = HALF / 8, KT = HALF / 16, VT = HD / 8;          // a warp's tiles of scores, of keys, of columns
+    constexpr int QPLANE = AR_ROWS * LD, KPLANE = KEYS * LD;             // bfloat16 numbers of a part
+    constexpr int U = KEYS * (HD / 4) / AR_THREADS;                      // fours of floats a thread fetches
+    extern __shared__ __align__(16) float ar_smem[];
+    bf16* q_p = reinterpret_cast<bf16*>(ar_smem);                        // [3][ROWS][LD]
+    const int group = threadIdx.x / AR_THREADS, tid = threadIdx.x % AR_THREADS;
+    bf16* k_p = q_p + 3 * QPLANE + group * 6 * KPLANE;                   // [3][KEYS][LD]
+    bf16* v_p = k_p + 3 * KPLANE;
+    const int lane = tid & 31, warp = tid >> 5, rt = warp & 3, half = warp >> 2;
+    const int g = lane >> 2, c4 = lane & 3;
+    auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(AR_THREADS) : "memory"); };
+    const int kvh = blockIdx.x;
+    const int G = a.nq / a.nkv, TPB = AR_ROWS / G;
+    // (the tokens with the most keys first)
+    const int t0 = (int)(gridDim.y - 1 - blockIdx.y) * TPB;
+    const int ntok = min(TPB, num_tokens - t0), nrows = ntok * G;
+    const size_t page_elems = (size_t)2 * a.nkv * a.page_size * HD;
+    const size_t v_off = (size_t)a.nkv * a.page_size * HD;
+    const float* head_base = kv_cache + (size_t)kvh * a.page_size * HD;
+    bool finite = true;
+    auto put = [&](bf16* to, int plane, const float4 v) {
+        uint32_t x[3], y[3];
+        finite = ap_split(v.x, v.y, x) && finite;
+        finite = ap_split(v.z, v.w, y) && finite;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(to + i * plane) = make_uint2(x[i], y[i]);
+    };
+    for (int c = threadIdx.x; c < AR_ROWS * (HD / 4); c += AR_GROUPS * AR_THREADS) {
+        const int r = c / (HD / 4), d = (c % (HD / 4)) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < nrows)
+            v = *reinterpret_cast<const float4*>(q + (size_t)(t0 + r / G) * a.q_stride + (size_t)(kvh * G + r % G) * HD + d);
+        put(q_p + r * LD + d, QPLANE, v);
+    }
+    __syncthreads();
+
+    for (int s0 = 0; s0 < ntok;) {
+        // tokens s0 .. s1-1 of the block belong to one request; every warp looks at them all, a token a lane (one
+        // after the other 16 of them took 3 us)
+        const int req = token_req[t0 + s0];
+        int s1 = s0, lo_min = 0x7fffffff, hi_max = 0;
+        for (bool more = true; more && s1 < ntok;) {
+            const int tk = s1 + lane;
+            const bool same = tk < ntok && token_req[t0 + min(tk, ntok - 1)] == req;
+            const int run = __ffs(~__ballot_sync(0xffffffffu, same)) - 1;          // (-1: all 32)
+            const bool in = run < 0 || lane < run;
+            const int hi = in ? cache_pos[t0 + tk] + 1 : 0;
+            const int lo = !in ? 0x7fffffff : (a.window > 0 && hi > a.window) ? hi - a.window : 0;
+            lo_min = min(lo_min, (int)__reduce_min_sync(0xffffffffu, (unsigned)lo));
+            hi_max = max(hi_max, (int)__reduce_max_sync(0xffffffffu, (unsigned)hi));
+            more = run < 0;
+            s1 += run < 0 ? 32 : run;
+        }
+        const int* bt = block_table + (size_t)req * a.bt_stride;
+        int lo_r[2], hi_r[2];                      // the keys that this thread's rows see
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int r = rt * 16 + g + 8 * i, tk = r / G;
+            lo_r[i] = hi_r[i] = 0;                 // a row of another request: idle
+            if (r < nrows && tk >= s0 && tk < s1) {
+                hi_r[i] = cache_pos[t0 + tk] + 1;
+                lo_r[i] = (a.window > 0 && hi_r[i] > a.window) ? hi_r[i] - a.window : 0;
+            }
+        }
+        const int warp_hi = (int)__reduce_max_sync(0xffffffffu, (unsigned)max(hi_r[0], hi_r[1]));
+        float4 k_next[U], v_next[U];
+        auto fetch = [&](int key0) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int c = tid + u * AR_THREADS, key = key0 + c / (HD / 4), d = (c % (HD / 4)) * 4;
+                k_next[u] = v_next[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (key >= lo_min && key < hi_max) {
+                    const float* src = head_base + (size_t)bt[key / a.page_size] * page_elems +
+                                       (size_t)(key % a.page_size) * HD + d;
+                    k_next[u] = *reinterpret_cast<const float4*>(src);
+                    v_next[u] = *reinterpret_cast<const float4*>(src + v_off);
+                }
+            }
+        };
+        float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, o[VT][4];
+#pragma unroll
+        for (int v = 0; v < VT; ++v) o[v][0] = o[v][1] = o[v][2] = o[v][3] = 0.f;
+        const int tile0 = lo_min / KEYS;
+        const int first = (tile0 + ((tile0 ^ group) & 1)) * KEYS;       // even tiles: group 0
+        if (first < hi_max) fetch(first);
+        for (int key0 = first; key0 < hi_max; key0 += AR_GROUPS * KEYS) {
+            group_sync();                          // the tile before is done with
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int c = tid + u * AR_THREADS, at = c / (HD / 4) * LD + (c % (HD / 4)) * 4;
+                put(k_p + at, KPLANE, k_next[u]);
+                put(v_p + at, KPLANE, v_next[u]);
+            }
+            group_sync();
+            if (key0 + AR_GROUPS * KEYS < hi_max) fetch(key0 + AR_GROUPS * KEYS);
+            const int mine = key0 + half * HALF;                         // this warp's first key
+            if (mine >= warp_hi || mine + HALF <= lo_min) continue;
+            float s[NT][4], rest[NT][4];
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) s[n][i] = rest[n][i] = 0.f;
+            const uint32_t q_at = smem_u32(q_p + (rt * 16 + (lane & 15)) * LD + (lane >> 4) * 8);
+            const uint32_t k_at = smem_u32(k_p + (half * HALF + (lane & 7) + (lane >> 4) * 8) * LD + ((lane >> 3) & 1) * 8);
+#pragma unroll
+            for (int k = 0; k < HD / 16; ++k) {
+                uint32_t A[3][4];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) ldmatrix_x4(A[i], q_at + (i * QPLANE + k * 16) * 2);
+#pragma unroll
+                for (int n = 0; n < NT; n += 2)
+#pragma unroll
+                    for (int i = 2; i >= 0; --i) {
+                        uint32_t B[4];
+                        ldmatrix_x4(B, k_at + (i * KPLANE + n * 8 * LD + k * 16) * 2);
+#pragma unroll
+                        for (int j = 2 - i; j >= 0; --j) {
+                            float (&x)[4] = i + j == 0 ? s[n] : rest[n];
+                            float (&y)[4] = i + j == 0 ? s[n + 1] : rest[n + 1];
+                            mma_bf16_16816(x, A[j], B[0], B[1]);
+                            mma_bf16_16816(y, A[j], B[2], B[3]);
+                        }
+                    }
+            }
+            float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int key = mine + n * 8 + 2 * c4 + (i & 1), r = i >> 1;
+                    s[n][i] = key >= lo_r[r] && key < hi_r[r] ? (s[n][i] + rest[n][i]) * a.scale : -INFINITY;
+                    mx[r] = fmaxf(mx[r], s[n][i]);
+                }
+            float alpha[2];
+            bool none[2];
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
+                mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
+                const float m_new = fmaxf(m[r], mx[r]);
+                none[r] = m_new == -INFINITY;                  // the row has seen no key yet
+                alpha[r] = none[r] ? 1.f : expf(m[r] - m_new);
+                m[r] = m_new;
+                l[r] *= alpha[r];
+            }
+            uint32_t P[3][KT][4];
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const float x = none[r] ? 0.f : expf(s[n][2 * r] - m[r]), y = none[r] ? 0.f : expf(s[n][2 * r + 1] - m[r]);
+                    l[r] += x + y;
+                    uint32_t p[3];
+                    ap_split(x, y, p);
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) P[i][n / 2][(n & 1) * 2 + r] = p[i];
+                }
+            const uint32_t v_at = smem_u32(v_p + (half * HALF + (lane & 7) + ((lane >> 3) & 1) * 8) * LD + (lane >> 4) * 8);
+#pragma unroll
+            for (int v = 0; v < VT; v += 2) {
+                float x[2][4], y[2][4];
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) x[n][i] = y[n][i] = 0.f;
+#pragma unroll
+                for (int k = 0; k < KT; ++k)
+#pragma unroll
+                    for (int i = 2; i >= 0; --i) {
+                        uint32_t B[4];
+                        ldmatrix_x4_trans(B, v_at + (i * KPLANE + k * 16 * LD + v * 8) * 2);
+#pragma unroll
+                        for (int j = 2 - i; j >= 0; --j) {
+                            mma_bf16_16816(i + j == 0 ? x[0] : y[0], P[j][k], B[0], B[1]);
+                            mma_bf16_16816(i + j == 0 ? x[1] : y[1], P[j][k], B[2], B[3]);
+                        }
+                    }
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) o[v + n][i] = fmaf(o[v + n][i], alpha[i >> 1], x[n][i] + y[n][i]);
+            }
+        }
+        // the shares of all warps but the first four pass through the tiles' place
+        constexpr int OLD = HD + 8;                // floats between rows of a share: eight rows meet no bank twice
+        float* shares = reinterpret_cast<float*>(q_p + 3 * QPLANE);      // [3][ROWS][OLD]
+        float2* share_ml = reinterpret_cast<float2*>(shares + 3 * AR_ROWS * OLD);    // [3][ROWS]
+        const int share = group * 2 + half - 1;
+        __syncthreads();                           // all tiles are done with
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1);
+            l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
+            if (share < 0) continue;
+            const int row = share * AR_ROWS + rt * 16 + g + 8 * r;
+            if (c4 == 0) share_ml[row] = make_float2(m[r], l[r]);
+#pragma unroll
+            for (int v = 0; v < VT; ++v)
+                *reinterpret_cast<float2*>(shares + row * OLD + v * 8 + 2 * c4) = make_float2(o[v][2 * r], o[v][2 * r + 1]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            if (share >= 0 || hi_r[r] == 0) continue;
+            const int row = rt * 16 + g + 8 * r;
+            float2 ml[3];
+            float top = m[r];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                ml[i] = share_ml[i * AR_ROWS + row];
+                top = fmaxf(top, ml[i].x);
+            }
+            const float w[4] = {expf(m[r] - top), expf(ml[0].x - top), expf(ml[1].x - top), expf(ml[2].x - top)};  // (no key: 0)
+            float sum = l[r] * w[0];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) sum = fmaf(ml[i].y, w[i + 1], sum);
+            float* dst = out + (size_t)(t0 + row / G) * a.nq * HD + (size_t)(kvh * G + row % G) * HD + 2 * c4;
+#pragma unroll
+            for (int v = 0; v < VT; ++v) {
+                float x = o[v][2 * r] * w[0], y = o[v][2 * r + 1] * w[0];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const float2 f = *reinterpret_cast<const float2*>(shares + (i * AR_ROWS + row) * OLD + v * 8 + 2 * c4);
+                    x = fmaf(f.x, w[i + 1], x);
+                    y = fmaf(f.y, w[i + 1], y);
+                }
+                *reinterpret_cast<float2*>(dst + v * 8) = make_float2(x / sum, y / sum);
+            }
+        }
+        __syncthreads();                           // the shares have been read
+        s0 = s1;
+    }
+    if (__syncthreads_or(!finite))
+        ar_block_fma<HD>(q, out, kv_cache, block_table, token_req, cache_pos, a, num_tokens);
+}
+
 // ------------------------------------------------------------------ float single tokens
 // One token's attention, a block for four query heads of a kv head (blockIdx.z: which four of its
 // group): scores of up to 512 keys into shared memory, their softmax statistics, then the values.  HD / 16
@@ -562,9 +833,10 @@ template <int HD>
 static int launch_rows_f32(const float* q, float* out, const float* kv, const int* block_table,
                            const int* token_req, const int* cache_pos, const AttnArgs& a, int num_tokens,
                            cudaStream_t s) {
-    constexpr int smem = (int)sizeof(float) *
-                         (AR_ROWS * (HD + 4) +
-                          AR_GROUPS * (AR_KEYS * (HD + 4) + AR_KEYS * HD + AR_ROWS * (AR_KEYS + 4)));
+    constexpr int fma = (int)sizeof(float) * (AR_ROWS * (HD + 4) +
+                                              AR_GROUPS * (AR_KEYS * (HD + 4) + AR_KEYS * HD + AR_ROWS * (AR_KEYS + 4)));
+    constexpr int smem = fma > ap_smem<HD>() ? fma : ap_smem<HD>();
+    static_assert(smem - 6 * AR_ROWS * (HD + 8) >= 3 * AR_ROWS * ((HD + 8) * 4 + 8), "room for the shares");
     static bool configured = false;
     if (!configured) {
         const cudaError_t e = cudaFuncSetAttribute(attention_rows_f32_kernel<HD>,

@@ -167,6 +167,33 @@ def test_latent_attention_of_single_tokens(kv, heads, rank, rot):
         assert (got[t].double() - want).abs().max() < 2 ** -16 * 2 * 5
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("where,value", [("q", float("inf")), ("key", float("nan")), ("key", -float("inf")),
+                                         ("value", float("inf")), ("value", 3.4e38), ("none", 0.0)])
+def test_float_attention_of_portions_keeps_what_is_not_finite(hd, where, value):
+    """As the kernel of a block per token has it; the largest floats, whose first part is not finite, too."""
+    from mstar_b200 import ops
+
+    T, heads = 150, 2
+    q, kv = rnd(T, heads * hd, seed=1), rnd(10, 2, 1, 16, hd, seed=2)
+    if where == "q":
+        q[70, 3] = value
+    elif where != "none":
+        kv[4, int(where == "value"), 0, 5, 3] = value            # key 69
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    outs = []
+    for entries in (1, T):                                  # (as many entries as tokens: a block per token)
+        out = torch.empty(T, heads * hd, device=DEV)
+        ops.paged_attention_generic(q, heads * hd, out, kv, i32([list(range(10))]), i32([0] * T), i32(list(range(T))), T,
+                                    heads, 1, hd, 16, 0, hd ** -0.5, entries=entries)
+        outs.append(out)
+    got, want = outs
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    both = want.isfinite()
+    assert both.any(dim=1)[:69].all()
+    torch.testing.assert_close(got[both], want[both], rtol=2e-5, atol=2e-6)
+
+
 @pytest.mark.parametrize("tokens,width,ff,experts,identity,top,form,on_input", [
     (200, 72, 8, 2, 0, 2, "silu", False),         # k-blocks that end early, one narrow column tile
     (300, 128, 264, 5, 1, 3, "silu", True),       # column tiles that end inside, identity experts
