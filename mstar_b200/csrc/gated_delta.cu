@@ -671,8 +671,7 @@ struct DeltaHeadArgs {
     const int* qo_indptr;
     const int* slots;
     // [pieces][G][2 C][D + 4]: the k rows, then the q rows; zeros past the end.  CHANNEL: [pieces][H][
-    // 3 C + 1][D + 4]: P_t k_t, P_t q_t, dec(C, t) k_t and P_C.  Key sizes of GP_TAKES: the same rows in
-    // bfloat16 parts, [3][2 C or 3 C][D + 8], then (CHANNEL) P_C as floats
+    // 3 C + 1][D + 4]: P_t k_t, P_t q_t, dec(C, t) k_t and P_C
     float* rows;
     float* mats;                // [pieces][H][C][GH_MROW]
     float* state;
@@ -683,31 +682,6 @@ struct DeltaHeadArgs {
     int* error_word;
     ConvAdvance conv;
 };
-
-// Key sizes whose scan runs on the tensor cores; the other ones take the float kernel.
-#define GP_TAKES(D) ((D) == 64 || (D) == 128 || (D) == 256)
-#define GP_LD(D) ((D) + 8)                  // bfloat16 numbers between rows: 16 bytes past a multiple of 128
-__host__ __device__ constexpr size_t gp_row_bytes(int D, bool channel) {
-    return (size_t)3 * (channel ? 3 : 2) * GC_TOKENS * GP_LD(D) * 2 + (channel ? (size_t)D * 4 : 0);
-}
-// floats of a piece's rows (of a head, or of a group of heads)
-__host__ __device__ constexpr size_t gh_row_floats(int D, bool channel) {
-    return GP_TAKES(D) ? gp_row_bytes(D, channel) / 4 : (size_t)(channel ? 3 * GC_TOKENS + 1 : 2 * GC_TOKENS) * (D + 4);
-}
-// Two floats as three pairs of bfloat16 numbers, their 24 bits eight at a time.
-__device__ __forceinline__ void gp_split(float x, float y, uint32_t (&p)[3]) {
-    p[0] = pack_bf16(x, y);
-    const float rx = x - __uint_as_float(p[0] << 16), ry = y - __uint_as_float(p[0] & 0xffff0000u);
-    p[1] = pack_bf16(rx, ry);
-    p[2] = pack_bf16(rx - __uint_as_float(p[1] << 16), ry - __uint_as_float(p[1] & 0xffff0000u));
-}
-// Numbers d, d + 1 of a row in parts; plane: bfloat16 numbers of a part's rows.
-__device__ __forceinline__ void gp_store(bf16* row, size_t plane, int d, float x, float y) {
-    uint32_t p[3];
-    gp_split(x, y, p);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(row + i * plane + d) = p[i];
-}
 
 // Pieces are numbered over the batch so that an entry's are consecutive: at most tokens / C + entries.
 __device__ __forceinline__ size_t gh_first_piece(int start, int e) { return (size_t)(start / GC_TOKENS + e); }
@@ -779,18 +753,9 @@ __global__ void __launch_bounds__(256) delta_head_pieces_kernel(DeltaHeadArgs a)
         }
         *reinterpret_cast<float4*>(ks + t * LD + d) = kv;
         *reinterpret_cast<float4*>(qs + t * LD + d) = qv;
-        float* dst = a.rows + ((gh_first_piece(start, e) + piece) * a.G + grp) * gh_row_floats(D, false);
-        if (GP_TAKES(D)) {
-            bf16* rk = reinterpret_cast<bf16*>(dst) + t * GP_LD(D);
-            const size_t plane = (size_t)2 * C * GP_LD(D);
-            gp_store(rk, plane, d, kv.x, kv.y);
-            gp_store(rk, plane, d + 2, kv.z, kv.w);
-            gp_store(rk + C * GP_LD(D), plane, d, qv.x, qv.y);
-            gp_store(rk + C * GP_LD(D), plane, d + 2, qv.z, qv.w);
-        } else {
-            *reinterpret_cast<float4*>(dst + t * LD + d) = kv;
-            *reinterpret_cast<float4*>(dst + (C + t) * LD + d) = qv;
-        }
+        float* dst = a.rows + (((gh_first_piece(start, e) + piece) * a.G + grp) * 2 * C + t) * LD + d;
+        *reinterpret_cast<float4*>(dst) = kv;
+        *reinterpret_cast<float4*>(dst + C * LD) = qv;
     }
     __syncthreads();
     {
@@ -894,47 +859,31 @@ __global__ void __launch_bounds__(256, 3) delta_channel_pieces_kernel(DeltaHeadA
     }
     __syncthreads();
     const size_t at = (gh_first_piece(start, e) + piece) * a.H + h;
-    // half of the threads the rows for the scan (a thread two channels, from the start or from the end), half
-    // those for the sums here (a thread a channel)
+    // a thread a channel: half of the threads the rows for the scan, half those for the sums here
     for (int i = tid; i < 2 * D; i += 256) {
+        const int d = i % D;
+        float kd[C], gd[C];
+#pragma unroll
+        for (int t = 0; t < C; ++t) {
+            kd[t] = ks[t * LD + d];
+            gd[t] = gs[t * LD + d];
+        }
         if (i < D) {
-            const int d = i % (D / 2) * 2;
-            float* dst = a.rows + at * gh_row_floats(D, true);
-            bf16* parts = reinterpret_cast<bf16*>(dst) + d;
-            constexpr int ROWS = 3 * C;
-            const size_t plane = (size_t)ROWS * GP_LD(D);
-            const bool takes = GP_TAKES(D);
-            auto put = [&](int row, float2 v) {
-                if (takes) gp_store(parts + row * GP_LD(D), plane, 0, v.x, v.y);
-                else *reinterpret_cast<float2*>(dst + row * LD + d) = v;
-            };
-            float2 P = make_float2(1.f, 1.f);
-            if (i < D / 2) {
-                for (int t = 0; t < C; ++t) {
-                    const float2 k2 = *reinterpret_cast<const float2*>(ks + t * LD + d);
-                    const float2 q2 = *reinterpret_cast<const float2*>(qs + t * LD + d);
-                    const float2 g2 = *reinterpret_cast<const float2*>(gs + t * LD + d);
-                    P.x *= g2.x, P.y *= g2.y;
-                    put(t, make_float2(k2.x * P.x, k2.y * P.y));
-                    put(C + t, make_float2(q2.x * P.x, q2.y * P.y));
-                }
-                *reinterpret_cast<float2*>(takes ? dst + (gp_row_bytes(D, true) / 4 - D) + d : dst + 3 * C * LD + d) = P;
-            } else {
-                for (int t = C - 1; t >= 0; --t) {
-                    const float2 k2 = *reinterpret_cast<const float2*>(ks + t * LD + d);
-                    const float2 g2 = *reinterpret_cast<const float2*>(gs + t * LD + d);
-                    put(2 * C + t, make_float2(k2.x * P.x, k2.y * P.y));
-                    P.x *= g2.x, P.y *= g2.y;
-                }
-            }
-        } else {
-            const int d = i - D;
-            float kd[C], gd[C];
+            float* dst = a.rows + at * GK_ROWS(C) * LD + d;
+            float P = 1.f, S = 1.f;
 #pragma unroll
             for (int t = 0; t < C; ++t) {
-                kd[t] = ks[t * LD + d];
-                gd[t] = gs[t * LD + d];
+                P *= gd[t];
+                dst[t * LD] = kd[t] * P;
+                dst[(C + t) * LD] = qs[t * LD + d] * P;
             }
+            dst[3 * C * LD] = P;
+#pragma unroll
+            for (int t = C - 1; t >= 0; --t) {
+                dst[(2 * C + t) * LD] = kd[t] * S;
+                S *= gd[t];
+            }
+        } else {
             float y[C - 4];                      // Y of the four that comes next
 #pragma unroll
             for (int f = 0; f < C / 4; ++f) {
@@ -1025,7 +974,9 @@ __device__ __forceinline__ void gh_bulk(float* dst, const float* src, uint32_t b
 
 //
 // CHANNEL: the rows hold the decays (P and dec are 1 in the matrices), the new state takes rows of its own,
-// and P_C is a row.  For key sizes of 32 and 96 (the others: the kernel below), bound by shared loads.
+// and P_C is a row.  2,048 tokens, 16 heads of 128 x 128: 173 us (a scan that gave a warp a column and a lane a
+// token's dot products, every warp reading all of the piece's rows, took 430 us: shared loads, which bound
+// this one too: with eight warps and half the columns of S a thread, 195 us).
 template <int D, int COLS, bool CHANNEL>
 __global__ void __launch_bounds__(GH_THREADS, 2) delta_head_scan_kernel(DeltaHeadArgs a) {
     extern __shared__ __align__(16) float sm[];
@@ -1262,298 +1213,6 @@ __global__ void __launch_bounds__(GH_THREADS, 2) delta_head_scan_kernel(DeltaHea
     gd_advance_conv(a.conv, waited, state + (size_t)a.slots[e] * a.state_stride, start, n, h, a.H);
 }
 
-// The same scan for key sizes of 64, 128 and 256 on the tensor cores (mma.sync m16n8k16), every float in three
-// bfloat16 parts, of whose products the six of 2^-16 or more of the whole are made, small ones first.  A block
-// owns 16 value columns of one head of one entry, a warp a quarter of the key channels: it keeps S^T of those in the
-// layout of a product's result, [columns x channels], which is also that of the right operand of the next
-// piece's [k; q] S0, so that the state stays in registers from piece to piece; only the warps' shares of [r; p] and u
-// pass through shared memory.  c, u = T c and o are made as above.  A piece's change of S is summed by itself
-// and then added to P_C S, rounded once: the tensor core cuts its sums off instead of rounding them.
-// Bound by the latency of a piece's steps: of some 2,300 cycles the 72 products take 860 (one in ten cycles a
-// scheduler), the state's parts 230, the shares' exchange 390, u and o 440.  2,048 tokens, 16 heads of 128 x 128,
-// a decay a key channel: 157 us (float products out of shared memory, the kernel above: 178); three portions of
-// up to 600 with one decay a head: 82 (117).  Eight warps of 16 channels: 165 and 118.
-#define GP_BUFS 5                           // pieces on their way, at most
-template <int D, bool CHANNEL>
-__global__ void __launch_bounds__(GH_THREADS) delta_parts_scan_kernel(DeltaHeadArgs a, int bufs) {
-    extern __shared__ __align__(16) float sm[];
-    constexpr int C = GC_TOKENS, COLS = 16, LD = GP_LD(D), WARPS = GH_THREADS / 32;
-    constexpr int TN = C * COLS / GH_THREADS; // columns a thread makes of c, u and o
-    constexpr int ROWS = (CHANNEL ? 3 : 2) * C, PLANE = ROWS * LD;                 // bfloat16 numbers
-    constexpr int row_floats = (int)(gp_row_bytes(D, CHANNEL) / 4), per_buf = row_floats + C * GH_MROW;
-    constexpr int DW = D / WARPS, KS = DW / 16, NT = DW / 8;      // a warp's channels, in sixteens and eights
-    constexpr int PLD = COLS + 8, ULD = C + 8;
-    float* part = sm + bufs * per_buf;              // [WARPS][2 C][PLD] shares of r and p
-    float* cs = part + WARPS * 2 * C * PLD;      // [C][COLS]
-    bf16* us = reinterpret_cast<bf16*>(cs + C * COLS);            // [3][COLS][ULD] dec(C, t) u_t in parts, a column a row
-    __shared__ __align__(8) unsigned long long full[GP_BUFS];
-    const int e = blockIdx.x, h = blockIdx.y;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int col0 = blockIdx.z * COLS;
-    const unsigned long long waited = pdl_wait();
-    const float* v = pdl_after(a.v, waited);
-    const float* rows = pdl_after((const float*)a.rows, waited);
-    const float* mats = pdl_after((const float*)a.mats, waited);
-    float* state = pdl_after(a.state, waited);
-    const int start = a.qo_indptr[e], n = a.qo_indptr[e + 1] - start;
-    if (n <= 0) return;
-    const int vv = a.H * a.VD, grp = h / (a.H / a.G);
-    const size_t first = gh_first_piece(start, e);
-
-    auto fetch = [&](int buf, int piece) {       // one thread; both copies complete on the buffer's barrier
-        const uint32_t bar = tc_smem(full + buf);
-        float* dst = sm + buf * per_buf;
-        mbar_expect_tx(bar, (uint32_t)(per_buf * sizeof(float)));
-        gh_bulk(dst, rows + (CHANNEL ? (first + piece) * a.H + h : (first + piece) * a.G + grp) * row_floats,
-                row_floats * sizeof(float), bar);
-        gh_bulk(dst + row_floats, mats + ((first + piece) * a.H + h) * C * GH_MROW, C * GH_MROW * sizeof(float), bar);
-    };
-
-    const int pieces = (n + C - 1) / C;
-    if (tid == 0) {
-        for (int i = 0; i < bufs; ++i) mbar_init(tc_smem(full + i), 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        for (int i = 0; i < min(bufs, pieces); ++i) fetch(i, i);
-    }
-    __syncthreads();
-    // S^T: s[j][0, 1] column g, channels 8 j + 2 q, + 1 of the warp's; [2, 3] column g + 8
-    const int g = lane >> 2, q = lane & 3, d0 = warp * DW;
-    float* s_head = state + (size_t)a.slots[e] * a.state_stride + a.state_offset + ((size_t)h * a.VD + col0) * D + d0;
-    float s[NT][4];
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            float2 f = make_float2(0.f, 0.f);
-            if (col0 + g + 8 * half < a.VD)
-                f = *reinterpret_cast<const float2*>(s_head + (size_t)(g + 8 * half) * D + 8 * j + 2 * q);
-            s[j][2 * half] = f.x;
-            s[j][2 * half + 1] = f.y;
-        }
-    // thread (token t, columns tc .. tc + TN - 1) between the products
-    const int t = tid / (COLS / TN), tc = tid % (COLS / TN) * TN;
-    float v_next[TN];
-#pragma unroll
-    for (int x = 0; x < TN; ++x) v_next[x] = 0.f;
-    auto ahead = [&](int piece) {                // the values the thread itself needs of a piece
-        const int at = piece * C + t;
-        if (at < n) {
-            const float* src = v + (size_t)(start + at) * vv + (size_t)h * a.VD + col0 + tc;
-#pragma unroll
-            for (int x = 0; x < TN; ++x)
-                if (col0 + tc + x < a.VD) v_next[x] = src[x];
-        }
-    };
-    ahead(0);
-    int buf = 0;
-    uint32_t parity = 0;
-    for (int piece = 0; piece < pieces; ++piece) {
-        if (!__all_sync(0xffffffffu, mbar_wait(tc_smem(full + buf), parity))) {
-            if (lane == 0) atomicExch(a.error_word, GH_WAIT_CODE);
-            // no copy in flight outlives the block
-            for (int i = 0; i < bufs && piece + i < pieces; ++i) {
-                mbar_wait(tc_smem(full + buf), parity);
-                if (++buf == bufs) buf = 0, parity ^= 1;
-            }
-            return;
-        }
-        float vt[TN];
-#pragma unroll
-        for (int x = 0; x < TN; ++x) vt[x] = v_next[x];
-        if (piece + 1 < pieces) ahead(piece + 1);
-        const int here = min(C, n - piece * C);
-        const bf16* ks = reinterpret_cast<const bf16*>(sm + buf * per_buf);        // (the q rows follow the k rows)
-        const float* ms = sm + buf * per_buf + row_floats;
-        const float P = ms[t * GH_MROW + 2 * C], dec = ms[t * GH_MROW + 2 * C + 1];
-        {
-            float acc[2][2][4];                  // [k rows, q rows][columns 0 .., 8 ..]
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int c = 0; c < 2; ++c) acc[m][c][0] = acc[m][c][1] = acc[m][c][2] = acc[m][c][3] = 0.f;
-            // parts of S, in the right operand's layout: [channels of a sixteen][columns]
-            uint32_t sp[KS][2][2][3];
-#pragma unroll
-            for (int k = 0; k < KS; ++k)
-#pragma unroll
-                for (int c = 0; c < 2; ++c)
-#pragma unroll
-                    for (int b = 0; b < 2; ++b) gp_split(s[2 * k + b][2 * c], s[2 * k + b][2 * c + 1], sp[k][c][b]);
-            const uint32_t at = smem_u32(ks) + ((lane & 15) * LD + d0 + (lane >> 4) * 8) * 2;
-            // left part pa by right parts last .. 0; products into one sum stand four or more apart (one
-            // after the other each would wait for the one before it)
-            auto products = [&](int pa, int last) {
-                uint32_t A[KS][2][4];
-#pragma unroll
-                for (int k = 0; k < KS; ++k)
-#pragma unroll
-                    for (int m = 0; m < 2; ++m) ldmatrix_x4(A[k][m], at + (pa * PLANE + m * C * LD + k * 16) * 2);
-#pragma unroll
-                for (int pb = last; pb >= 0; --pb)
-#pragma unroll
-                    for (int k = 0; k < KS; ++k)
-#pragma unroll
-                        for (int m = 0; m < 2; ++m)
-#pragma unroll
-                            for (int c = 0; c < 2; ++c)
-                                mma_bf16_16816(acc[m][c], A[k][m], sp[k][c][0][pb], sp[k][c][1][pb]);
-            };
-            products(2, 0);
-            products(1, 1);
-            products(0, 2);
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    float* to = part + (warp * 2 * C + m * C + g) * PLD + c * 8 + 2 * q;
-                    *reinterpret_cast<float2*>(to) = make_float2(acc[m][c][0], acc[m][c][1]);
-                    *reinterpret_cast<float2*>(to + 8 * PLD) = make_float2(acc[m][c][2], acc[m][c][3]);
-                }
-        }
-        __syncthreads();
-        // (the piece before this one is done with in all warps: its buffer is free)
-        if (piece >= 1 && piece - 1 + bufs < pieces && tid == GH_THREADS - 32) fetch(buf == 0 ? bufs - 1 : buf - 1, piece - 1 + bufs);
-        float r[TN], p[TN];
-#pragma unroll
-        for (int x = 0; x < TN; ++x) r[x] = p[x] = 0.f;
-#pragma unroll
-        for (int w = 0; w < WARPS; ++w) {
-            float rs[TN], ps[TN];
-            gh_load(part + (w * 2 * C + t) * PLD + tc, rs);
-            gh_load(part + (w * 2 * C + C + t) * PLD + tc, ps);
-#pragma unroll
-            for (int x = 0; x < TN; ++x) {
-                r[x] += rs[x];
-                p[x] += ps[x];
-            }
-        }
-        // (a token past the piece has c = 0: its row and column of T and B T are not used)
-        float ct[TN];
-#pragma unroll
-        for (int x = 0; x < TN; ++x) ct[x] = t < here ? fmaf(-P, r[x], vt[x]) : 0.f;
-        gh_store(cs + t * COLS + tc, ct);
-        __syncthreads();
-        {
-            float u[TN], o[TN];
-#pragma unroll
-            for (int x = 0; x < TN; ++x) {
-                u[x] = 0.f;
-                o[x] = P * p[x];
-            }
-            const float* trow = ms + t * GH_MROW;
-            const float* brow = trow + C;
-#pragma unroll
-            for (int i = 0; i < C; i += 4) {
-                // up to t only, not with the zeros behind: a later token's value that is not finite stays out
-                // (0 times it would be no 0)
-                float t4[4], b4[4];
-                load4(trow + i, t4);
-                load4(brow + i, b4);
-#pragma unroll
-                for (int w = 0; w < 4; ++w) {
-                    float c[TN];
-                    gh_load(cs + (i + w) * COLS + tc, c);
-                    const bool seen = i + w <= t;
-                    if (!seen) t4[w] = b4[w] = 0.f;
-#pragma unroll
-                    for (int x = 0; x < TN; ++x) {
-                        if (!seen) c[x] = 0.f;
-                        u[x] = fmaf(t4[w], c[x], u[x]);
-                        o[x] = fmaf(b4[w], c[x], o[x]);
-                    }
-                }
-            }
-            uint32_t up[3];
-            gp_split(t < here ? dec * u[0] : 0.f, t < here ? dec * u[1] : 0.f, up);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                us[(i * COLS + tc) * ULD + t] = __ushort_as_bfloat16((unsigned short)up[i]);
-                us[(i * COLS + tc + 1) * ULD + t] = __ushort_as_bfloat16((unsigned short)(up[i] >> 16));
-            }
-            if (t < here) {
-                float* dst = a.out + (size_t)(start + piece * C + t) * vv + (size_t)h * a.VD + col0 + tc;
-#pragma unroll
-                for (int x = 0; x < TN; ++x)
-                    if (col0 + tc + x < a.VD) dst[x] = o[x];
-            }
-        }
-        __syncthreads();
-        {
-            // the change of S^T: u^T [columns x tokens] by the rows that enter [tokens x channels]
-            const bf16* news = CHANNEL ? ks + 2 * C * LD : ks;
-            uint32_t U[3][4];
-#pragma unroll
-            for (int i = 0; i < 3; ++i)
-                ldmatrix_x4(U[i], smem_u32(us + (i * COLS + (lane & 15)) * ULD + (lane >> 4) * 8));
-            float more[NT][4];
-#pragma unroll
-            for (int j = 0; j < NT; ++j) more[j][0] = more[j][1] = more[j][2] = more[j][3] = 0.f;
-            const uint32_t at = smem_u32(news) + ((lane & 15) * LD + d0 + (lane >> 4) * 8) * 2;
-            auto products = [&](int pb, int last) {
-                uint32_t B[KS][4];
-#pragma unroll
-                for (int k = 0; k < KS; ++k) ldmatrix_x4_trans(B[k], at + (pb * PLANE + k * 16) * 2);
-#pragma unroll
-                for (int pa = last; pa >= 0; --pa)
-#pragma unroll
-                    for (int k = 0; k < KS; ++k) {
-                        mma_bf16_16816(more[2 * k], U[pa], B[k][0], B[k][1]);
-                        mma_bf16_16816(more[2 * k + 1], U[pa], B[k][2], B[k][3]);
-                    }
-            };
-            products(2, 0);
-            products(1, 1);
-            products(0, 2);
-            if (++buf == bufs) buf = 0, parity ^= 1;
-            const float whole = ms[(here - 1) * GH_MROW + 2 * C];
-#pragma unroll
-            for (int j = 0; j < NT; ++j) {
-                float2 pc = make_float2(whole, whole);
-                if (CHANNEL)
-                    pc = *reinterpret_cast<const float2*>(ms - D + d0 + 8 * j + 2 * q);
-                s[j][0] = fmaf(pc.x, s[j][0], more[j][0]);
-                s[j][1] = fmaf(pc.y, s[j][1], more[j][1]);
-                s[j][2] = fmaf(pc.x, s[j][2], more[j][2]);
-                s[j][3] = fmaf(pc.y, s[j][3], more[j][3]);
-            }
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-#pragma unroll
-        for (int half = 0; half < 2; ++half)
-            if (col0 + g + 8 * half < a.VD)
-                *reinterpret_cast<float2*>(s_head + (size_t)(g + 8 * half) * D + 8 * j + 2 * q) =
-                    make_float2(s[j][2 * half], s[j][2 * half + 1]);
-    gd_advance_conv(a.conv, waited, state + (size_t)a.slots[e] * a.state_stride, start, n, h, a.H);
-}
-
-template <int D, bool CHANNEL>
-static int launch_parts_scan(const DeltaHeadArgs& a, int entries, cudaStream_t s) {
-    constexpr size_t buf = gp_row_bytes(D, CHANNEL) + GC_TOKENS * GH_MROW * 4;
-    constexpr size_t rest = ((GH_THREADS / 32) * 2 * GC_TOKENS * 24 + GC_TOKENS * 16) * 4 + 3 * 16 * (GC_TOKENS + 8) * 2;
-    constexpr size_t most = 225 * 1024;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(delta_parts_scan_kernel<D, CHANNEL>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
-    const dim3 grid(entries, a.H, (a.VD + 15) / 16);
-    if (grid.z > 65535) return -1;
-    // as many pieces on their way as the blocks that an SM gets leave room for
-    const long long blocks = (long long)grid.x * grid.y * grid.z, sms = device_sm_count();
-    const long long share = (long long)most / ((blocks + sms - 1) / sms) - 1024 - (long long)rest;
-    const long long room = share / (long long)buf;       // (2 or fewer where there are more blocks than fit at once)
-    const int bufs = room >= GP_BUFS ? GP_BUFS : room >= 2 ? (int)room : 2;
-    mstar_launch((delta_parts_scan_kernel<D, CHANNEL>), grid, dim3(GH_THREADS), bufs * buf + rest, s, a, bufs);
-    return launch_status();
-}
-template <int D> static int launch_parts_scan_kind(const DeltaHeadArgs& a, int entries, bool channel, cudaStream_t s) {
-    return channel ? launch_parts_scan<D, true>(a, entries, s) : launch_parts_scan<D, false>(a, entries, s);
-}
-
 template <int D, int COLS, bool CHANNEL>
 static int launch_head_scan(const DeltaHeadArgs& a, int entries, cudaStream_t s) {
     constexpr int rows = CHANNEL ? GK_ROWS(GC_TOKENS) : 2 * GC_TOKENS;
@@ -1603,7 +1262,7 @@ MSTAR_API int mstar_delta_scan_pieces(const float* q, const float* k, const floa
         return -1;
     const int max_pieces = (max_q_len + GC_TOKENS - 1) / GC_TOKENS;
     const size_t most = (size_t)(tokens / GC_TOKENS + entries);
-    const size_t row_floats = most * (head_decay ? G : H) * gh_row_floats(D, !head_decay);
+    const size_t row_floats = head_decay ? most * G * 2 * GC_TOKENS * (D + 4) : most * H * GK_ROWS(GC_TOKENS) * (D + 4);
     DeltaHeadArgs a{q, k, v, beta, decay, qo_indptr, slots, work, work + row_floats, state, state_stride, state_offset, out,
                     H, G, D, VD, tokens, error_word, {taps > 1 ? conv_raw : nullptr, conv_ld, channels, taps}};
     cudaStream_t s = (cudaStream_t)stream;
@@ -1630,10 +1289,10 @@ MSTAR_API int mstar_delta_scan_pieces(const float* q, const float* k, const floa
     const int code = launch_status();
     if (code != 0) return code;
     if (D == 32) return launch_head_scan_kind<32>(a, entries, !head_decay, s);
+    if (D == 64) return launch_head_scan_kind<64>(a, entries, !head_decay, s);
     if (D == 96) return launch_head_scan_cols<96, false>(a, entries, s);
-    if (D == 64) return launch_parts_scan_kind<64>(a, entries, !head_decay, s);
-    if (D == 128) return launch_parts_scan_kind<128>(a, entries, !head_decay, s);
-    return launch_parts_scan_kind<256>(a, entries, !head_decay, s);
+    if (D == 128) return launch_head_scan_kind<128>(a, entries, !head_decay, s);
+    return launch_head_scan_kind<256>(a, entries, !head_decay, s);
 }
 
 // ------------------------------------------------------------------ finish

@@ -2028,7 +2028,6 @@ def delta_prepare(proj: torch.Tensor, conv_w: torch.Tensor, a_proj: torch.Tensor
 DELTA_PIECE = 16            # tokens of a piece of the delta-rule scan
 DELTA_PIECES_FROM = 64      # entries of this many tokens or more are scanned in pieces
 DELTA_PIECES_DIMS = (32, 64, 128, 256)     # key sizes the scan in pieces takes
-DELTA_PARTS_DIMS = (64, 128, 256)   # ... and takes on the tensor cores
 DELTA_HEAD_PIECES_DIMS = (32, 64, 96, 128, 256)    # with one decay a head
 
 
@@ -2069,13 +2068,8 @@ def delta_scan(q, k, v, beta, decay, qo_indptr, slots, state: torch.Tensor, entr
     aligned = all(t.data_ptr() % 16 == 0 for t in (q, k, state)) and (head_decay or decay.data_ptr() % 16 == 0)
     if (pieces and dim in (DELTA_HEAD_PIECES_DIMS if head_decay else DELTA_PIECES_DIMS) and tokens > 0 and offset % 4 == 0
             and state.stride(0) % 4 == 0 and (aligned or head_decay)):
-        # a piece's rows as the scan wants them: floats, or three bfloat16 parts of each
-        kinds = 2 if head_decay else 3
-        if dim in DELTA_PARTS_DIMS:
-            row = kinds * DELTA_PIECE * (dim + 8) * 3 // 2 + (0 if head_decay else dim)
-        else:
-            row = (kinds * DELTA_PIECE + (0 if head_decay else 1)) * (dim + 4)
-        per_piece = (kv_heads if head_decay else heads) * row + heads * DELTA_PIECE * (2 * DELTA_PIECE + 4)
+        rows = (kv_heads * 2 * DELTA_PIECE if head_decay else heads * (3 * DELTA_PIECE + 1)) * (dim + 4)
+        per_piece = rows + heads * DELTA_PIECE * (2 * DELTA_PIECE + 4)
         work = q.new_empty((tokens // DELTA_PIECE + entries) * per_piece, dtype=torch.float32)
         code = lib.get("gated_delta").mstar_delta_scan_pieces(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), beta.data_ptr(), decay.data_ptr(),

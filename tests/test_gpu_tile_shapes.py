@@ -321,6 +321,33 @@ def test_delta_rule_in_pieces_with_decays_per_channel(lens, heads, kv_heads, dim
 
 
 @pytest.mark.parametrize("head_decay", [False, True])
+@pytest.mark.parametrize("dim,vdim", [(32, 32), (64, 48), (128, 128), (256, 64)])
+def test_delta_rule_in_pieces_rounds_to_nearest(dim, vdim, head_decay):
+    """Under decays that leave a few tokens in the state, its errors favour neither side (sums that are
+    cut off come out 2^-25 of themselves too small)."""
+    from mstar_b200 import ops
+
+    T, heads = 64, 2
+    q, k = (torch.nn.functional.normalize(rnd(T, heads, dim, seed=s), dim=-1).view(T, -1) for s in (1, 2))
+    v, beta = rnd(T, heads * vdim, seed=3), torch.sigmoid(rnd(T, heads, seed=4))
+    decay = torch.exp(-torch.exp(2 * rnd(T, heads * (1 if head_decay else dim), seed=5)))
+    state = torch.zeros(1, ops.gated_delta_state_size(heads, heads, dim, vdim, 1), device=DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    ops.delta_scan(q, k, v, beta, decay, i32([0, T]), i32([0]), state, 1, heads, heads, dim, vdim, 1, max_q_len=T)
+    kd, gd = k.double().view(T, heads, dim), decay.double().view(T, heads, -1)
+    S = torch.zeros(heads, dim, vdim, dtype=torch.float64, device=DEV)
+    for t in range(T):
+        S *= gd[t][:, :, None]
+        u = beta[t].double()[:, None] * (v[t].double().view(heads, vdim) - (kd[t][:, None] @ S)[:, 0])
+        S += kd[t][:, :, None] * u[:, None]
+    far = (state.view(heads, vdim, dim).transpose(1, 2).double() - S) / S
+    far = far[S.abs() > S.abs().mean() / 8]
+    # a column of the last token's u is off by 2^-24 at most either way: 2^-24 / sqrt(heads * vdim) in the mean,
+    # times a margin of 2
+    assert far.mean().abs() < 2 ** -23 / (heads * vdim) ** 0.5
+
+
+@pytest.mark.parametrize("head_decay", [False, True])
 @pytest.mark.parametrize("heads,dim,vdim", [(1, 32, 8), (2, 128, 40), (80, 64, 32)])     # 8 and 16 columns a block
 def test_delta_rule_in_pieces_leaves_later_values_out(head_decay, heads, dim, vdim):
     """A value that is not finite reaches no earlier token's output, wherever it lies in its piece."""
