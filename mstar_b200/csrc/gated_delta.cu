@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(256) delta_prepare_kernel(DeltaPrepArgs a) {
     }
 }
 
-// Prompts, with four taps and heads of up to 128: a warp takes a unit of DP_RUN tokens in a row, so that a
+// Prompts, with four taps and heads of 128: a warp takes a unit of DP_RUN tokens in a row, so that a
 // projected row is read once instead of four times and the taps' weights once instead of DP_RUN times.  The
 // arithmetic of a token is that of the kernel above.  Bound by instructions (the exponentials' and the IEEE
 // quotients'): 2,048 tokens, 16 heads of 128 with a decay a key channel: 45 us, 55 above; 3 x 600 with one a head: 18, 21.
@@ -328,8 +328,13 @@ MSTAR_API int mstar_delta_prepare(const float* proj, int row_stride, const void*
     bool vec = D % 4 == 0 && VD % 4 == 0 && row_stride % 4 == 0 && state_stride % 4 == 0;
     const void* ptrs[] = {proj, conv_w, state, q, k, v};
     for (const void* p : ptrs) vec = vec && (uintptr_t)p % 16 == 0;
-    // runs of tokens where there are enough to fill the SMs with (64 tokens of 64 units: 64 blocks)
-    if (vec && taps == 4 && D <= 128 && VD <= 128 && tokens >= 64 &&
+    // Runs of tokens (the same bits) where a head keeps all lanes of a warp busy (heads of 64: 98 us against 68, 32 heads,
+    // 2,000 tokens) and there are enough of them, since a run is a chain: with a decay a key channel 7.4 against 11.1 us
+    // for 12,800 (200 tokens of 64 units), 43 against 55 for 128,000, but 6.3 against 4.5 for 3,840; with one a head 6.8
+    // against 10.4 for 13,000, 11.1 against 12.7 for 30,600, but 6.1 against 5.5 for 8,500 and 52.7 against 48.1 for
+    // 130,000.
+    const long long all = (long long)tokens * units;
+    if (vec && taps == 4 && D == 128 && VD == 128 && (head_decay ? all >= 9000 && all <= 64000 : all >= 12000) &&
         (head_decay || (((uintptr_t)a_proj | (uintptr_t)dt_bias | (uintptr_t)decay) % 16 == 0))) {
         const dim3 runs((tokens + DP_RUN - 1) / DP_RUN, (units + 7) / 8);
         mstar_launch(weight_dtype == MSTAR_F32 ? delta_prepare_run_kernel<float> : delta_prepare_run_kernel<bf16>, runs,

@@ -373,6 +373,52 @@ def test_delta_rule_in_pieces_leaves_later_values_out(head_decay, heads, dim, vd
     ops.check_error_word(DEV)
 
 
+@pytest.mark.parametrize("head_decay", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_delta_inputs_by_runs_of_tokens(head_decay, dtype):
+    """Enough tokens for a warp to take eight in a row, entries that meet inside such a run or are shorter than the
+    convolution, no multiple of eight in all: against double precision, and each entry by itself (a token a warp there,
+    and an entry that begins a run) with the same bits."""
+    from mstar_b200 import ops
+
+    lens, heads, kv_heads, dim, taps = [300, 2, 5, 241, 1], 8, 4, 128, 4
+    T, qk, vv = sum(lens), kv_heads * dim, heads * dim
+    channels = 2 * qk + vv
+    proj = rnd(T, channels + 2 * heads + 8, seed=1)
+    w = (0.3 * rnd(channels, taps, seed=2)).to(dtype)
+    decays = heads if head_decay else heads * dim
+    a_proj = None if head_decay else rnd(T, decays, seed=3)
+    bias, rate = rnd(decays, seed=4) - 3, torch.rand(heads, device=DEV) * 15 + 1
+    state = rnd(len(lens), ops.gated_delta_state_size(heads, kv_heads, dim, dim, taps), seed=5)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    starts = [sum(lens[:e]) for e in range(len(lens) + 1)]
+
+    def run(first, last, slots):
+        rows = slice(starts[first], starts[last])
+        req = [e for e in range(last - first) for _ in range(lens[first + e])]
+        return ops.delta_prepare(proj[rows], w, None if head_decay else a_proj[rows], bias, rate, i32(req),
+                                 i32([s - starts[first] for s in starts[first:last + 1]]), i32(slots), state, heads,
+                                 kv_heads, dim, dim, taps, 1e-6)
+
+    got = run(0, len(lens), list(range(len(lens))))
+    for e in range(len(lens)):
+        alone = run(e, e + 1, [e])
+        assert all(torch.equal(x[starts[e]:starts[e + 1]], y) for x, y in zip(got, alone)), e
+    past = state[:, :(taps - 1) * channels].double().view(-1, taps - 1, channels)
+    x = torch.cat([torch.cat([past[e], proj[starts[e]:starts[e + 1], :channels].double()]).unfold(0, taps, 1)
+                   for e in range(len(lens))])
+    y = torch.nn.functional.silu((x * w.double()).sum(2))
+    unit = lambda z: (z / (z.pow(2).sum(2, keepdim=True) + 1e-6).sqrt()).view(T, -1)
+    b = proj[:, channels:channels + heads].double()
+    z = proj[:, channels + heads:channels + 2 * heads].double() if head_decay else a_proj.double()
+    step = torch.nn.functional.softplus(z + bias.double()).view(T, heads, -1)
+    want = (unit(y[:, :qk].view(T, kv_heads, dim)) * dim ** -0.5, unit(y[:, qk:2 * qk].view(T, kv_heads, dim)),
+            y[:, 2 * qk:], torch.sigmoid(b), torch.exp(-rate.double()[:, None] * step).view(T, -1))
+    for g, v in zip(got, want):
+        # four products and a SiLU, each rounded once or twice, of sums of about 1 (exponents of up to some 50)
+        assert (g.double() - v).abs().max() < 2 ** -24 * 64
+
+
 @pytest.mark.parametrize("temperature,opts", [(0.6, {"top_p": 0.8}), (3.0, {"top_p": 0.95}), (0.05, {"top_p": 0.999}),
                                               (1.0, {"top_p": 1e-6}), (1.5, {"top_k": 3000, "top_p": 0.9}),
                                               (1.0, {"top_k": 700})])
