@@ -91,10 +91,10 @@ __device__ __forceinline__ void mark(const float* p, size_t step, int rows, uint
         }
 }
 
-// A sum v that is not finite, of rows with these marks.
-__device__ __forceinline__ float not_finite(float v, uint32_t kind, const float* a, const float* w, int K) {
+// A sum that is not finite, of rows with these marks.  (Without a mark: finite numbers whose products pass the
+// largest float; those of the middle parts may then be infinities of the other sign.)
+__device__ __forceinline__ float not_finite(uint32_t kind, const float* a, const float* w, int K) {
     if (kind & 2) return __uint_as_float(0x7fffffffu);
-    if (kind == 0) return v;                  // finite numbers with a sum past the largest float
     float even = 0.f, odd = 0.f;
 #pragma unroll 1
     for (int k = 0; k < K; k += 2) {          // K is a multiple of 4
@@ -306,7 +306,7 @@ sgemm_parts_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
                 const int m = m0 + part * PART + j;
                 if (m < M) {
                     if (!isfinite(total[j]))
-                        total[j] = not_finite(total[j], w_kind[row] | a_kind[part * PART + j], A + (size_t)m * lda,
+                        total[j] = not_finite(w_kind[row] | a_kind[part * PART + j], A + (size_t)m * lda,
                                               W + (size_t)n * ldw, K);
                     C[(size_t)m * ldc + n] = total[j];
                 }
@@ -380,7 +380,7 @@ sgemm_parts_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
                     uint32_t kind = 0;
                     for (int q = 0; q < cluster; ++q)
                         kind |= cl.map_shared_rank(w_kind, q)[row] | cl.map_shared_rank(a_kind, q)[col];
-                    v = not_finite(v, kind, A + (size_t)(m0 + col) * lda, W + (size_t)n * ldw, K);
+                    v = not_finite(kind, A + (size_t)(m0 + col) * lda, W + (size_t)n * ldw, K);
                 }
                 C[(size_t)(m0 + col) * ldc + n] = v;
             }

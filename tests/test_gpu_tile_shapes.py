@@ -80,6 +80,19 @@ def test_sgemm_by_parts_keeps_infinities(m, k):
     torch.testing.assert_close(got[both], want[both], rtol=1e-5, atol=1e-3)
 
 
+@pytest.mark.parametrize("m,k", [(5, 1024), (100, 2048), (40, 4096)])
+def test_sgemm_by_parts_of_products_past_the_largest_float(m, k):
+    """Finite operands: where products with the lesser parts pass it too, they may be infinities of the other sign."""
+    from mstar_b200 import ops
+
+    a, w = rnd(m, k, seed=7), rnd(256, k, seed=8)
+    a[1, 3], a[2, 3], w[:, 3] = 1.3e23, -3.7e30, 2.9e20 * (1 + rnd(256, seed=9).abs())
+    a[3, 40], w[:, 40] = 1e25, 1e25 * rnd(256, seed=10).sign()
+    got, want = ops.sgemm_nt(a, w), _sgemm(a, w)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf()) and want[1:4].isinf().all()
+    assert torch.equal(got[want.isinf()], want[want.isinf()])
+
+
 @pytest.mark.parametrize("lens_q,lens_kv,nq,nkv,hd,page,window", [
     ([70, 9], [70, 200], 4, 1, 64, 16, 0),          # several blocks, a border between requests in one
     ([33, 4, 64], [100, 4, 129], 6, 2, 128, 8, 0),  # a group of 3: 63 of 64 rows
