@@ -160,29 +160,30 @@ MSTAR_API int mstar_sgemm_nt(const float* A, const float* W, float* C, int M, in
     if (M <= 0 || N <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     // Wide matrices of aligned rows go to the tensor cores, three bfloat16 parts a float (gemm_f32_tc.cu, with both
-    // sides measured; no error word: never).  From K = 512 on: the start and end of a tile there take some
-    // 8 us, as long as the FMAs of a shorter row ([1536, 128] x [4096, 128]: 47 to 49 against 50 us).
+    // sides measured; no error word: never).  From K = 1,024 on: the start and end of a tile there take some
+    // 8 us, and a row alone takes 8.7 with K = 512 where the FMAs take 6.7 to 8.0 (N = 128 to 3,072; at 1,024: 8.7 to 11 against
+    // 11 to 12), while matrices alone decide, so that a row's sums are the same in every batch.  Below that the FMAs are
+    // as near to 64 bits as well.
     if (error != nullptr && sgemm_parts_takes(A, W, N, K, lda, ldw))
         return sgemm_parts(A, W, C, M, N, K, lda, ldw, ldc, 0, 0, error, s);
     const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
                      ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0;
     const int sms = device_sm_count();
     auto tiles = [&](int bm, int bn) { return (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
-    // Few rows: the stream of W counts, so narrow tiles (a block an SM or more) with deep stages.
-    // [8, 2048] x [3072, 2048]: 21 us, [8, 3072] x [16384, 3072]: 78 us (64 x 64 tiles of 16 k, no
-    // stages in flight: 248 and 640 us); with 16 rows a tile these two take 25 and 120 us.
+    // What comes here has a short K, few columns or rows off 16 bytes.
+    // Few rows: the stream of W counts, so narrow tiles with deep stages.  [1, 512] x [3072, 512] 7.6 us, 8.6 with 16
+    // rows a tile, 13 with 32; [8, 2048] x [64, 2048] 19, 23 and 43.
     if (M <= 8) return launch_sgemm<8, 16, 2, 1, 128, 4>(A, W, C, M, N, K, lda, ldw, ldc, vec, s);
-    // up to 32 rows: 30 against 40 to 52 us for tiles of 32 rows at [30, 2048] x [3072, 2048];
-    // twice as wide where that still makes two blocks an SM
+    // up to 32 rows: 10.6 us against 13.7 for tiles of 32 rows at [30, 512] x [3072, 512], 31 against 58 at [30, 2047] x
+    // [2048, 2047] off 16 bytes; twice as wide where that still makes two blocks an SM ([30, 512] x [16384, 512]: 35 against 41)
     if (M <= 32) {
         if (tiles(16, 32) >= 2 * sms)
             return launch_sgemm<16, 32, 2, 2, 64, 4>(A, W, C, M, N, K, lda, ldw, ldc, vec, s);
         return launch_sgemm<16, 16, 2, 2, 64, 4>(A, W, C, M, N, K, lda, ldw, ldc, vec, s);
     }
-    // 64 x 64 tiles with 8 x 4 outputs a thread where they give every SM more than one block (several
-    // share an SM): 46 TFLOP/s at [2048, 4096] x [4096, 4096], 36 at [512, 2048] x [3072, 2048], against
-    // 40 to 42 and 26 to 29 for 128 x 128 and 64 x 128 tiles of 8 x 8.  Below that 32 x 32 tiles: 51
-    // against 75 us at [64, 2048] x [3072, 2048].
+    // 64 x 64 tiles with 8 x 4 outputs a thread where they give every SM more than one block (several share an SM): 46
+    // us against 53 for 32 x 32 at [1536, 128] x [4096, 128], 389 against 445 at [2048, 512] x [8192, 512] (44 TFLOP/s).  Below
+    // that 32 x 32 tiles: 14 against 21 us at [64, 512] x [1024, 512].
     if (tiles(64, 64) * 2 >= 3 * sms)
         return launch_sgemm<64, 64, 8, 4, 32, 3>(A, W, C, M, N, K, lda, ldw, ldc, vec, s);
     return launch_sgemm<32, 32, 4, 4, 32, 4>(A, W, C, M, N, K, lda, ldw, ldc, vec, s);

@@ -3,11 +3,12 @@
 // A float is the sum of three bfloat16 numbers, its 24 bits eight at a time.  Of the nine products of such
 // parts the six that are 2^-16 or more of the whole are made (tcgen05.mma kind::f16): the leading
 // one into one accumulator, the others into two more, since a tensor-core accumulator is cut off rather
-// than rounded and every sum into it costs half a bit of its last place.  After a slice of K (128
-// positions, more from K = 2,048 on) the three are read out of tensor memory and added, rounded to nearest,
-// to the sums in registers.  Error against 64 bits (2-norm over 2-norm, normal operands; the FMA kernel of
-// gemm_f32.cu in brackets): 1.4e-7 (5.8e-7) at K = 2,048, 4.8e-7 (1.2e-6) at K = 8,192.  Operands of one sign
-// are where the cutting off shows most: 1.7e-7 (3.3e-7) and 8.5e-7 (6.6e-7).
+// than rounded and every sum into it costs half a bit of its last place, all on the same side where products have one
+// sign.  After 128 positions of K, however long it is, the three are read out of tensor memory and added, rounded
+// to nearest, to the sums in registers.  Error against 64 bits (2-norm over 2-norm; the FMA kernel of gemm_f32.cu in
+// brackets): normal operands 1.3e-7 (3.9e-7) at K = 1,024, 1.4e-7 (1.1e-6) at 8,192, 1.6e-7 (2.1e-6) at 28,672; operands of
+// one sign 1.75e-7 at every K (2.3e-7, 7.1e-7, 1.3e-6).  With sums of 512 positions at K = 8,192 those took 8.9e-7; with sums of 64
+// they have 9.3e-8, and the product takes 1.4 times as long.
 //
 // A CTA has 128 rows of W (the M side of the product, lanes of tensor memory) and BN rows of A (the
 // N side, columns).  Two groups of eight warps, one for the even and one for the odd k-blocks of 64,
@@ -15,8 +16,8 @@
 // parts, put these into the group's stage in shared memory in the layout the products read (K-major,
 // 128-byte swizzle) and add up the slices; one more warp issues the products.
 //
-// Every element is the sum, in this order, of its slices.  Where there are few tiles, the CTAs of a
-// cluster share K slice by slice, keep each slice's sum in tensor memory and add them in the same
+// Every element is the sum, in this order, of its slices of K, which the two matrices' widths cut.  Where there are few
+// tiles, the CTAs of a cluster share K slice by slice, keep each slice's sum and add them in the same
 // order through distributed shared memory, so a row's result depends neither on what else is in
 // the batch nor on how the work was cut.
 //
@@ -27,9 +28,13 @@
 // What bounds it: the way of a block through the splitters, its fence, the products and back, 1.1 us with 16
 // rows of A and 1.5 with 80 where the products alone take 0.3 and 0.5; shared memory, which the splitters
 // fill and the products read, and instruction slots (half of them) are what the two groups compete for.
-// Measured, against the FMA kernel: [448, 2048] x [3072, 2048] 55 (183) us, [50, 2048] x [16384, 2048] 49 (129),
-// [7, 2048] x [16384, 2048] 41 (57), [1, 2048] x [3072, 2048] 19 (23).  Slower: a warpgroup of its own for the sums,
-// blocks of 32 in five stages (70 us where this takes 55), three stages of 64.
+// Measured, against the FMA kernel: [448, 2048] x [3072, 2048] 55 (177) us, [50, 2048] x [16384, 2048] 44 (128),
+// [7, 2048] x [16384, 2048] 39 (57), [1, 2048] x [3072, 2048] 17 (20); with a long K [256, 8192] x [3072, 8192] 150 (422), [1, 8192] x
+// [3072, 8192] 41 (70).  One row of 4,100 to 9,400 columns and K up to 2,048 is slower: [1, 2048] x [5632, 2048] 25 (22).  What
+// several slices cost a CTA that has them all: [448, 3072] x [3072, 3072] takes 89 us, 75 if K were one slice, since the sums that
+// wait in shared memory leave L1 and registers short; a second set in registers 83, waiting in C for more than one
+// slice 102.  Slower too: a warpgroup of its own for the sums, blocks of 32 in five stages (70 us where this takes 55), three
+// stages of 64, leading products alone read out every 128 positions (the issuer's loop is what all wait for: 58).
 #include "common.cuh"
 #include "tcgen05_util.cuh"
 #include "tma_util.cuh"
@@ -46,12 +51,25 @@ constexpr int GROUP = 256;           // threads that fill a stage
 constexpr int WORKERS = 2 * GROUP;   // then the issuer's warp
 constexpr int THREADS = WORKERS + 32;
 constexpr int ISSUER = WORKERS / 32;
-// k-blocks a tensor-core sum runs over: 128 positions up to K = 2,048, so that at most 16 sums make an element
-__host__ __device__ constexpr int slice_blocks(int k) { return 2 * ((k + 2047) / 2048); }
+// A tensor-core sum runs over a pair of k-blocks, 128 positions, whatever K is.  Pairs are added up in slices of K, which
+// are what CTAs can share, and these in their order: a pair each up to K = 2,048; of a longer K as many as CTAs can
+// share K with a tile each of W and no more rows of A than a tile has, on 148 SMs less what GPCs leave over.
+__host__ __device__ constexpr bool is_long(int k) { return k > 2048; }
+__host__ __device__ constexpr int pairs_of(int k) { return (k + 2 * BK - 1) / (2 * BK); }
+int slices_of(int n, int k) {
+    const int tiles = (n + BW - 1) / BW;
+    return !is_long(k) ? pairs_of(k) : tiles <= 13 ? 8 : tiles <= 32 ? 4 : tiles <= 74 ? 2 : 1;
+}
+__host__ __device__ constexpr int slice_start(int s, int slices, int pairs) { return s * pairs / slices; }
+// What a CTA does with the sums of pairs and slices: it has all of K and adds pairs to a sum in registers (ALL); of a long
+// K in two slices the first one's sum waits in C for the second's (HALVES), of more they wait in shared memory
+// (OUTSIDE; few registers are left).  CTAs that share K have an accumulator a pair and read none before the end
+// (RAW), or where these do not fit keep the slices' sums in tensor memory behind two accumulators (KEPT).
+enum Mode { ALL, HALVES, OUTSIDE, RAW, KEPT };
 constexpr int W_PLANE = BW * 128;     // bytes of a part of the W tile
 
 __host__ __device__ constexpr int stage_bytes(int bn) { return 3 * (W_PLANE + bn * 128); }
-constexpr int smem_bytes(int bn) { return 2 * stage_bytes(bn) + 1024; }
+constexpr int smem_bytes(int bn, Mode mode) { return 2 * stage_bytes(bn) + (mode == OUTSIDE ? bn * BW * 4 : 0) + 1024; }
 
 // Two floats into their three parts, packed, each part rounded to nearest; t collects the last
 // remainders: they are tiny unless a float was not finite, or so large that its first part is not,
@@ -117,6 +135,12 @@ __device__ __forceinline__ void tc_ld(uint32_t taddr, float (&r)[4]) {
                  : "memory");
 }
 
+__device__ __forceinline__ void tc_st(uint32_t taddr, const float (&r)[4]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};"
+                 ::"r"(taddr), "f"(r[0]), "f"(r[1]), "f"(r[2]), "f"(r[3])
+                 : "memory");
+}
+
 // Whether a phase is over, without waiting.
 __device__ __forceinline__ bool is_over(uint32_t bar, uint32_t parity) {
     uint32_t ok;
@@ -130,10 +154,11 @@ __device__ __forceinline__ bool is_over(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
-template <int BN, bool SPLIT>
+template <int BN, Mode MODE>
 __global__ void __launch_bounds__(THREADS, 1)
 sgemm_parts_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N,
-                   int K, int lda, int ldw, int ldc, int cluster, uint32_t tmem_cols, int* error) {
+                   int K, int lda, int ldw, int ldc, int cluster, int slices, uint32_t tmem_cols, int* error) {
+    constexpr bool SPLIT = MODE == RAW || MODE == KEPT;
     constexpr int STAGE = stage_bytes(BN), A_PLANE = BN * 128;
     constexpr int PART = BN / 4;                                 // columns a thread adds up
     constexpr int UW = BW * 16 / GROUP, UA = BN * 16 / GROUP;    // fours of floats a thread
@@ -150,10 +175,12 @@ sgemm_parts_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
     // the last tile of W may cover rows of the one before again
     const int m0 = (SPLIT ? blockIdx.x / cluster : blockIdx.x) * BN, n0 = min((int)blockIdx.y * BW, N - BW);
 
-    const int slice = slice_blocks(K), blocks = (K + BK - 1) / BK, slices = (blocks + slice - 1) / slice;
+    const int blocks = (K + BK - 1) / BK, pairs = pairs_of(K);
     const int per = SPLIT ? (slices + cluster - 1) / cluster : slices;
-    const int s0 = min(rank * per, slices), my_slices = min(per, slices - s0);
-    const int kb0 = s0 * slice, kb1 = min(blocks, (s0 + my_slices) * slice);
+    const int s0 = rank * per, my_slices = min(per, slices - s0);
+    const int pair0 = SPLIT ? slice_start(s0, slices, pairs) : 0;
+    const int my_pairs = SPLIT ? slice_start(s0 + my_slices, slices, pairs) - pair0 : pairs;
+    const int kb0 = 2 * pair0, kb1 = min(blocks, kb0 + 2 * my_pairs);
 
     // Splitters: four numbers of row r; a thread keeps its place in k and walks down the rows, 16 apart.
     // Rows of A past the matrix are never stored, so the last one stands in for them; numbers past K are
@@ -259,7 +286,7 @@ sgemm_parts_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
             arrive(full + stage * 8);
             return ok;
         };
-        // this thread's columns of its row of a slice whose accumulators begin at a column
+        // this thread's columns of its row of a pair with this accumulator
         constexpr int STEP = PART % 8 == 0 ? 8 : 4;
         const int row = (warp & 3) * 32 + lane, part = warp >> 2, n = n0 + row;
         const uint32_t my_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16) + part * PART;
@@ -276,48 +303,105 @@ sgemm_parts_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
             }
         };
         bool ok = true;
-        if constexpr (!SPLIT) {
-            float total[PART];
+        float total[PART];
 #pragma unroll
-            for (int j = 0; j < PART; ++j) total[j] = 0.f;
-            int done = 0, left = slice;                          // slices added up, blocks to the next one
-            auto drain = [&]() {
-                const int b = done & 1;
-                ok = ok && wait(ready + b * 8, (done >> 1) & 1);
-                tc_fence_after_sync();
-                sums(b, [&](int j, float v) { total[j] += v; });
-                tc_fence_before_sync();
-                arrive(drained + b * 8);
-                ++done;
-            };
-            for (int kb = kb0 + stage; kb < kb1 && ok; kb += 2) {
-                ok = fill(kb);
-                // the slice before this block's, while this one's products run
-                if (left == 0) {
-                    drain();
-                    left = slice;
+        for (int j = 0; j < PART; ++j) total[j] = 0.f;
+        int done = 0, left = 2;                                  // pairs added up, blocks to the next one
+        int s = 0, s_end = 0;                                    // of a long K: the slice, its end
+        if (MODE == HALVES || MODE == OUTSIDE || MODE == KEPT) s_end = slice_start(s0 + 1, slices, pairs) - pair0;
+        float* outside = reinterpret_cast<float*>(smem + 2 * STAGE) + part * PART * BW + row;      // [column][row]
+        const uint32_t kept = my_tmem + 6 * BN;
+        auto drain = [&]() {
+            const int b = done & 1;
+            ok = ok && wait(ready + b * 8, (done >> 1) & 1);
+            tc_fence_after_sync();
+            sums(b, [&](int j, float v) { total[j] += v; });
+            tc_fence_before_sync();
+            arrive(drained + b * 8);
+            ++done;
+            if constexpr (MODE == HALVES) {
+                if (done != s_end) return;
+                // (where the last tile of W is shifted back the tile before has these rows)
+                const int first = m0 + (warp >> 2) * PART, rows = n0 + row < (int)blockIdx.y * BW ? 0 : M - first;
+                float* at = C + (size_t)first * ldc + n0 + row;
+#pragma unroll
+                for (int j = 0; j < PART; ++j) {
+                    if (j < rows) *at = total[j];
+                    at += ldc;
+                    total[j] = 0.f;
                 }
-                left -= 2;
             }
-            while (done < my_slices && ok) drain();
+            if constexpr (MODE == OUTSIDE || MODE == KEPT) {
+                if (done != s_end) return;
+#pragma unroll
+                for (int j = 0; j < PART; j += 4) {
+                    const float v[4] = {total[j], total[j + 1], total[j + 2], total[j + 3]};
+                    if constexpr (MODE == KEPT) tc_st(kept + s * BN + j, v);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        if constexpr (MODE == OUTSIDE) outside[(j + i) * BW] = (s == 0 ? 0.f : outside[(j + i) * BW]) + v[i];
+                        total[j + i] = 0.f;
+                    }
+                }
+                ++s;
+                s_end = slice_start(s0 + s + 1, slices, pairs) - pair0;
+            }
+        };
+        for (int kb = kb0 + stage; kb < kb1 && ok; kb += 2) {
+            ok = fill(kb);
+            // the pair before this block's, while this one's products run
+            if (MODE != RAW && left == 0) {
+                drain();
+                left = 2;
+            }
+            left -= 2;
+        }
+        if constexpr (MODE != RAW)
+            while (done < my_pairs && ok) drain();
+        if constexpr (!SPLIT) {
             asm volatile("bar.sync 1, 512;" ::: "memory");       // all marks are made
 #pragma unroll
             for (int j = 0; j < PART; ++j) {
                 const int m = m0 + part * PART + j;
-                if (m < M) {
-                    if (!isfinite(total[j]))
-                        total[j] = not_finite(w_kind[row] | a_kind[part * PART + j], A + (size_t)m * lda,
-                                              W + (size_t)n * ldw, K);
-                    C[(size_t)m * ldc + n] = total[j];
+                if (m < M && (MODE != HALVES || n >= (int)blockIdx.y * BW)) {
+                    float v = MODE == OUTSIDE ? outside[j * BW] : total[j];
+                    if (MODE == HALVES) v = C[(size_t)m * ldc + n] + v;
+                    if (!isfinite(v))
+                        v = not_finite(w_kind[row] | a_kind[part * PART + j], A + (size_t)m * lda, W + (size_t)n * ldw, K);
+                    C[(size_t)m * ldc + n] = v;
                 }
             }
         } else {
-            for (int kb = kb0 + stage; kb < kb1 && ok; kb += 2) ok = fill(kb);
-            ok = ok && wait(ready, 0);
-            tc_fence_after_sync();
-            float* out = reinterpret_cast<float*>(smem);         // [slice][column][row], in the stages' place
-            for (int s = 0; s < my_slices; ++s)
-                sums(s, [&](int j, float v) { out[(s * BN + part * PART + j) * BW + row] = v; });
+            // [slice][column][row], in the stages' place: their last products are done
+            float* out = reinterpret_cast<float*>(smem) + part * PART * BW + row;
+            if constexpr (MODE == RAW) {
+                ok = ok && wait(ready, 0);
+                tc_fence_after_sync();
+                for (int i = 0, at = 0; i < my_slices; ++i) {
+                    const int end = slice_start(s0 + i + 1, slices, pairs) - pair0;
+                    if (end == at + 1) {
+                        sums(at++, [&](int j, float v) { out[(i * BN + j) * BW] = v; });
+                        continue;
+                    }
+                    for (; at < end; ++at) sums(at, [&](int j, float v) { total[j] += v; });
+#pragma unroll
+                    for (int j = 0; j < PART; ++j) {
+                        out[(i * BN + j) * BW] = total[j];
+                        total[j] = 0.f;
+                    }
+                }
+            } else {
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                for (int i = 0; i < my_slices; ++i)
+#pragma unroll
+                    for (int j = 0; j < PART; j += 4) {
+                        float v[4];
+                        tc_ld(kept + i * BN + j, v);
+                        tc_wait_ld();
+#pragma unroll
+                        for (int x = 0; x < 4; ++x) out[(i * BN + j + x) * BW] = v[x];
+                    }
+            }
         }
         if (!ok) atomicExch(error, 28);
         tc_fence_before_sync();
@@ -327,13 +411,13 @@ sgemm_parts_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
             constexpr uint32_t one = instr_desc_bf16(BW, BN);
             bool ok = true;
             const int mine = kb1 - kb0;
-            int left = slice, at = 0, st = 0;                    // blocks of the slice to come, slices begun
+            int left = 2, at = 0, st = 0;                        // blocks of the pair to come, pairs begun
             uint32_t lead = tmem, parity = 0;
             bool there = false;                                  // this block is known to be there
             for (int it = 0; it < mine; ++it) {
-                const bool first = left == slice;
+                const bool first = left == 2;
                 // a buffer that was never used is free: the wait for the phase before its first passes
-                if (!SPLIT && first) ok = mbar_wait(drained + (at & 1) * 8, ((at >> 1) & 1) ^ 1);
+                if (MODE != RAW && first) ok = mbar_wait(drained + (at & 1) * 8, ((at >> 1) & 1) ^ 1);
                 if (!there) ok = ok && mbar_wait(full + st * 8, parity);
                 if (!ok) break;
                 const int next = st ^ 1;
@@ -351,10 +435,10 @@ sgemm_parts_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
                 }
                 tc_commit(empty + st * 8);
                 if (--left == 0 || it + 1 == mine) {
-                    if (!SPLIT || it + 1 == mine) tc_commit(ready + (SPLIT ? 0 : at & 1) * 8);
-                    left = slice;
+                    if (MODE != RAW || it + 1 == mine) tc_commit(ready + (MODE == RAW ? 0 : at & 1) * 8);
+                    left = 2;
                     ++at;
-                    lead = SPLIT ? lead + 3 * BN : tmem + (at & 1) * 3 * BN;
+                    lead = MODE == RAW ? lead + 3 * BN : tmem + (at & 1) * 3 * BN;
                 }
                 st = next;
                 parity = next_parity;
@@ -394,13 +478,25 @@ sgemm_parts_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
     }
 }
 
-int slices_of(int K) { return ((K + BK - 1) / BK + slice_blocks(K) - 1) / slice_blocks(K); }
+// Columns of tensor memory that a CTA takes (512 there are).
+int columns(int bn, int per_slices, int per_pairs, Mode mode) {
+    return bn * (mode == RAW ? 3 * per_pairs : mode == KEPT ? 6 + per_slices : 6);
+}
+// The way for this many columns of a tile and CTAs that share K, or -1: the slices have to fit, also as floats in the
+// stages' shared memory, and no CTA may be without one.
+int mode_of(int bn, int cluster, int N, int K) {
+    const int slices = slices_of(N, K), pairs = pairs_of(K), per = (slices + cluster - 1) / cluster;
+    if (cluster == 1) return !is_long(K) || slices == 1 ? ALL : slices == 2 ? HALVES : OUTSIDE;
+    if (per * bn * BW * 4 > 2 * stage_bytes(bn) || (cluster - 1) * per >= slices) return -1;
+    const int per_pairs = (per * pairs + slices - 1) / slices;
+    return columns(bn, per, per_pairs, RAW) <= 512 ? RAW : columns(bn, per, per_pairs, KEPT) <= 512 ? KEPT : -1;
+}
 
-template <int BN, bool SPLIT>
+template <int BN, Mode MODE>
 int launch(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int cluster,
            int* error, cudaStream_t s) {
-    constexpr int smem = smem_bytes(BN);
-    auto kernel = sgemm_parts_kernel<BN, SPLIT>;
+    constexpr int smem = smem_bytes(BN, MODE);
+    auto kernel = sgemm_parts_kernel<BN, MODE>;
     static bool configured[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -409,9 +505,10 @@ int launch(const float* A, const float* W, float* C, int M, int N, int K, int ld
         if (e != cudaSuccess) return (int)e;
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    const int slices = slices_of(K), per = (slices + cluster - 1) / cluster;
+    const int slices = slices_of(N, K), per = (slices + cluster - 1) / cluster;
+    const int need = columns(BN, per, (per * pairs_of(K) + slices - 1) / slices, MODE);
     uint32_t cols = 32;
-    while (cols < (uint32_t)(3 * BN * (SPLIT ? per : 2))) cols *= 2;
+    while ((int)cols < need) cols *= 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)((M + BN - 1) / BN * cluster), (unsigned)((N + BW - 1) / BW));
     cfg.blockDim = dim3(THREADS);
@@ -422,62 +519,48 @@ int launch(const float* A, const float* W, float* C, int M, int N, int K, int ld
     attr[0].val.clusterDim = {(unsigned)cluster, 1, 1};
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, A, W, C, M, N, K, lda, ldw, ldc, cluster, cols, error);
+    cudaLaunchKernelEx(&cfg, kernel, A, W, C, M, N, K, lda, ldw, ldc, cluster, slices, cols, error);
     return launch_status();
-}
-
-// Whether BN columns and a cluster of this size hold all slices of a CTA: in tensor memory (512 columns)
-// and, as floats, in the stages' shared memory.
-bool fits(int bn, int cluster, int slices) {
-    if (cluster == 1) return true;
-    const int per = (slices + cluster - 1) / cluster;
-    return 3 * bn * per <= 512 && per * bn * BW * 4 <= 2 * stage_bytes(bn) &&
-           (cluster - 1) * per < slices;
 }
 
 }  // namespace
 
 bool sgemm_parts_takes(const float* A, const float* W, int N, int K, int lda, int ldw) {
-    return N >= BW && K >= 512 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
+    return N >= BW && K >= 1024 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
            ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0;
 }
 
 int sgemm_parts(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int bn,
                 int cluster, int* error, cudaStream_t s) {
-    const int slices = slices_of(K);
+    const int blocks = (K + BK - 1) / BK;
     if (bn <= 0) {
         // Microseconds, from measured products: 6 for the start and end of a tile, 1.1 (BN 16) to 1.5
         // (BN 80) a k-block, 4 for adding up a cluster's sums; clusters of 4 and 8 leave SMs of a
-        // GPC over.  It gives 18 for [1, 2048] x [3072, 2048] (measured: 19), 45 for [50, 8192] x [2048, 8192] (45),
-        // 53 for [448, 2048] x [3072, 2048] (55).
+        // GPC over.  Of 60 products of 1 to 1,000 rows it chose one that was slower than the best by 10 % twice.
         const int sms = device_sm_count();
         double best = 1e30;
         for (int b : {16, 32, 48, 64, 80})
             for (int c : {1, 2, 4, 8}) {
-                if (!fits(b, c, slices)) continue;
-                const int per = (slices + c - 1) / c;
+                if (mode_of(b, c, N, K) < 0) continue;
                 const long long ctas = (long long)((M + b - 1) / b) * ((N + BW - 1) / BW) * c;
                 const int there = c == 8 ? sms * 3 / 4 : c == 4 ? sms * 7 / 8 : sms;
                 const double block = 0.9 + 0.0075 * b > 1.1 ? 0.9 + 0.0075 * b : 1.1;
-                const double t = (double)((ctas + there - 1) / there) * (per * slice_blocks(K) * block + 6.0) +
+                const double t = (double)((ctas + there - 1) / there) * ((double)blocks / c * block + 6.0) +
                                  (c > 1 ? 4.0 : 0.0);
                 if (t < best) best = t, bn = b, cluster = c;
             }
-    } else if (!fits(bn, cluster, slices)) {
-        return -1;
     }
-#define CASE(B)                                                                                                   \
-    case B:                                                                                                       \
-        return cluster > 1 ? launch<B, true>(A, W, C, M, N, K, lda, ldw, ldc, cluster, error, s)                  \
-                           : launch<B, false>(A, W, C, M, N, K, lda, ldw, ldc, 1, error, s);
-    switch (bn) {
-        CASE(16)
-        CASE(32)
-        CASE(48)
-        CASE(64)
-        CASE(80)
-    }
+    const int mode = mode_of(bn, cluster, N, K);
+#define GO(B, MODE) \
+    if (bn == B && mode == MODE) return launch<B, MODE>(A, W, C, M, N, K, lda, ldw, ldc, cluster, error, s);
+#define CASE(B) GO(B, ALL) GO(B, HALVES) GO(B, OUTSIDE) GO(B, RAW) GO(B, KEPT)
+    CASE(16)
+    CASE(32)
+    CASE(48)
+    CASE(64)
+    GO(80, ALL) GO(80, HALVES) GO(80, OUTSIDE) GO(80, RAW)          // (80 columns leave no tensor memory to keep slices in)
 #undef CASE
+#undef GO
     return -1;
 }
 

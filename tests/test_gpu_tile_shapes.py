@@ -42,30 +42,36 @@ def _sgemm(a, w, *tile):
     return out if code == 0 else None
 
 
-# one row, a row past every tile width, the last tile of W shifted back by all but one row, K that ends inside
-# a block, inside a slice and on its border, longer slices
-@pytest.mark.parametrize("m,n,k,pad", [(1, 128, 512, 0), (17, 129, 516, 4), (80, 300, 1000, 0), (81, 255, 2112, 0),
-                                       (33, 256, 4100, 8), (200, 640, 1024, 0)])
-def test_sgemm_by_parts(m, n, k, pad):
-    """Three bfloat16 parts a float: no further from 64 bits than the FMA kernel, the same bits from every
-    tile, however K is shared, and for a row alone."""
+# one row, a row past every tile width, the last tile of W shifted back by all but one row, K that ends inside a block,
+# inside a pair of them and on its border, an odd number of pairs; slices of one pair (up to 2,048) and of several
+@pytest.mark.parametrize("m,n,k,pad", [(1, 128, 1024, 0), (17, 129, 1028, 4), (80, 300, 1500, 0), (81, 255, 2112, 0),
+                                       (33, 256, 4100, 8), (200, 640, 1024, 0), (49, 200, 2048, 0), (90, 130, 9000, 0)])
+@pytest.mark.parametrize("one_sign", [False, True])
+def test_sgemm_by_parts(m, n, k, pad, one_sign):
+    """Three bfloat16 parts a float: no further from 64 bits than the FMA kernel, operands of one sign (whose sums are
+    all cut off to the same side) among them, the same bits from every tile, however K is shared, and for a row alone."""
     from mstar_b200 import ops
 
     a, w = rnd(m, k + pad, seed=5)[:, :k], rnd(n, k + pad, seed=6)[:, :k]
+    if one_sign:
+        a.abs_(), w.abs_()
     want = a.double() @ w.double().T
     got = ops.sgemm_nt(a, w)
     far = lambda c: ((c.double() - want).norm() / want.norm()).item()
     assert far(got) <= far(_sgemm(a, w))
+    # an element of one sign: eight sums of growing numbers cut off, half a last place (2^-24 and less) each in the mean,
+    # then 24 at most that are rounded
+    assert not one_sign or far(got) < 2 ** -24 * (8 / 2 + 24 ** 0.5 / 4)
     # every sum into an accumulator cuts off at most a last place (2^-23) of what is there, every sum of
-    # slices rounds: at most K / 16 + 16 of them
-    assert ((got.double() - want).abs() <= 2 ** -23 * (k / 16 + 16) * (a.double().abs() @ w.double().abs().T)).all()
+    # slices rounds: 8 a pair, and 24 at most
+    assert ((got.double() - want).abs() <= 2 ** -23 * (8 + 24) * (a.double().abs() @ w.double().abs().T)).all()
     assert torch.equal(ops.sgemm_nt(a[m - 1:], w), got[m - 1:])
     tiles = [_sgemm(a, w, bn, cluster) for bn in (16, 32, 48, 64, 80) for cluster in (1, 2, 4, 8)]
     assert all(torch.equal(t, got) for t in tiles if t is not None) and sum(t is not None for t in tiles) >= 6
     ops.check_error_word(DEV)
 
 
-@pytest.mark.parametrize("m,k", [(5, 512), (100, 2048)])
+@pytest.mark.parametrize("m,k", [(5, 1024), (100, 2048), (40, 4096)])
 def test_sgemm_by_parts_keeps_infinities(m, k):
     from mstar_b200 import ops
 
