@@ -161,8 +161,8 @@ paged_attention_generic_kernel(const A* __restrict__ q, A* __restrict__ out,
 // the few keys that some rows see and others don't are taken one by one (the last tile of every row is such a one).
 // Tiles start at multiples of 64 keys whatever the block's rows are, and a tile that a row does
 // not see leaves its sums as they are, so a row's result does not depend on what else is in the
-// batch.  Bound by the shared loads that feed the FMA pipe (of 16 bytes, no bank met twice).  It makes the blocks
-// whose operands are not finite; the others go to the tensor cores (below, both sides measured).
+// batch.  Bound by the shared loads that feed the FMA pipe (of 16 bytes, no bank met twice).  It makes the rows (`bad`) that
+// the tensor cores (below, both sides measured) cannot, for operands that are not finite.
 #define AR_ROWS 64
 #define AR_KEYS 64
 #define AR_THREADS 256                         // of a group
@@ -208,7 +208,7 @@ template <int HD>
 __device__ __noinline__ void ar_block_fma(const float* __restrict__ q, float* __restrict__ out,
                                           const float* __restrict__ kv_cache, const int* __restrict__ block_table,
                                           const int* __restrict__ token_req, const int* __restrict__ cache_pos,
-                                          const AttnArgs& a, int num_tokens) {
+                                          const AttnArgs& a, int num_tokens, unsigned long long bad) {
     constexpr int QL = HD + 4, PL = AR_KEYS + 4;   // floats between rows: 16-byte reads of 8 rows
     extern __shared__ __align__(16) float ar_smem[];
     float* q_s = ar_smem;                          // [ROWS][QL]
@@ -240,6 +240,10 @@ __device__ __noinline__ void ar_block_fma(const float* __restrict__ q, float* __
     for (int s0 = 0; s0 < ntok;) {
         // tokens s0 .. s1-1 of the block belong to one request
         const int req = token_req[t0 + s0];
+        if ((bad >> (s0 * G) & ((2ull << (G - 1)) - 1)) == 0) {        // nothing to make for this token
+            ++s0;
+            continue;
+        }
         int s1 = s0, lo_min = 0x7fffffff, hi_max = 0;      // the keys that any of them sees
         int full_lo = 0, full_hi = 0x7fffffff;             // ... and those that all of them see
         for (; s1 < ntok && token_req[t0 + s1] == req; ++s1) {
@@ -380,8 +384,8 @@ __device__ __noinline__ void ar_block_fma(const float* __restrict__ q, float* __
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            if (group != 0 || hi_r[i] == 0) continue;
             const int r = ty + 16 * i;
+            if (group != 0 || hi_r[i] == 0 || !(bad >> r & 1)) continue;
             const float2 ml = other_ml[r];
             const float top = fmaxf(m[i], ml.x);
             const float w0 = expf(m[i] - top), w1 = expf(ml.x - top);      // (a group that saw no key: 0)
@@ -408,13 +412,18 @@ __device__ __noinline__ void ar_block_fma(const float* __restrict__ q, float* __
 // shares of a row are added up at the end in their order.  A tile's keys and values are fetched into registers under
 // the products of the tile before it, cut into their parts and put into shared memory by the whole group;
 // probabilities go from the scores' registers into the products' without passing through memory.
-// Operands that are not finite leave no sum behind in their parts (infinity less infinity): a block that met one
-// makes its rows again with plain FMAs.
+// Operands that are not finite leave no sum behind in their parts (infinity less infinity): zeros stand in for those of a
+// key or value, and the rows that see one, or whose result is not finite (an own query, products of finite numbers
+// past the largest float), are made again with plain FMAs, no others, so that a row's result does not depend on
+// what else is in the batch.
 // Bound by latencies where prompts are short (of a block's 10 us with one tile the queries take 1.2, the first
 // keys 2, the tile 3, the shares 2) and by the warp-level tensor path and the splitting where they are long.  448
 // prompt tokens with 32 / 8 heads of 64 (requests of 256 and 192): 26.5 us, with FMAs 33, and 41 in one group with
 // whole tiles; 1,500 tokens: 211, 283, 283; one of 250 tokens on 250 cached keys, 24 / 8 heads of 128: 72, 89, 121;
-// 2,000 tokens: 695, 876, 1,258.  Error against 64 bits as with FMAs (the layer: 5.0e-7, 4.9e-7).
+// 2,000 tokens: 695, 876, 1,258.  512 threads leave 128 registers each: 160 (HD 64) and 300 (128) bytes of them are spilled.
+// Error against 64 bits, FMAs in brackets: 256 tokens of normal numbers 1.2e-7 (1.9e-7) with heads of 64 and 1.8e-7 (2.2e-7)
+// of 128, 2,000 tokens 1.5e-7 (3.6e-7) and 2.2e-7 (3.9e-7), values of one sign 7.4e-8 (4.7e-7); tokens that see two keys
+// of even weight 2.8e-8 (2.7e-8).
 template <int HD> __host__ __device__ constexpr int ap_keys() { return HD == 64 ? 64 : 32; }     // of a tile
 template <int HD> __host__ __device__ constexpr int ap_smem() {
     return 3 * 2 * (HD + 8) * (AR_ROWS + AR_GROUPS * 2 * ap_keys<HD>());
@@ -428,6 +437,19 @@ __device__ __forceinline__ bool ap_split(float x, float y, uint32_t (&p)[3]) {
     const float sx = rx - __uint_as_float(p[1] << 16), sy = ry - __uint_as_float(p[1] & 0xffff0000u);
     p[2] = pack_bf16(sx, sy);
     return isfinite(sx + sy);
+}
+
+// Zeros for the parts of four floats if one of them is not finite, and a bit set.  (Out of line: this is rare.)
+__device__ __noinline__ void ap_zero(bf16* to, int plane, const float* v, unsigned long long* bad, int bit) {
+    uint32_t p[3];
+    if (ap_split(v[0], v[1], p) && ap_split(v[2], v[3], p)) return;
+    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(to + i * plane) = make_uint2(0u, 0u);
+    atomicOr(bad, 1ull << bit);
+}
+// The row, if it sees one of these keys.
+__device__ __noinline__ void ap_mark(unsigned long long keys, int key0, int lo, int hi, int row, unsigned long long* bad) {
+    for (int key = max(lo - key0, 0); key < min(hi - key0, 64); ++key)
+        if (keys >> key & 1) atomicOr(bad, 1ull << row);
 }
 
 template <int HD>
@@ -448,6 +470,14 @@ attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
     const int lane = tid & 31, warp = tid >> 5, rt = warp & 3, half = warp >> 2;
     const int g = lane >> 2, c4 = lane & 3;
     auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(AR_THREADS) : "memory"); };
+    // a group's sync that tells it whether this holds for any thread
+    auto any_of_group = [&](bool here) {
+        uint32_t any;
+        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\t"
+                     "barrier.cta.red.or.pred q, %2, %3, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                     : "=r"(any) : "r"((uint32_t)here), "r"(1 + group), "n"(AR_THREADS) : "memory");
+        return any != 0;
+    };
     const int kvh = blockIdx.x;
     const int G = a.nq / a.nkv, TPB = AR_ROWS / G;
     // (the tokens with the most keys first)
@@ -456,14 +486,18 @@ attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
     const size_t page_elems = (size_t)2 * a.nkv * a.page_size * HD;
     const size_t v_off = (size_t)a.nkv * a.page_size * HD;
     const float* head_base = kv_cache + (size_t)kvh * a.page_size * HD;
-    bool finite = true;
+    // rows to make again; keys of a tile that are not finite, while the rows that see them are marked
+    __shared__ unsigned long long bad_rows, bad_keys[AR_GROUPS];
+    if (threadIdx.x == 0) bad_rows = bad_keys[0] = bad_keys[1] = 0ull;
     auto put = [&](bf16* to, int plane, const float4 v) {
         uint32_t x[3], y[3];
-        finite = ap_split(v.x, v.y, x) && finite;
+        bool finite = ap_split(v.x, v.y, x);
         finite = ap_split(v.z, v.w, y) && finite;
 #pragma unroll
         for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(to + i * plane) = make_uint2(x[i], y[i]);
+        return finite;
     };
+    // (a query that is not finite spoils its own row alone, whose result tells)
     for (int c = threadIdx.x; c < AR_ROWS * (HD / 4); c += AR_GROUPS * AR_THREADS) {
         const int r = c / (HD / 4), d = (c % (HD / 4)) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -524,13 +558,30 @@ attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
         if (first < hi_max) fetch(first);
         for (int key0 = first; key0 < hi_max; key0 += AR_GROUPS * KEYS) {
             group_sync();                          // the tile before is done with
+            bool finite = true;
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int c = tid + u * AR_THREADS, at = c / (HD / 4) * LD + (c % (HD / 4)) * 4;
-                put(k_p + at, KPLANE, k_next[u]);
-                put(v_p + at, KPLANE, v_next[u]);
+                finite = put(k_p + at, KPLANE, k_next[u]) && finite;
+                finite = put(v_p + at, KPLANE, v_next[u]) && finite;
             }
-            group_sync();
+            if (any_of_group(!finite)) {
+#pragma unroll 1
+                for (int c = tid; c < KEYS * (HD / 4); c += AR_THREADS) {
+                    const int key = c / (HD / 4), d = (c % (HD / 4)) * 4, there = key0 + key;
+                    if (there < lo_min || there >= hi_max) continue;
+                    const float* src = head_base + (size_t)bt[there / a.page_size] * page_elems +
+                                       (size_t)(there % a.page_size) * HD + d;
+                    ap_zero(k_p + key * LD + d, KPLANE, src, &bad_keys[group], key);
+                    ap_zero(v_p + key * LD + d, KPLANE, src + v_off, &bad_keys[group], key);
+                }
+                group_sync();
+                const unsigned long long keys = bad_keys[group];
+                ap_mark(keys, key0, lo_r[0], hi_r[0], rt * 16 + g, &bad_rows);
+                ap_mark(keys, key0, lo_r[1], hi_r[1], rt * 16 + g + 8, &bad_rows);
+                group_sync();
+                if (tid == 0) bad_keys[group] = 0ull;
+            }
             if (key0 + AR_GROUPS * KEYS < hi_max) fetch(key0 + AR_GROUPS * KEYS);
             const int mine = key0 + half * HALF;                         // this warp's first key
             if (mine >= warp_hi || mine + HALF <= lo_min) continue;
@@ -650,7 +701,7 @@ attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
                 top = fmaxf(top, ml[i].x);
             }
             const float w[4] = {expf(m[r] - top), expf(ml[0].x - top), expf(ml[1].x - top), expf(ml[2].x - top)};  // (no key: 0)
-            float sum = l[r] * w[0];
+            float sum = l[r] * w[0], all = 0.f;
 #pragma unroll
             for (int i = 0; i < 3; ++i) sum = fmaf(ml[i].y, w[i + 1], sum);
             float* dst = out + (size_t)(t0 + row / G) * a.nq * HD + (size_t)(kvh * G + row % G) * HD + 2 * c4;
@@ -663,14 +714,18 @@ attention_rows_f32_kernel(const float* __restrict__ q, float* __restrict__ out,
                     x = fmaf(f.x, w[i + 1], x);
                     y = fmaf(f.y, w[i + 1], y);
                 }
-                *reinterpret_cast<float2*>(dst + v * 8) = make_float2(x / sum, y / sum);
+                x /= sum;
+                y /= sum;
+                all += x + y;
+                *reinterpret_cast<float2*>(dst + v * 8) = make_float2(x, y);
             }
+            if (!isfinite(all)) atomicOr(&bad_rows, 1ull << row);
         }
         __syncthreads();                           // the shares have been read
         s0 = s1;
     }
-    if (__syncthreads_or(!finite))
-        ar_block_fma<HD>(q, out, kv_cache, block_table, token_req, cache_pos, a, num_tokens);
+    if (const unsigned long long bad = bad_rows)      // (written before the last sync)
+        ar_block_fma<HD>(q, out, kv_cache, block_table, token_req, cache_pos, a, num_tokens, bad);
 }
 
 // ------------------------------------------------------------------ float single tokens

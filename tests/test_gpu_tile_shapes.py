@@ -213,6 +213,48 @@ def test_float_attention_of_portions_keeps_what_is_not_finite(hd, where, value):
     torch.testing.assert_close(got[both], want[both], rtol=2e-5, atol=2e-6)
 
 
+@pytest.mark.parametrize("hd,window", [(64, 0), (128, 0), (64, 20)])
+@pytest.mark.parametrize("where,value", [("q", float("nan")), ("key", float("inf")), ("value", float("nan")),
+                                         ("key", 1e30)])
+def test_float_attention_of_portions_keeps_the_bits_of_rows_that_see_finite_numbers(hd, window, where, value):
+    """An operand that is not finite (or scores past the largest float) changes the bits of no row that does not see it,
+    of its own request or of another in the same block of 64 rows."""
+    from mstar_b200 import ops
+
+    lens, heads, page = [21, 40, 30], 2, 16                      # 32 tokens a block: each meets two requests
+    T = sum(lens)
+    q, kv = rnd(T, heads * hd, seed=1), rnd(9, 2, 1, page, hd, seed=2)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    table = i32([[0, 1, 2], [3, 4, 5], [6, 7, 8]])
+    req, pos = [r for r, n in enumerate(lens) for _ in range(n)], [t for n in lens for t in range(n)]
+
+    def run():
+        out = torch.empty(T, heads * hd, device=DEV)
+        ops.paged_attention_generic(q, heads * hd, out, kv, table, i32(req), i32(pos), T, heads, 1, hd, page, window,
+                                    hd ** -0.5, entries=len(lens))
+        return out
+
+    want = run()
+    at = 12                                                      # of the second request
+    if where == "q":
+        q[lens[0] + at, 3] = value
+    else:
+        kv[3, int(where == "value"), 0, at, 3] = value
+        if value == 1e30:
+            q[lens[0] + at:lens[0] + lens[1], 3::hd] = -1e30     # the rows that see the key
+    got = run()
+    sees = torch.tensor([r == 1 and (t == at if where == "q" else t >= at and not (window and t >= at + window))
+                         for r, t in zip(req, pos)], device=DEV)
+    if value == 1e30:
+        sees = torch.tensor([r == 1 and t >= at for r, t in zip(req, pos)], device=DEV)     # (their queries changed)
+    assert torch.equal(got[~sees], want[~sees])
+    if value != 1e30:
+        rows = got[sees].view(-1, heads, hd)                     # (a key of plus infinity may have a score of minus infinity)
+        assert not torch.isfinite(rows).all() and (where == "key" or not torch.isfinite(rows).all(2).all(1).any())
+    else:                                                        # a score of minus infinity: the key has no weight
+        assert torch.isfinite(got[sees]).all()
+
+
 @pytest.mark.parametrize("tokens,width,ff,experts,identity,top,form,on_input", [
     (200, 72, 8, 2, 0, 2, "silu", False),         # k-blocks that end early, one narrow column tile
     (300, 128, 264, 5, 1, 3, "silu", True),       # column tiles that end inside, identity experts
