@@ -636,25 +636,29 @@ __global__ void convert_kernel(const S* __restrict__ src, D* __restrict__ dst, s
         dst[i] = from_float<D>(to_float(src[i]));
 }
 
-// the same for rows of `cols` elements that lie `ld` apart
+// the same for rows of `cols` elements that lie `ld` apart: the first `left` of each go to one matrix, the rest to another
 template <typename S, typename D>
-__global__ void convert_rows_kernel(const S* __restrict__ src, D* __restrict__ dst, size_t n, int cols, int ld) {
+__global__ void convert_rows_kernel(const S* __restrict__ src, D* __restrict__ dst, D* __restrict__ dst2, size_t n, int cols,
+                                    int left, int ld) {
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const size_t row = i / cols;
-        dst[i] = from_float<D>(to_float(src[row * ld + (i - row * cols)]));
+        const int col = (int)(i - row * cols);
+        const D v = from_float<D>(to_float(src[row * ld + col]));
+        if (col < left) dst[row * left + col] = v;
+        else dst2[row * (cols - left) + (col - left)] = v;
     }
 }
 
-MSTAR_API int mstar_convert_rows(const void* src, int src_dtype, void* dst, int dst_dtype, long long rows, int cols,
-                                 int ld, void* stream) {
+MSTAR_API int mstar_convert_rows(const void* src, int src_dtype, void* dst, void* dst2, int dst_dtype, long long rows,
+                                 int cols, int left, int ld, void* stream) {
     if (rows <= 0 || cols <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     const size_t n = (size_t)rows * cols, most = (size_t)device_sm_count() * 32;
     const int blocks = (int)((n + 255) / 256 < most ? (n + 255) / 256 : most);
     if (src_dtype == MSTAR_F32 && dst_dtype == MSTAR_BF16)
-        convert_rows_kernel<<<blocks, 256, 0, s>>>((const float*)src, (bf16*)dst, n, cols, ld);
+        convert_rows_kernel<<<blocks, 256, 0, s>>>((const float*)src, (bf16*)dst, (bf16*)dst2, n, cols, left, ld);
     else if (src_dtype == MSTAR_BF16 && dst_dtype == MSTAR_F32)
-        convert_rows_kernel<<<blocks, 256, 0, s>>>((const bf16*)src, (float*)dst, n, cols, ld);
+        convert_rows_kernel<<<blocks, 256, 0, s>>>((const bf16*)src, (float*)dst, (float*)dst2, n, cols, left, ld);
     else
         return -1;
     return launch_status();

@@ -201,16 +201,26 @@ def convert(src: torch.Tensor, dtype: torch.dtype):
     _need_cuda(src)
     if src.dtype == dtype:
         return src
-    out = src.new_empty(src.shape, dtype=dtype)
     if src.dim() == 2 and src.stride(1) == 1 and src.shape[1] < src.stride(0) < 1 << 31:    # columns of wider rows
-        check(lib.get("elementwise").mstar_convert_rows(
-            src.data_ptr(), _dt(src), out.data_ptr(), _dt(out), src.shape[0], src.shape[1], src.stride(0),
-            _stream()), "convert_rows")
-        return out
+        return convert_columns(src, dtype, src.shape[1])[0]
+    out = src.new_empty(src.shape, dtype=dtype)
     assert src.is_contiguous()
     check(lib.get("elementwise").mstar_convert(
         src.data_ptr(), _dt(src), out.data_ptr(), _dt(out), src.numel(), _stream()), "convert")
     return out
+
+
+def convert_columns(src: torch.Tensor, dtype: torch.dtype, left: int) -> tuple:
+    """(the first ``left`` columns, the other ones) of a matrix in another dtype, each a matrix of its own: columns of
+    a wider one could start off the 16 bytes that the products want."""
+    _need_cuda(src)
+    rows, cols = src.shape
+    assert src.dtype != dtype and src.stride(1) == 1 and src.stride(0) < 1 << 31 and 0 <= left <= cols
+    a, b = src.new_empty((rows, left), dtype=dtype), src.new_empty((rows, cols - left), dtype=dtype)
+    check(lib.get("elementwise").mstar_convert_rows(
+        src.data_ptr(), _dt(src), a.data_ptr(), b.data_ptr(), _DT[dtype], rows, cols, left, src.stride(0),
+        _stream()), "convert_rows")
+    return a, b
 
 
 def rope_kv_write(qkv: torch.Tensor, positions, cache_pos, token_req, block_table,

@@ -26,7 +26,7 @@ _SIGNATURES = {
         "mstar_add_rmsnorm": [_vp, _vp, _vp, _i, _vp, _i, _i, _i, _f, _f, _i, _vp],
         "mstar_gather_add_rows": [_vp, _vp, _i, _vp, _vp, _i, _i, _vp],
         "mstar_silu_mul": [_vp, _vp, _i, _i, _i, _i, _f, _f, _vp],
-        "mstar_convert_rows": [_vp, _i, _vp, _i, _ll, _i, _i, _vp],
+        "mstar_convert_rows": [_vp, _i, _vp, _vp, _i, _ll, _i, _i, _i, _vp],
         "mstar_convert": [_vp, _i, _vp, _i, _ll, _vp],
         "mstar_rope_kv_write": [_vp, _i, _vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i,
                                 _i, _i, _vp],

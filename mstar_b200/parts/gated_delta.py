@@ -100,8 +100,7 @@ class GatedDelta:
                                                   else s.gate_rank)]
         narrow = self.runtime.dtype != torch.float32
         if a_proj is not None and not s.full_gate and narrow:
-            low = ops.convert(proj[:, at:at + a_cols + s.gate_rank], self.runtime.dtype)
-            a_proj, gate = low[:, :a_cols], low[:, a_cols:]
+            a_proj, gate = ops.convert_columns(proj[:, at:at + a_cols + s.gate_rank], self.runtime.dtype, a_cols)
         if a_proj is not None:
             a_proj = ops.linear(ops.convert(a_proj, self.runtime.dtype) if narrow else a_proj.contiguous(),
                                 self.w_a2, out_dtype=torch.float32, static_weights=True)

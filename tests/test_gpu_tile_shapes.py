@@ -480,6 +480,27 @@ def test_delta_inputs_by_runs_of_tokens(head_decay, dtype):
         assert (g.double() - v).abs().max() < 2 ** -24 * 64
 
 
+@pytest.mark.parametrize("decay_rank,gate_rank", [(12, 64), (8, 8), (64, 20), (128, 128)])
+def test_low_rank_inputs_of_the_delta_rule_are_matrices_of_their_own(decay_rank, gate_rank, monkeypatch):
+    """On 16 bytes and without gaps between rows, as the package's own products want them, whatever the ranks are."""
+    import types
+
+    from mstar_b200.parts import gated_delta
+
+    part = object.__new__(gated_delta.GatedDelta)
+    part.spec = types.SimpleNamespace(head_decay=False, full_gate=False, num_heads=2, v_dim=16, decay_rank=decay_rank,
+                                      gate_rank=gate_rank)
+    part.runtime = types.SimpleNamespace(dtype=torch.bfloat16)
+    part.w_a2, part.w_g2 = rnd(32, decay_rank, dtype=torch.bfloat16), rnd(32, gate_rank, dtype=torch.bfloat16)
+    linear, inputs = gated_delta.ops.linear, []
+    monkeypatch.setattr(gated_delta.ops, "linear", lambda x, w, **kw: inputs.append(x) or linear(x, w, **kw))
+    proj = rnd(9, 101 + decay_rank + gate_rank + 4, seed=2)
+    part._decay_and_gate(proj, 101)
+    want = proj[:, 101:101 + decay_rank + gate_rank].bfloat16().split([decay_rank, gate_rank], dim=1)
+    for got, w in zip(inputs, want):
+        assert torch.equal(got, w) and got.is_contiguous() and got.data_ptr() % 16 == 0
+
+
 @pytest.mark.parametrize("temperature,opts", [(0.6, {"top_p": 0.8}), (3.0, {"top_p": 0.95}), (0.05, {"top_p": 0.999}),
                                               (1.0, {"top_p": 1e-6}), (1.5, {"top_k": 3000, "top_p": 0.9}),
                                               (1.0, {"top_k": 700})])
