@@ -34,8 +34,9 @@ __global__ void embed_rows_kernel(const W* __restrict__ table, const int* __rest
     }
     const W* row = table + (size_t)id * hidden;
     // Eight numbers a thread where rows lie on 16 bytes, so that a decoded token's row is one round of loads:
-    // what a row takes is their latency (one of 2,048 numbers: 4.4 us a number at a time, 2.2 so).
-    if (hidden % 8 == 0 && ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
+    // what a row takes is their latency (one of 2,048 numbers: 2.6 us a number at a time, 1.6 so).  With thousands of rows
+    // it is the order of the writes: 4,000 of 2,048 take 10.0 us a number at a time, 11.3 so (of 3,072: 19.6 and 15.5).
+    if ((gridDim.x <= 1024 || hidden > 2048) && hidden % 8 == 0 && ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
         for (int i = threadIdx.x * 8; i < hidden; i += blockDim.x * 8) {
             float v[8];
             load8(row + i, v);
@@ -443,8 +444,9 @@ __global__ void gather_add_rows_kernel(const float* __restrict__ resid, const A*
     const size_t src = (size_t)rows[blockIdx.x] * hidden;
     const size_t dst = (size_t)blockIdx.x * hidden;
     // eight numbers a thread where rows lie on 16 bytes: both rows in one round of loads (one row of 2,048
-    // numbers, all between the last product and the final norm: 6.1 us a number at a time, 2.7 so)
-    if (hidden % 8 == 0 && ((reinterpret_cast<uintptr_t>(resid) | reinterpret_cast<uintptr_t>(delta) |
+    // numbers, all between the last product and the final norm: 2.8 us a number at a time, 1.6 so), unless
+    // there are many rows (1,000 of 3,072: 4.9 and 5.9; of 8,192: 22 and 13)
+    if ((gridDim.x <= 512 || hidden >= 4096) && hidden % 8 == 0 && ((reinterpret_cast<uintptr_t>(resid) | reinterpret_cast<uintptr_t>(delta) |
                              reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
         for (int i = threadIdx.x * 8; i < hidden; i += blockDim.x * 8) {
             float v[8], d[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -849,7 +851,9 @@ MSTAR_API int mstar_rope_kv_write(void* qkv, int act_dtype, const int* positions
     // table aligned: the vector kernel; else one pair per item
     const bool vec = !interleaved && rotary_dim > 0 && rotary_dim <= 256 && (rotary_dim / 2) % 8 == 0 && hd % 8 == 0 &&
                      (hd - rotary_dim) % 8 == 0 && ((uintptr_t)qkv % 32 == 0) &&
-                     ((uintptr_t)inv_freq % 32 == 0) && (kv_cache == nullptr || (uintptr_t)kv_cache % 32 == 0);
+                     ((uintptr_t)inv_freq % 32 == 0) && (kv_cache == nullptr || (uintptr_t)kv_cache % 32 == 0) &&
+                     // (floats: a few tokens are over sooner a pair a thread, 8 tokens 2.6 us against 3.1; 256: 6.1 and 3.8)
+                     (act_dtype == MSTAR_BF16 || num_tokens >= 64);
     if (vec) {
         const int items = (nq + nkv) * (rotary_dim / 16) + nkv * ((hd - rotary_dim) / 8) + nkv * (hd / 8);
         int slices = (items + threads - 1) / threads;

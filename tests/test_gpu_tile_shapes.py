@@ -501,6 +501,36 @@ def test_low_rank_inputs_of_the_delta_rule_are_matrices_of_their_own(decay_rank,
         assert torch.equal(got, w) and got.is_contiguous() and got.data_ptr() % 16 == 0
 
 
+@pytest.mark.parametrize("heads,kv_heads,dim,rotary", [(4, 2, 64, 64), (3, 1, 128, 64), (2, 2, 64, 16)])
+def test_float_rotation_of_few_and_many_tokens(heads, kv_heads, dim, rotary):
+    """63 tokens a pair a thread, 64 by eights: the same bits, in the rows and in the cache."""
+    from mstar_b200 import ops
+
+    page, T = 16, 64
+    qkv, freq = rnd(T, (heads + 2 * kv_heads) * dim, seed=1), torch.rand(rotary // 2, device=DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    table, pos, cached = i32([list(range(40))]), [5 + 9 * t for t in range(T)], []
+    for n in (T, T - 1):
+        rows, kv = qkv[:n].clone(), torch.zeros(40, 2, kv_heads, page, dim, device=DEV)
+        ops.rope_kv_write(rows, i32(pos[:n]), i32(pos[:n]), i32([0] * n), table, freq, kv, heads, kv_heads, dim, rotary,
+                          False, page)
+        if n == T:
+            kv[pos[-1] // page, :, :, pos[-1] % page] = 0        # the token that the other run leaves out
+        cached.append((rows[:T - 1, :heads * dim], kv))
+    assert all(torch.equal(x, y) for x, y in zip(*cached)) and cached[0][1].any()
+
+
+# on both sides of the counts from which rows go a number a thread
+@pytest.mark.parametrize("rows,hidden", [(1024, 64), (1025, 64), (1025, 2056), (512, 2056), (513, 2056), (513, 4096)])
+def test_rows_by_eights_and_one_by_one(rows, hidden):
+    from mstar_b200 import ops
+
+    table, ids = rnd(50, hidden, dtype=torch.bfloat16, seed=1), torch.arange(rows, device=DEV, dtype=torch.int32) % 50
+    assert torch.equal(ops.embed_rows(table, ids, scale=0.5), table.float()[ids.long()] * 0.5)
+    resid, delta = rnd(50, hidden, seed=2), rnd(50, hidden, dtype=torch.bfloat16, seed=3)
+    assert torch.equal(ops.gather_add_rows(resid, delta, ids), (resid + delta.float())[ids.long()])
+
+
 @pytest.mark.parametrize("temperature,opts", [(0.6, {"top_p": 0.8}), (3.0, {"top_p": 0.95}), (0.05, {"top_p": 0.999}),
                                               (1.0, {"top_p": 1e-6}), (1.5, {"top_k": 3000, "top_p": 0.9}),
                                               (1.0, {"top_k": 700})])
