@@ -1126,14 +1126,16 @@ def latent_fill(q, dkv, norm_weight, freq: torch.Tensor, positions, cache_pos, t
 
 
 def latent_attention_plan(tokens: int, heads: int, rank: int, max_keys: int,
-                          sms: int | None = None) -> tuple:
+                          sms: int | None = None, tensor: bool = True) -> tuple:
     """(heads per block, splits of a token's keys) for the latent attention kernels.  The
     tensor-core kernel takes up to 16 heads a block whatever the first number says; the
     CUDA-core kernels take as many heads as a thread's 32 sums allow (they share the rows a
     block loads), fewer when tokens are few.  With few tokens a token's keys are shared among
     blocks until there are some two blocks per SM, a split keeping at least one tile of 32
     keys (a tile is a chain of some 4 us: 7 tokens on 200 keys take 13.3 us with a tile a split, 23.5
-    with two or more)."""
+    with two or more).  Not ``tensor``, the CUDA-core kernels: the same while their blocks of heads leave SMs
+    over (7 tokens of 16 float heads of 512 on 70 keys: 24.6 us, 50.8 with two), else two tiles (64 tokens of these on
+    70 keys: 66.7 us with one, 55.6 with two)."""
     if sms is None:
         sms = num_sms()
     group = max(1, min(heads, 16 if rank <= 256 else (8 if rank <= 512 else 4)))
@@ -1142,7 +1144,8 @@ def latent_attention_plan(tokens: int, heads: int, rank: int, max_keys: int,
         group = max(4, group // 2)
     blocks = tokens * -(-heads // 16)
     tiles = max(1, -(-max_keys // 32))
-    splits = max(1, min(want // max(blocks, 1), tiles, 32))
+    least = 1 if tensor or tokens * -(-heads // group) < sms else 2
+    splits = max(1, min(want // max(blocks, 1), tiles // least, 32))
     return group, splits
 
 
@@ -1168,7 +1171,8 @@ def latent_attention(q_abs: torch.Tensor, q_rot: torch.Tensor, cache: torch.Tens
         max_keys = window or 32
     if window:
         max_keys = min(max_keys, window)
-    group, splits = latent_attention_plan(tokens, heads, rank, max_keys, num_sms(q_abs.device))
+    tensor = cache.dtype == torch.bfloat16 and rank % 32 == 0 and (rank + rot) % 16 == 0
+    group, splits = latent_attention_plan(tokens, heads, rank, max_keys, num_sms(q_abs.device), tensor)
     out = q_abs.new_empty((tokens, heads, rank), dtype=torch.float32)
     scratch = None
     if splits > 1:

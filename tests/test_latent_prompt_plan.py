@@ -67,3 +67,12 @@ def test_the_cache_leaves_room_for_prompts(dtype, v_dim, need, monkeypatch):
     monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: (1 << 30, 1 << 31))
     page = 16 * 128 * dtype.itemsize
     assert llm._pages_from_memory(16, 0.9) == [int(((1 << 30) - need) * 0.9) // page]
+
+
+def test_splits_of_a_token_s_keys():
+    """A tile of 32 keys a split, or two where the CUDA-core kernels' blocks of heads fill the SMs by themselves."""
+    plan = ops.latent_attention_plan
+    assert plan(7, 16, 512, 70, sms=148)[1] == 3 and plan(64, 16, 512, 70, sms=148)[1] == 3
+    assert plan(7, 16, 512, 70, sms=148, tensor=False)[1] == 3
+    assert plan(64, 16, 512, 70, sms=148, tensor=False)[1] == 1 and plan(64, 16, 512, 200, sms=148, tensor=False)[1] == 3
+    assert plan(1, 16, 512, 5, sms=148)[1] == plan(64, 16, 512, 20, sms=148, tensor=False)[1] == 1
