@@ -568,22 +568,26 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int c
             }
         });
         if (cs_pick_few(cluster, rank, hist, offered, result, need(), above)) return (unsigned)result[0];
+        // Keys from the least that a logit of this bin can have (a bin to either side makes up for all rounding; the lowest
+        // bin also has the row's smallest ones), so that 22 bits, two rounds, hold most bins.
+        unsigned low = 0u, range = 0xffffffffu;
+        if (bin > 0u && per_bin < INFINITY) {
+            low = ordered_bits(__fadd_rd(base_v, __fdiv_rd((float)(bin - 1u), per_bin)));
+            range = ordered_bits(__fadd_ru(base_v, __fdiv_ru((float)(bin + 2u), per_bin))) - low;
+        }
         unsigned prefix = 0u;
-        int decided = 0;
-        for (int round = 0; round < 3; ++round) {
-            const int bits = round < 2 ? 11 : 10;
-            const int shift = 32 - decided - bits;
+        for (int left = range < 1u << 11 ? 11 : range < 1u << 22 ? 22 : 32; left > 0;) {
+            const int bits = left < 11 ? left : 11, all = left;
+            left -= bits;
             cs_clear(hist);
             each([&](float v) {
                 if (!among(v) || bin_of(v) != bin) return;
-                const unsigned key = key_of(v);
-                if (decided == 0 || (key >> (32 - decided)) == prefix)
-                    cs_add(hist, (key >> shift) & ((1u << bits) - 1u), weight_of(v));
+                const unsigned key = key_of(v) - low;
+                if (all == 32 || (key >> all) == prefix) cs_add(hist, (key >> left) & ((1u << bits) - 1u), weight_of(v));
             });
             prefix = (prefix << bits) | (unsigned)cs_pick_bin(cluster, rank, hist, scratch, slot, result, need, above);
-            decided += bits;
         }
-        return prefix;
+        return low + prefix;
     };
     const bool choose_k = k > 0 && k < vocab;
 

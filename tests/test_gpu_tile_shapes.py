@@ -560,6 +560,27 @@ def test_sampling_where_the_threshold_is_hard_to_find(temperature, opts):
         assert (cdf[tok - 1].item() if tok else 0.0) - 1e-4 <= u <= cdf[tok].item() + 1e-4, (r, tok, u)
 
 
+@pytest.mark.parametrize("opts", [{"top_p": 0.9}, {"top_k": 900}])
+def test_sampling_of_more_tied_logits_than_a_list_holds(opts):
+    """Logits in steps of an eighth over rows of 157 k, at offsets at which their keys take one, two and three rounds."""
+    import plain_llama as P
+    from mstar_b200 import ops
+
+    vocab = 156940
+    x = torch.round(3 * rnd(6, vocab, seed=3) * 8) / 8
+    for r, (scale, off) in enumerate(((1, 0), (1, 3000), (1e-3, 1), (1, -40), (1e-6, 1), (64, 0))):
+        x[r] = x[r] * scale + off
+    seeds, offsets = torch.arange(50, 56, device=DEV), torch.arange(6, device=DEV)
+    temperature = torch.tensor([1, 1, 1e-3, 1, 1e-6, 64], device=DEV)
+    extra = {k: torch.full((6,), v, dtype=torch.int32 if k == "top_k" else torch.float32, device=DEV) for k, v in opts.items()}
+    got = ops.sample(x, temperature, seed=seeds, offset=offsets, **extra).tolist()
+    for r, tok in enumerate(got):
+        p = P.plain_sampling_distribution(x[r].cpu(), temperature[r].item(), **opts)
+        assert p[tok] > 0, f"row {r}: token {tok} is outside the kept set"
+        cdf, u = torch.cumsum(p.double(), 0), P.plain_uniform(50 + r, r)
+        assert (cdf[tok - 1].item() if tok else 0.0) - 1e-4 <= u <= cdf[tok].item() + 1e-4, (r, tok, u)
+
+
 def test_delta_rule_in_pieces_with_more_blocks_than_fit():
     """So many blocks an SM (34,816 in all) that a share of its shared memory holds no piece."""
     from mstar_b200 import ops
