@@ -211,9 +211,11 @@ __device__ __forceinline__ void cp_async_all_done() {
 // portion's own length alone, so that its sums do not depend on the batch (600 tokens of 2,048 channels:
 // 44 us in pieces of 64, 52 of 128; 2,048 of 4,096: 217 of 128, 223 and 226 of 64 and 256; 8,192: 809 of
 // 256, 832 of 128).
-// Shorter portions stay whole: one of 130 tokens of 4,096 channels takes 32 us either way, one of 100 28 us
+// Shorter portions stay whole: one of 130 tokens of 4,096 channels took 32 us either way, one of 100 28 us
 // against 30 in two pieces, one of 333 58 against 46; with several of them the SMs are full and whole is
-// faster (three of 333: 85 against 97).
+// faster (three of 333: 85 against 97).  At the line, 191 tokens whole and 192 in three pieces: 37 and 31 us of 4,096 channels,
+// 35 and 25 of 2,048, 31 and 21 of 1,024, 57 and 55 of 8,192.  The whole ones pay some 4 of that for an exponential that
+// is nearer (error of the outputs against 64 bits, one portion of 60 tokens: 7.7e-8, with 2^x 1.3e-7).
 #define SCAN_CUT_FROM 192
 __host__ __device__ __forceinline__ int scan_piece(int n) {
     if (n < SCAN_CUT_FROM) return SCAN_CUT_FROM;
@@ -558,6 +560,11 @@ __device__ __forceinline__ float sx_ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// The decays of two states, of dt A (exact) or of dt A log2(e): portions that are not cut keep the exponential of the
+// kernel for any state, whose error the few roundings of a short portion do not hide.
+template <bool EXACT> __device__ __forceinline__ unsigned long long sx_decays(unsigned long long z) {
+    return EXACT ? sx_pack(expf(sx_lo(z)), expf(sx_hi(z))) : sx_pack(sx_ex2(sx_lo(z)), sx_ex2(sx_hi(z)));
+}
 __device__ __forceinline__ float sx_silu(float v, bf16) { return silu_bf16(v); }
 __device__ __forceinline__ float sx_silu(float v, float) { return silu_f(v); }
 
@@ -638,11 +645,12 @@ selective_scan16_kernel(const A* __restrict__ xc, const A* __restrict__ xz, cons
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
 
-    // A in units of log2(e): the decays are then 2^(dt A)
+    // A in units of log2(e): the decays are then 2^(dt A); exact: A as it is
+    const bool exact = PASS != 1 && pieces == 1 && e_tok < SCAN_CUT_FROM;
     unsigned long long S[2], An[2];
     {
         const float4 an = *reinterpret_cast<const float4*>(a_neg + (size_t)c * 16 + 4 * sub);
-        constexpr float L = 1.4426950408889634f;
+        const float L = exact ? 1.f : 1.4426950408889634f;
         An[0] = sx_pack(an.x * L, an.y * L);
         An[1] = sx_pack(an.z * L, an.w * L);
     }
@@ -677,8 +685,8 @@ selective_scan16_kernel(const A* __restrict__ xc, const A* __restrict__ xz, cons
     // The step sizes that pass 1 made lie where it found their products.
     const bool made = PASS == 2 && piece < pieces - 1;
 
-    auto walk = [&](auto whole, ScanStage<A>& st, int t0, int nt) {
-        constexpr bool WHOLE = decltype(whole)::value;
+    auto walk = [&](auto whole, auto exactly, ScanStage<A>& st, int t0, int nt) {
+        constexpr bool WHOLE = decltype(whole)::value, EXACT = decltype(exactly)::value;
         if (!made || !WHOLE) {
             // the softplus of a channel's step sizes is dealt out among its lanes
 #pragma unroll
@@ -709,7 +717,7 @@ selective_scan16_kernel(const A* __restrict__ xc, const A* __restrict__ xz, cons
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
                     const unsigned long long z = sx_mul(dt2, An[i]);
-                    da[kk][i] = sx_pack(sx_ex2(sx_lo(z)), sx_ex2(sx_hi(z)));
+                    da[kk][i] = sx_decays<EXACT>(z);
                     db[kk][i] = here ? sx_mul(dx2, i == 0 ? B.x : B.y) : 0ull;
                 }
             }
@@ -745,8 +753,12 @@ selective_scan16_kernel(const A* __restrict__ xc, const A* __restrict__ xz, cons
         ScanStage<A>& st = stage[(t0 / SS_TC) % SX_STAGES];
         const int nt = min(SS_TC, n_tok - t0);
         // whole chunks ask for no token's place in them
-        if (nt == SS_TC) walk(std::true_type(), st, t0, nt);
-        else walk(std::false_type(), st, t0, nt);
+        auto one = [&](auto exactly) {
+            if (nt == SS_TC) walk(std::true_type(), exactly, st, t0, nt);
+            else walk(std::false_type(), exactly, st, t0, nt);
+        };
+        if (PASS != 1 && exact) one(std::true_type());
+        else one(std::false_type());
     }
     if (PASS == 1) {                           // this piece alone, for the pieces after it
         const size_t at = at0 + piece;
@@ -777,8 +789,8 @@ selective_scan16_kernel(const A* __restrict__ xc, const A* __restrict__ xz, cons
 // token, summed in the order of the product for many tokens (gemm_f32.cu: even and odd places apart), so that a
 // token's bits do not depend on which of the two made them.  Every entry reads W_dt again then, which
 // costs less than a launch up to some 32 tokens.  Bound by the stream of the states and by two dependent
-// rounds of loads: 20 entries of one token, 4,096 channels: 18 us (34 in the kernel for any state, whose lanes read
-// W_dt from global memory, 28 in the kernel above, 10 of them the product's launch); 64: 30 (84, 56).
+// rounds of loads: 20 entries of one token, 4,096 channels and rank 128: 12.9 us (24.8 in the kernel for any state, whose
+// lanes read W_dt from global memory), 64: 20.8 (68); 1,024 channels and rank 64: 4.5 (7.9) and 8.6 (16.3).
 #define SCAN_FEW 8
 #define SCAN_FEW_RANK 256           // rows of W_dt that a block can hold
 template <typename A, bool MAKE>
@@ -832,8 +844,7 @@ selective_scan16_few_kernel(const A* __restrict__ xc, const A* __restrict__ xz, 
     float* slot = state + (size_t)slots[e] * a.state_stride;
     float* s_slot = slot + (size_t)(a.taps - 1) * a.inner + (size_t)c * 16 + 4 * sub;
     const float4 an = *reinterpret_cast<const float4*>(a_neg + (size_t)c * 16 + 4 * sub);
-    constexpr float L = 1.4426950408889634f;
-    const unsigned long long An[2] = {sx_pack(an.x * L, an.y * L), sx_pack(an.z * L, an.w * L)};
+    const unsigned long long An[2] = {sx_pack(an.x, an.y), sx_pack(an.z, an.w)};
     const float bias = dt_bias[c], dsk = d_skip[c];
     const bool wide = (reinterpret_cast<uintptr_t>(s_slot) & 15) == 0;
     unsigned long long S[2];
@@ -888,7 +899,7 @@ selective_scan16_few_kernel(const A* __restrict__ xc, const A* __restrict__ xz, 
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const unsigned long long p = sx_mul(d2, An[i]);
-                S[i] = sx_fma(sx_pack(sx_ex2(sx_lo(p)), sx_ex2(sx_hi(p))), S[i], sx_mul(dx2, i == 0 ? B[k].x : B[k].y));
+                S[i] = sx_fma(sx_decays<true>(p), S[i], sx_mul(dx2, i == 0 ? B[k].x : B[k].y));
             }
             const unsigned long long y2 = sx_fma(S[1], C[k].y, sx_mul(S[0], C[k].x));
             float y = sx_lo(y2) + sx_hi(y2);

@@ -1796,10 +1796,13 @@ SCAN_PIECE = 128
 SCAN_PIECES_FROM = 512
 # The same for the kernels for 16 states (the csrc constant of this name says what was measured).
 SCAN_CUT_FROM = 192
-# Portions of at most so many tokens go to a kernel that stages nothing, and a step of at most so many
-# tokens in all needs no launch of its own for the step sizes' product there.
+# Portions of at most so many tokens go to a kernel that stages nothing (csrc has the same number), and a step of at most
+# so many tokens in all, or so many numbers of W_dt read in all, needs no launch of its own for the step sizes' product
+# there (33 tokens of 512 channels and rank 32: 3.7 us without, 6.5 with, 64 of 1,024 and 64 8.6 and 10.6; but 64 of 2,048
+# and 64 14.5 and 12.6).
 SCAN_FEW = 8
 SCAN_FEW_TOKENS = 32
+SCAN_FEW_NUMBERS = 1 << 22
 
 
 def scan_most_pieces(longest: int) -> int:
@@ -1855,8 +1858,8 @@ def selective_scan(xc: torch.Tensor, xz: torch.Tensor, proj: torch.Tensor, w_dt,
         # true-32-bit product of its own (a third of the scan's instructions otherwise, and W_dt read
         # again for every entry)
         # (portions of a few tokens: the scan makes its own, in the same order, up to so many of them)
-        if not (sixteen and max_q_len <= SCAN_FEW and tokens <= SCAN_FEW_TOKENS and rank <= 256
-                and w_dt.data_ptr() % 16 == 0):
+        if not (sixteen and max_q_len <= SCAN_FEW and rank <= 256 and w_dt.data_ptr() % 16 == 0
+                and (tokens <= SCAN_FEW_TOKENS or tokens * inner * rank <= SCAN_FEW_NUMBERS)):
             dt_tokens = tokens
     if piece:
         # (cut by their own lengths, portions have a piece for every started 64 tokens at most)
