@@ -162,8 +162,8 @@ MSTAR_API int mstar_sgemm_nt(const float* A, const float* W, float* C, int M, in
     // Wide matrices of aligned rows go to the tensor cores, three bfloat16 parts a float (gemm_f32_tc.cu, with both
     // sides measured; no error word: never).  From K = 1,024 on: the start and end of a tile there take some
     // 8 us, and a row alone takes 8.7 with K = 512 where the FMAs take 6.7 to 8.0 (N = 128 to 3,072; at 1,024: 8.7 to 11 against
-    // 11 to 12), while matrices alone decide, so that a row's sums are the same in every batch.  Below that the FMAs are
-    // as near to 64 bits as well.
+    // 11 to 12), while matrices alone decide, so that a row's sums are the same in every batch.  From 75 tiles of W on, where no
+    // CTAs share K, from K = 512: one row of 10,240 columns 12.6 against 14.6 us (of 8,192, 64 tiles: 10.6 against 9.3).
     if (error != nullptr && sgemm_parts_takes(A, W, N, K, lda, ldw))
         return sgemm_parts(A, W, C, M, N, K, lda, ldw, ldc, 0, 0, error, s);
     const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&

@@ -287,7 +287,7 @@ sgemm_parts_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
             return ok;
         };
         // this thread's columns of its row of a pair with this accumulator
-        constexpr int STEP = PART % 8 == 0 ? 8 : 4;
+        constexpr int STEP = PART == 8 ? 8 : 4;                  // (of 16 columns at once more would be spilled)
         const int row = (warp & 3) * 32 + lane, part = warp >> 2, n = n0 + row;
         const uint32_t my_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16) + part * PART;
         auto sums = [&](int b, auto&& use) {
@@ -306,7 +306,8 @@ sgemm_parts_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
         float total[PART];
 #pragma unroll
         for (int j = 0; j < PART; ++j) total[j] = 0.f;
-        int done = 0, left = 2;                                  // pairs added up, blocks to the next one
+        int done = 0;                                            // pairs added up
+        bool second = false;                                     // a block of this thread's is under way
         int s = 0, s_end = 0;                                    // of a long K: the slice, its end
         if (MODE == HALVES || MODE == OUTSIDE || MODE == KEPT) s_end = slice_start(s0 + 1, slices, pairs) - pair0;
         float* outside = reinterpret_cast<float*>(smem + 2 * STAGE) + part * PART * BW + row;      // [column][row]
@@ -350,11 +351,8 @@ sgemm_parts_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
         for (int kb = kb0 + stage; kb < kb1 && ok; kb += 2) {
             ok = fill(kb);
             // the pair before this block's, while this one's products run
-            if (MODE != RAW && left == 0) {
-                drain();
-                left = 2;
-            }
-            left -= 2;
+            if (MODE != RAW && second) drain();
+            second = true;
         }
         if constexpr (MODE != RAW)
             while (done < my_pairs && ok) drain();
@@ -526,7 +524,7 @@ int launch(const float* A, const float* W, float* C, int M, int N, int K, int ld
 }  // namespace
 
 bool sgemm_parts_takes(const float* A, const float* W, int N, int K, int lda, int ldw) {
-    return N >= BW && K >= 1024 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
+    return N >= BW && K >= (N > 74 * BW ? 512 : 1024) && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
            ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0;
 }
 

@@ -45,7 +45,8 @@ def _sgemm(a, w, *tile):
 # one row, a row past every tile width, the last tile of W shifted back by all but one row, K that ends inside a block,
 # inside a pair of them and on its border, an odd number of pairs; slices of one pair (up to 2,048) and of several
 @pytest.mark.parametrize("m,n,k,pad", [(1, 128, 1024, 0), (17, 129, 1028, 4), (80, 300, 1500, 0), (81, 255, 2112, 0),
-                                       (33, 256, 4100, 8), (200, 640, 1024, 0), (49, 200, 2048, 0), (90, 130, 9000, 0)])
+                                       (33, 256, 4100, 8), (200, 640, 1024, 0), (49, 200, 2048, 0), (90, 130, 9000, 0),
+                                       (18, 9500, 516, 0)])
 @pytest.mark.parametrize("one_sign", [False, True])
 def test_sgemm_by_parts(m, n, k, pad, one_sign):
     """Three bfloat16 parts a float: no further from 64 bits than the FMA kernel, operands of one sign (whose sums are
