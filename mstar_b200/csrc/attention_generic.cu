@@ -1,6 +1,6 @@
 // Paged grouped-query attention for any mix of prompt portions and decoded tokens,
-// in float arithmetic on CUDA cores.  It is the attention of the true 32-bit path
-// and the fallback of the bfloat16 path for shapes the tensor-core kernels refuse.
+// in float arithmetic: on CUDA cores, and for prompt portions of floats by bfloat16 parts on the tensor cores (below).  It is
+// the attention of the true 32-bit path and the fallback of the bfloat16 path for shapes the tensor-core kernels refuse.
 //
 // Semantics (mstar/engine/cache_manager.py:653-701 for the call, scale 1/sqrt(hd)
 // as in mstar/utils/attention.py:116-117): query head i uses key/value head
